@@ -101,6 +101,8 @@ RLC_API int rlc_device_count(void);
 /* ---- maps: OMap (RangeLib.h:121-322) ---------------------------------- */
 /* OMap(int w, int h) + grid fill (RangeLib.h:143-156; PyOMap(ndarray), RangeLibc.pyx:140-145). */
 RLC_API int rlc_map_create(const uint8_t* occ, int width, int height, rlc_map** out);
+/* The same from image rows, rows[y * width + x] (a [row, col] array as PyOMap(ndarray) takes it). */
+RLC_API int rlc_map_create_rows(const uint8_t* rows, int width, int height, rlc_map** out);
 /* OMap(std::string filename, float threshold) (RangeLib.h:158-201): the PNG's pixel (x, y) is
  * occupied when (int)rgb2gray(r, g, b) < threshold, with r, g, b the pixel's blue, green and red
  * (the reference reads bytes 2, 1, 0 of each RGBA pixel).  Host code, no GPU.  Call with

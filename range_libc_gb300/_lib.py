@@ -50,6 +50,7 @@ SIGNATURES = {
     "rlc_last_error": (C.c_char_p, []),
     "rlc_device_count": (C.c_int, []),
     "rlc_map_create": (C.c_int, [_u8p, C.c_int, C.c_int, C.POINTER(_vp)]),
+    "rlc_map_create_rows": (C.c_int, [_vp, C.c_int, C.c_int, C.POINTER(_vp)]),
     "rlc_png_occupancy": (C.c_int, [C.c_char_p, C.c_float, _vp, C.POINTER(C.c_int), C.POINTER(C.c_int)]),
     "rlc_png_save_occupancy": (C.c_int, [C.c_char_p, _vp, C.c_int, C.c_int]),
     "rlc_map_set_world": (C.c_int, [_vp] + [C.c_float] * 6),

@@ -75,58 +75,55 @@ struct rlc_map {
     std::atomic<int> refs{1};
     std::mutex mu;
 
+    void* d_layouts = nullptr;    // one allocation behind every distance-transform layout
+
     ~rlc_map() {
         cudaFree(d_bits);
-        cudaFree(d_dt);
-        cudaFree(d_dt_tiled);
-        cudaFree(d_dt16);
-        cudaFree(d_dt8);
-        cudaFree(d_step);
-        cudaFree(d_runs);
+        cudaFree(d_layouts);
     }
-    // distance transform on first use (RayMarching constructor, RangeLib.h:924)
+    // Distance transform and its layouts on first use (RayMarching constructor, RangeLib.h:924).
+    // All of them share one allocation (a cudaMalloc + cudaFree pair of 4 MB or more costs ~110 us
+    // whatever its size, seven of them cost more than every kernel here), and the searches'
+    // scratch is the run map's space, which is written last.
     int ensure_dt() {
         std::lock_guard<std::mutex> lk(mu);
         if (d_dt) return RLC_OK;
-        size_t n = (size_t)W * H;
-        size_t tiled = (size_t)((W + 7) >> 3) * TY * 64;
-        float* dt = nullptr;
-        float* dtt = nullptr;
-        uint16_t* dt16 = nullptr;
-        uint8_t* dt8 = nullptr;
-        float* step = nullptr;
-        uint32_t* runs = nullptr;
-        void* scratch = nullptr;
-        size_t sb = edt_scratch_bytes(W, H);
-        cudaError_t e = cudaMalloc(&dt, (n ? n : 1) * sizeof(float));
-        if (e == cudaSuccess) e = cudaMalloc(&dtt, (tiled ? tiled : 1) * sizeof(float));
-        if (e == cudaSuccess) e = cudaMalloc(&dt16, (tiled ? tiled : 1) * sizeof(uint16_t));
-        if (e == cudaSuccess) e = cudaMalloc(&dt8, (tiled ? tiled : 1) * sizeof(uint8_t));
-        if (e == cudaSuccess) e = cudaMalloc(&step, (n ? n : 1) * sizeof(float));
-        if (e == cudaSuccess) e = cudaMalloc(&runs, (n ? n : 1) * sizeof(uint32_t));
-        if (e == cudaSuccess) e = cudaMalloc(&scratch, sb);
-        if (e == cudaSuccess) e = launch_edt(d_bits, W, H, TY, dt, scratch, sb, 0);
-        if (e == cudaSuccess) e = launch_dt_to_tiled(dt, W, H, dtt, 0);
-        if (e == cudaSuccess) e = launch_dt_to_u16(dt, W, H, dt16, 0);
-        if (e == cudaSuccess) e = launch_dt_to_u8(dt, W, H, dt8, 0);
-        if (e == cudaSuccess) e = launch_dt_to_step(dt, W, H, step, 0);
-        if (e == cudaSuccess) e = launch_step_runs(step, W, H, runs, 0);
+        const size_t n = (size_t)W * H, tiled = (size_t)((W + 7) >> 3) * TY * 64;
+        size_t total = 0;
+        auto room = [&](size_t bytes) {
+            const size_t at = total;
+            total += (bytes + 255) & ~(size_t)255;
+            return at;
+        };
+        const size_t o_dt = room(n * sizeof(float)), o_step = room(n * sizeof(float));
+        const size_t o_tiled = room(tiled * sizeof(float)), o_u16 = room(tiled * sizeof(uint16_t)), o_u8 = room(tiled);
+        const size_t o_runs = room(n * sizeof(uint32_t)), o_eq = room(step_eq_words(W, H) * sizeof(uint32_t));
+        const size_t sb = edt_scratch_bytes(W, H);
+        void* extra = nullptr;   // maps with a side above 16384 need more scratch than the run map holds
+        char* base = nullptr;
+        cudaError_t e = cudaMalloc(&base, total);
+        if (e == cudaSuccess && sb > n * sizeof(uint32_t)) e = cudaMalloc(&extra, sb);
+        DtOut o;
+        o.dt = (float*)(base + o_dt);
+        o.step = (float*)(base + o_step);
+        o.tiled = (float*)(base + o_tiled);
+        o.u16 = (uint16_t*)(base + o_u16);
+        o.u8 = (uint8_t*)(base + o_u8);
+        uint32_t* runs = (uint32_t*)(base + o_runs);
+        if (e == cudaSuccess) e = launch_edt(d_bits, W, H, TY, o, extra ? extra : runs, sb, 0);
+        if (e == cudaSuccess) e = launch_step_runs(o.step, W, H, (uint32_t*)(base + o_eq), runs, 0);
         if (e == cudaSuccess) e = cudaStreamSynchronize(0);
-        cudaFree(scratch);
+        cudaFree(extra);
         if (e != cudaSuccess) {
-            cudaFree(dt);
-            cudaFree(dtt);
-            cudaFree(dt16);
-            cudaFree(dt8);
-            cudaFree(step);
-            cudaFree(runs);
+            cudaFree(base);
             return cuda_fail(e, "distance transform");
         }
-        d_dt = dt;
-        d_dt_tiled = dtt;
-        d_dt16 = dt16;
-        d_dt8 = dt8;
-        d_step = step;
+        d_layouts = base;
+        d_dt = o.dt;
+        d_dt_tiled = o.tiled;
+        d_dt16 = o.u16;
+        d_dt8 = o.u8;
+        d_step = o.step;
         d_runs = runs;
         return RLC_OK;
     }
@@ -334,6 +331,17 @@ bool host_direct() {
     return c == 2;
 }
 
+// makes `device` current until the end of the scope
+struct DeviceGuard {
+    int before = -1;
+    explicit DeviceGuard(int device) {
+        if (cudaGetDevice(&before) != cudaSuccess || before == device || cudaSetDevice(device) != cudaSuccess) before = -1;
+    }
+    ~DeviceGuard() {
+        if (before >= 0) cudaSetDevice(before);
+    }
+};
+
 int finish_launch(cudaError_t e, const char* what) {
     if (e != cudaSuccess) return cuda_fail(e, what);
     return RLC_OK;
@@ -366,7 +374,7 @@ int rlc_device_count(void) {
     return n;
 }
 
-int rlc_map_create(const uint8_t* occ, int width, int height, rlc_map** out) {
+static int map_create(const uint8_t* occ, int width, int height, bool rows, rlc_map** out) {
     if (!out) return fail(RLC_ERR_ARG, "null output handle");
     *out = nullptr;
     if (width <= 0 || height <= 0) return fail(RLC_ERR_ARG, "map size %dx%d must be positive", width, height);
@@ -379,11 +387,15 @@ int rlc_map_create(const uint8_t* occ, int width, int height, rlc_map** out) {
     m->TY = (height + 7) >> 3;
     size_t n = (size_t)width * height;
     size_t words = (size_t)((width + 7) >> 3) * m->TY;
+    // the grid is read once: in place where the GPU reads host memory, else staged
+    const bool direct = host_direct();
     uint8_t* d_occ = nullptr;
-    cudaError_t e = cudaMalloc(&d_occ, n);
-    if (e == cudaSuccess) e = cudaMalloc(&m->d_bits, words * sizeof(uint64_t));
-    if (e == cudaSuccess) e = cudaMemcpy(d_occ, occ, n, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = launch_pack_bits(d_occ, width, height, m->d_bits, 0);
+    cudaError_t e = cudaMalloc(&m->d_bits, words * sizeof(uint64_t));
+    if (!direct) {
+        if (e == cudaSuccess) e = cudaMalloc(&d_occ, n);
+        if (e == cudaSuccess) e = cudaMemcpy(d_occ, occ, n, cudaMemcpyHostToDevice);
+    }
+    if (e == cudaSuccess) e = launch_pack_bits(direct ? occ : d_occ, width, height, rows, m->d_bits, 0);
     if (e == cudaSuccess) e = cudaStreamSynchronize(0);
     cudaFree(d_occ);
     if (e != cudaSuccess) {
@@ -392,6 +404,14 @@ int rlc_map_create(const uint8_t* occ, int width, int height, rlc_map** out) {
     }
     *out = m;
     return RLC_OK;
+}
+
+int rlc_map_create(const uint8_t* occ, int width, int height, rlc_map** out) {
+    return map_create(occ, width, height, false, out);
+}
+
+int rlc_map_create_rows(const uint8_t* rows, int width, int height, rlc_map** out) {
+    return map_create(rows, width, height, true, out);
 }
 
 int rlc_map_set_world(rlc_map* map, float scale, float angle, float ox, float oy, float sin_angle,
@@ -420,6 +440,7 @@ int rlc_map_size(const rlc_map* map, int* width, int* height) {
 
 int rlc_map_occupancy(rlc_map* map, uint8_t* occ_out) {
     if (!map || !occ_out) return fail(RLC_ERR_ARG, "null argument");
+    const DeviceGuard on(map->device);   // PyOMap.occupancy may be asked with another device current
     size_t n = (size_t)map->W * map->H;
     uint8_t* d = nullptr;
     CUDA_OR_FAIL(cudaMalloc(&d, n), "occupancy export");

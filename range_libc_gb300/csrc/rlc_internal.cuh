@@ -93,21 +93,26 @@ struct SensorDev {
 };
 
 // ---- map preprocessing (rlc_map.cu) ----
-cudaError_t launch_pack_bits(const uint8_t* d_occ, int W, int H, uint64_t* d_bits, cudaStream_t s);
-cudaError_t launch_edt(const uint64_t* d_bits, int W, int H, int tiles_y, float* d_dt_linear,
+// rows: occ[y * W + x], else occ[x * H + y]
+cudaError_t launch_pack_bits(const uint8_t* d_occ, int W, int H, bool rows, uint64_t* d_bits, cudaStream_t s);
+// the distance transform's device arrays: the linear floats, and (all or none) the derived layouts
+struct DtOut {
+    float* dt = nullptr;         // [W * H]
+    float* step = nullptr;       // [W * H]
+    float* tiled = nullptr;      // [ceil(W / 8) * tiles_y * 64], as u16 and u8
+    uint16_t* u16 = nullptr;
+    uint8_t* u8 = nullptr;
+};
+cudaError_t launch_edt(const uint64_t* d_bits, int W, int H, int tiles_y, const DtOut& out,
                        void* scratch, size_t scratch_bytes, cudaStream_t s);
 size_t edt_scratch_bytes(int W, int H);
 // upper bound of edt_scratch_bytes(W, H) over all W * H <= cells with W, H <= side
 constexpr size_t edt_scratch_bound(size_t cells, size_t side) {
     return ((cells * 4 + 255) & ~(size_t)255) + cells * 4 + (cells + side) * 8 + 256;
 }
-cudaError_t launch_dt_to_tiled(const float* d_lin, int W, int H, float* d_tiled, cudaStream_t s);
-cudaError_t launch_dt_to_u16(const float* d_lin, int W, int H, uint16_t* d_u16, cudaStream_t s);
-// the ray-marching step of every cell (linear layout), as RayMarching::calc_range forms it
-cudaError_t launch_dt_to_step(const float* d_lin, int W, int H, float* d_step, cudaStream_t s);
-// equal-step run lengths of the step map along both axes (MapDev::runs)
-cudaError_t launch_step_runs(const float* d_step, int W, int H, uint32_t* d_runs, cudaStream_t s);
-cudaError_t launch_dt_to_u8(const float* d_lin, int W, int H, uint8_t* d_u8, cudaStream_t s);
+// equal-step run lengths of the step map along both axes (MapDev::runs); d_eq: step_eq_words scratch
+size_t step_eq_words(int W, int H);
+cudaError_t launch_step_runs(const float* d_step, int W, int H, uint32_t* d_eq, uint32_t* d_runs, cudaStream_t s);
 cudaError_t launch_edge_map(const uint64_t* d_bits, int W, int H, int tiles_y, uint8_t* d_edge, cudaStream_t s);
 cudaError_t launch_unpack_bits(const uint64_t* d_bits, int W, int H, int tiles_y, uint8_t* d_occ, cudaStream_t s);
 

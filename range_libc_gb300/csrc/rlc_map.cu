@@ -9,10 +9,8 @@
 // f[q] + q*q are float (they round above 2^24, which matters on large
 // maps), breakpoints are double, and the per-line output is a float.
 // Pass 1 runs along y for every x, pass 2 along x for every y.  Maps with
-// both sides <= 4096 take k_edt_cols_exact/k_edt_rows_exact instead: the same
-// results from a closed form of pass 1 and from pass 2 with its breakpoint
-// comparisons decided in integer arithmetic (the argument is given above
-// those kernels).
+// both sides <= 16384 take k_edt_cols/k_edt_rows instead: the same values from
+// a search per cell (the argument is given above those kernels).
 #include "rangelibc.h"
 #include "rlc_internal.cuh"
 
@@ -25,22 +23,47 @@ namespace {
 
 constexpr double kDblMax = 1.7976931348623157e308;
 
-__global__ void k_pack_bits(const uint8_t* __restrict__ occ, int W, int H, int TY, uint64_t* __restrict__ bits) {
-    int TX = (W + 7) >> 3;
-    long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+// bit j set where byte j of v is not 0
+__device__ __forceinline__ unsigned nonzero_bytes(uint64_t v) {
+    const uint64_t low = 0x7f7f7f7f7f7f7f7full;
+    const uint64_t top = (((v & low) + low) | v) & ~low;                 // 0x80 in every such byte
+    return (unsigned)(((top >> 7) * 0x0102040810204080ull) >> 56);
+}
+
+// Occupancy bytes to bit tiles, one thread per tile.  ROWS: the grid as image rows, occ[y * W + x]
+// (numpy's [row, col]); otherwise occ[x * H + y].  A tile's eight lines of eight bytes are read as
+// 8-byte words where the lines are aligned to them, and consecutive lanes read consecutive words:
+// the grid may be host memory read in place over NVLink-C2C, so the transposition that image rows
+// need costs nothing here (4.9 ms in numpy for 2048^2, 29 us for this kernel).
+template <bool ROWS>
+__global__ void __launch_bounds__(256) k_pack_bits(const uint8_t* __restrict__ occ, int W, int H, int TY,
+                                                   uint64_t* __restrict__ bits) {
+    const int TX = (W + 7) >> 3;
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= (long long)TX * TY) return;
-    int tx = (int)(t / TY), ty = (int)(t - (long long)tx * TY);
+    const int tx = ROWS ? (int)(t % TX) : (int)(t / TY), ty = ROWS ? (int)(t / TX) : (int)(t % TY);
+    const int inner = ROWS ? W : H, outer = ROWS ? H : W;             // contiguous axis, line count
+    const int i0 = (ROWS ? tx : ty) << 3, o0 = (ROWS ? ty : tx) << 3;
+    const bool wide = i0 + 8 <= inner && inner % 8 == 0 && (reinterpret_cast<uintptr_t>(occ) & 7) == 0;
     uint64_t w = 0;
-    for (int i = 0; i < 8; ++i) {
-        int x = (tx << 3) + i;
-        if (x >= W) break;
-        for (int j = 0; j < 8; ++j) {
-            int y = (ty << 3) + j;
-            if (y >= H) break;
-            if (occ[(size_t)x * H + y]) w |= 1ull << ((i << 3) | j);
+#pragma unroll
+    for (int o = 0; o < 8; ++o) {
+        if (o0 + o >= outer) break;
+        const uint8_t* line = occ + (size_t)(o0 + o) * inner + i0;
+        unsigned m = 0;
+        if (wide) {
+            m = nonzero_bytes(*reinterpret_cast<const uint64_t*>(line));
+        } else {
+            for (int i = 0; i < 8; ++i)
+                if (i0 + i < inner && line[i]) m |= 1u << i;
+        }
+        if (ROWS) {   // line o is row y & 7 = o: its bits i are x & 7, at bit (i << 3) | o
+            for (int i = 0; i < 8; ++i) w |= (uint64_t)((m >> i) & 1u) << ((i << 3) | o);
+        } else {
+            w |= (uint64_t)m << (o << 3);
         }
     }
-    bits[t] = w;
+    bits[(size_t)tx * TY + ty] = w;
 }
 
 __device__ __forceinline__ bool occ_bit(const uint64_t* __restrict__ bits, int TY, int x, int y) {
@@ -115,28 +138,30 @@ __global__ void k_edt_pass_x(const float* g, int W, int H, float* dt, uint32_t* 
     fh_line(RowInput{g, H, y}, RowSqrtOutput{dt, H, y}, (unsigned)W, v + y, z + y, (size_t)H);
 }
 
-// ---- exact-comparison passes for maps with both sides <= 16384 --------------------------------
+// ---- maps with both sides <= 16384 -------------------------------------------------------------
 //
 // For such maps a cheaper computation of the F-H steps above gives the same results bit for bit.
-// Every finite key f(q) + q*q (a float sum, as in the reference) is an integer below 2^29, and
-// every breakpoint is a quotient a / b of integers with |a| < 2^29 and 2 <= b <= 2 (n - 1) < 2^15,
-// computed in double exactly up to the final rounding.  Rounding moves a / b by at most
+// Every finite key K(q) = f(q) + q*q (a float sum, as in the reference) is an integer below 2^29,
+// and every breakpoint is a quotient a / b of integers with |a| < 2^29 and 2 <= b <= 2 (n - 1) <
+// 2^15, computed in double exactly up to the final rounding.  Rounding moves a / b by at most
 // 2^-53 |a| / b, while two different quotients a / b and c / d differ by at least 1 / (b d);
 // since |a| d + |c| b < 2^45 < 2^53, rounding never reverses or merges two different quotients,
 // and equal quotients round alike.  A comparison of rounded breakpoints (s <= z[k],
-// z[k + 1] < q) therefore has the outcome of the exact comparison of the quotients, which integer
-// cross-multiplication decides.  Comparisons with a FLT_MAX key are evaluated in double exactly
-// as the reference does.  The stack holds (v, f(v)) only; breakpoints are recomputed from it.
-//  * sides <= 4096, pass 1 (input 0 on occupied cells, FLT_MAX elsewhere): q*q < 2^24 is exact,
-//    a breakpoint between two occupied cells p < q is (p + q) / 2, a FLT_MAX parabola is popped
-//    by the next occupied cell (their breakpoint is below -FLT_MAX / 8192) or lies beyond the
-//    line's end (its breakpoint is above FLT_MAX / 8192), so the envelope picks the nearest
-//    occupied cell p and stores (q - p)^2, or FLT_MAX + (q - p)^2 = FLT_MAX in a column without
-//    one: a closed form per column (edt_col_exact);
-//  * sides <= 4096, pass 2: the stack of each row in shared memory (k_edt_rows_exact);
-//  * a side above 4096: q*q rounds, the closed form no longer holds, and both passes run the
-//    exact-comparison steps with the stack in global memory (k_edt_cols_fh, k_edt_rows_fh).
-constexpr int kEdtExactSide = 4096;           // closed-form pass 1, shared-memory pass 2
+// z[k + 1] < q) therefore has the outcome of the exact comparison of the quotients.
+//  * edt_col_exact and fh_line_exact are the reference's steps with those comparisons decided in
+//    integers, one line after the other; comparisons with a FLT_MAX key run in double as in the
+//    reference.  No kernel runs them: they state the rule that the searches below are tested with.
+//  * So the envelope is the exact lower envelope of the lines K(p) - 2 p q, and at an integer q it
+//    takes the smallest p among those with the least K(p) - 2 p q: `s <= z[k]` drops a vertex that
+//    is nowhere strictly least, `z[k + 1] < q` stays with the left vertex where two tie.  A
+//    FLT_MAX vertex is never taken while a finite one exists (its breakpoints lie beyond
+//    +-FLT_MAX / 2^15), and a line without a finite input gives FLT_MAX.
+//  * K(p) - 2 p q + q*q = f(p) + (p - q)^2 + e(p), where e(p) is what rounding added to the key: 0
+//    while keys stay below 2^24, at most 1 below 2^25 (sides <= 4096: q*q is exact), at most
+//    8 + 16 below 2^29.  Since f >= 0, no vertex further from q than the square root of (the least
+//    value found so far + the bound of e) can be least: each cell is found by searching outward
+//    from it, all cells in parallel (edt_col_search, edt_row_search).
+constexpr int kEdtExactSide = 4096;           // q*q is exact
 constexpr int kEdtIntSide = 16384;            // integer comparisons
 constexpr float kEdtExactKey = 536870912.0f;  // 2^29: finite keys are below it
 
@@ -289,100 +314,341 @@ __host__ __device__ void fh_line_exact(const In& f, const Out& out, unsigned n, 
     }
 }
 
-// one thread per column; dynamic shared memory: blockDim.x * (TY + 1) uint16
-__global__ void k_edt_cols_exact(const uint64_t* __restrict__ bits, int W, int H, int TY, float* __restrict__ g) {
-    extern __shared__ uint16_t s_next[];
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
-    if (x >= W) return;
-    edt_col_exact(bits + (size_t)(x >> 3) * TY, (x & 7) << 3, H, TY, s_next + (size_t)threadIdx.x * (TY + 1),
-                  g + (size_t)x * H);
+// ---- the searches
+constexpr unsigned kEdtNone = 0xFFFFu;   // "no occupied cell in the column"
+constexpr int kEdtNear = 32;             // distances searched one by one before whole blocks
+constexpr int kEdtBlock = 32;            // cells of a row whose least pass-1 distance is kept together
+
+// f of a pass-1 distance d: the float square (pass 1 stores 0 + (q - v)^2), FLT_MAX for none
+__host__ __device__ __forceinline__ float edt_f(unsigned d) {
+    return d == kEdtNone ? FLT_MAX : edt_fmul((float)d, (float)d);
 }
 
-// one thread per row; dynamic shared memory: blockDim.x * W * (4 + 2) bytes
-__global__ void k_edt_rows_exact(const float* __restrict__ g, int W, int H, float* __restrict__ dt) {
-    extern __shared__ __align__(16) unsigned char s_stack[];
-    const int y = blockIdx.x * blockDim.x + threadIdx.x;
-    if (y >= H) return;
-    float* sf = reinterpret_cast<float*>(s_stack) + (size_t)threadIdx.x * W;
-    uint16_t* sv = reinterpret_cast<uint16_t*>(reinterpret_cast<float*>(s_stack) + (size_t)blockDim.x * W) +
-                   (size_t)threadIdx.x * W;
-    fh_line_exact(RowInput{g, H, y}, RowSqrtOutput{dt, H, y}, (unsigned)W, sv, sf, 1);
+// Pass 1 at row q: the distance to the vertex F-H takes.  prev / next: the last occupied row <= q
+// (-1: none) and the first >= q (kEdtNone: none).  Up to 4096 rows that is the nearest of them;
+// above, q*q rounds (e <= 8 either way), so that a vertex up to sqrt(d*d + 16) away can win.
+template <class Occ>
+__host__ __device__ __forceinline__ unsigned edt_col_search(int prev, unsigned next, int q, int H, const Occ& occ) {
+    int d = 0x7FFFFFFF;
+    if (prev >= 0) d = q - prev;
+    if (next != kEdtNone && (int)next - q < d) d = (int)next - q;
+    if (d == 0x7FFFFFFF) return kEdtNone;
+    if (H <= kEdtExactSide) return (unsigned)d;
+    const int limit = d * d + 16;
+    int best = 0x7FFFFFFF, at = 0;
+    for (int e = d; e * e <= limit; ++e)
+        for (int side = 0; side < 2; ++side) {
+            const int p = side ? q + e : q - e;
+            if (p < 0 || p >= H || !occ(p)) continue;
+            const int cost = (int)(float)(p * p) - 2 * p * q;
+            if (cost < best || (cost == best && p < at)) {
+                best = cost;
+                at = p;
+            }
+        }
+    return (unsigned)(at < q ? q - at : at - q);
 }
 
-// a side above 4096: one thread per line, the lines' stacks interleaved in global memory
-// (entry k of line l at k * lines + l)
-__global__ void k_edt_cols_fh(const uint64_t* __restrict__ bits, int W, int H, int TY, float* g, uint16_t* sv,
-                              float* sf) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
-    if (x >= W) return;
-    fh_line_exact(OccInput{bits, TY, x}, ColOutput{g, (size_t)x * H}, (unsigned)H, sv + x, sf + x, (size_t)W);
-}
-
-__global__ void k_edt_rows_fh(const float* g, int W, int H, float* dt, uint16_t* sv, float* sf) {
-    const int y = blockIdx.x * blockDim.x + threadIdx.x;
-    if (y >= H) return;
-    fh_line_exact(RowInput{g, H, y}, RowSqrtOutput{dt, H, y}, (unsigned)W, sv + y, sf + y, (size_t)H);
-}
-
-__global__ void k_dt_to_tiled(const float* __restrict__ lin, int W, int H, int TY, float* __restrict__ tiled) {
-    long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    int TX = (W + 7) >> 3;
-    if (i >= (long long)TX * TY * 64) return;
-    long long tile = i >> 6;
-    int within = (int)(i & 63);
-    int tx = (int)(tile / TY), ty = (int)(tile - (long long)tx * TY);
-    int x = (tx << 3) + (within >> 3), y = (ty << 3) + (within & 7);
-    tiled[i] = (x < W && y < H) ? lin[(size_t)x * H + y] : 0.0f;
-}
-
-// compact distance transform: uint16 d^2 in 8x8 tiles, 4x4 cells per 32-B sector
-__global__ void k_dt_to_u16(const float* __restrict__ lin, int W, int H, int TY, uint16_t* __restrict__ out) {
-    long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    int TX = (W + 7) >> 3;
-    if (i >= (long long)TX * TY * 64) return;
-    long long tile = i >> 6;
-    int within = (int)(i & 63);
-    int sector = within >> 4, cell = within & 15;
-    int tx = (int)(tile / TY), ty = (int)(tile - (long long)tx * TY);
-    int x = (tx << 3) + ((sector >> 1) << 2) + (cell >> 2);
-    int y = (ty << 3) + ((sector & 1) << 2) + (cell & 3);
-    uint16_t v = 0xFFFF;
-    if (x < W && y < H) {
-        // dt = sqrtf(D) for an integer D; D is recovered exactly while D < 2^22
-        double d = (double)lin[(size_t)x * H + y];
-        double d2 = rint(d * d);
-        if (d2 < 65535.0 && __fsqrt_rn((float)d2) == (float)d) v = (uint16_t)d2;
+// Pass 2 at column q of a row of W pass-1 distances g(p): the value whose square root is the
+// distance transform.  gmin(b): the least distance of columns [32 b, 32 b + 32).  Distances up to
+// kEdtNear are searched one by one (most cells of a map with walls end there), farther ones a
+// block at a time, so that an empty map costs W / 32 block reads per cell and not W.
+//
+// Keys below 2^24: the value is the least f(p) + (p - q)^2, and which p gives it does not matter.
+// So the near search runs in groups of four distances with one exit test, and a position past the
+// row's end reads its last cell instead (which at that distance is never less than it is itself).
+template <class G, class GMin>
+__host__ __device__ __forceinline__ float edt_row_search_exact(const G& g, const GMin& gmin, int W, int q) {
+    // 65535^2 + e^2 < 2^32 for e <= 256 stands for "none"; every true value is below 2^24
+    unsigned best = g(q) * g(q);
+    int e = 1;
+    for (; e <= kEdtNear && (unsigned)(e * e) < best; e += 4) {
+        unsigned d[8];
+#ifdef __CUDA_ARCH__
+#pragma unroll
+#endif
+        for (int u = 0; u < 4; ++u) {
+            d[2 * u] = g(q - e - u > 0 ? q - e - u : 0);
+            d[2 * u + 1] = g(q + e + u < W ? q + e + u : W - 1);
+        }
+#ifdef __CUDA_ARCH__
+#pragma unroll
+#endif
+        for (int u = 0; u < 4; ++u) {
+            const unsigned e2 = (unsigned)((e + u) * (e + u));
+            const unsigned l = d[2 * u] * d[2 * u] + e2, r = d[2 * u + 1] * d[2 * u + 1] + e2;
+            const unsigned m = l < r ? l : r;
+            best = m < best ? m : best;
+        }
     }
-    out[i] = v;
+    if (e > kEdtNear && (unsigned)(e * e) < best) {
+        const int own = q / kEdtBlock, nb = (W + kEdtBlock - 1) / kEdtBlock;
+        for (int k = 1;; ++k) {
+            bool open = false;
+            for (int side = 0; side < 2; ++side) {
+                const int b = side ? own + k : own - k;
+                if (b < 0 || b >= nb) continue;
+                const unsigned gap = (unsigned)(side ? b * kEdtBlock - q : q - (b * kEdtBlock + kEdtBlock - 1));
+                if (gap * gap >= best) continue;
+                open = true;
+                const unsigned m = gmin(b);
+                if (m == kEdtNone || gap * gap + m * m >= best) continue;
+                const int end = b * kEdtBlock + kEdtBlock < W ? b * kEdtBlock + kEdtBlock : W;
+                for (int p = b * kEdtBlock; p < end; ++p) {
+                    const unsigned d = g(p);
+                    if (d == kEdtNone) continue;
+                    const unsigned c = d * d + (unsigned)((p - q) * (p - q));
+                    best = c < best ? c : best;
+                }
+            }
+            if (!open) break;
+        }
+    }
+    return best < (1u << 24) ? (float)best : FLT_MAX;
 }
 
-// step of the march from each cell, RangeLib.h:957 (t += max(distance * 0.999, 1)); 0 marks an
-// occupied cell (distance 0), where the march ends
-__global__ void k_dt_to_step(const float* __restrict__ lin, long long n, float* __restrict__ step) {
+// Keys that round: they are formed as the reference rounds them, `slack` bounds e, and the smallest
+// p of the least keys is the one taken.
+template <class G, class GMin>
+__host__ __device__ __forceinline__ float edt_row_search_rounded(const G& g, const GMin& gmin, int W, int q, int slack) {
+    int best = 0x7FFFFFFF, at = q;   // best: K(p) - 2 p q + q q
+    unsigned d_at = kEdtNone;
+    auto take = [&](int p) {
+        const unsigned d = g(p);
+        if (d == kEdtNone) return;
+        const int cost = (int)edt_key(edt_f(d), (unsigned)p) - 2 * p * q + q * q;
+        if (cost < best || (cost == best && p < at)) {
+            best = cost;
+            at = p;
+            d_at = d;
+        }
+    };
+    take(q);
+    int e = 1;
+    for (; e <= kEdtNear && e * e - slack <= best; ++e) {
+        if (q - e >= 0) take(q - e);
+        if (q + e < W) take(q + e);
+    }
+    if (e > kEdtNear && e * e - slack <= best) {
+        const int own = q / kEdtBlock, nb = (W + kEdtBlock - 1) / kEdtBlock;
+        for (int k = 1;; ++k) {
+            bool open = false;
+            for (int side = 0; side < 2; ++side) {
+                const int b = side ? own + k : own - k;
+                if (b < 0 || b >= nb) continue;
+                const int gap = side ? b * kEdtBlock - q : q - (b * kEdtBlock + kEdtBlock - 1);
+                if (gap * gap - slack > best) continue;
+                open = true;
+                const unsigned m = gmin(b);
+                if (m == kEdtNone || gap * gap - slack > best - (int)edt_f(m)) continue;
+                const int end = b * kEdtBlock + kEdtBlock < W ? b * kEdtBlock + kEdtBlock : W;
+                for (int p = b * kEdtBlock; p < end; ++p) take(p);
+            }
+            if (!open) break;
+        }
+    }
+    if (d_at == kEdtNone) return FLT_MAX;
+    const float dq = edt_fsub((float)q, (float)at);
+    return edt_fadd(edt_f(d_at), edt_fmul(dq, dq));
+}
+
+template <bool EXACT, class G, class GMin>
+__host__ __device__ __forceinline__ float edt_row_search(const G& g, const GMin& gmin, int W, int q, int slack) {
+    return EXACT ? edt_row_search_exact(g, gmin, W, q) : edt_row_search_rounded(g, gmin, W, q, slack);
+}
+
+// Pass 1, a few blocks per 8 columns (a row of bit tiles), each answering a share of the rows.  Bound by its 2 bytes per cell written.  A
+// warp per column finds, for every tile, the last occupied row before it and the first one at or
+// after it (a ballot per 32 tiles); every thread then answers its rows from the tile's byte and
+// those two.  2048^2: 121 us with one thread per column -> 17 us.
+__global__ void __launch_bounds__(256) k_edt_cols(const uint64_t* __restrict__ bits, int W, int H, int TY,
+                                                  uint16_t* __restrict__ g) {
+    extern __shared__ uint16_t s_near[];   // per column: before[TY], from[TY]
+    const int tx = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint64_t* col = bits + (size_t)tx * TY;
+    const unsigned full = 0xffffffffu;
+    {
+        uint16_t* before = s_near + (size_t)warp * 2 * TY;
+        uint16_t* from = before + TY;
+        const int chunks = (TY + 31) >> 5, sh = warp << 3;
+        unsigned carry = kEdtNone;
+        for (int k = 0; k < chunks; ++k) {
+            const int c = (k << 5) + lane;
+            const unsigned b = c < TY ? (unsigned)(col[c] >> sh) & 0xFFu : 0u;
+            const unsigned row = b ? ((unsigned)c << 3) + (unsigned)edt_msb(b) : 0u;
+            const unsigned mask = __ballot_sync(full, b != 0), below = mask & ((1u << lane) - 1u);
+            const unsigned v = __shfl_sync(full, row, below ? 31 - __clz(below) : 0);
+            if (c < TY) before[c] = (uint16_t)(below ? v : carry);
+            const unsigned lastv = __shfl_sync(full, row, mask ? 31 - __clz(mask) : 0);
+            if (mask) carry = lastv;
+        }
+        carry = kEdtNone;
+        for (int k = chunks - 1; k >= 0; --k) {
+            const int c = (k << 5) + lane;
+            const unsigned b = c < TY ? (unsigned)(col[c] >> sh) & 0xFFu : 0u;
+            const unsigned row = b ? ((unsigned)c << 3) + (unsigned)edt_lsb(b) : 0u;
+            const unsigned mask = __ballot_sync(full, b != 0), at = mask & ~((1u << lane) - 1u);
+            const unsigned v = __shfl_sync(full, row, at ? __ffs(at) - 1 : 0);
+            if (c < TY) from[c] = (uint16_t)(at ? v : carry);
+            const unsigned firstv = __shfl_sync(full, row, mask ? __ffs(mask) - 1 : 0);
+            if (mask) carry = firstv;
+        }
+    }
+    __syncthreads();
+    for (int j = 0; j < 8; ++j) {
+        const int x = (tx << 3) + j;
+        if (x >= W) break;
+        const uint16_t* before = s_near + (size_t)j * 2 * TY;
+        const uint16_t* from = before + TY;
+        const auto occ = [&](int p) { return (col[p >> 3] >> ((j << 3) | (p & 7))) & 1ull; };
+        for (int q = blockIdx.y * blockDim.x + threadIdx.x; q < H; q += gridDim.y * blockDim.x) {
+            const int c = q >> 3, in = q & 7;
+            const unsigned b = (unsigned)(col[c] >> (j << 3)) & 0xFFu;
+            const unsigned lo = b & ((2u << in) - 1u), hi = b >> in;
+            int prev = lo ? (c << 3) + edt_msb(lo) : (before[c] == kEdtNone ? -1 : (int)before[c]);
+            unsigned next = hi ? (unsigned)(q + edt_lsb(hi)) : (c + 1 < TY ? from[c + 1] : kEdtNone);
+            g[(size_t)x * H + q] = (uint16_t)edt_col_search(prev, next, q, H, occ);
+        }
+    }
+}
+
+// the least pass-1 distance of every block of kEdtBlock columns, per row: gmin[b * H + y]
+__global__ void __launch_bounds__(256) k_edt_block_min(const uint16_t* __restrict__ g, int W, int H,
+                                                       uint16_t* __restrict__ gmin) {
+    const int y = blockIdx.x * blockDim.x + threadIdx.x, b = blockIdx.y;
+    if (y >= H) return;
+    const int x0 = b * kEdtBlock, x1 = min(x0 + kEdtBlock, W);
+    unsigned m = kEdtNone;
+#pragma unroll 8
+    for (int x = x0; x < x1; ++x) m = min(m, (unsigned)__ldg(g + (size_t)x * H + y));
+    gmin[(size_t)b * H + y] = (uint16_t)m;
+}
+
+// Every form of the distance transform at cell (x, y), value dt; padding cells of the tiles too.
+//  * tiled: the float in 8x8 tiles (0 in the padding);
+//  * u16: d^2 in 8x8 tiles, 4x4 cells per 32-byte sector, u8: d^2 in 8x8 tiles of 64 bytes; all
+//    ones = "read the float" (and in the padding).  dt = sqrtf(D) of an integer D, and for D <
+//    2^16 the float product dt * dt is within 0.02 of it;
+//  * step: the march step max(dt * 0.999, 1) of RangeLib.h:957, 0 on occupied cells.
+__device__ __forceinline__ void store_layouts(const DtOut& o, int W, int H, int TY, int x, int y, float dt) {
+    const bool in = x < W && y < H;
+    const size_t tile = ((size_t)(x >> 3) * TY + (y >> 3)) << 6;
+    const float d2 = rintf(__fmul_rn(dt, dt));
+    if (in) {
+        const size_t i = (size_t)x * H + y;
+        o.dt[i] = dt;
+        const float v = __fmul_rn(dt, 0.999f);
+        o.step[i] = dt <= 0.0f ? 0.0f : (v < 1.0f ? 1.0f : v);
+    }
+    o.tiled[tile + ((x & 7) << 3) + (y & 7)] = in ? dt : 0.0f;
+    o.u16[tile + ((((x >> 2) & 1) << 1 | ((y >> 2) & 1)) << 4) + (((x & 3) << 2) | (y & 3))] =
+        in && d2 < 65535.0f ? (uint16_t)d2 : (uint16_t)0xFFFF;
+    o.u8[tile + ((x & 7) << 3) + (y & 7)] = in && d2 <= 254.0f ? (uint8_t)d2 : (uint8_t)0xFF;
+}
+
+// Pass 2, one thread per cell, 32 consecutive y per warp (the searched distances of a warp are
+// whole 64-byte pieces) x 8 x per block (which share them in the L1).  Bound by the search's
+// instructions: about 2 x (mean distance) reads per cell.  ALL: writes every layout, straight from
+// the search (60 MB at 2048^2; four more kernels read the linear one back before).
+// 2048^2 with the layouts: 1553 + 117 us with one thread per row -> 118 us.
+template <bool EXACT, bool ALL>
+__global__ void __launch_bounds__(256) k_edt_rows(const uint16_t* __restrict__ g, const uint16_t* __restrict__ gmin,
+                                                  int W, int H, int TY, int slack, DtOut o) {
+    const int y = blockIdx.x * 32 + threadIdx.x, x = blockIdx.y * 8 + threadIdx.y;
+    float dt = 0.0f;
+    if (x < W && y < H)
+        dt = __fsqrt_rn(edt_row_search<EXACT>([&](int p) { return (unsigned)__ldg(g + (size_t)p * H + y); },
+                                              [&](int b) { return (unsigned)__ldg(gmin + (size_t)b * H + y); }, W, x,
+                                              slack));
+    if (ALL) {
+        if ((y >> 3) < TY) store_layouts(o, W, H, TY, x, y, dt);
+    } else if (x < W && y < H) {
+        o.dt[(size_t)x * H + y] = dt;
+    }
+}
+
+// the layouts of a linear distance transform (maps with a side above 16384)
+__global__ void __launch_bounds__(256) k_dt_layouts(const float* __restrict__ lin, int W, int H, int TY, DtOut o) {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float d = lin[i];
-    const float v = __fmul_rn(d, 0.999f);
-    step[i] = d <= 0.0f ? 0.0f : (v < 1.0f ? 1.0f : v);
+    const int TX = (W + 7) >> 3;
+    if (i >= (long long)TX * TY * 64) return;
+    const long long tile = i >> 6;
+    const int within = (int)(i & 63), tx = (int)(tile / TY), ty = (int)(tile - (long long)tx * TY);
+    const int x = (tx << 3) + (within >> 3), y = (ty << 3) + (within & 7);
+    store_layouts(o, W, H, TY, x, y, x < W && y < H ? lin[(size_t)x * H + y] : 0.0f);
 }
 
-// 8-bit squared distance in 8x8 tiles of 64 bytes (x-major within the tile):
-// d^2 <= 254 exactly, 255 = "read the float"
-__global__ void k_dt_to_u8(const float* __restrict__ lin, int W, int H, int TY, uint8_t* __restrict__ out) {
-    long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    int TX = (W + 7) >> 3;
-    if (i >= (long long)TX * TY * 64) return;
-    long long tile = i >> 6;
-    int within = (int)(i & 63);
-    int tx = (int)(tile / TY), ty = (int)(tile - (long long)tx * TY);
-    int x = (tx << 3) + (within >> 3), y = (ty << 3) + (within & 7);
-    uint8_t v = 0xFF;
-    if (x < W && y < H) {
-        double d = (double)lin[(size_t)x * H + y];
-        double d2 = rint(d * d);
-        if (d2 <= 254.0 && __fsqrt_rn((float)d2) == (float)d) v = (uint8_t)d2;
+// ---- equal-step runs
+// Which neighbouring cells have equal steps, one bit per cell and axis: bit y & 31 of eqy[x * HW +
+// (y >> 5)] is step(x, y - 1) == step(x, y), bit x & 31 of eqx[(x >> 5) * H + y] is step(x - 1, y)
+// == step(x, y).  A warp reads a 32 x 32 patch once, 32 independent coalesced rows.
+__global__ void __launch_bounds__(256) k_step_eq(const float* __restrict__ step, int W, int H, int HW,
+                                                 uint32_t* __restrict__ eqx, uint32_t* __restrict__ eqy) {
+    const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31, XW = (W + 31) >> 5;
+    if (w >= (long long)XW * HW) return;
+    const int xw = (int)(w / HW), yw = (int)(w - (long long)xw * HW), x0 = xw << 5, y = (yw << 5) + lane;
+    const bool in = y < H;
+    const float none = __int_as_float(0x7fc00000);   // equal to nothing
+    // lane j: the cell before this patch's rows in column x0 + j
+    const float edge = yw > 0 && x0 + lane < W ? __ldg(step + (size_t)(x0 + lane) * H + (yw << 5) - 1) : none;
+    float prev = in && x0 > 0 ? __ldg(step + (size_t)(x0 - 1) * H + y) : none;
+    uint32_t mx = 0, my = 0;
+#pragma unroll
+    for (int j0 = 0; j0 < 32; j0 += 8) {
+        float v[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = in && x0 + j0 + j < W ? __ldg(step + (size_t)(x0 + j0 + j) * H + y) : none;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            float left = __shfl_up_sync(0xffffffffu, v[j], 1);
+            const float before = __shfl_sync(0xffffffffu, edge, j0 + j);
+            if (lane == 0) left = before;
+            const uint32_t m = __ballot_sync(0xffffffffu, left == v[j]);
+            if (lane == j0 + j) my = m;   // lane j keeps column x0 + j's word
+            mx |= (uint32_t)(prev == v[j]) << (j0 + j);
+            prev = v[j];
+        }
     }
-    out[i] = v;
+    if (x0 + lane < W) eqy[(size_t)(x0 + lane) * HW + yw] = my;
+    if (in) eqx[(size_t)xw * H + y] = mx;
+}
+
+// consecutive set bits at position j and below (down) or at j and above (up) of a bit line whose
+// word w is word(w), at most 255; up stops at the line's end (nw words)
+template <class Word>
+__device__ __forceinline__ unsigned bits_down(const Word& word, int j) {
+    unsigned n = 0;
+    for (int w = j >> 5, l = j & 31;; --w, l = 31) {
+        const unsigned t = (unsigned)__clz((int)~(word(w) << (31 - l)));
+        n += min(t, (unsigned)(l + 1));
+        if (t < (unsigned)(l + 1) || w == 0 || n >= 255u) break;
+    }
+    return min(n, 255u);
+}
+template <class Word>
+__device__ __forceinline__ unsigned bits_up(const Word& word, int j, int nw) {
+    unsigned n = 0;
+    for (int w = j >> 5, l = j & 31; w < nw; ++w, l = 0) {
+        const unsigned z = ~(word(w) >> l), t = min(z ? (unsigned)__ffs((int)z) - 1u : 32u, 32u - (unsigned)l);
+        n += t;
+        if (t < 32u - (unsigned)l || n >= 255u) break;
+    }
+    return min(n, 255u);
+}
+
+// runs[x * H + y]: how many cells after (x, y) along +y, -y, +x and -x have its step (bits 0-7,
+// 8-15, 16-23, 24-31; at most 255 each), counted in the bit lines: one or two words per direction
+// where a thread per line walked the map before.  2048^2: 2106 us -> 51 us with k_step_eq.
+__global__ void __launch_bounds__(256) k_step_runs(const uint32_t* __restrict__ eqx, const uint32_t* __restrict__ eqy,
+                                                   int W, int H, int HW, uint32_t* __restrict__ runs) {
+    const unsigned yb = ((unsigned)H + 31u) >> 5, bx = blockIdx.x / yb;   // 32 y x 8 x cells per block
+    const int x = (int)(bx * 8 + threadIdx.y), y = (int)((blockIdx.x - bx * yb) * 32 + threadIdx.x);
+    if (x >= W || y >= H) return;
+    const auto wx = [&](int w) { return __ldg(eqx + (size_t)w * H + y); };
+    const auto wy = [&](int w) { return __ldg(eqy + (size_t)x * HW + w); };
+    runs[(size_t)x * H + y] = bits_up(wy, y + 1, HW) | bits_down(wy, y) << 8 | bits_up(wx, x + 1, (W + 31) >> 5) << 16 |
+              bits_down(wx, x) << 24;
 }
 
 // RangeLib.h:293-312: an occupied cell with any in-grid free 8-neighbour.
@@ -413,15 +679,18 @@ inline unsigned blocks_for(long long n, int b) { return (unsigned)((n + b - 1) /
 
 }  // namespace
 
-cudaError_t launch_pack_bits(const uint8_t* d_occ, int W, int H, uint64_t* d_bits, cudaStream_t s) {
+cudaError_t launch_pack_bits(const uint8_t* d_occ, int W, int H, bool rows, uint64_t* d_bits, cudaStream_t s) {
     int TY = (H + 7) >> 3, TX = (W + 7) >> 3;
     long long n = (long long)TX * TY;
     if (n == 0) return cudaSuccess;
-    k_pack_bits<<<blocks_for(n, 256), 256, 0, s>>>(d_occ, W, H, TY, d_bits);
+    if (rows) k_pack_bits<true><<<blocks_for(n, 256), 256, 0, s>>>(d_occ, W, H, TY, d_bits);
+    else k_pack_bits<false><<<blocks_for(n, 256), 256, 0, s>>>(d_occ, W, H, TY, d_bits);
     return cudaGetLastError();
 }
 
 size_t edt_scratch_bytes(int W, int H) {
+    if (W <= kEdtIntSide && H <= kEdtIntSide)   // pass-1 distances and their block minima, uint16
+        return ((size_t)W + (size_t)((W + kEdtBlock - 1) / kEdtBlock)) * H * sizeof(uint16_t);
     // pass-1 output g (W*H floats) + per-line v (n uint32) and z (n+1 doubles);
     // both passes reuse the same v/z region sized for the larger pass
     size_t g = (size_t)W * H * sizeof(float);
@@ -431,38 +700,37 @@ size_t edt_scratch_bytes(int W, int H) {
     return ((g + 255) & ~(size_t)255) + vz + 256;
 }
 
-cudaError_t launch_edt(const uint64_t* d_bits, int W, int H, int TY, float* d_dt, void* scratch,
+cudaError_t launch_edt(const uint64_t* d_bits, int W, int H, int TY, const DtOut& o, void* scratch,
                        size_t scratch_bytes, cudaStream_t s) {
     if (W <= 0 || H <= 0) return cudaSuccess;
     if (scratch_bytes < edt_scratch_bytes(W, H)) return cudaErrorInvalidValue;
+    const bool all = o.step != nullptr;
     char* base = static_cast<char*>(scratch);
-    float* g = reinterpret_cast<float*>(base);
-    if (W <= kEdtExactSide && H <= kEdtExactSide) {
-        k_edt_cols_exact<<<blocks_for(W, 32), 32, 32 * (TY + 1) * sizeof(uint16_t), s>>>(d_bits, W, H, TY, g);
-        cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) return e;
-        // rows per block: the stack's shared memory, and about one block per SM of a 152-SM part
-        constexpr int kSmemCap = 227 * 1024;
-        const int per_line = W * (int)(sizeof(float) + sizeof(uint16_t));
-        int lines = (H + 151) / 152;
-        lines = lines < kSmemCap / per_line ? lines : kSmemCap / per_line;
-        lines = lines < 32 ? (lines > 0 ? lines : 1) : 32;
+    if (W <= kEdtIntSide && H <= kEdtIntSide) {
+        uint16_t* g = reinterpret_cast<uint16_t*>(base);
+        uint16_t* gmin = g + (size_t)W * H;
+        const size_t smem = (size_t)8 * 2 * TY * sizeof(uint16_t);   // at most 64 KB
         static std::atomic<unsigned long long> attr_done{0};
-        e = ensure_smem_attr(k_edt_rows_exact, kSmemCap, attr_done);
+        cudaError_t e = ensure_smem_attr(k_edt_cols, 8 * 2 * (kEdtIntSide / 8) * (int)sizeof(uint16_t), attr_done);
         if (e != cudaSuccess) return e;
-        k_edt_rows_exact<<<blocks_for(H, lines), lines, (size_t)lines * per_line, s>>>(g, W, H, d_dt);
+        k_edt_cols<<<dim3((W + 7) >> 3, min(4, (H + 255) / 256)), 256, smem, s>>>(d_bits, W, H, TY, g);
+        e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+        k_edt_block_min<<<dim3(blocks_for(H, 256), (W + kEdtBlock - 1) / kEdtBlock), 256, 0, s>>>(g, W, H, gmin);
+        e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+        const dim3 grid(blocks_for((long long)TY * 8, 32), (W + 7) >> 3), block(32, 8);
+        // keys below 2^24 are exact; see above for the bounds of what rounding adds
+        const bool exact = (long long)(W - 1) * (W - 1) + (long long)(H - 1) * (H - 1) < (1ll << 24);
+        const int slack = exact ? 0 : (W <= kEdtExactSide && H <= kEdtExactSide ? 1 : 24);
+        if (exact && all) k_edt_rows<true, true><<<grid, block, 0, s>>>(g, gmin, W, H, TY, slack, o);
+        else if (exact) k_edt_rows<true, false><<<grid, block, 0, s>>>(g, gmin, W, H, TY, slack, o);
+        else if (all) k_edt_rows<false, true><<<grid, block, 0, s>>>(g, gmin, W, H, TY, slack, o);
+        else k_edt_rows<false, false><<<grid, block, 0, s>>>(g, gmin, W, H, TY, slack, o);
         return cudaGetLastError();
     }
+    float* g = reinterpret_cast<float*>(base);
     size_t goff = ((size_t)W * H * sizeof(float) + 255) & ~(size_t)255;
-    if (W <= kEdtIntSide && H <= kEdtIntSide) {   // stacks: W * H floats, then W * H uint16 (either pass)
-        float* sf = reinterpret_cast<float*>(base + goff);
-        uint16_t* sv = reinterpret_cast<uint16_t*>(base + goff + (size_t)W * H * sizeof(float));
-        k_edt_cols_fh<<<blocks_for(W, 32), 32, 0, s>>>(d_bits, W, H, TY, g, sv, sf);
-        cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) return e;
-        k_edt_rows_fh<<<blocks_for(H, 32), 32, 0, s>>>(g, W, H, d_dt, sv, sf);
-        return cudaGetLastError();
-    }
     // per pass: z (n+1 doubles per line) first, then v (n uint32 per line)
     double* z1 = reinterpret_cast<double*>(base + goff);
     uint32_t* v1 = reinterpret_cast<uint32_t*>(base + goff + (size_t)W * (H + 1) * sizeof(double));
@@ -471,86 +739,26 @@ cudaError_t launch_edt(const uint64_t* d_bits, int W, int H, int TY, float* d_dt
     if (e != cudaSuccess) return e;
     double* z2 = reinterpret_cast<double*>(base + goff);
     uint32_t* v2 = reinterpret_cast<uint32_t*>(base + goff + (size_t)H * (W + 1) * sizeof(double));
-    k_edt_pass_x<<<blocks_for(H, 64), 64, 0, s>>>(g, W, H, d_dt, v2, z2);
+    k_edt_pass_x<<<blocks_for(H, 64), 64, 0, s>>>(g, W, H, o.dt, v2, z2);
+    e = cudaGetLastError();
+    if (e != cudaSuccess || !all) return e;
+    k_dt_layouts<<<blocks_for((long long)((W + 7) >> 3) * TY * 64, 256), 256, 0, s>>>(o.dt, W, H, TY, o);
     return cudaGetLastError();
 }
 
-cudaError_t launch_dt_to_tiled(const float* d_lin, int W, int H, float* d_tiled, cudaStream_t s) {
-    int TY = (H + 7) >> 3, TX = (W + 7) >> 3;
-    long long n = (long long)TX * TY * 64;
-    if (n == 0) return cudaSuccess;
-    k_dt_to_tiled<<<blocks_for(n, 256), 256, 0, s>>>(d_lin, W, H, TY, d_tiled);
-    return cudaGetLastError();
+size_t step_eq_words(int W, int H) {
+    return (size_t)W * ((H + 31) >> 5) + (size_t)((W + 31) >> 5) * H;
 }
 
-cudaError_t launch_dt_to_u16(const float* d_lin, int W, int H, uint16_t* d_u16, cudaStream_t s) {
-    int TY = (H + 7) >> 3, TX = (W + 7) >> 3;
-    long long n = (long long)TX * TY * 64;
-    if (n == 0) return cudaSuccess;
-    k_dt_to_u16<<<blocks_for(n, 256), 256, 0, s>>>(d_lin, W, H, TY, d_u16);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_dt_to_step(const float* d_lin, int W, int H, float* d_step, cudaStream_t s) {
-    const long long n = (long long)W * H;
-    if (n == 0) return cudaSuccess;
-    k_dt_to_step<<<blocks_for(n, 256), 256, 0, s>>>(d_lin, n, d_step);
-    return cudaGetLastError();
-}
-
-// Equal-step runs along y: one thread per column x walks it both ways; bits 0-7 of runs[x * H + y]
-// count the cells y + 1, y + 2, ... whose step equals the step of (x, y), bits 8-15 the cells
-// y - 1, y - 2, ... (at most 255 each); bits 16-31 are cleared for the x pass.
-__global__ void k_step_runs_y(const float* __restrict__ step, int W, int H, uint32_t* __restrict__ runs) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
-    if (x >= W) return;
-    const float* col = step + (size_t)x * H;
-    uint32_t* out = runs + (size_t)x * H;
-    unsigned run = 0;
-    for (int y = 1; y < H; ++y) {   // -y: run ending just below y
-        run = col[y - 1] == col[y] ? min(run + 1u, 255u) : 0u;
-        out[y] = run << 8;
-    }
-    out[0] = 0u;
-    run = 0;
-    for (int y = H - 2; y >= 0; --y) {   // +y
-        run = col[y + 1] == col[y] ? min(run + 1u, 255u) : 0u;
-        out[y] |= run;
-    }
-}
-
-// the same along x, one thread per row y: bits 16-23 (+x) and 24-31 (-x)
-__global__ void k_step_runs_x(const float* __restrict__ step, int W, int H, uint32_t* __restrict__ runs) {
-    const int y = blockIdx.x * blockDim.x + threadIdx.x;
-    if (y >= H) return;
-    unsigned run = 0;
-    for (int x = 1; x < W; ++x) {
-        const size_t i = (size_t)x * H + y;
-        run = step[i - H] == step[i] ? min(run + 1u, 255u) : 0u;
-        runs[i] |= run << 24;
-    }
-    run = 0;
-    for (int x = W - 2; x >= 0; --x) {
-        const size_t i = (size_t)x * H + y;
-        run = step[i + H] == step[i] ? min(run + 1u, 255u) : 0u;
-        runs[i] |= run << 16;
-    }
-}
-
-cudaError_t launch_step_runs(const float* d_step, int W, int H, uint32_t* d_runs, cudaStream_t s) {
+cudaError_t launch_step_runs(const float* d_step, int W, int H, uint32_t* d_eq, uint32_t* d_runs, cudaStream_t s) {
     if ((long long)W * H == 0) return cudaSuccess;
-    k_step_runs_y<<<blocks_for(W, 128), 128, 0, s>>>(d_step, W, H, d_runs);
+    const int HW = (H + 31) >> 5, XW = (W + 31) >> 5;
+    uint32_t* eqy = d_eq;
+    uint32_t* eqx = d_eq + (size_t)W * HW;
+    k_step_eq<<<blocks_for((long long)XW * HW, 8), 256, 0, s>>>(d_step, W, H, HW, eqx, eqy);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    k_step_runs_x<<<blocks_for(H, 128), 128, 0, s>>>(d_step, W, H, d_runs);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_dt_to_u8(const float* d_lin, int W, int H, uint8_t* d_u8, cudaStream_t s) {
-    int TY = (H + 7) >> 3, TX = (W + 7) >> 3;
-    long long n = (long long)TX * TY * 64;
-    if (n == 0) return cudaSuccess;
-    k_dt_to_u8<<<blocks_for(n, 256), 256, 0, s>>>(d_lin, W, H, TY, d_u8);
+    k_step_runs<<<blocks_for(H, 32) * blocks_for(W, 8), dim3(32, 8), 0, s>>>(eqx, eqy, W, H, HW, d_runs);
     return cudaGetLastError();
 }
 
@@ -683,9 +891,9 @@ extern "C" int rlc_distance_transform_noalloc(const uint8_t* d_occ, int width, i
     uint64_t* bits = static_cast<uint64_t*>(base);
     void* edt_scratch = static_cast<char*>(base) + kNoAllocBitsBytes;
     const int TY = (height + 7) >> 3;
-    cudaError_t e = launch_pack_bits(d_occ, width, height, bits, s);
+    cudaError_t e = launch_pack_bits(d_occ, width, height, false, bits, s);
     if (e == cudaSuccess)
-        e = launch_edt(bits, width, height, TY, d_dt, edt_scratch, kNoAllocScratchBytes - kNoAllocBitsBytes, s);
+        e = launch_edt(bits, width, height, TY, DtOut{d_dt}, edt_scratch, kNoAllocScratchBytes - kNoAllocBitsBytes, s);
     if (e != cudaSuccess) {
         snprintf(msg, sizeof(msg), "rlc_distance_transform_noalloc: %s", cudaGetErrorString(e));
         return set_last_error(RLC_ERR_CUDA, msg);

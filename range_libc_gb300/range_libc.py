@@ -243,11 +243,18 @@ class PyOMap:
         self._error = False
         self.fn = ""   # the PNG's path, as OMap::fn
         world = (1.0, 0.0, 0.0, 0.0, 0.0, 1.0)
+        grid = None
         if arg1 is not None and arg2 is not None and isinstance(arg1, (int, np.integer)):
             occ = np.zeros((int(arg1), int(arg2)), np.uint8)
         elif arg1 is not None and arg2 is not None:
             self.fn = str(arg1)
             occ = self._from_png(str(arg1), float(arg2))
+        elif isinstance(arg1, np.ndarray) and arg1.ndim == 2 and arg1.size:
+            # handed over as it lies in memory, rows or columns; grid[x][y] is made on the device, and
+            # read back if it is asked for
+            cells = arg1 if arg1.dtype.kind in "bui" and arg1.itemsize == 1 else arg1 != 0
+            by_rows = cells.flags.c_contiguous or abs(cells.strides[0]) >= abs(cells.strides[1])
+            grid = np.ascontiguousarray(cells if by_rows else cells.T)
         elif isinstance(arg1, np.ndarray):
             occ = np.ascontiguousarray((arg1 != 0).T, dtype=np.uint8)
         elif hasattr(arg1, "info") and hasattr(arg1, "data"):
@@ -258,14 +265,22 @@ class PyOMap:
         else:
             print("Failed to construct PyOMap, check argument types.")
             occ = np.zeros((1, 1), np.uint8)
-        if occ.size == 0:
-            occ = np.zeros((1, 1), np.uint8)
-            self._error = True
-        self._occ = np.ascontiguousarray(occ, dtype=np.uint8)
         self.world = tuple(float(np.float32(v)) for v in world)
         h = C.c_void_p()
-        W, H = self._occ.shape
-        call("rlc_map_create", self._occ.ctypes.data_as(_lib._u8p), W, H, C.byref(h))
+        if grid is not None:
+            self._occ = None
+            self._shape = (int(arg1.shape[1]), int(arg1.shape[0]))
+            if by_rows:
+                call("rlc_map_create_rows", grid.ctypes.data, *self._shape, C.byref(h))
+            else:
+                call("rlc_map_create", grid.ctypes.data_as(_lib._u8p), *self._shape, C.byref(h))
+        else:
+            if occ.size == 0:
+                occ = np.zeros((1, 1), np.uint8)
+                self._error = True
+            self._occ = np.ascontiguousarray(occ, dtype=np.uint8)
+            self._shape = self._occ.shape
+            call("rlc_map_create", self._occ.ctypes.data_as(_lib._u8p), *self._shape, C.byref(h))
         self._h = h
         call("rlc_map_set_world", self._h, *self.world)
 
@@ -302,28 +317,32 @@ class PyOMap:
     @property
     def occupancy(self) -> np.ndarray:
         """grid[x][y] as a uint8 array of shape (width, height)."""
+        if self._occ is None:
+            occ = np.empty(self._shape, np.uint8)
+            call("rlc_map_occupancy", self._h, occ.ctypes.data_as(_lib._u8p))
+            self._occ = occ
         return self._occ
 
     def save(self, fn) -> bool:
         """PNG with white = free, black = occupied (OMap::save, RangeLib.h:263-291); False on
         success, like the reference's encoder status."""
-        W, H = self._occ.shape
-        rc = lib().rlc_png_save_occupancy(fn.encode() if isinstance(fn, str) else bytes(fn), self._occ.ctypes.data, W, H)
+        occ = self.occupancy
+        rc = lib().rlc_png_save_occupancy(fn.encode() if isinstance(fn, str) else bytes(fn), occ.ctypes.data, *occ.shape)
         if rc != _lib.RLC_OK:
             print(f"encoder error {rc}: {lib().rlc_last_error().decode()}")
         return rc != _lib.RLC_OK
 
     def isOccupied(self, x: int, y: int) -> bool:
-        return bool(self._occ[x, y])
+        return bool(self.occupancy[x, y])
 
     def error(self) -> bool:
         return self._error
 
     def width(self) -> int:
-        return int(self._occ.shape[0])
+        return int(self._shape[0])
 
     def height(self) -> int:
-        return int(self._occ.shape[1])
+        return int(self._shape[1])
 
 
 # ---------------------------------------------------------------- methods
