@@ -170,6 +170,9 @@ struct rlc_method {
     int prefetch = 0;
     int fused_block = 256;
     int tile = 0;             // particles per tile of the fused kernels (0 = auto)
+    // no schedule asked for or autotuned yet: every call picks its kernels by size (results do not
+    // depend on the schedule; rlc_method_get_schedule reports the values above meanwhile)
+    bool pick = true;
     bool autotune_pending = false;
     // the last autotune: every candidate's schedule and median times (ms) of both stages
     struct TuneResult { int layout, block, prefetch, tile; float first_ms, final_ms; };
@@ -349,6 +352,26 @@ int finish_launch(cudaError_t e, const char* what) {
 
 // layout used by the per-ray kernels (the staged schedule only changes the fused update)
 int cast_layout(const rlc_method* m) { return m->layout == DT_STAGED ? DT_LINEAR : m->layout; }
+
+// layout of a cast of `rays` rays.  Without a schedule, ray marching takes the step map, with its
+// equal-step runs where the call waits for its longest rays: independent queries (their warps mix
+// long and short rays: 2 M queries on 2048^2 linear / step / runs 121 / 119 / 94 us, 10,000 21 / 19 /
+// 17 us, 1,000 on 512^2 33 / 33 / 15 us), and repeat-angle calls between 16 K and 1 M rays (4,000 x
+// 61 27 / 27 / 21 us; 1 x 1,081 9.7 / 9.3 / 10.0 us, 20,000 x 61 43 / 41 / 46 us, 20,000 x 1,081
+// 267 / 257 / 336 us).
+int cast_layout(const rlc_method* m, long long rays, bool independent) {
+    if (!m->pick || m->dkind != K_RM) return cast_layout(m);
+    return independent || (rays >= (1ll << 14) && rays < (1ll << 20)) ? DT_RUNS : DT_STEP;
+}
+
+// layout of a fused call.  Without a schedule, ray marching takes the step map, with its equal-step
+// runs while the call waits for its longest rays (below 2 M rays): 4,000 x 61 linear / step / runs
+// 43 / 43 / 34 us, 4,000 x 271 73 / 72 / 65 us; 4,000 x 1,081 160 / 157 / 166 us, 20,000 x 1,081
+// 438 / 423 / 496 us (2048^2 corridor map).
+int fused_layout(const rlc_method* m, long long rays) {
+    if (!m->pick || m->dkind != K_RM) return cast_layout(m);
+    return rays < (2ll << 20) ? DT_RUNS : DT_STEP;
+}
 
 int check_trig(const rlc_method* m, long long rays) {
     if (m->d_trig && m->trig_count < rays)
@@ -769,9 +792,9 @@ int rlc_calc_range_many(rlc_method* m, const float* ins, float* outs, int n, uns
     CastParams p = m->params();
     bool world = !(flags & RLC_NO_WORLD);
     if (flags & RLC_DEVICE_PTRS)
-        return finish_launch(launch_calc_range_many(p, cast_layout(m), m->prefetch, world, ins, outs, n, s), "calc_range_many");
+        return finish_launch(launch_calc_range_many(p, cast_layout(m, n, true), m->prefetch, world, ins, outs, n, s), "calc_range_many");
     if (host_direct()) {
-        CUDA_OR_FAIL(launch_calc_range_many(p, cast_layout(m), m->prefetch, world, ins, outs, n, s), "calc_range_many");
+        CUDA_OR_FAIL(launch_calc_range_many(p, cast_layout(m, n, true), m->prefetch, world, ins, outs, n, s), "calc_range_many");
         CUDA_OR_FAIL(cudaStreamSynchronize(s), "calc_range_many");
         return RLC_OK;
     }
@@ -781,7 +804,7 @@ int rlc_calc_range_many(rlc_method* m, const float* ins, float* outs, int n, uns
     float* d_in = (float*)st;
     float* d_out = (float*)((char*)st + bin);
     CUDA_OR_FAIL(cudaMemcpyAsync(d_in, ins, (size_t)n * 3 * sizeof(float), cudaMemcpyHostToDevice, s), "H2D");
-    CUDA_OR_FAIL(launch_calc_range_many(p, cast_layout(m), m->prefetch, world, d_in, d_out, n, s), "calc_range_many");
+    CUDA_OR_FAIL(launch_calc_range_many(p, cast_layout(m, n, true), m->prefetch, world, d_in, d_out, n, s), "calc_range_many");
     CUDA_OR_FAIL(cudaMemcpyAsync(outs, d_out, (size_t)n * sizeof(float), cudaMemcpyDeviceToHost, s), "D2H");
     CUDA_OR_FAIL(cudaStreamSynchronize(s), "calc_range_many");
     return RLC_OK;
@@ -798,9 +821,9 @@ int rlc_calc_range_repeat_angles(rlc_method* m, const float* ins, const float* a
     cudaStream_t s = (cudaStream_t)stream;
     CastParams p = m->params();
     if (flags & RLC_DEVICE_PTRS)
-        return finish_launch(launch_repeat_angles(p, cast_layout(m), m->prefetch, ins, angles, outs, n, na, s), "repeat_angles");
+        return finish_launch(launch_repeat_angles(p, cast_layout(m, (long long)n * na, false), m->prefetch, ins, angles, outs, n, na, s), "repeat_angles");
     if (host_direct()) {
-        CUDA_OR_FAIL(launch_repeat_angles(p, cast_layout(m), m->prefetch, ins, angles, outs, n, na, s), "repeat_angles");
+        CUDA_OR_FAIL(launch_repeat_angles(p, cast_layout(m, (long long)n * na, false), m->prefetch, ins, angles, outs, n, na, s), "repeat_angles");
         CUDA_OR_FAIL(cudaStreamSynchronize(s), "repeat_angles");
         return RLC_OK;
     }
@@ -813,7 +836,7 @@ int rlc_calc_range_repeat_angles(rlc_method* m, const float* ins, const float* a
     float* d_out = (float*)((char*)st + b0 + b1);
     CUDA_OR_FAIL(cudaMemcpyAsync(d_in, ins, (size_t)n * 3 * sizeof(float), cudaMemcpyHostToDevice, s), "H2D");
     CUDA_OR_FAIL(cudaMemcpyAsync(d_ang, angles, (size_t)na * sizeof(float), cudaMemcpyHostToDevice, s), "H2D");
-    CUDA_OR_FAIL(launch_repeat_angles(p, cast_layout(m), m->prefetch, d_in, d_ang, d_out, n, na, s), "repeat_angles");
+    CUDA_OR_FAIL(launch_repeat_angles(p, cast_layout(m, (long long)n * na, false), m->prefetch, d_in, d_ang, d_out, n, na, s), "repeat_angles");
     CUDA_OR_FAIL(cudaMemcpyAsync(outs, d_out, (size_t)n * na * sizeof(float), cudaMemcpyDeviceToHost, s), "D2H");
     CUDA_OR_FAIL(cudaStreamSynchronize(s), "repeat_angles");
     return RLC_OK;
@@ -931,8 +954,8 @@ static int fused_device(rlc_method* m, const float* ins, const float* angles, co
         return finish_launch(launch_fused_staged(p, sm, ins, angles, obs, w, n, na, m->tile, m->d_bins, s),
                              "fused sensor model (staged)");
     }
-    return finish_launch(launch_fused(p, cast_layout(m), m->prefetch, sm, ins, angles, obs, w, n, na, m->fused_block,
-                                      m->tile, s),
+    return finish_launch(launch_fused(p, fused_layout(m, (long long)n * na), m->prefetch, sm, ins, angles, obs, w, n, na,
+                                      m->fused_block, m->tile, m->pick, s),
                          "fused sensor model");
 }
 
@@ -1002,6 +1025,7 @@ int rlc_method_set_schedule(rlc_method* m, int dt_layout, int fused_block, int p
         m->layout = dt_layout;
         m->prefetch = prefetch;
         m->tile = tile;
+        m->pick = false;
     }
     if (fused_block) m->fused_block = fused_block;
     return RLC_OK;
@@ -1079,7 +1103,7 @@ int rlc_method_autotune_ex(rlc_method* m, const float* ins, const float* angles,
         m->layout = c.layout;
         CastParams p = m->params();
         if (c.layout == DT_STAGED) return launch_fused_staged(p, sm, ins, angles, obs, w, n, na, 0, m->d_bins, s);
-        return launch_fused(p, c.layout, c.prefetch, sm, ins, angles, obs, w, n, na, c.block, c.tile, s);
+        return launch_fused(p, c.layout, c.prefetch, sm, ins, angles, obs, w, n, na, c.block, c.tile, false, s);
     };
     unsigned flush_round = 0;
     auto time_once = [&](const Cand& c, float* ms) -> cudaError_t {
@@ -1129,6 +1153,7 @@ int rlc_method_autotune_ex(rlc_method* m, const float* ins, const float* angles,
     if (err != cudaSuccess) return cuda_fail(err, "autotune");
     if (best >= 0) {
         const Cand& b = cands[best];
+        m->pick = false;
         m->layout = b.layout;
         if (b.block) m->fused_block = b.block;
         m->prefetch = b.prefetch;

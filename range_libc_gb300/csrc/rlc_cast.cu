@@ -747,29 +747,10 @@ __global__ void __launch_bounds__(256) k_repeat_angles(CastParams p, const float
 // ------------------------------------------------------------ sensor model
 // The weight of a particle is the product of its beams' table values in beam
 // order (RangeLib.h:533-555, 558-612), in double, exactly as the reference
-// multiplies -- so weights are bit-identical.  A tile holds P particles
-// and the products run one particle per lane: each double multiply
-// instruction then serves up to 32 particles instead of one (the FP64 pipe
-// spends the same time on a warp instruction with one active lane as with
-// 32).  In eval_sensor_model's tiles the given ranges' 16-bit bins sit in
-// shared memory (sdi, particle-major) beside the beams' observation bins
-// (sri): (P * na + na) * 2 bytes per block; the fused update keeps each
-// ray's table factor instead (k_fused).
-struct TileSmem {
-    uint16_t* sdi;   // [P * na] range bins
-    uint16_t* sri;   // [na] observation bins
-};
-
-__host__ __device__ inline size_t tile_smem(int P, int na) {
-    return (((size_t)P * na + (size_t)na) * sizeof(uint16_t) + 15) & ~(size_t)15;
-}
-
-__device__ __forceinline__ TileSmem tile_layout(unsigned char* base, int P, int na) {
-    TileSmem t;
-    t.sdi = reinterpret_cast<uint16_t*>(base);
-    t.sri = t.sdi + (size_t)P * na;
-    return t;
-}
+// multiplies -- so weights are bit-identical.  The products run one particle
+// per lane: each double multiply instruction then serves up to 32 particles
+// instead of one (the FP64 pipe spends the same ~19 cycles on a warp
+// instruction with one active lane as with 32).
 
 // In-order product of the table factors table[sri(a) * K + bin(a)], a = 0 ..
 // na - 1, as a three-stage software pipeline over groups of kGroup beams: in
@@ -780,7 +761,7 @@ __device__ __forceinline__ TileSmem tile_layout(unsigned char* base, int P, int 
 // group_bins(g, b) delivers the kGroup bins of group g (entries past na are
 // not used).  Registers: 2 x kGroup doubles and 2 x kGroup bins.
 template <int kGroup, class SriF, class GroupF>
-__device__ __forceinline__ double product_chain(const SensorDev& sm, int na, SriF sri, GroupF group_bins) {
+__device__ __forceinline__ double product_chain(const SensorDev& sm, int na, SriF sri, GroupF group_bins, double w = 1.0) {
     unsigned bx[kGroup], by[kGroup];
     double f0[kGroup], f1[kGroup];
     const int ng = (na + kGroup - 1) / kGroup;
@@ -799,7 +780,6 @@ __device__ __forceinline__ double product_chain(const SensorDev& sm, int na, Sri
         for (int u = 0; u < kGroup; ++u) w = __dmul_rn(w, f[u]);
         return w;
     };
-    double w = 1.0;
     load_bins(bx, 0);
     load_factors(f0, bx, 0);
     load_bins(bx, 1);
@@ -815,41 +795,71 @@ __device__ __forceinline__ double product_chain(const SensorDev& sm, int na, Sri
     return w;
 }
 
-// one lane per particle; a short unrolled gather keeps the fused kernels' registers low
-__device__ __forceinline__ void tile_products(const SensorDev& sm, const TileSmem& ts, int na, int P, int first,
-                                              int n, double* __restrict__ weights) {
-    for (int li = threadIdx.x; li < P; li += blockDim.x) {
-        const int i = first + li;
-        if (i >= n) continue;
-        const uint16_t* row = ts.sdi + (size_t)li * na;
-        double w = 1.0;
-#pragma unroll 8
-        for (int a = 0; a < na; ++a) w = __dmul_rn(w, __ldg(sm.table + (size_t)ts.sri[a] * sm.K + row[a]));
-        weights[i] = w;
-    }
-}
+// RangeLib.h:533-555 on given ranges (world units), 32 particles per block.  Warps 1-7 prepare the
+// table factors of kEvalBeams beams at a time -- lane = beam, a few particles' rows per warp, so that
+// the ranges are read coalesced whatever the row length -- into shared memory, while warp 0
+// multiplies the beams before them, lane = particle.  The ranges of the chunk after are requested
+// before the factors of this one, so that a chunk waits for one read and not for two.  Bound by the
+// chain of in-order double multiplies (86 cycles each: 4.9 us for 108 beams) and, for many
+// particles, by the FP64 pipe.  Tiles of 256 / na particles per block (before) ran the same chain
+// with 2 lanes per multiply, or one from 256 beams on, after all bins were made.
+// 4,000 x 108, kernel (ncu): 25.1 -> 8.9 us; 20,000 x 1,081 63 us a call.
+constexpr int kEvalBeams = 32;
+constexpr int kEvalWarps = 8;
+constexpr int kEvalRows = (32 + kEvalWarps - 2) / (kEvalWarps - 1);   // particles per preparing warp
 
-__device__ __forceinline__ void tile_obs_bins(const CastParams& p, const SensorDev& sm, const float* __restrict__ obs,
-                                              int na, uint16_t* sri) {
-    for (int a = threadIdx.x; a < na; a += blockDim.x)
-        sri[a] = (uint16_t)sensor_bin(__fmul_rn(__ldg(obs + a), p.world.inv_s), sm.K, p.err);
-}
-
-// RangeLib.h:533-555 on given ranges (world units)
-__global__ void __launch_bounds__(512) k_eval_sensor(CastParams p, SensorDev sm, const float* __restrict__ obs,
-                                                     const float* __restrict__ ranges, double* __restrict__ outs,
-                                                     int na, int n, int P) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const TileSmem ts = tile_layout(smem_raw, P, na);
-    const int first = blockIdx.x * P;
-    tile_obs_bins(p, sm, obs, na, ts.sri);
-    const int nr = P * na;
-    for (int r = threadIdx.x; r < nr; r += blockDim.x) {
-        int li = r / na, a = r - li * na, i = first + li;
-        if (i < n) ts.sdi[r] = (uint16_t)sensor_bin(__fmul_rn(__ldg(ranges + (size_t)i * na + a), p.world.inv_s), sm.K, p.err);
+__global__ void __launch_bounds__(32 * kEvalWarps) k_eval_sensor(CastParams p, SensorDev sm,
+                                                                 const float* __restrict__ obs,
+                                                                 const float* __restrict__ ranges,
+                                                                 double* __restrict__ outs, int na, int n) {
+    __shared__ double s_f[2][kEvalBeams][33];   // [beam][particle]; a row is 33 doubles: no bank conflicts either way
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int first = blockIdx.x * 32, np = min(32, n - first);
+    const float* rows = ranges + (size_t)first * na;
+    const int chunks = (na + kEvalBeams - 1) / kEvalBeams;
+    if (warp > 0) {
+        const int i0 = (warp - 1) * kEvalRows;
+        float r[kEvalRows], o = 0.0f;
+        const auto request = [&](int k) {   // chunk k's ranges and observation, lane = beam
+            const int a = k * kEvalBeams + lane;
+            if (a < na) {
+                o = __ldg(obs + a);
+#pragma unroll
+                for (int u = 0; u < kEvalRows; ++u) r[u] = i0 + u < np ? __ldg(rows + (size_t)(i0 + u) * na + a) : 0.0f;
+            }
+        };
+        const auto factors = [&](int k) {
+            if (k * kEvalBeams + lane < na) {
+                const double* row = sm.table + (size_t)sensor_bin(__fmul_rn(o, p.world.inv_s), sm.K, p.err) * sm.K;
+                int bin[kEvalRows];
+#pragma unroll
+                for (int u = 0; u < kEvalRows; ++u) bin[u] = sensor_bin(__fmul_rn(r[u], p.world.inv_s), sm.K, p.err);
+                if (k + 1 < chunks) request(k + 1);
+#pragma unroll
+                for (int u = 0; u < kEvalRows; ++u)
+                    if (i0 + u < np) s_f[k & 1][lane][i0 + u] = __ldg(row + bin[u]);
+            }
+        };
+        if (chunks > 0) {
+            request(0);
+            factors(0);
+        }
+        __syncthreads();
+        for (int k = 0; k < chunks; ++k) {
+            if (k + 1 < chunks) factors(k + 1);
+            __syncthreads();
+        }
+        return;
     }
     __syncthreads();
-    tile_products(sm, ts, na, P, first, n, outs);
+    double w = 1.0;
+    for (int k = 0; k < chunks; ++k) {
+        const int nb = min(kEvalBeams, na - k * kEvalBeams);
+#pragma unroll 8
+        for (int a = 0; a < nb; ++a) w = __dmul_rn(w, s_f[k & 1][a][lane]);
+        __syncthreads();
+    }
+    if (lane < np) outs[first + lane] = w;
 }
 
 // range of ray (particle i, beam a) in pixels (RangeLib.h:558-612)
@@ -918,6 +928,142 @@ __global__ void __launch_bounds__(512, KIND == K_CDDT ? 1 : 4) k_fused(CastParam
     }
 }
 
+// cos/sin of a ray of heading fl(th - ang): the caller's override, else from the float pairs of the
+// particle heading's and the beam angle's sin and cos (rlc_trig::sincos_diff: the correctly rounded
+// values of the ray's heading, for about a third of the instructions of computing them from the
+// heading), else -- where no pairs exist or their rounding is not certain -- from the heading.
+__device__ __forceinline__ void ray_direction(const float* trig, long long ray, float th, float ang, float4 pt,
+                                              float4 bt, float& c, float& s) {
+    if (trig) {
+        c = trig[2 * ray];
+        s = trig[2 * ray + 1];
+    } else if (isnan(pt.x) || isnan(bt.x) ||
+               !rlc_trig::sincos_diff(th, ang, rlc_trig::F2{pt.x, pt.y}, rlc_trig::F2{pt.z, pt.w},
+                                      rlc_trig::F2{bt.x, bt.y}, rlc_trig::F2{bt.z, bt.w}, &s, &c)) {
+        rlc_trig::sincos_cr(__fsub_rn(th, ang), &s, &c);
+    }
+}
+
+// {sin hi, sin lo, cos hi, cos lo} of x; a NaN sin hi where x has no pairs
+__device__ __forceinline__ float4 trig_record(float x) {
+    rlc_trig::F2 sn, cs;
+    return rlc_trig::sincos_pairs(x, &sn, &cs) ? make_float4(sn.h, sn.l, cs.h, cs.l)
+                                               : make_float4(__int_as_float(0x7fc00000), 0.0f, 0.0f, 0.0f);
+}
+
+// the four range bins of beams 4g .. 4g + 3 of tile particle li: one 8-byte read (bins in groups of
+// four beams, particles innermost but for the four)
+__device__ __forceinline__ void tile_bins4(const uint16_t* tile, int P, int li, int g, unsigned* b) {
+    const uint2 v = *reinterpret_cast<const uint2*>(tile + ((size_t)g * P + li) * 4);
+    b[0] = v.x & 0xFFFFu;
+    b[1] = v.x >> 16;
+    b[2] = v.y & 0xFFFFu;
+    b[3] = v.y >> 16;
+}
+
+// Fused update of many rays: a block takes P particles through all beams, C beams at a time.  While
+// the block's warps cast the rays of chunk k (32 at a time from a shared counter), warp 0 first
+// multiplies chunk k - 1, one particle per lane, from the 16-bit bins in shared memory; it joins the
+// cast when it is done.  P (up to 32) is chosen so that all blocks are resident at once (or in few
+// equal waves): no tail, and as many lanes share each FP64 multiply as the particle count allows.
+// Poses and, for the kinds that need a ray's cos/sin, the trig records of the particles are made
+// once per block, those of the beams once per chunk.  Before, blocks held 256 / na particles: from
+// 256 beams on a single lane multiplied, and since a double multiply costs the FP64 pipe ~19 cycles
+// whatever its active lanes, 20,000 x 1,081 rays took the pipe's 1.36 ms (82 % busy, 25 % of the
+// issue slots used).  Now 384 us.
+constexpr int kWideThreads = 256;
+constexpr int kWideParticles = 32;
+
+struct WideSmem {   // byte offsets of the dynamic shared memory
+    int part, beam, ang, row, bins, total;
+};
+__host__ __device__ inline WideSmem wide_smem(int P, int C) {
+    WideSmem w;
+    w.part = 0;                        // [P] pose, trig record
+    w.beam = w.part + P * 32;          // [2][C] trig record
+    w.ang = w.beam + 2 * C * 16;       // [2][C] beam angle
+    w.bins = w.ang + 2 * C * 4;        // [2][C / 4][P][4] range bins
+    w.row = w.bins + 2 * C * P * 2;    // [3][C] observation bin
+    w.total = w.row + 3 * C * 2;
+    return w;
+}
+
+template <int KIND, int LAYOUT, int PF>
+__global__ void __launch_bounds__(kWideThreads, KIND == K_CDDT ? 4 : 8)
+k_fused_wide(CastParams p, SensorDev sm, const float* __restrict__ ins, const float* __restrict__ angles,
+             const float* __restrict__ obs, double* __restrict__ weights, int n, int na, int P, int C) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ unsigned s_next[2];
+    constexpr bool kTrig = KIND == K_RM || KIND == K_BL;
+    const WideSmem off = wide_smem(P, C);
+    float4* part = reinterpret_cast<float4*>(smem_raw + off.part);
+    float4* beam = reinterpret_cast<float4*>(smem_raw + off.beam);
+    float* ang = reinterpret_cast<float*>(smem_raw + off.ang);
+    uint16_t* bins = reinterpret_cast<uint16_t*>(smem_raw + off.bins);
+    uint16_t* row = reinterpret_cast<uint16_t*>(smem_raw + off.row);
+    const int lane = threadIdx.x & 31, first = blockIdx.x * P, np = min(P, n - first);
+    const int chunks = (na + C - 1) / C;
+    if ((int)threadIdx.x < np) {
+        const float* q = ins + 3 * (size_t)(first + threadIdx.x);
+        float ax, ay, th;
+        world_to_grid(p.world, __ldg(q), __ldg(q + 1), __ldg(q + 2), ax, ay, th);
+        part[2 * threadIdx.x] = make_float4(ax, ay, th, 0.0f);
+        if (kTrig && !p.trig) part[2 * threadIdx.x + 1] = trig_record(th);
+    }
+    const auto beams = [&](int k, int t) {   // records of chunk k's beams, thread t of 64 or more
+        for (int j = t; j < min(C, na - k * C); j += 64) {
+            const float an = __ldg(angles + k * C + j);
+            ang[(k & 1) * C + j] = an;
+            if (kTrig && !p.trig) beam[(k & 1) * C + j] = trig_record(an);
+            row[(k % 3) * C + j] = (uint16_t)sensor_bin(__fmul_rn(__ldg(obs + k * C + j), p.world.inv_s), sm.K, p.err);
+        }
+    };
+    if (threadIdx.x >= kWideThreads - 64) beams(0, threadIdx.x - (kWideThreads - 64));
+    if (threadIdx.x == 0) s_next[0] = 0u;
+    __syncthreads();
+    double w = 1.0;
+    for (int k = 0; k <= chunks; ++k) {
+        if (threadIdx.x < 32 && k > 0 && lane < np) {
+            const uint16_t* tile = bins + ((k - 1) & 1) * C * P;
+            const uint16_t* rw = row + ((k - 1) % 3) * C;
+            w = product_chain<4>(sm, min(C, na - (k - 1) * C), [&](int a) { return (unsigned)rw[a]; },
+                                 [&](int g, unsigned* b) { tile_bins4(tile, P, lane, g, b); }, w);
+        }
+        if (k == chunks) break;
+        if (k + 1 < chunks && threadIdx.x >= kWideThreads - 64) beams(k + 1, threadIdx.x - (kWideThreads - 64));
+        if (threadIdx.x == 0) s_next[(k + 1) & 1] = 0u;
+        const int nb = min(C, na - k * C), nr = np * nb;
+        const float inv_nb = __frcp_rn(__int2float_rn(nb));
+        uint16_t* tile = bins + (k & 1) * C * P;
+        for (;;) {
+            unsigned base = 0u;
+            if (lane == 0) base = atomicAdd(&s_next[k & 1], 32u);
+            base = __shfl_sync(0xffffffffu, base, 0);
+            if (base >= (unsigned)nr) break;
+            const int r = (int)base + lane;
+            if (r >= nr) continue;
+            const int li = div_small(r, nb, inv_nb), a = r - li * nb;
+            const float4 pose = part[2 * li];
+            const float an = ang[(k & 1) * C + a];
+            float d;
+            if (KIND == K_CDDT) {
+                d = cddt_cast<PF == 2>(p, pose.x, pose.y, __fsub_rn(pose.z, an));
+            } else if (KIND == K_GLT) {
+                d = glt_cast(p, pose.x, pose.y, __fsub_rn(pose.z, an));
+            } else {
+                float c, s;
+                ray_direction(p.trig, (long long)(first + li) * na + k * C + a, pose.z, an, part[2 * li + 1],
+                              beam[(k & 1) * C + a], c, s);
+                d = KIND == K_RM ? rm_cast<LAYOUT, PF>(p.map, p.mr, pose.x, pose.y, c, s)
+                                 : bl_cast(p.map, p.mr, pose.x, pose.y, c, s, p.err);
+            }
+            tile[((size_t)(a >> 2) * P + li) * 4 + (a & 3)] = (uint16_t)sensor_bin(d, sm.K, p.err);
+        }
+        __syncthreads();   // the chunk's bins and the next chunk's records are written
+    }
+    if (threadIdx.x < 32 && lane < np) weights[first + lane] = w;
+}
+
 // ------------------------------------------------- persistent multi-filter
 // Every block loops: take the next tile index from the device queue and
 // cast the tile's rays (P particles of one filter) into the filter's range
@@ -930,15 +1076,6 @@ __global__ void __launch_bounds__(512, KIND == K_CDDT ? 1 : 4) k_fused(CastParam
 // descending per-tile cost, so heavy tiles are handed out first.  There is
 // no waiting on other blocks: a block that finds the queue exhausted
 // multiplies its last tile and exits.
-// the four range bins of beams 4g .. 4g + 3 of tile particle li: one 8-byte read (batch bin layout)
-__device__ __forceinline__ void tile_bins4(const uint16_t* tile, int P, int li, int g, unsigned* b) {
-    const uint2 v = *reinterpret_cast<const uint2*>(tile + ((size_t)g * P + li) * 4);
-    b[0] = v.x & 0xFFFFu;
-    b[1] = v.x >> 16;
-    b[2] = v.y & 0xFFFFu;
-    b[3] = v.y >> 16;
-}
-
 __device__ __forceinline__ void batch_products(const FilterDev& F, int tile, int np) {
     const int lane = threadIdx.x & 31;
     const uint16_t* obs_bins = F.obs_bins;
@@ -960,27 +1097,12 @@ __device__ __forceinline__ void batch_store(const FilterDev& F, int first, uint1
 }
 
 // Ray (particle i, beam a) of a ray-marching filter at the start of its march (RangeLib.h:558-612,
-// 927-931); r is the tile's index of the ray.  The particle's grid-frame pose comes from its
-// record; the ray's cos/sin from the caller's override, else from the float pairs of the particle
-// heading's and the beam angle's sin and cos (rlc_trig::sincos_diff: the correctly rounded values
-// of the ray's heading fl(th - a), for about a third of the instructions of computing them from
-// the heading), else -- where no pairs exist or their rounding is not certain -- from the heading.
+// 927-931); r is the tile's index of the ray.  The particle's grid-frame pose and the trig pairs
+// come from the filter's records.
 __device__ __forceinline__ RmRay rm_ray_start(const FilterDev& F, int i, int a, int r) {
-    const float4 pose = __ldg(F.part_rec + 2 * (size_t)i);
-    const float ang = __ldg(F.angles + a);
-    const float h = __fsub_rn(pose.z, ang);
+    const float4 pose = __ldg(F.part_rec + 2 * (size_t)i), pt = __ldg(F.part_rec + 2 * (size_t)i + 1);
     float c, s;
-    if (F.p.trig) {
-        const long long ray = (long long)i * F.na + a;
-        c = F.p.trig[2 * ray];
-        s = F.p.trig[2 * ray + 1];
-    } else {
-        const float4 pt = __ldg(F.part_rec + 2 * (size_t)i + 1), bt = __ldg(F.beam_rec + a);
-        if (isnan(pt.x) || isnan(bt.x) ||
-            !rlc_trig::sincos_diff(pose.z, ang, rlc_trig::F2{pt.x, pt.y}, rlc_trig::F2{pt.z, pt.w},
-                                   rlc_trig::F2{bt.x, bt.y}, rlc_trig::F2{bt.z, bt.w}, &s, &c))
-            rlc_trig::sincos_cr(h, &s, &c);
-    }
+    ray_direction(F.p.trig, (long long)i * F.na + a, pose.z, __ldg(F.angles + a), pt, __ldg(F.beam_rec + a), c, s);
     return RmRay{pose.x, pose.y, c, s, 0.0f, -1.0f, 0, r};
 }
 
@@ -1114,7 +1236,7 @@ __global__ void __launch_bounds__(512, 4) k_batch(const FilterDev* __restrict__ 
 // Products of every particle of the batch in one launch after the cast (the
 // alternative to k_batch's overlapped products): one thread per particle,
 // 32 particles per warp, the bins read back from global memory.
-__global__ void __launch_bounds__(256) k_batch_products(const FilterDev* __restrict__ filters, int nf,
+__global__ void __launch_bounds__(64) k_batch_products(const FilterDev* __restrict__ filters, int nf,
                                                         unsigned total_particles) {
     const unsigned g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= total_particles) return;
@@ -1146,11 +1268,7 @@ __global__ void k_batch_obs_bins(const FilterDev* __restrict__ filters, bool rec
     const FilterDev& F = filters[blockIdx.x];
     for (int a = threadIdx.x; a < F.na; a += blockDim.x) {
         F.obs_bins[a] = (uint16_t)sensor_bin(__fmul_rn(__ldg(F.obs + a), F.p.world.inv_s), F.sm.K, F.p.err);
-        if (records) {
-            rlc_trig::F2 sn, cs;
-            F.beam_rec[a] = rlc_trig::sincos_pairs(__ldg(F.angles + a), &sn, &cs) ? make_float4(sn.h, sn.l, cs.h, cs.l)
-                                                                                    : make_float4(__int_as_float(0x7fc00000), 0.0f, 0.0f, 0.0f);
-        }
+        if (records) F.beam_rec[a] = trig_record(__ldg(F.angles + a));
     }
 }
 
@@ -1171,10 +1289,7 @@ __global__ void __launch_bounds__(256) k_batch_particles(const FilterDev* __rest
     float ax, ay, th;
     world_to_grid(F.p.world, __ldg(F.ins + 3 * i), __ldg(F.ins + 3 * i + 1), __ldg(F.ins + 3 * i + 2), ax, ay, th);
     F.part_rec[2 * i] = make_float4(ax, ay, th, 0.0f);
-    rlc_trig::F2 sn, cs;
-    F.part_rec[2 * i + 1] = !F.p.trig && rlc_trig::sincos_pairs(th, &sn, &cs)
-                                ? make_float4(sn.h, sn.l, cs.h, cs.l)
-                                : make_float4(__int_as_float(0x7fc00000), 0.0f, 0.0f, 0.0f);
+    F.part_rec[2 * i + 1] = F.p.trig ? make_float4(__int_as_float(0x7fc00000), 0.0f, 0.0f, 0.0f) : trig_record(th);
 }
 
 
@@ -1416,14 +1531,13 @@ struct RunAngles {
 
 // particles per tile (P) and threads per block: P = tile if given, else the
 // most particles whose rays fit one ray per thread; P is capped so that the
-// tile's per-ray entries (ray_bytes each: a 16-bit bin, or the fused update's
-// 8-byte factor) and the beams' 16-bit observation bins fit kTileSmem bytes
+// tile's 8-byte factors (and two more bytes per beam) fit kTileSmem bytes
 constexpr size_t kTileSmem = 48 * 1024;
-inline void product_shape(int na, int block, int tile, int& P, int& threads, size_t ray_bytes = sizeof(uint16_t)) {
+inline void product_shape(int na, int block, int tile, int& P, int& threads) {
     if (block <= 0) block = 256;
     if (na <= 0) { P = block; threads = block; return; }   // empty product: weight 1.0
     P = tile > 0 ? tile : (na >= block ? 1 : block / na);
-    int cap = (int)((kTileSmem - (size_t)na * sizeof(uint16_t)) / ((size_t)na * ray_bytes));
+    int cap = (int)((kTileSmem - (size_t)na * sizeof(uint16_t)) / ((size_t)na * sizeof(double)));
     if (cap < 1) cap = 1;
     if (P > cap) P = cap;
     int nr = P * na;
@@ -1437,13 +1551,46 @@ cudaError_t set_smem(K kernel, size_t bytes) {
     return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
+// Which fused calls go wide, where the caller has not asked for a schedule: from 1 M rays on, if a
+// block of k_fused would hold a single particle (one lane per multiply), and then with at least two
+// particles per lane set.  Ray marching on a 2048^2 corridor map, us per call before / wide:
+// 20,000 x 1,081 1365 / 401, 4,000 x 1,081 329 / 155, 4,000 x 271 88 / 65; below the line
+// 20,000 x 61 62 / 68, 2,000 x 108 26 / 32, 1,000 x 1,081 101 / 108.  CDDT: 8,000 x 1,081 634 / 187,
+// 4,000 x 271 97 / 46.  Bresenham's walks are too uneven for a barrier per chunk (8,000 x 1,081
+// 722 / 869).
+constexpr long long kWideRays = 1 << 20;
+constexpr int kWideMinBeams = 192, kWideMinParticles = 2000;
+constexpr int kWideChunk = 2048;   // rays of a chunk: 17 x 64 / 128 / 256 beams 425 / 401 / 475 us
+
+inline bool fused_wide(int kind, int n, int na) {
+    return kind != K_BL && (long long)n * na >= kWideRays && na >= kWideMinBeams && n >= kWideMinParticles;
+}
+
 template <int KIND, int LAYOUT, int PF>
 struct RunFused {
     static cudaError_t run(const CastParams& p, const SensorDev& sm, const float* ins, const float* angles,
-                           const float* obs, double* w, int n, int na, int block, int tile, cudaStream_t s) {
+                           const float* obs, double* w, int n, int na, int block, int tile, bool pick, cudaStream_t s) {
         if (n <= 0) return cudaSuccess;
+        // the kernels that a call without a schedule can come to (pick_layout)
+        constexpr bool kPicked = KIND == K_GLT || (KIND == K_CDDT && PF == 0) ||
+                                 (KIND == K_RM && PF == 0 && (LAYOUT == DT_STEP || LAYOUT == DT_RUNS));
+        if constexpr (kPicked) {
+            if (pick && fused_wide(KIND, n, na)) {
+                int dev = 0, sms = 0;
+                cudaError_t e = cudaGetDevice(&dev);
+                if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+                if (e != cudaSuccess) return e;
+                const long long resident = (long long)sms * (KIND == K_CDDT ? 4 : 8);
+                const long long waves = (n + resident * kWideParticles - 1) / (resident * kWideParticles);
+                const int P = (int)((n + resident * waves - 1) / (resident * waves));
+                const int C = min(max(32, min(512, (kWideChunk / P + 31) / 32 * 32)), (na + 3) / 4 * 4);
+                k_fused_wide<KIND, LAYOUT, PF><<<blocks_for(n, P), kWideThreads, wide_smem(P, C).total, s>>>(
+                    p, sm, ins, angles, obs, w, n, na, P, C);
+                return cudaGetLastError();
+            }
+        }
         int P, threads;
-        product_shape(na, block, tile, P, threads, sizeof(double));
+        product_shape(na, block, tile, P, threads);
         const size_t smem = (size_t)P * na * sizeof(double);
         cudaError_t e = set_smem(k_fused<KIND, LAYOUT, PF>, smem);
         if (e != cudaSuccess) return e;
@@ -1467,24 +1614,19 @@ cudaError_t launch_repeat_angles(const CastParams& p, int layout, int pf, const 
 cudaError_t launch_eval_sensor(const CastParams& p, const SensorDev& sm, const float* obs, const float* ranges,
                                double* outs, int na, int n, cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
-    int P, threads;
-    product_shape(na, 256, 0, P, threads);
-    size_t smem = tile_smem(P, na);
-    cudaError_t e = set_smem(k_eval_sensor, smem);
-    if (e != cudaSuccess) return e;
-    k_eval_sensor<<<blocks_for(n, P), threads, smem, s>>>(p, sm, obs, ranges, outs, na, n, P);
+    k_eval_sensor<<<blocks_for(n, 32), 32 * kEvalWarps, 0, s>>>(p, sm, obs, ranges, outs, na, n);
     return cudaGetLastError();
 }
 
 cudaError_t launch_fused(const CastParams& p, int layout, int pf, const SensorDev& sm, const float* ins,
                          const float* angles, const float* obs, double* weights, int n, int na, int block, int tile,
-                         cudaStream_t s) {
-    return dispatch<RunFused>(p.kind, layout, pf, p, sm, ins, angles, obs, weights, n, na, block, tile, s);
+                         bool pick, cudaStream_t s) {
+    return dispatch<RunFused>(p.kind, layout, pf, p, sm, ins, angles, obs, weights, n, na, block, tile, pick, s);
 }
 
 int tile_particles(int na, int block, int tile) {
     int P, threads;
-    product_shape(na, block, tile, P, threads, sizeof(double));
+    product_shape(na, block, tile, P, threads);
     return P;
 }
 
@@ -1541,7 +1683,7 @@ cudaError_t launch_fused_staged(const CastParams& p, const SensorDev& sm, const 
                                 const float* obs, double* weights, int n, int na, int chunks,
                                 uint16_t* bins, cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
-    if (na <= 0) return launch_fused(p, DT_LINEAR, 0, sm, ins, angles, obs, weights, n, na, 0, 0, s);
+    if (na <= 0) return launch_fused(p, DT_LINEAR, 0, sm, ins, angles, obs, weights, n, na, 0, 0, false, s);
     if (chunks <= 0) {   // one block per SM: beams x chunks ~ SM count
         int dev = 0, sms = 152;
         cudaGetDevice(&dev);
@@ -1616,7 +1758,7 @@ cudaError_t launch_batch(const FilterDev* d_filters, int nf, unsigned total_tile
     k<<<grid, block, smem, s>>>(d_filters, nf, total_tiles, queue);
     e = cudaGetLastError();
     if (e != cudaSuccess || !separate || total_particles == 0) return e;
-    k_batch_products<<<blocks_for(total_particles, 256), 256, 0, s>>>(d_filters, nf, total_particles);
+    k_batch_products<<<blocks_for(total_particles, 64), 64, 0, s>>>(d_filters, nf, total_particles);
     return cudaGetLastError();
 }
 

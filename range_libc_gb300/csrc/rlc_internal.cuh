@@ -124,10 +124,11 @@ cudaError_t launch_repeat_angles(const CastParams& p, int layout, int pf, const 
                                  float* outs, int n, int na, cudaStream_t s);
 cudaError_t launch_eval_sensor(const CastParams& p, const SensorDev& sm, const float* obs,
                                const float* ranges, double* outs, int na, int n, cudaStream_t s);
-// block: threads per block (0 = 256); tile: particles per tile (0 = auto)
+// block: threads per block (0 = 256); tile: particles per tile (0 = auto); pick: the caller has
+// asked for neither, the launch chooses its kernel by size
 cudaError_t launch_fused(const CastParams& p, int layout, int pf, const SensorDev& sm, const float* ins,
                          const float* angles, const float* obs, double* weights, int n, int na,
-                         int block, int tile, cudaStream_t s);
+                         int block, int tile, bool pick, cudaStream_t s);
 // particles per tile the fused kernel uses
 int tile_particles(int na, int block, int tile);
 
