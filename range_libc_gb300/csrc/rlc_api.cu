@@ -356,21 +356,21 @@ int cast_layout(const rlc_method* m) { return m->layout == DT_STAGED ? DT_LINEAR
 // layout of a cast of `rays` rays.  Without a schedule, ray marching takes the step map, with its
 // equal-step runs where the call waits for its longest rays: independent queries (their warps mix
 // long and short rays: 2 M queries on 2048^2 linear / step / runs 121 / 119 / 94 us, 10,000 21 / 19 /
-// 17 us, 1,000 on 512^2 33 / 33 / 15 us), and repeat-angle calls between 16 K and 1 M rays (4,000 x
-// 61 27 / 27 / 21 us; 1 x 1,081 9.7 / 9.3 / 10.0 us, 20,000 x 61 43 / 41 / 46 us, 20,000 x 1,081
-// 267 / 257 / 336 us).
+// 17 us, 1,000 on 512^2 33 / 33 / 15 us), and repeat-angle calls between 16 K and 256 K rays (4,000 x
+// 61 27 / 27 / 21 us; 1 x 1,081 9.7 / 9.3 / 10.0 us, 1,588 x 199 29 / 29 / 31 us, 20,000 x 61
+// 43 / 41 / 46 us, 20,000 x 1,081 267 / 257 / 336 us).
 int cast_layout(const rlc_method* m, long long rays, bool independent) {
     if (!m->pick || m->dkind != K_RM) return cast_layout(m);
-    return independent || (rays >= (1ll << 14) && rays < (1ll << 20)) ? DT_RUNS : DT_STEP;
+    return independent || (rays >= (1ll << 14) && rays < (1ll << 18)) ? DT_RUNS : DT_STEP;
 }
 
 // layout of a fused call.  Without a schedule, ray marching takes the step map, with its equal-step
-// runs while the call waits for its longest rays (below 2 M rays): 4,000 x 61 linear / step / runs
-// 43 / 43 / 34 us, 4,000 x 271 73 / 72 / 65 us; 4,000 x 1,081 160 / 157 / 166 us, 20,000 x 1,081
-// 438 / 423 / 496 us (2048^2 corridor map).
-int fused_layout(const rlc_method* m, long long rays) {
+// runs while the call waits for its longest rays and not for its products: 4,000 x 61 linear / step /
+// runs 43 / 43 / 34 us, 500 x 300 50 / 50 / 38, 4,000 x 271 - / 69 / 60; 637 x 849 72 / 72 / 78,
+// 4,000 x 1,081 - / 140 / 157, 20,000 x 1,081 438 / 423 / 496 us.
+int fused_layout(const rlc_method* m, int n, int na) {
     if (!m->pick || m->dkind != K_RM) return cast_layout(m);
-    return rays < (2ll << 20) ? DT_RUNS : DT_STEP;
+    return (long long)n * na < (2ll << 20) && (na < 512 || n >= 2000) ? DT_RUNS : DT_STEP;
 }
 
 int check_trig(const rlc_method* m, long long rays) {
@@ -954,7 +954,7 @@ static int fused_device(rlc_method* m, const float* ins, const float* angles, co
         return finish_launch(launch_fused_staged(p, sm, ins, angles, obs, w, n, na, m->tile, m->d_bins, s),
                              "fused sensor model (staged)");
     }
-    return finish_launch(launch_fused(p, fused_layout(m, (long long)n * na), m->prefetch, sm, ins, angles, obs, w, n, na,
+    return finish_launch(launch_fused(p, fused_layout(m, n, na), m->prefetch, sm, ins, angles, obs, w, n, na,
                                       m->fused_block, m->tile, m->pick, s),
                          "fused sensor model");
 }

@@ -963,8 +963,8 @@ __device__ __forceinline__ void tile_bins4(const uint16_t* tile, int P, int li, 
 
 // Fused update of many rays: a block takes P particles through all beams, C beams at a time.  While
 // the block's warps cast the rays of chunk k (32 at a time from a shared counter), warp 0 first
-// multiplies chunk k - 1, one particle per lane, from the 16-bit bins in shared memory; it joins the
-// cast when it is done.  P (up to 32) is chosen so that all blocks are resident at once (or in few
+// multiplies chunk k - 1, one particle per lane, from the bins (or table factors) in shared memory; it
+// joins the cast when it is done.  P (up to 32) is chosen so that all blocks are resident at once (or in few
 // equal waves): no tail, and as many lanes share each FP64 multiply as the particle count allows.
 // Poses and, for the kinds that need a ray's cos/sin, the trig records of the particles are made
 // once per block, those of the beams once per chunk.  Before, blocks held 256 / na particles: from
@@ -977,25 +977,25 @@ constexpr int kWideParticles = 32;
 struct WideSmem {   // byte offsets of the dynamic shared memory
     int part, beam, ang, row, bins, total;
 };
-__host__ __device__ inline WideSmem wide_smem(int P, int C) {
+__host__ __device__ inline WideSmem wide_smem(int P, int C, bool factors) {
     WideSmem w;
     w.part = 0;                        // [P] pose, trig record
     w.beam = w.part + P * 32;          // [2][C] trig record
     w.ang = w.beam + 2 * C * 16;       // [2][C] beam angle
-    w.bins = w.ang + 2 * C * 4;        // [2][C / 4][P][4] range bins
-    w.row = w.bins + 2 * C * P * 2;    // [3][C] observation bin
+    w.bins = w.ang + 2 * C * 4;        // [2][C / 4][P][4] range bins, or [2][P][C] table factors
+    w.row = w.bins + 2 * C * P * (factors ? 8 : 2);   // [3][C] observation bin
     w.total = w.row + 3 * C * 2;
     return w;
 }
 
-template <int KIND, int LAYOUT, int PF>
+template <int KIND, int LAYOUT, int PF, bool FACTORS>
 __global__ void __launch_bounds__(kWideThreads, KIND == K_CDDT ? 4 : 8)
 k_fused_wide(CastParams p, SensorDev sm, const float* __restrict__ ins, const float* __restrict__ angles,
              const float* __restrict__ obs, double* __restrict__ weights, int n, int na, int P, int C) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ unsigned s_next[2];
     constexpr bool kTrig = KIND == K_RM || KIND == K_BL;
-    const WideSmem off = wide_smem(P, C);
+    const WideSmem off = wide_smem(P, C, FACTORS);
     float4* part = reinterpret_cast<float4*>(smem_raw + off.part);
     float4* beam = reinterpret_cast<float4*>(smem_raw + off.beam);
     float* ang = reinterpret_cast<float*>(smem_raw + off.ang);
@@ -1023,7 +1023,13 @@ k_fused_wide(CastParams p, SensorDev sm, const float* __restrict__ ins, const fl
     __syncthreads();
     double w = 1.0;
     for (int k = 0; k <= chunks; ++k) {
-        if (threadIdx.x < 32 && k > 0 && lane < np) {
+        if (FACTORS && threadIdx.x < 32 && k > 0 && lane < np) {
+            const double* f = reinterpret_cast<const double*>(bins) + (((k - 1) & 1) * P + lane) * C;
+            const int nb = min(C, na - (k - 1) * C);
+#pragma unroll 8
+            for (int a = 0; a < nb; ++a) w = __dmul_rn(w, f[a]);
+        }
+        if (!FACTORS && threadIdx.x < 32 && k > 0 && lane < np) {
             const uint16_t* tile = bins + ((k - 1) & 1) * C * P;
             const uint16_t* rw = row + ((k - 1) % 3) * C;
             w = product_chain<4>(sm, min(C, na - (k - 1) * C), [&](int a) { return (unsigned)rw[a]; },
@@ -1057,7 +1063,12 @@ k_fused_wide(CastParams p, SensorDev sm, const float* __restrict__ ins, const fl
                 d = KIND == K_RM ? rm_cast<LAYOUT, PF>(p.map, p.mr, pose.x, pose.y, c, s)
                                  : bl_cast(p.map, p.mr, pose.x, pose.y, c, s, p.err);
             }
-            tile[((size_t)(a >> 2) * P + li) * 4 + (a & 3)] = (uint16_t)sensor_bin(d, sm.K, p.err);
+            const int bin = sensor_bin(d, sm.K, p.err);
+            if (FACTORS)
+                reinterpret_cast<double*>(bins)[((k & 1) * P + li) * C + a] =
+                    __ldg(sm.table + (size_t)row[(k % 3) * C + a] * sm.K + bin);
+            else
+                tile[((size_t)(a >> 2) * P + li) * 4 + (a & 3)] = (uint16_t)bin;
         }
         __syncthreads();   // the chunk's bins and the next chunk's records are written
     }
@@ -1551,20 +1562,26 @@ cudaError_t set_smem(K kernel, size_t bytes) {
     return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
-// Which fused calls go wide, where the caller has not asked for a schedule: from 1 M rays on, if a
-// block of k_fused would hold a single particle (one lane per multiply), and then with at least two
-// particles per lane set.  Ray marching on a 2048^2 corridor map, us per call before / wide:
-// 20,000 x 1,081 1365 / 401, 4,000 x 1,081 329 / 155, 4,000 x 271 88 / 65; below the line
-// 20,000 x 61 62 / 68, 2,000 x 108 26 / 32, 1,000 x 1,081 101 / 108.  CDDT: 8,000 x 1,081 634 / 187,
-// 4,000 x 271 97 / 46.  Bresenham's walks are too uneven for a barrier per chunk (8,000 x 1,081
-// 722 / 869).
-constexpr long long kWideRays = 1 << 20;
-constexpr int kWideMinBeams = 192, kWideMinParticles = 2000;
-constexpr int kWideChunk = 2048;   // rays of a chunk: 17 x 64 / 128 / 256 beams 425 / 401 / 475 us
-
+// Which fused calls go wide, where the caller has not asked for a schedule: those where a block of
+// k_fused would multiply with one or two lanes, from the particle count on at which that costs more
+// than the shorter blocks gain.  Ray marching on a 2048^2 corridor map, us per call before / wide:
+// 20,000 x 1,081 1365 / 379, 4,000 x 1,081 329 / 140, 4,000 x 271 88 / 60, 2,000 x 1,081 178 / 107,
+// 2,000 x 300 61 / 48, 6,000 x 150 70 / 51, 2,000 x 150 41 / 35; below the line 1,000 x 1,081
+// 100 / 97, 1,000 x 300 38 / 43, 600 x 150 28 / 30, 20,000 x 61 62 / 68.  CDDT: 8,000 x 1,081
+// 634 / 187, 4,000 x 271 97 / 46.  Bresenham's walks are too uneven for a barrier per chunk (8,000 x
+// 1,081 722 / 869).
 inline bool fused_wide(int kind, int n, int na) {
-    return kind != K_BL && (long long)n * na >= kWideRays && na >= kWideMinBeams && n >= kWideMinParticles;
+    const long long rays = (long long)n * na;
+    if (kind == K_BL || n < 2000) return false;
+    return kind == K_RM ? na >= 128 && rays >= (1ll << 18) : na >= 192 && rays >= (1ll << 20);
 }
+// Its shape: as few particles per block as keep all blocks resident at once.  Up to kWideFactors
+// particles the rays' threads read the table factors themselves (a lone product chain that reads
+// them waits for each: 2,000 x 1,081 137 us, 110 with the factors at hand), in chunks of 128 beams;
+// with more, 16-bit bins keep the chunk's shared memory small (17 particles x 64 / 128 / 256 beams
+// 425 / 401 / 475 us).
+constexpr int kWideFactors = 8;
+constexpr int kWideChunk = 2048;
 
 template <int KIND, int LAYOUT, int PF>
 struct RunFused {
@@ -1583,9 +1600,11 @@ struct RunFused {
                 const long long resident = (long long)sms * (KIND == K_CDDT ? 4 : 8);
                 const long long waves = (n + resident * kWideParticles - 1) / (resident * kWideParticles);
                 const int P = (int)((n + resident * waves - 1) / (resident * waves));
-                const int C = min(max(32, min(512, (kWideChunk / P + 31) / 32 * 32)), (na + 3) / 4 * 4);
-                k_fused_wide<KIND, LAYOUT, PF><<<blocks_for(n, P), kWideThreads, wide_smem(P, C).total, s>>>(
-                    p, sm, ins, angles, obs, w, n, na, P, C);
+                const bool factors = P <= kWideFactors;
+                const int C = min(factors ? (P <= 2 ? 256 : 128) : max(32, (kWideChunk / P + 31) / 32 * 32), (na + 3) / 4 * 4);
+                const int smem = wide_smem(P, C, factors).total;
+                const auto kernel = factors ? k_fused_wide<KIND, LAYOUT, PF, true> : k_fused_wide<KIND, LAYOUT, PF, false>;
+                kernel<<<blocks_for(n, P), kWideThreads, smem, s>>>(p, sm, ins, angles, obs, w, n, na, P, C);
                 return cudaGetLastError();
             }
         }
