@@ -95,7 +95,8 @@ struct rlc_map {
             total += (bytes + 255) & ~(size_t)255;
             return at;
         };
-        const size_t o_dt = room(n * sizeof(float)), o_step = room(n * sizeof(float));
+        const size_t steps = step_map_cells(W, H);
+        const size_t o_dt = room(n * sizeof(float)), o_step = room(steps * sizeof(float));
         const size_t o_tiled = room(tiled * sizeof(float)), o_u16 = room(tiled * sizeof(uint16_t)), o_u8 = room(tiled);
         const size_t o_runs = room(n * sizeof(uint32_t)), o_eq = room(step_eq_words(W, H) * sizeof(uint32_t));
         const size_t sb = edt_scratch_bytes(W, H);
@@ -105,13 +106,13 @@ struct rlc_map {
         if (e == cudaSuccess && sb > n * sizeof(uint32_t)) e = cudaMalloc(&extra, sb);
         DtOut o;
         o.dt = (float*)(base + o_dt);
-        o.step = (float*)(base + o_step);
+        o.step = steps ? (float*)(base + o_step) : nullptr;
         o.tiled = (float*)(base + o_tiled);
         o.u16 = (uint16_t*)(base + o_u16);
         o.u8 = (uint8_t*)(base + o_u8);
         uint32_t* runs = (uint32_t*)(base + o_runs);
         if (e == cudaSuccess) e = launch_edt(d_bits, W, H, TY, o, extra ? extra : runs, sb, 0);
-        if (e == cudaSuccess) e = launch_step_runs(o.step, W, H, (uint32_t*)(base + o_eq), runs, 0);
+        if (e == cudaSuccess && steps) e = launch_step_runs(o.step, W, H, (uint32_t*)(base + o_eq), runs, 0);
         if (e == cudaSuccess) e = cudaStreamSynchronize(0);
         cudaFree(extra);
         if (e != cudaSuccess) {
@@ -350,8 +351,13 @@ int finish_launch(cudaError_t e, const char* what) {
     return RLC_OK;
 }
 
+// `layout`, or the linear one where the map is too large for a step map
+int map_layout(const rlc_map* map, int layout) {
+    return (layout == DT_STEP || layout == DT_RUNS) && !map->d_step ? DT_LINEAR : layout;
+}
+
 // layout used by the per-ray kernels (the staged schedule only changes the fused update)
-int cast_layout(const rlc_method* m) { return m->layout == DT_STAGED ? DT_LINEAR : m->layout; }
+int cast_layout(const rlc_method* m) { return m->layout == DT_STAGED ? DT_LINEAR : map_layout(m->map, m->layout); }
 
 // layout of a cast of `rays` rays.  Without a schedule, ray marching takes the step map, with its
 // equal-step runs where the call waits for its longest rays: independent queries (their warps mix
@@ -361,7 +367,7 @@ int cast_layout(const rlc_method* m) { return m->layout == DT_STAGED ? DT_LINEAR
 // 43 / 41 / 46 us, 20,000 x 1,081 267 / 257 / 336 us).
 int cast_layout(const rlc_method* m, long long rays, bool independent) {
     if (!m->pick || m->dkind != K_RM) return cast_layout(m);
-    return independent || (rays >= (1ll << 14) && rays < (1ll << 18)) ? DT_RUNS : DT_STEP;
+    return map_layout(m->map, independent || (rays >= (1ll << 14) && rays < (1ll << 18)) ? DT_RUNS : DT_STEP);
 }
 
 // layout of a fused call.  Without a schedule, ray marching takes the step map, with its equal-step
@@ -370,7 +376,7 @@ int cast_layout(const rlc_method* m, long long rays, bool independent) {
 // 4,000 x 1,081 - / 140 / 157, 20,000 x 1,081 438 / 423 / 496 us.
 int fused_layout(const rlc_method* m, int n, int na) {
     if (!m->pick || m->dkind != K_RM) return cast_layout(m);
-    return (long long)n * na < (2ll << 20) && (na < 512 || n >= 2000) ? DT_RUNS : DT_STEP;
+    return map_layout(m->map, (long long)n * na < (2ll << 20) && (na < 512 || n >= 2000) ? DT_RUNS : DT_STEP);
 }
 
 int check_trig(const rlc_method* m, long long rays) {
@@ -1103,7 +1109,7 @@ int rlc_method_autotune_ex(rlc_method* m, const float* ins, const float* angles,
         m->layout = c.layout;
         CastParams p = m->params();
         if (c.layout == DT_STAGED) return launch_fused_staged(p, sm, ins, angles, obs, w, n, na, 0, m->d_bins, s);
-        return launch_fused(p, c.layout, c.prefetch, sm, ins, angles, obs, w, n, na, c.block, c.tile, false, s);
+        return launch_fused(p, map_layout(m->map, c.layout), c.prefetch, sm, ins, angles, obs, w, n, na, c.block, c.tile, false, s);
     };
     unsigned flush_round = 0;
     auto time_once = [&](const Cand& c, float* ms) -> cudaError_t {
@@ -1197,6 +1203,15 @@ struct rlc_batch {
     // schedule
     int layout = DT_LINEAR, prefetch = 0, block = 256, tile = 0;
     bool separate = false;    // products in a second launch instead of inside the persistent kernel
+    // nothing asked for or autotuned yet: a batch of ray-marching filters runs with the products
+    // inside the launch (k_batch_wide), on the step map with its equal-step runs while the run waits
+    // for its longest rays (below 2 M rays: one filter of 1,198 x 120 36 against 51 us without), and
+    // the getters report the values above meanwhile.  8 filters of 512^2 - 4096^2, 23 M rays: those
+    // values 987 us, the best schedule of k_batch 649, this 575.  From 48 M rays on, that schedule of
+    // k_batch, whose march budget gains what its second launch costs: 45 M rays 1003 against 1012 us,
+    // 73 M 1504 / 1577, 122 M 2529 / 2772.
+    bool pick = true;
+    struct Schedule { int layout, prefetch, block, tile; bool separate, wide; } run{};   // what is run
     // built state
     int nf = 0;
     FilterDev* d_filters = nullptr;
@@ -1234,11 +1249,29 @@ struct rlc_batch {
     // (re)build the device filter table for the current schedule
     int build() {
         drop_graph();
+        int dev = 0, sms = 0;
+        CUDA_OR_FAIL(cudaGetDevice(&dev), "batch setup");
+        CUDA_OR_FAIL(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "batch setup");
+        run = Schedule{layout, prefetch, block, tile, separate, false};
+        bool steps = true;   // every ray-marching filter's map has a step map
+        long long particles = 0;
+        for (const rlc_filter_desc& d : descs) {
+            if (d.method->dkind == K_RM && map_layout(d.method->map, DT_STEP) != DT_STEP) steps = false;
+            particles += d.n_particles;
+        }
+        if (!steps && (layout == DT_STEP || layout == DT_RUNS)) run.layout = DT_LINEAR;
+        if (pick && rm_only && steps) {
+            if (rays < (48ll << 20))
+                run = Schedule{rays < (2ll << 20) ? DT_RUNS : DT_STEP, 0, 256, batch_wide_tile(particles, sms), false, true};
+            else
+                run = Schedule{DT_STEP, 0, 256, 8, true, false};
+        }
         struct Item { FilterDev f; double cost; };
         std::vector<Item> items;
-        const int ppb = tile > 0 ? tile : 32;   // 32 particles: one full lane set of the product warp
+        const int ppb = run.tile > 0 ? run.tile : 32;   // 32 particles: one full lane set of the product warp
         size_t need = 0, nobs = 0, nrec = 0;
         for (const rlc_filter_desc& d : descs) {
+            if (run.wide) break;   // no bins, no records
             need += (size_t)((d.n_particles + ppb - 1) / ppb) * batch_tile_bins(d.n_angles, ppb);
             nobs += (size_t)d.n_angles;
             nrec += 2 * (size_t)d.n_particles + (size_t)d.n_angles;
@@ -1250,19 +1283,19 @@ struct rlc_batch {
             CUDA_OR_FAIL(cudaMalloc(&d_bins, (need ? need : 1) * sizeof(uint16_t)), "batch range bins");
             bins_cap = need;
         }
-        if (!d_obs_bins) CUDA_OR_FAIL(cudaMalloc(&d_obs_bins, (nobs ? nobs : 1) * sizeof(uint16_t)), "batch observation bins");
-        if (!d_rec) CUDA_OR_FAIL(cudaMalloc(&d_rec, (nrec ? nrec : 1) * sizeof(float4)), "batch particle and beam records");
+        if (!run.wide && !d_obs_bins) CUDA_OR_FAIL(cudaMalloc(&d_obs_bins, (nobs ? nobs : 1) * sizeof(uint16_t)), "batch observation bins");
+        if (!run.wide && !d_rec) CUDA_OR_FAIL(cudaMalloc(&d_rec, (nrec ? nrec : 1) * sizeof(float4)), "batch particle and beam records");
         size_t bin_ofs = 0, obs_ofs = 0, rec_ofs = 0;
         for (const rlc_filter_desc& d : descs) {
             rlc_method* m = d.method;
             Item it{};
             CastParams p = m->params();
             if (m->dkind == K_RM) {   // the batch schedule's layout for every ray-marching filter
-                p.map.dt = layout == DT_TILED ? m->map->d_dt_tiled : m->map->d_dt;
+                p.map.dt = run.layout == DT_TILED ? m->map->d_dt_tiled : m->map->d_dt;
             }
             it.f.p = p;
-            it.f.layout = layout;
-            it.f.prefetch = prefetch;
+            it.f.layout = run.layout;
+            it.f.prefetch = run.prefetch;
             it.f.sm = SensorDev{m->d_table, m->K};
             it.f.ins = d.ins;
             it.f.angles = d.angles;
@@ -1273,14 +1306,16 @@ struct rlc_batch {
             it.f.na = d.n_angles;
             it.f.inv_na = d.n_angles > 0 ? 1.0f / (float)d.n_angles : 0.0f;
             it.f.ppb = ppb;
-            it.f.bins = d_bins + bin_ofs;
-            bin_ofs += (size_t)((d.n_particles + ppb - 1) / ppb) * batch_tile_bins(d.n_angles, ppb);
-            it.f.obs_bins = d_obs_bins + obs_ofs;
-            obs_ofs += (size_t)d.n_angles;
-            it.f.part_rec = d_rec + rec_ofs;
-            rec_ofs += 2 * (size_t)d.n_particles;
-            it.f.beam_rec = d_rec + rec_ofs;
-            rec_ofs += (size_t)d.n_angles;
+            if (!run.wide) {
+                it.f.bins = d_bins + bin_ofs;
+                bin_ofs += (size_t)((d.n_particles + ppb - 1) / ppb) * batch_tile_bins(d.n_angles, ppb);
+                it.f.obs_bins = d_obs_bins + obs_ofs;
+                obs_ofs += (size_t)d.n_angles;
+                it.f.part_rec = d_rec + rec_ofs;
+                rec_ofs += 2 * (size_t)d.n_particles;
+                it.f.beam_rec = d_rec + rec_ofs;
+                rec_ofs += (size_t)d.n_angles;
+            }
             // heavier tiles first: rays per tile x march length
             it.cost = (double)it.f.ppb * (d.n_angles > 0 ? d.n_angles : 1) * (double)(m->mr > 1.0f ? m->mr : 1.0f);
             items.push_back(it);
@@ -1299,11 +1334,12 @@ struct rlc_batch {
             if (tiles >= 0xffffffffull) return fail(RLC_ERR_ARG, "too many tiles in one batch");
             hf.push_back(it.f);
         }
-        int dev = 0, sms = 0, per_sm = 0;
-        cudaError_t e = cudaGetDevice(&dev);
-        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        smem = batch_smem(block, rm_only);
-        if (e == cudaSuccess) e = batch_occupancy(block, smem, rm_only, layout, prefetch, separate, &per_sm);
+        int per_sm = 0;
+        cudaError_t e = cudaSuccess;
+        smem = batch_smem(run.block, rm_only);
+        if (run.wide) e = batch_wide_occupancy(run.layout, run.tile, &per_sm);
+        else
+            e = batch_occupancy(run.block, smem, rm_only, run.layout, run.prefetch, run.separate, &per_sm);
         if (e == cudaSuccess && per_sm <= 0) e = cudaErrorInvalidConfiguration;
         if (e == cudaSuccess && !d_filters) e = cudaMalloc(&d_filters, descs.size() * sizeof(FilterDev));
         if (e == cudaSuccess)
@@ -1336,9 +1372,11 @@ struct rlc_batch {
         if (!exec) {
             CUDA_OR_FAIL(cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal), "batch capture");
             cudaError_t e = cudaMemsetAsync(d_queue, 0, sizeof(unsigned), cap);
-            if (e == cudaSuccess)
-                e = launch_batch(d_filters, nf, total_tiles, d_queue, grid, block, smem, rm_only, layout, prefetch,
-                                 separate, total_particles, cap);
+            if (e == cudaSuccess && run.wide)
+                e = launch_batch_wide(d_filters, nf, total_tiles, d_queue, grid, run.layout, run.tile, cap);
+            else if (e == cudaSuccess)
+                e = launch_batch(d_filters, nf, total_tiles, d_queue, grid, run.block, smem, rm_only, run.layout,
+                                 run.prefetch, run.separate, total_particles, cap);
             cudaGraph_t g = nullptr;
             cudaError_t e2 = cudaStreamEndCapture(cap, &g);
             if (e == cudaSuccess) e = e2;
@@ -1361,7 +1399,8 @@ int rlc_batch_create(const rlc_filter_desc* fd, int nf, int block, rlc_batch** o
     if (!out) return fail(RLC_ERR_ARG, "null output handle");
     *out = nullptr;
     if (nf <= 0 || !fd) return fail(RLC_ERR_ARG, "a batch needs at least one filter");
-    if (block == 0) block = 256;
+    const bool asked = block != 0;
+    if (!asked) block = 256;
     if (block < 32 || block > 512 || block % 32) return fail(RLC_ERR_ARG, "block must be a multiple of 32 in [32, 512]");
     long long rays = 0;
     bool rm_only = true;
@@ -1384,6 +1423,7 @@ int rlc_batch_create(const rlc_filter_desc* fd, int nf, int block, rlc_batch** o
     b->descs.assign(fd, fd + nf);
     b->rm_only = rm_only;
     b->block = block;
+    b->pick = !asked;
     b->rays = rays;
     if (int rc = b->build()) {
         delete b;
@@ -1400,6 +1440,7 @@ int rlc_batch_set_schedule(rlc_batch* b, int dt_layout, int prefetch, int block,
     if (prefetch < 0 || prefetch > 1) return fail(RLC_ERR_ARG, "prefetch must be 0 or 1");
     if (block != 0 && (block < 32 || block > 512 || block % 32)) return fail(RLC_ERR_ARG, "block must be a multiple of 32 in [32, 512]");
     if (tile < 0 || tile > 512) return fail(RLC_ERR_ARG, "tile must be in [0, 512]");
+    b->pick = false;
     b->layout = dt_layout;
     b->prefetch = prefetch;
     if (block) b->block = block;
@@ -1410,6 +1451,7 @@ int rlc_batch_set_schedule(rlc_batch* b, int dt_layout, int prefetch, int block,
 int rlc_batch_set_product_mode(rlc_batch* b, int mode) {
     if (!b) return fail(RLC_ERR_ARG, "null batch handle");
     if (mode != RLC_PRODUCTS_OVERLAPPED && mode != RLC_PRODUCTS_SEPARATE) return fail(RLC_ERR_ARG, "product mode %d", mode);
+    b->pick = false;
     b->separate = mode == RLC_PRODUCTS_SEPARATE;
     return b->build();
 }
@@ -1450,7 +1492,8 @@ int rlc_batch_autotune(rlc_batch* b, void* stream) {
                         if (!b->rm_only && (kLayouts[lk] != 0 || pf != 0)) continue;
                         cands.push_back(Cand{sp != 0, kLayouts[lk], pf, blocks[bi], tiles[ti], 0.0f});
                     }
-    const bool s0 = b->separate;
+    const bool s0 = b->separate, pick0 = b->pick;
+    b->pick = false;
     const int l0 = b->layout, p0 = b->prefetch, b0 = b->block, t0 = b->tile;
     auto apply = [&](const Cand& c) {
         b->separate = c.sep;
@@ -1506,6 +1549,7 @@ int rlc_batch_autotune(rlc_batch* b, void* stream) {
         int rc2 = apply(cands[best]);
         return rc ? rc : rc2;
     }
+    b->pick = pick0;
     b->separate = s0;
     b->layout = l0;
     b->prefetch = p0;

@@ -65,7 +65,6 @@ __device__ __forceinline__ float dt_at(const MapDev& m, int x, int y) {
     }
     if (LAYOUT == DT_TILED)
         return __ldg(m.dt + (((size_t)(x >> 3) * m.tiles_y + (y >> 3)) << 6) + ((x & 7) << 3) + (y & 7));
-    if (LAYOUT == DT_STEP || LAYOUT == DT_RUNS) return __ldg(m.step + (size_t)x * m.H + y);   // the step (0 on walls)
     return __ldg(m.dt + (size_t)x * m.H + y);
 }
 
@@ -74,7 +73,7 @@ __device__ __forceinline__ const void* dt_ptr(const MapDev& m, int x, int y) {
     if (LAYOUT == DT_U16) return m.dt16 + u16_index(m, x, y);
     if (LAYOUT == DT_TILED)
         return m.dt + (((size_t)(x >> 3) * m.tiles_y + (y >> 3)) << 6) + ((x & 7) << 3) + (y & 7);
-    if (LAYOUT == DT_STEP || LAYOUT == DT_RUNS) return m.step + (size_t)x * m.H + y;
+    if (LAYOUT == DT_STEP || LAYOUT == DT_RUNS) return m.step + ((size_t)x * (m.H + 1) + y);
     return m.dt + (size_t)x * m.H + y;
 }
 
@@ -99,14 +98,14 @@ __device__ __forceinline__ bool occ_at(const MapDev& m, int x, int y) {
 //
 // DT_RUNS: the step map plus equal-step runs (run_skip below).
 constexpr int kMinRun = 12;       // shortest run worth a skip
-constexpr int kRunTrigger = 6;    // equal steps in a row before the run map is read
+constexpr int kUnroll = 4;        // steps of the step map between two looks at the budget and the run map
 
 // Exact skip over a run of equal steps (DT_RUNS).  A ray running beside a wall keeps the same
 // distance to it, so its march repeats one step value v for many iterations: the longest rays of
 // a particle-filter step repeat a step of 1 (one pixel) or 1.998 over a hundred times.  Once a
-// ray has taken kRunTrigger equal steps in a row, at cell (px, py), the run map says how many
-// cells after it along the ray's major axis (L, direction of travel) have step v too (only then:
-// the read would lengthen the march of every other ray).  The march parameters of such a
+// ray takes a step equal to the one kUnroll steps before, at cell (px, py), the run map says how
+// many cells after it along the ray's major axis (L, direction of travel) have step v too (only
+// then: the read would lengthen the march of every other ray).  The march parameters of such a
 // run are known without reading a cell: t_j+1 = t_j + v rounded as the reference's addition.  An
 // estimate J of how many positions t_1 .. t_J stay in the box {the current row or column} x {the
 // run} is checked exactly at t_J with the march's own float operations; positions are monotone in
@@ -143,28 +142,79 @@ __device__ __forceinline__ float run_skip(float mr, float x0, float y0, float c,
 }
 
 // A ray's march state (RangeLib.h:927-962): origin, direction, the parameter t, and for DT_RUNS
-// the last step and how many equal steps in a row ended with it; r is the caller's ray index.
+// the last step looked at; r is the caller's ray index.
 struct __align__(16) RmRay {
     float x0, y0, c, s, t, prev;
-    int rep, r;
+    int r, unused;
 };
+
+// The march over the step map, which decides a step by one comparison: an occupied cell holds NaN
+// and the row and column past the grid +inf, so that t + step < max_range fails at a hit, off the
+// grid (a position off the grid reads that row or column) and at max_range alike, and what the cell
+// holds says which it was.  15 instructions a step instead of 24 with the grid tests and the hit
+// test beside it; the budget and the run map are looked at every kUnroll steps.  2 M queries on
+// 2048^2 with runs 94 -> 87 us, 20,000 x 1,081 fused 401 -> 365, 23 M rays batched 707 -> 649.
+template <int LAYOUT, int PF, bool BUDGETED>
+__device__ __forceinline__ bool rm_advance_steps(const MapDev& m, float mr, RmRay& q, int budget, float* out, int* steps) {
+    const float x0 = q.x0, y0 = q.y0, c = q.c, s = q.s;
+    float t = q.t, prev = q.prev;
+    const unsigned W = (unsigned)m.W, H = (unsigned)m.H, pitch = H + 1u;
+    // DT_RUNS: the byte of the run word that lies along the ray (major axis, direction of travel)
+    const unsigned run_shift = fabsf(s) >= fabsf(c) ? (s > 0.0f ? 0u : 8u) : (c > 0.0f ? 16u : 24u);
+    for (int round = 0;; round += kUnroll) {
+        if (BUDGETED && round >= budget) {
+            q.t = t;
+            q.prev = prev;
+            return false;
+        }
+        unsigned px, py;
+        float st;
+#pragma unroll
+        for (int u = 0; u < kUnroll; ++u) {
+            px = min((unsigned)__float2int_rz(__fadd_rn(x0, __fmul_rn(c, t))), W);
+            py = min((unsigned)__float2int_rz(__fadd_rn(y0, __fmul_rn(s, t))), H);
+            if (PF > 0) {
+                const float tp = t + (float)PF;
+                const int qx = __float2int_rz(x0 + c * tp), qy = __float2int_rz(y0 + s * tp);
+                if ((unsigned)qx < W && (unsigned)qy < H) prefetch_l1(dt_ptr<LAYOUT>(m, qx, qy));
+            }
+            st = __ldg(m.step + (px * pitch + py));
+            if (steps && !isinf(st)) ++*steps;
+            const float tn = __fadd_rn(t, st);
+            if (!(tn < mr)) {
+                if (isnan(st)) {
+                    const float xd = __fsub_rn(__int2float_rn((int)px), x0), yd = __fsub_rn(__int2float_rn((int)py), y0);
+                    *out = __fsqrt_rn(__fadd_rn(__fmul_rn(xd, xd), __fmul_rn(yd, yd)));
+                } else {
+                    *out = mr;
+                }
+                return true;
+            }
+            t = tn;
+        }
+        if (LAYOUT == DT_RUNS) {
+            if (st == prev) {   // a ray repeating one step (beside a wall): look for the run
+                const int L = (int)((__ldg(m.runs + (px * H + py)) >> run_shift) & 255u);
+                if (L >= kMinRun) t = run_skip(mr, x0, y0, c, s, (int)px, (int)py, L, st, t, steps);
+            }
+            prev = st;
+        }
+    }
+}
 
 // Marches q from its parameter q.t.  BUDGETED: at most `budget` rounds of the loop (a run skip is
 // one round), after which it returns false with q holding the state of the next round, exactly
 // where the reference's loop stands; otherwise (and when the ray ends first) it returns true with
-// the range in *out.  One exit test per step: an off-grid position reads cell (0, 0) and leaves.
+// the range in *out.  Distance layouts: one exit test per step, an off-grid position reads cell
+// (0, 0) and leaves; the linear layout forms the cell index in 32 bits (W * H < 2^31).
 template <int LAYOUT, int PF, bool BUDGETED>
 __device__ __forceinline__ bool rm_advance(const MapDev& m, float mr, RmRay& q, int budget, float* out, int* steps) {
+    if (LAYOUT == DT_STEP || LAYOUT == DT_RUNS) return rm_advance_steps<LAYOUT, PF, BUDGETED>(m, mr, q, budget, out, steps);
     const float x0 = q.x0, y0 = q.y0, c = q.c, s = q.s;
-    float t = q.t, prev = q.prev;
-    int rep = q.rep;   // equal steps in a row
-    // DT_RUNS: the byte of the run word that lies along the ray (major axis, direction of travel)
-    const unsigned run_shift = fabsf(s) >= fabsf(c) ? (s > 0.0f ? 0u : 8u) : (c > 0.0f ? 16u : 24u);
+    float t = q.t;
     for (int round = 0;; ++round) {
         if (BUDGETED && round >= budget) {
             q.t = t;
-            q.prev = prev;
-            q.rep = rep;
             return false;
         }
         const int px = __float2int_rz(__fadd_rn(x0, __fmul_rn(c, t)));
@@ -175,19 +225,16 @@ __device__ __forceinline__ bool rm_advance(const MapDev& m, float mr, RmRay& q, 
             const int qx = __float2int_rz(x0 + c * tp), qy = __float2int_rz(y0 + s * tp);
             if ((unsigned)qx < (unsigned)m.W && (unsigned)qy < (unsigned)m.H) prefetch_l1(dt_ptr<LAYOUT>(m, qx, qy));
         }
-        // DT_STEP reads the step max(d * 0.999, 1) precomputed per cell (0 where d = 0).  The
-        // linear layouts form the cell index in 32 bits (W * H < 2^31) and select it once.
-        constexpr bool kStepMap = LAYOUT == DT_STEP || LAYOUT == DT_RUNS;
         float d;
         unsigned cell = 0u;
-        if (LAYOUT == DT_LINEAR || kStepMap) {
+        if (LAYOUT == DT_LINEAR) {
             cell = out_of_grid ? 0u : (unsigned)px * (unsigned)m.H + (unsigned)py;
-            d = __ldg((kStepMap ? m.step : m.dt) + cell);
+            d = __ldg(m.dt + cell);
         } else {
             d = dt_at<LAYOUT>(m, out_of_grid ? 0 : px, out_of_grid ? 0 : py);
         }
         if (steps && !out_of_grid) ++*steps;
-        const float st = kStepMap ? d : ref_maxf(__fmul_rn(d, 0.999f), 1.0f);
+        const float st = ref_maxf(__fmul_rn(d, 0.999f), 1.0f);
         const float tn = __fadd_rn(t, st);
         const bool hit = d <= 0.0f;
         if (out_of_grid | hit | !(tn < mr)) {
@@ -201,15 +248,6 @@ __device__ __forceinline__ bool rm_advance(const MapDev& m, float mr, RmRay& q, 
             return true;
         }
         t = tn;
-        if (LAYOUT == DT_RUNS) {
-            rep = st == prev ? rep + 1 : 0;
-            prev = st;
-            if (rep == kRunTrigger) {   // a ray repeating one step (beside a wall): look for the run
-                rep = 0;
-                const int L = (int)((__ldg(m.runs + cell) >> run_shift) & 255u);
-                if (L >= kMinRun) t = run_skip(mr, x0, y0, c, s, px, py, L, st, t, steps);
-            }
-        }
     }
 }
 
@@ -546,8 +584,8 @@ __device__ __forceinline__ float glt_cast(const CastParams& p, float x, float y,
     return __fmul_rn(__int2float_rn(__ldg(g.lut + cell * g.td + b)), g.max_div_limits);
 }
 
-// one ray per (cell corner, angle bin), angle bins fastest: lut[(x * H + y) * td + i]; the march reads
-// the per-cell step map (the same steps as the distance transform's, two instructions fewer)
+// one ray per (cell corner, angle bin), angle bins fastest: lut[(x * H + y) * td + i]
+template <int LAYOUT>
 __global__ void __launch_bounds__(256) k_glt_build(MapDev m, float mr, unsigned td, const float* __restrict__ cosv,
                                                    const float* __restrict__ sinv, float limits_div_max,
                                                    uint16_t* __restrict__ lut, long long total) {
@@ -556,7 +594,7 @@ __global__ void __launch_bounds__(256) k_glt_build(MapDev m, float mr, unsigned 
     const long long cell = idx / td;
     const int i = (int)(idx - cell * td);
     const int x = (int)(cell / m.H), y = (int)(cell - (long long)x * m.H);
-    float r = rm_cast<DT_STEP, 0>(m, mr, __int2float_rn(x), __int2float_rn(y), __ldg(cosv + i), __ldg(sinv + i));
+    float r = rm_cast<LAYOUT, 0>(m, mr, __int2float_rn(x), __int2float_rn(y), __ldg(cosv + i), __ldg(sinv + i));
     r = r < mr ? r : mr;   // std::min(max_range, r)
     lut[idx] = (uint16_t)__float2uint_rz(__fmul_rn(r, limits_div_max));
 }
@@ -988,20 +1026,21 @@ __host__ __device__ inline WideSmem wide_smem(int P, int C, bool factors) {
     return w;
 }
 
+// Particles [first, first + np) of one filter through all its beams, by a whole block; ranges (pixels,
+// optional) as ranges[i * na + a].  s_next: two counters of the block.
 template <int KIND, int LAYOUT, int PF, bool FACTORS>
-__global__ void __launch_bounds__(kWideThreads, KIND == K_CDDT ? 4 : 8)
-k_fused_wide(CastParams p, SensorDev sm, const float* __restrict__ ins, const float* __restrict__ angles,
-             const float* __restrict__ obs, double* __restrict__ weights, int n, int na, int P, int C) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ unsigned s_next[2];
+__device__ __forceinline__ void wide_tile(const CastParams& p, const SensorDev& sm, const float* __restrict__ ins,
+                                          const float* __restrict__ angles, const float* __restrict__ obs,
+                                          float* __restrict__ ranges, double* __restrict__ weights, int first, int np,
+                                          int na, int P, int C, unsigned char* smem, unsigned* s_next) {
     constexpr bool kTrig = KIND == K_RM || KIND == K_BL;
     const WideSmem off = wide_smem(P, C, FACTORS);
-    float4* part = reinterpret_cast<float4*>(smem_raw + off.part);
-    float4* beam = reinterpret_cast<float4*>(smem_raw + off.beam);
-    float* ang = reinterpret_cast<float*>(smem_raw + off.ang);
-    uint16_t* bins = reinterpret_cast<uint16_t*>(smem_raw + off.bins);
-    uint16_t* row = reinterpret_cast<uint16_t*>(smem_raw + off.row);
-    const int lane = threadIdx.x & 31, first = blockIdx.x * P, np = min(P, n - first);
+    float4* part = reinterpret_cast<float4*>(smem + off.part);
+    float4* beam = reinterpret_cast<float4*>(smem + off.beam);
+    float* ang = reinterpret_cast<float*>(smem + off.ang);
+    uint16_t* bins = reinterpret_cast<uint16_t*>(smem + off.bins);
+    uint16_t* row = reinterpret_cast<uint16_t*>(smem + off.row);
+    const int lane = threadIdx.x & 31;
     const int chunks = (na + C - 1) / C;
     if ((int)threadIdx.x < np) {
         const float* q = ins + 3 * (size_t)(first + threadIdx.x);
@@ -1010,7 +1049,7 @@ k_fused_wide(CastParams p, SensorDev sm, const float* __restrict__ ins, const fl
         part[2 * threadIdx.x] = make_float4(ax, ay, th, 0.0f);
         if (kTrig && !p.trig) part[2 * threadIdx.x + 1] = trig_record(th);
     }
-    const auto beams = [&](int k, int t) {   // records of chunk k's beams, thread t of 64 or more
+    const auto beams = [&](int k, int t) {   // records of chunk k's beams, thread t of 64
         for (int j = t; j < min(C, na - k * C); j += 64) {
             const float an = __ldg(angles + k * C + j);
             ang[(k & 1) * C + j] = an;
@@ -1063,6 +1102,7 @@ k_fused_wide(CastParams p, SensorDev sm, const float* __restrict__ ins, const fl
                 d = KIND == K_RM ? rm_cast<LAYOUT, PF>(p.map, p.mr, pose.x, pose.y, c, s)
                                  : bl_cast(p.map, p.mr, pose.x, pose.y, c, s, p.err);
             }
+            if (ranges) ranges[(size_t)(first + li) * na + k * C + a] = d;
             const int bin = sensor_bin(d, sm.K, p.err);
             if (FACTORS)
                 reinterpret_cast<double*>(bins)[((k & 1) * P + li) * C + a] =
@@ -1073,6 +1113,17 @@ k_fused_wide(CastParams p, SensorDev sm, const float* __restrict__ ins, const fl
         __syncthreads();   // the chunk's bins and the next chunk's records are written
     }
     if (threadIdx.x < 32 && lane < np) weights[first + lane] = w;
+}
+
+template <int KIND, int LAYOUT, int PF, bool FACTORS>
+__global__ void __launch_bounds__(kWideThreads, KIND == K_CDDT ? 4 : 8)
+k_fused_wide(CastParams p, SensorDev sm, const float* __restrict__ ins, const float* __restrict__ angles,
+             const float* __restrict__ obs, double* __restrict__ weights, int n, int na, int P, int C) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ unsigned s_next[2];
+    const int first = blockIdx.x * P;
+    wide_tile<KIND, LAYOUT, PF, FACTORS>(p, sm, ins, angles, obs, nullptr, weights, first, min(P, n - first), na, P, C,
+                                         smem_raw, s_next);
 }
 
 // ------------------------------------------------- persistent multi-filter
@@ -1114,7 +1165,7 @@ __device__ __forceinline__ RmRay rm_ray_start(const FilterDev& F, int i, int a, 
     const float4 pose = __ldg(F.part_rec + 2 * (size_t)i), pt = __ldg(F.part_rec + 2 * (size_t)i + 1);
     float c, s;
     ray_direction(F.p.trig, (long long)i * F.na + a, pose.z, __ldg(F.angles + a), pt, __ldg(F.beam_rec + a), c, s);
-    return RmRay{pose.x, pose.y, c, s, 0.0f, -1.0f, 0, r};
+    return RmRay{pose.x, pose.y, c, s, 0.0f, -1.0f, r, 0};
 }
 
 // A tile's rays in a ray-marching batch, with a march budget.  A warp takes 32 rays at a time;
@@ -1244,10 +1295,48 @@ __global__ void __launch_bounds__(512, 4) k_batch(const FilterDev* __restrict__ 
 }
 
 
+// The ray-marching batch without a schedule: every block draws tiles of the device queue and takes
+// each through all its beams like the wide fused update, products included, so that a run is one
+// launch and holds no bins (the separate products of k_batch were a fifth of its step: 179 of 690
+// us, 8 filters).  Tiles of 4 to 16 particles (batch_wide_tile): fewer share each FP64 multiply with
+// fewer lanes, more leave blocks without a tile at the end -- 8 filters, 46,730 particles, us at
+// 4 / 8 / 12 / 16 / 20: 839 / 641 / 589 / 575 / 621; 3 filters, 11,049: 298 / 319 / 313 / 382.  A march
+// budget as in k_batch loses here (651 against 575 us): its rays would have to be finished at every
+// chunk.
+constexpr int kBatchWideBeams = 128;   // a chunk's beams (64 / 96 / 128 / 192 at 16 particles: 619 / 585 / 575 / 604 us)
+
+template <int LAYOUT, bool FACTORS>
+__global__ void __launch_bounds__(kWideThreads, 8) k_batch_wide(const FilterDev* __restrict__ filters, int nf,
+                                                               unsigned total_tiles, unsigned* __restrict__ queue, int C) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ unsigned s_next[2], s_tile;
+    __shared__ int s_f;
+    for (;;) {
+        if (threadIdx.x == 0) {
+            const unsigned t = atomicAdd(queue, 1u);
+            s_tile = t;
+            int lo = 0, hi = nf - 1;   // last filter with tile_begin <= t
+            while (lo < hi) {
+                const int mid = (lo + hi + 1) >> 1;
+                if (filters[mid].tile_begin <= t) lo = mid; else hi = mid - 1;
+            }
+            s_f = lo;
+        }
+        __syncthreads();
+        const unsigned t = s_tile;
+        if (t >= total_tiles) break;
+        const FilterDev& F = filters[s_f];
+        const int first = (int)(t - F.tile_begin) * F.ppb;
+        wide_tile<K_RM, LAYOUT, 0, FACTORS>(F.p, F.sm, F.ins, F.angles, F.obs, F.ranges, F.weights, first,
+                                            min(F.ppb, F.n - first), F.na, F.ppb, C, smem_raw, s_next);
+        __syncthreads();   // s_tile, s_f and the tile's memory may be reused
+    }
+}
+
 // Products of every particle of the batch in one launch after the cast (the
 // alternative to k_batch's overlapped products): one thread per particle,
 // 32 particles per warp, the bins read back from global memory.
-__global__ void __launch_bounds__(64) k_batch_products(const FilterDev* __restrict__ filters, int nf,
+__global__ void __launch_bounds__(256) k_batch_products(const FilterDev* __restrict__ filters, int nf,
                                                         unsigned total_particles) {
     const unsigned g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= total_particles) return;
@@ -1729,7 +1818,8 @@ cudaError_t launch_glt_build(const MapDev& map, float mr, unsigned td, const flo
                              float limits_div_max, uint16_t* lut, cudaStream_t s) {
     const long long total = (long long)map.W * map.H * td;
     if (total <= 0) return cudaSuccess;
-    k_glt_build<<<blocks_for(total, 256), 256, 0, s>>>(map, mr, td, cosv, sinv, limits_div_max, lut, total);
+    const auto kernel = map.step ? k_glt_build<DT_STEP> : k_glt_build<DT_LINEAR>;
+    kernel<<<blocks_for(total, 256), 256, 0, s>>>(map, mr, td, cosv, sinv, limits_div_max, lut, total);
     return cudaGetLastError();
 }
 
@@ -1744,6 +1834,36 @@ cudaError_t launch_cddt_radial(const CastParams& p, const float* ins, const floa
     const long long total = (long long)n * A;
     if (total <= 0 || num_rays <= 0) return cudaSuccess;
     k_cddt_radial<<<blocks_for(total, 256), 256, 0, s>>>(p, ins, angles, outs, n, num_rays, mp, off, A);
+    return cudaGetLastError();
+}
+
+// particles per tile of a wide batch of `particles` in all
+int batch_wide_tile(long long particles, int sms) {
+    const long long slots = 8ll * sms;
+    const long long fine = (particles + slots / 2 - 1) / (slots / 2), coarse = (particles + slots * 5 / 2 - 1) / (slots * 5 / 2);
+    return (int)max(min(fine, 4ll), min(coarse, 16ll));
+}
+
+typedef void (*BatchWideKernel)(const FilterDev*, int, unsigned, unsigned*, int);
+static BatchWideKernel batch_wide_kernel(int layout, int tile, int* smem) {
+    const bool factors = tile <= 4;   // as in the wide fused update: a short tile's product chain is alone
+    *smem = wide_smem(tile, kBatchWideBeams, factors).total;
+    if (layout == DT_RUNS) return factors ? k_batch_wide<DT_RUNS, true> : k_batch_wide<DT_RUNS, false>;
+    return factors ? k_batch_wide<DT_STEP, true> : k_batch_wide<DT_STEP, false>;
+}
+
+cudaError_t batch_wide_occupancy(int layout, int tile, int* blocks_per_sm) {
+    int smem;
+    const BatchWideKernel k = batch_wide_kernel(layout, tile, &smem);
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k, kWideThreads, smem);
+}
+
+cudaError_t launch_batch_wide(const FilterDev* d_filters, int nf, unsigned total_tiles, unsigned* queue, int grid,
+                              int layout, int tile, cudaStream_t s) {
+    if (total_tiles == 0 || nf == 0) return cudaSuccess;
+    int smem;
+    const BatchWideKernel k = batch_wide_kernel(layout, tile, &smem);
+    k<<<grid, kWideThreads, smem, s>>>(d_filters, nf, total_tiles, queue, kBatchWideBeams);
     return cudaGetLastError();
 }
 
@@ -1777,7 +1897,7 @@ cudaError_t launch_batch(const FilterDev* d_filters, int nf, unsigned total_tile
     k<<<grid, block, smem, s>>>(d_filters, nf, total_tiles, queue);
     e = cudaGetLastError();
     if (e != cudaSuccess || !separate || total_particles == 0) return e;
-    k_batch_products<<<blocks_for(total_particles, 64), 64, 0, s>>>(d_filters, nf, total_particles);
+    k_batch_products<<<blocks_for(total_particles, 256), 256, 0, s>>>(d_filters, nf, total_particles);
     return cudaGetLastError();
 }
 

@@ -44,7 +44,9 @@ struct MapDev {
     const float* dt;          // distance transform (DT_LINEAR / DT_TILED; linear for DT_U16)
     const uint16_t* dt16;     // compact squared distances (DT_U16)
     const uint8_t* dt8;       // 8-bit squared distances (DT_STAGED windows)
-    const float* step;        // march step per cell, max(dt * 0.999, 1), 0 on occupied cells (DT_STEP, DT_RUNS)
+    // march step per cell, max(dt * 0.999, 1), NaN on occupied cells, in a (W + 1) x (H + 1) grid whose
+    // last row and column are +inf (DT_STEP, DT_RUNS); null where that grid's index needs more than 32 bits
+    const float* step;
     // DT_RUNS: per cell, how many consecutive cells after it have the same step value, along +y,
     // -y, +x and -x (bits 0-7, 8-15, 16-23, 24-31; at most 255)
     const uint32_t* runs;
@@ -95,10 +97,11 @@ struct SensorDev {
 // ---- map preprocessing (rlc_map.cu) ----
 // rows: occ[y * W + x], else occ[x * H + y]
 cudaError_t launch_pack_bits(const uint8_t* d_occ, int W, int H, bool rows, uint64_t* d_bits, cudaStream_t s);
-// the distance transform's device arrays: the linear floats, and (all or none) the derived layouts
+// the distance transform's device arrays: the linear floats, and (all but step, or none) the derived
+// layouts
 struct DtOut {
     float* dt = nullptr;         // [W * H]
-    float* step = nullptr;       // [W * H]
+    float* step = nullptr;       // [step_map_cells(W, H)], null where that is 0
     float* tiled = nullptr;      // [ceil(W / 8) * tiles_y * 64], as u16 and u8
     uint16_t* u16 = nullptr;
     uint8_t* u8 = nullptr;
@@ -110,6 +113,8 @@ size_t edt_scratch_bytes(int W, int H);
 constexpr size_t edt_scratch_bound(size_t cells, size_t side) {
     return ((cells * 4 + 255) & ~(size_t)255) + cells * 4 + (cells + side) * 8 + 256;
 }
+// cells of the step map, 0 where their 32-bit index does not reach
+size_t step_map_cells(int W, int H);
 // equal-step run lengths of the step map along both axes (MapDev::runs); d_eq: step_eq_words scratch
 size_t step_eq_words(int W, int H);
 cudaError_t launch_step_runs(const float* d_step, int W, int H, uint32_t* d_eq, uint32_t* d_runs, cudaStream_t s);
@@ -217,6 +222,12 @@ inline size_t cddt_zeros_bytes(size_t nz) { return ((nz + 7) / 8 + (nz == 0)) * 
 cudaError_t launch_batch(const FilterDev* d_filters, int nf, unsigned total_tiles, unsigned* queue, int grid,
                          int block, size_t smem, bool rm_only, int layout, int pf, bool separate,
                          unsigned total_particles, cudaStream_t s);
+// The same with the products inside the launch (ray marching on the step map or its runs; the filters'
+// bins and records are not used): tiles of batch_wide_tile particles, at most 32.
+int batch_wide_tile(long long particles, int sms);
+cudaError_t batch_wide_occupancy(int layout, int tile, int* blocks_per_sm);
+cudaError_t launch_batch_wide(const FilterDev* d_filters, int nf, unsigned total_tiles, unsigned* queue, int grid,
+                              int layout, int tile, cudaStream_t s);
 // dynamic shared memory of a batch launch (the ray-marching kernel's per-warp slots of handed-on rays)
 size_t batch_smem(int block, bool rm_only);
 cudaError_t batch_occupancy(int block, size_t smem, bool rm_only, int layout, int pf, bool separate,

@@ -529,7 +529,8 @@ __global__ void __launch_bounds__(256) k_edt_block_min(const uint16_t* __restric
 //  * u16: d^2 in 8x8 tiles, 4x4 cells per 32-byte sector, u8: d^2 in 8x8 tiles of 64 bytes; all
 //    ones = "read the float" (and in the padding).  dt = sqrtf(D) of an integer D, and for D <
 //    2^16 the float product dt * dt is within 0.02 of it;
-//  * step: the march step max(dt * 0.999, 1) of RangeLib.h:957, 0 on occupied cells.
+//  * step: the march step max(dt * 0.999, 1) of RangeLib.h:957, NaN on occupied cells, in a grid
+//    with one more row and column of +inf (what a march off the grid reads).
 __device__ __forceinline__ void store_layouts(const DtOut& o, int W, int H, int TY, int x, int y, float dt) {
     const bool in = x < W && y < H;
     const size_t tile = ((size_t)(x >> 3) * TY + (y >> 3)) << 6;
@@ -537,8 +538,14 @@ __device__ __forceinline__ void store_layouts(const DtOut& o, int W, int H, int 
     if (in) {
         const size_t i = (size_t)x * H + y;
         o.dt[i] = dt;
-        const float v = __fmul_rn(dt, 0.999f);
-        o.step[i] = dt <= 0.0f ? 0.0f : (v < 1.0f ? 1.0f : v);
+        if (o.step) {
+            const float v = __fmul_rn(dt, 0.999f), inf = __int_as_float(0x7f800000);
+            float* row = o.step + (size_t)x * (H + 1);
+            row[y] = dt <= 0.0f ? __int_as_float(0x7fc00000) : (v < 1.0f ? 1.0f : v);
+            if (y == H - 1) row[H] = inf;
+            if (x == W - 1) row[H + 1 + y] = inf;
+            if (x == W - 1 && y == H - 1) row[H + 1 + H] = inf;
+        }
     }
     o.tiled[tile + ((x & 7) << 3) + (y & 7)] = in ? dt : 0.0f;
     o.u16[tile + ((((x >> 2) & 1) << 1 | ((y >> 2) & 1)) << 4) + (((x & 3) << 2) | (y & 3))] =
@@ -588,17 +595,18 @@ __global__ void __launch_bounds__(256) k_step_eq(const float* __restrict__ step,
     const int lane = threadIdx.x & 31, XW = (W + 31) >> 5;
     if (w >= (long long)XW * HW) return;
     const int xw = (int)(w / HW), yw = (int)(w - (long long)xw * HW), x0 = xw << 5, y = (yw << 5) + lane;
+    const size_t pitch = (size_t)H + 1;   // of the step map
     const bool in = y < H;
     const float none = __int_as_float(0x7fc00000);   // equal to nothing
     // lane j: the cell before this patch's rows in column x0 + j
-    const float edge = yw > 0 && x0 + lane < W ? __ldg(step + (size_t)(x0 + lane) * H + (yw << 5) - 1) : none;
-    float prev = in && x0 > 0 ? __ldg(step + (size_t)(x0 - 1) * H + y) : none;
+    const float edge = yw > 0 && x0 + lane < W ? __ldg(step + (x0 + lane) * pitch + (yw << 5) - 1) : none;
+    float prev = in && x0 > 0 ? __ldg(step + (x0 - 1) * pitch + y) : none;
     uint32_t mx = 0, my = 0;
 #pragma unroll
     for (int j0 = 0; j0 < 32; j0 += 8) {
         float v[8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) v[j] = in && x0 + j0 + j < W ? __ldg(step + (size_t)(x0 + j0 + j) * H + y) : none;
+        for (int j = 0; j < 8; ++j) v[j] = in && x0 + j0 + j < W ? __ldg(step + (x0 + j0 + j) * pitch + y) : none;
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
             float left = __shfl_up_sync(0xffffffffu, v[j], 1);
@@ -704,7 +712,7 @@ cudaError_t launch_edt(const uint64_t* d_bits, int W, int H, int TY, const DtOut
                        size_t scratch_bytes, cudaStream_t s) {
     if (W <= 0 || H <= 0) return cudaSuccess;
     if (scratch_bytes < edt_scratch_bytes(W, H)) return cudaErrorInvalidValue;
-    const bool all = o.step != nullptr;
+    const bool all = o.tiled != nullptr;
     char* base = static_cast<char*>(scratch);
     if (W <= kEdtIntSide && H <= kEdtIntSide) {
         uint16_t* g = reinterpret_cast<uint16_t*>(base);
@@ -744,6 +752,11 @@ cudaError_t launch_edt(const uint64_t* d_bits, int W, int H, int TY, const DtOut
     if (e != cudaSuccess || !all) return e;
     k_dt_layouts<<<blocks_for((long long)((W + 7) >> 3) * TY * 64, 256), 256, 0, s>>>(o.dt, W, H, TY, o);
     return cudaGetLastError();
+}
+
+size_t step_map_cells(int W, int H) {
+    const unsigned long long cells = ((unsigned long long)W + 1) * ((unsigned long long)H + 1);
+    return cells < (1ull << 32) ? (size_t)cells : 0;
 }
 
 size_t step_eq_words(int W, int H) {

@@ -911,6 +911,8 @@ struct LearnedModel {
     float* y = nullptr;
     float* dy = nullptr;
     float* loss = nullptr;
+    float* ray_xyt = nullptr;          // the rays of a training step [cap x 3] and their targets
+    float* ray_t = nullptr;
     uint32_t* free_cells = nullptr;
     uint32_t n_free = 0;
     // query buffers (rays of one learned call)
@@ -938,8 +940,8 @@ struct LearnedModel {
         cudaFree(dZ[0]); cudaFree(dZ[1]);
         cudaFree(XT); cudaFree(dZT); cudaFree(wbfT);
         for (int l = 0; l < kLayers - 1; ++l) { cudaFree(HT[l]); HT[l] = nullptr; }
-        cudaFree(y); cudaFree(dy); cudaFree(loss);
-        X = nullptr; dZ[0] = dZ[1] = nullptr; y = dy = loss = nullptr;
+        cudaFree(y); cudaFree(dy); cudaFree(loss); cudaFree(ray_xyt); cudaFree(ray_t);
+        X = nullptr; dZ[0] = dZ[1] = nullptr; y = dy = loss = ray_xyt = ray_t = nullptr;
         XT = dZT = wbfT = nullptr;
         cap = 0;
     }
@@ -967,6 +969,8 @@ struct LearnedModel {
         TRY(cudaMalloc(&y, (size_t)rows * sizeof(float)));
         TRY(cudaMalloc(&dy, (size_t)rows * sizeof(float)));
         TRY(cudaMalloc(&loss, sizeof(float)));
+        TRY(cudaMalloc(&ray_xyt, (size_t)rows * 3 * sizeof(float)));
+        TRY(cudaMalloc(&ray_t, (size_t)rows * sizeof(float)));
         cap = rows;
         return cudaSuccess;
     }
@@ -1254,9 +1258,8 @@ int rlc_learned_train(rlc_learned* L, int steps, int batch, float lr, unsigned s
     LearnedModel& M = L->m;
     cudaStream_t s = (cudaStream_t)stream;
     LTRY(M.ensure(batch), "train buffers");
-    float *xyt = nullptr, *tt = nullptr;
-    LTRY(cudaMalloc(&xyt, (size_t)batch * 3 * sizeof(float)), "train buffers");
-    cudaError_t e = cudaMalloc(&tt, (size_t)batch * sizeof(float));
+    float *xyt = M.ray_xyt, *tt = M.ray_t;   // kept: two allocations and frees a call cost up to 150 us
+    cudaError_t e = cudaSuccess;
     float loss_acc = 0.0f;
     int loss_n = 0;
     for (int st = 0; st < steps && e == cudaSuccess; ++st) {
@@ -1282,8 +1285,6 @@ int rlc_learned_train(rlc_learned* L, int steps, int batch, float lr, unsigned s
         }
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    cudaFree(xyt);
-    cudaFree(tt);
     if (e != cudaSuccess) return lfail(RLC_ERR_CUDA, "training", e);
     unsigned err = 0;
     LTRY(cudaMemcpy(&err, M.err, sizeof(unsigned), cudaMemcpyDeviceToHost), "training");

@@ -84,3 +84,55 @@ def test_wide_fused_update(rl, oracle_mod, kind, n, na):
         ref.set_sensor_model(table)
         exp = ref.calc_range_repeat_angles_eval_sensor_model(ins, angles, obs, nthreads=NT)
         assert np.array_equal(_bits(w), _bits(exp))
+
+
+@pytest.mark.parametrize("scale", [1, 40])   # a few particles per tile, and 16
+def test_wide_batch(rl, oracle_mod, scale):
+    """A batch without a schedule against per-filter calls: tiles of 2 to 16 particles, chunks with one
+    beam, filters without particles or beams, poses off the map, ranges kept, cos/sin given."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(70 + scale)
+    filters, host = [], []
+    sizes = [(700, 129), (1, 300), (33, 1), (0, 50), (5, 0), (900, 128), (1300, 61)]
+    for k, (n, na) in enumerate(sizes):
+        n *= scale
+        mr = 50.0 + 9 * k
+        occ = np.ascontiguousarray(W.rect_disk_map(256, 80 + k)[:, :200 + k])
+        m = rl.PyOMap(np.ascontiguousarray(occ.T))
+        g = rl.PyRayMarching(m, mr)
+        table = W.sensor_table(int(mr) + 1) ** 0.1
+        g.set_sensor_model(table)
+        ins = np.empty((n, 3), np.float32)
+        ins[:, 0], ins[:, 1] = rng.uniform(-5, 210, n), rng.uniform(-5, 260, n)
+        ins[:, 2] = rng.uniform(-7, 7, n)
+        ins[::97, 2] = np.nan
+        angles = W.laser_angles(na) if na else np.zeros(0, np.float32)
+        obs = rng.uniform(0, mr, na).astype(np.float32)
+        if k == 5:
+            g.set_trig_override(oracle_mod.world_rays(m.world, ins, angles)[1])
+        t = [torch.from_numpy(a).cuda() for a in (ins, angles, obs)]
+        filters.append((g, *t, torch.full((n,), -1.0, dtype=torch.float64, device="cuda"),
+                        torch.full((n * na,), -1.0, device="cuda") if k % 2 == 0 else None))
+        host.append((ins, angles, obs, n, na))
+    batch = rl.PyFilterBatch(filters)
+    for _ in range(2):
+        batch.run()
+    torch.cuda.synchronize()
+    assert batch.schedule() == (0, 0, 256, 0) and batch.product_mode() == "overlapped"
+    first = [f[4].clone() for f in filters]
+    for f, (ins, angles, obs, n, na) in zip(filters, host):
+        g = f[0]
+        g.set_schedule(0, 0, 0, 0)
+        if n:
+            w = np.empty(n)
+            g.calc_range_repeat_angles_eval_sensor_model(ins, angles, obs, w)
+            assert np.array_equal(_bits(f[4].cpu().numpy()), _bits(w)), (n, na)
+        if f[5] is not None and n and na:
+            r = np.empty(n * na, np.float32)
+            g.calc_range_repeat_angles(ins, angles, r)
+            assert np.array_equal(f[5].cpu().numpy().view(np.uint32), r.view(np.uint32)), (n, na)
+    for separate in (False, True):   # the schedules that a caller can ask for afterwards
+        batch.set_product_mode(separate)
+        batch.run()
+        torch.cuda.synchronize()
+        assert all(torch.equal(a, f[4]) for a, f in zip(first, filters))
