@@ -151,6 +151,8 @@ struct rlc_method {
     float* d_cos = nullptr;
     float* d_sin = nullptr;
     CddtBuild tab;
+    CddtIndex index;
+    unsigned table_gen = 0;   // counts the tables of this method (a batch holds their device pointers)
     // GiantLUTCast
     uint16_t* d_lut = nullptr;
     float max_div_limits = 0.0f, limits_div_max = 0.0f;
@@ -187,6 +189,7 @@ struct rlc_method {
         cudaFree(tab.slice_base);
         cudaFree(tab.bin_start);
         cudaFree(tab.zeros);
+        cddt_index_free(&index);
         cudaFree(d_table);
         cudaFree(d_stage);
         cudaFree(d_err);
@@ -223,10 +226,20 @@ struct rlc_method {
         p.glt.max_div_limits = max_div_limits;
         p.cddt.bin_start = tab.bin_start;
         p.cddt.zeros = tab.zeros;
+        p.cddt.slices = index.slices;
+        p.cddt.index = index.index;
+        p.cddt.qz = index.qz;
         p.world = world;
         p.trig = d_trig;
         p.err = d_err;
         return p;
+    }
+
+    // the index of the current CDDT table
+    cudaError_t build_index() {
+        ++table_gen;
+        return cddt_index_build(tab, map->W, map->H, td, h_widths.data(), h_trans.data(), h_cos.data(), h_sin.data(),
+                                h_slice_base.data(), &index, 0);
     }
 
     int stage(size_t bytes, void** out) {
@@ -369,6 +382,10 @@ int cast_layout(const rlc_method* m, long long rays, bool independent) {
     if (!m->pick || m->dkind != K_RM) return cast_layout(m);
     return map_layout(m->map, independent || (rays >= (1ll << 14) && rays < (1ll << 18)) ? DT_RUNS : DT_STEP);
 }
+
+// search of a CDDT method's queries (the prefetch schedule) or prefetch of a ray-marching one:
+// without a schedule, CDDT queries go by the table's index where it has one
+int cast_search(const rlc_method* m) { return m->pick && m->dkind == K_CDDT && m->index.index ? 3 : m->prefetch; }
 
 // layout of a fused call.  Without a schedule, ray marching takes the step map, with its equal-step
 // runs while the call waits for its longest rays and not for its products: 4,000 x 61 linear / step /
@@ -566,6 +583,7 @@ static int method_create(rlc_map* map, int kind, float max_range, unsigned td, c
                            m->d_sin, &m->tab, 0);
             if (e != cudaSuccess) rc = cuda_fail(e, "CDDT prune");
         }
+        if (!rc && (e = m->build_index()) != cudaSuccess) rc = cuda_fail(e, "CDDT index");
     }
     if (rc) {
         delete m;
@@ -615,6 +633,7 @@ int rlc_cddt_prune(rlc_method* m, float max_range) {
     if (m->dkind != K_CDDT) return fail(RLC_ERR_STATE, "prune applies to CDDT methods");
     cudaError_t e = cddt_prune(m->map->d_bits, m->map->W, m->map->H, m->map->TY, m->td, max_range, m->d_widths,
                                m->d_trans, m->d_cos, m->d_sin, &m->tab, 0);
+    if (e == cudaSuccess) e = m->build_index();
     return finish_launch(e, "CDDT prune");
 }
 
@@ -677,6 +696,7 @@ int rlc_cddt_table_load(rlc_method* m, const float* trans, const int64_t* bin_le
     m->tab.nzeros = (uint32_t)num_zeros;
     std::memcpy(m->h_trans.data(), trans, m->td * sizeof(float));
     CUDA_OR_FAIL(cudaMemcpy(m->d_trans, trans, m->td * sizeof(float), cudaMemcpyHostToDevice), "CDDT load");
+    CUDA_OR_FAIL(m->build_index(), "CDDT load");
     return RLC_OK;
 }
 
@@ -798,9 +818,9 @@ int rlc_calc_range_many(rlc_method* m, const float* ins, float* outs, int n, uns
     CastParams p = m->params();
     bool world = !(flags & RLC_NO_WORLD);
     if (flags & RLC_DEVICE_PTRS)
-        return finish_launch(launch_calc_range_many(p, cast_layout(m, n, true), m->prefetch, world, ins, outs, n, s), "calc_range_many");
+        return finish_launch(launch_calc_range_many(p, cast_layout(m, n, true), cast_search(m), world, ins, outs, n, s), "calc_range_many");
     if (host_direct()) {
-        CUDA_OR_FAIL(launch_calc_range_many(p, cast_layout(m, n, true), m->prefetch, world, ins, outs, n, s), "calc_range_many");
+        CUDA_OR_FAIL(launch_calc_range_many(p, cast_layout(m, n, true), cast_search(m), world, ins, outs, n, s), "calc_range_many");
         CUDA_OR_FAIL(cudaStreamSynchronize(s), "calc_range_many");
         return RLC_OK;
     }
@@ -810,7 +830,7 @@ int rlc_calc_range_many(rlc_method* m, const float* ins, float* outs, int n, uns
     float* d_in = (float*)st;
     float* d_out = (float*)((char*)st + bin);
     CUDA_OR_FAIL(cudaMemcpyAsync(d_in, ins, (size_t)n * 3 * sizeof(float), cudaMemcpyHostToDevice, s), "H2D");
-    CUDA_OR_FAIL(launch_calc_range_many(p, cast_layout(m, n, true), m->prefetch, world, d_in, d_out, n, s), "calc_range_many");
+    CUDA_OR_FAIL(launch_calc_range_many(p, cast_layout(m, n, true), cast_search(m), world, d_in, d_out, n, s), "calc_range_many");
     CUDA_OR_FAIL(cudaMemcpyAsync(outs, d_out, (size_t)n * sizeof(float), cudaMemcpyDeviceToHost, s), "D2H");
     CUDA_OR_FAIL(cudaStreamSynchronize(s), "calc_range_many");
     return RLC_OK;
@@ -827,9 +847,9 @@ int rlc_calc_range_repeat_angles(rlc_method* m, const float* ins, const float* a
     cudaStream_t s = (cudaStream_t)stream;
     CastParams p = m->params();
     if (flags & RLC_DEVICE_PTRS)
-        return finish_launch(launch_repeat_angles(p, cast_layout(m, (long long)n * na, false), m->prefetch, ins, angles, outs, n, na, s), "repeat_angles");
+        return finish_launch(launch_repeat_angles(p, cast_layout(m, (long long)n * na, false), cast_search(m), ins, angles, outs, n, na, s), "repeat_angles");
     if (host_direct()) {
-        CUDA_OR_FAIL(launch_repeat_angles(p, cast_layout(m, (long long)n * na, false), m->prefetch, ins, angles, outs, n, na, s), "repeat_angles");
+        CUDA_OR_FAIL(launch_repeat_angles(p, cast_layout(m, (long long)n * na, false), cast_search(m), ins, angles, outs, n, na, s), "repeat_angles");
         CUDA_OR_FAIL(cudaStreamSynchronize(s), "repeat_angles");
         return RLC_OK;
     }
@@ -842,7 +862,7 @@ int rlc_calc_range_repeat_angles(rlc_method* m, const float* ins, const float* a
     float* d_out = (float*)((char*)st + b0 + b1);
     CUDA_OR_FAIL(cudaMemcpyAsync(d_in, ins, (size_t)n * 3 * sizeof(float), cudaMemcpyHostToDevice, s), "H2D");
     CUDA_OR_FAIL(cudaMemcpyAsync(d_ang, angles, (size_t)na * sizeof(float), cudaMemcpyHostToDevice, s), "H2D");
-    CUDA_OR_FAIL(launch_repeat_angles(p, cast_layout(m, (long long)n * na, false), m->prefetch, d_in, d_ang, d_out, n, na, s), "repeat_angles");
+    CUDA_OR_FAIL(launch_repeat_angles(p, cast_layout(m, (long long)n * na, false), cast_search(m), d_in, d_ang, d_out, n, na, s), "repeat_angles");
     CUDA_OR_FAIL(cudaMemcpyAsync(outs, d_out, (size_t)n * na * sizeof(float), cudaMemcpyDeviceToHost, s), "D2H");
     CUDA_OR_FAIL(cudaStreamSynchronize(s), "repeat_angles");
     return RLC_OK;
@@ -960,7 +980,7 @@ static int fused_device(rlc_method* m, const float* ins, const float* angles, co
         return finish_launch(launch_fused_staged(p, sm, ins, angles, obs, w, n, na, m->tile, m->d_bins, s),
                              "fused sensor model (staged)");
     }
-    return finish_launch(launch_fused(p, fused_layout(m, n, na), m->prefetch, sm, ins, angles, obs, w, n, na,
+    return finish_launch(launch_fused(p, fused_layout(m, n, na), cast_search(m), sm, ins, angles, obs, w, n, na,
                                       m->fused_block, m->tile, m->pick, s),
                          "fused sensor model");
 }
@@ -1228,7 +1248,8 @@ struct rlc_batch {
     cudaStream_t cap = nullptr;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
-    std::vector<const float*> trig_seen;   // each method's trig override when the table was built
+    // each method's trig override and CDDT table when the device table was built
+    std::vector<std::pair<const float*, unsigned>> seen;
 
     void drop_graph() {
         if (exec) cudaGraphExecDestroy(exec);
@@ -1320,8 +1341,8 @@ struct rlc_batch {
             it.cost = (double)it.f.ppb * (d.n_angles > 0 ? d.n_angles : 1) * (double)(m->mr > 1.0f ? m->mr : 1.0f);
             items.push_back(it);
         }
-        trig_seen.clear();
-        for (const rlc_filter_desc& d : descs) trig_seen.push_back(d.method->d_trig);
+        seen.clear();
+        for (const rlc_filter_desc& d : descs) seen.emplace_back(d.method->d_trig, d.method->table_gen);
         std::stable_sort(items.begin(), items.end(), [](const Item& a, const Item& b) { return a.cost > b.cost; });
         unsigned long long tiles = 0, parts = 0;
         std::vector<FilterDev> hf;
@@ -1359,11 +1380,11 @@ struct rlc_batch {
     // queue reset + persistent kernel, captured once as a CUDA graph
     int launch(cudaStream_t stream) {
         if (total_tiles == 0) return RLC_OK;
-        // a method whose trig override was set or cleared since the build: the device table holds
-        // the old (freed) override, so rebuild it (and the graph) first
+        // a method whose trig override was set or cleared, or whose CDDT table was pruned or loaded, since
+        // the build: the device table holds the old (freed) one, so rebuild it (and the graph) first
         for (size_t i = 0; i < descs.size(); ++i) {
             const rlc_method* m = descs[i].method;
-            if (i < trig_seen.size() && m->d_trig == trig_seen[i]) continue;
+            if (i < seen.size() && seen[i] == std::make_pair((const float*)m->d_trig, m->table_gen)) continue;
             if (m->d_trig && m->trig_count < (long long)descs[i].n_particles * descs[i].n_angles)
                 return fail(RLC_ERR_ARG, "filter %d: trig override too short", (int)i);
             if (int rc = build()) return rc;

@@ -35,6 +35,28 @@ constexpr float kMPiUpF = 0x1.921fb6p+1f;
 // all 8,388,608 floats of the interval (tests/test_float_identities.py).
 constexpr float kMPiHiF = 0x1.921fb6p+1f;     // (float)M_PI
 constexpr float kMPiLoF = -0x1.777a5cp-24f;   // (float)(M_PI - kMPiHiF)
+// (float)((double)t + M_2PI) for every float t in [-16, -2^-16] at least 2^-10 from -M_2PI, and
+// (float)((double)t - M_2PI) for every float t in (M_2PI, 64], from float operations alone: t +- kM2PiHiF as an exact pair, the low
+// part of the constant added to its error, one rounding -- checked for all floats of both intervals
+// (tests/test_cddt_index.py).  In double they kept
+// the FP64 pipe 43 % busy through 1 M GiantLUTCast queries (26.7 -> 25.0 us).
+constexpr float kM2PiHiF = 0x1.921fb6p+2f;    // (float)M_2PI
+constexpr float kM2PiLoF = -0x1.777a22p-23f;  // (float)(M_2PI - kM2PiHiF)
+
+// (out of line: the compiler would run the doubles beside the floats and select)
+__device__ __noinline__ float add_2pi_double(float t) { return __double2float_rn(__dadd_rn((double)t, kM2Pi)); }
+__device__ __noinline__ float sub_2pi_double(float t) { return __double2float_rn(__dsub_rn((double)t, kM2Pi)); }
+__device__ __forceinline__ float add_2pi(float t) {
+    const rlc_trig::F2 s = rlc_trig::two_sum(t, kM2PiHiF);
+    if (t >= -16.0f && t <= -0x1p-16f && fabsf(s.h) >= 0x1p-10f) return __fadd_rn(s.h, __fadd_rn(s.l, kM2PiLoF));
+    return add_2pi_double(t);
+}
+__device__ __forceinline__ float sub_2pi(float t) {   // t > kM2PiDownF
+    const rlc_trig::F2 s = rlc_trig::two_sum(t, -kM2PiHiF);
+    if (t <= 64.0f) return __fadd_rn(s.h, __fsub_rn(s.l, kM2PiLoF));
+    return sub_2pi_double(t);
+}
+
 constexpr int kPrefetch = 8;                        // RM prefetch distance (px) of the prefetching schedule
 constexpr int kAnyKind = -1;                        // k_batch: kind, layout and prefetch chosen per filter
 constexpr int kRmOnly = -2;                         // k_batch: every filter ray-marches (LAYOUT, PF given)
@@ -349,12 +371,12 @@ __device__ __forceinline__ void cddt_discretize(const CddtDev& c, float theta, i
     if (theta < 0.0f) {
         while (theta < 0.0f) {
             if (++it > kMaxWrap) { atomicOr(err, F_WRAP_BOUND); break; }
-            theta = __double2float_rn(__dadd_rn((double)theta, kM2Pi));
+            theta = add_2pi(theta);
         }
     } else if (theta > kM2PiDownF) {
         while (theta > kM2PiDownF) {
             if (++it > kMaxWrap) { atomicOr(err, F_WRAP_BOUND); break; }
-            theta = __double2float_rn(__dsub_rn((double)theta, kM2Pi));
+            theta = sub_2pi(theta);
         }
     }
     bool fl = false;
@@ -368,7 +390,8 @@ __device__ __forceinline__ void cddt_discretize(const CddtDev& c, float theta, i
         rounded = 0;
         fl = !fl;
     }
-    binned = (int)((unsigned)rounded % c.td);
+    // within [0, td) but after a bounded wrap: the remainder's ~20 instructions only there
+    binned = (unsigned)rounded < c.td ? rounded : (int)((unsigned)rounded % c.td);
     flipped = fl;
 }
 
@@ -531,6 +554,80 @@ __device__ float cddt_cast(const CastParams& p, float x, float y, float heading)
                                     : bound_g(q.bin, q.n, q.lx, upper));
 }
 
+// A query by the table's index (CddtDev::index; schedules that name a search keep theirs).  The
+// index holds, for every bin and every kCddtBucket pixels along it, where in the query's copy of the
+// zero points (CddtDev::qz: per bin -inf, the zero points, +inf up to a whole quad) those at or past
+// the bucket's start begin.  Bucket numbers are a monotone function of the position, so the bound
+// lies between the bucket's start and the next one's whatever that function rounds.  A query reads
+// the slice's two records (L1), one index entry and a quad or two of zero points, in which it keeps
+// the last value not past lx and the first past it without branches: 3 dependent reads and ~5
+// scattered requests, against ~10 and ~20 for slice entries, bin bounds, bin ends and a binary
+// search.  1 M queries on 2048^2, td 108: 42 -> 24.5 us (binary search / index; the sector search 39),
+// td 216 48 -> 31, pruned 36 -> 21, 512^2 32 -> 21; 4,000 x 500 beams and their weights 52 -> 46.
+__device__ __forceinline__ float cddt_cast_index(const CastParams& p, float x, float y, float heading) {
+    const CddtDev& c = p.cddt;
+    const float mr = p.mr, inf = __int_as_float(0x7f800000);
+    if (isnan(x) || isnan(y) || isnan(heading)) return mr;
+    const bool occ = (x > -1.0f) && (y > -1.0f) && occ_at(p.map, __float2int_rz(x), __float2int_rz(y));
+    int a;
+    bool fl;
+    cddt_discretize(c, -heading, a, fl, p.err);
+    const float4 g = __ldg(c.slices + 2 * a);                                                 // cos, sin, translation, start
+    const uint4 h = __ldg(reinterpret_cast<const uint4*>(c.slices) + 2 * a + 1);              // width, index base, row, -
+    const float lx = __fsub_rn(__fmul_rn(x, g.x), __fmul_rn(y, g.y));
+    const float ly = __fadd_rn(__fadd_rn(__fmul_rn(x, g.y), __fmul_rn(y, g.x)), g.z);
+    const unsigned li = (unsigned)__float2int_rz(ly);
+    if (li >= h.x || h.z == 0u) return mr;   // off the slice, or a slice without zero points
+    if (!(fabsf(lx) < inf)) return cddt_cast<false>(p, x, y, heading);   // an infinite coordinate
+    const int k = min(max(cddt_bucket(lx, g.w), 0), (int)h.z - 2);
+    const unsigned* e = c.index + (h.y + li * h.z + (unsigned)k);
+    // flipped: the last zero point <= lx (it may precede the bucket), else the first >= lx: the
+    // boundary between the values <= below and those past it
+    const float below = fl ? lx : (lx > 0.0f ? __int_as_float(__float_as_int(lx) - 1)
+                                             : (lx < 0.0f ? __int_as_float(__float_as_int(lx) + 1) : -__int_as_float(1)));
+    unsigned q = (__ldg(e) - (fl ? 1u : 0u)) >> 2;
+    const float4* quads = reinterpret_cast<const float4*>(c.qz);
+    float4 v = __ldg(quads + q);
+    float prev = -inf;
+    if (v.w <= below) {   // the whole quad precedes the boundary
+        prev = v.w;
+        v = __ldg(quads + ++q);
+        if (v.w <= below) {   // a crowded bucket: binary search over the quads up to the next bucket's start
+            unsigned lo = q + 1u, hi = __ldg(e + 1) >> 2;
+            while (lo < hi) {   // first quad whose last value is past the boundary
+                const unsigned mid = (lo + hi) >> 1;
+                if (__ldg(c.qz + 4 * (size_t)mid + 3) <= below) lo = mid + 1; else hi = mid;
+            }
+            q = lo;
+            v = __ldg(quads + q);
+            prev = __ldg(c.qz + 4 * (size_t)q - 1);
+        }
+    }
+    float next = v.w;
+    prev = v.x <= below ? v.x : prev;
+    prev = v.y <= below ? v.y : prev;
+    prev = v.z <= below ? v.z : prev;
+    next = v.z > below ? v.z : next;
+    next = v.y > below ? v.y : next;
+    next = v.x > below ? v.x : next;
+    const float near = fl ? prev : next;
+    if (fabsf(near) == inf) return mr;                                 // flipped: first > lx; else: last < lx
+    if (occ) {   // inside a wall, unless nothing lies beyond (flipped: last < lx, else: first > lx)
+        // (the first zero point follows the -inf that heads its bin, so it is never a quad's first value)
+        if (fl ? !(next == inf && prev < lx) : !(next > lx && prev == -inf && v.x == -inf)) return 0.0f;
+    } else if (!fl && next == lx) {   // on a zero point: bins of more than 65 entries take the next one above it
+        const unsigned b = __ldg(c.slice_base + a) + li;
+        if ((int)(__ldg(c.bin_start + b + 1) - __ldg(c.bin_start + b)) - 1 <= kBinarySearchThreshold) return 0.0f;
+        const float* z = c.qz + 4 * (size_t)q;
+        do next = __ldg(z++); while (next <= lx);
+        if (next == inf) {   // the reference reads past the bin
+            atomicOr(p.err, F_CDDT_PAST_END);
+            return 0.0f;
+        }
+    }
+    return fl ? __fsub_rn(lx, prev) : __fsub_rn(next, lx);
+}
+
 // warp-cooperative variant: every lane resolves its own query up to the bin,
 // then the warp searches the pending bins one query at a time
 __device__ __forceinline__ float cddt_cast_warp(const CastParams& p, bool active, float x, float y, float heading) {
@@ -562,16 +659,16 @@ __device__ __forceinline__ int glt_discretize(const GltDev& g, float theta, unsi
     if (theta < 0.0f) {
         while (theta < 0.0f) {
             if (++it > kMaxWrap) { atomicOr(err, F_WRAP_BOUND); break; }
-            theta = __double2float_rn(__dadd_rn((double)theta, kM2Pi));
+            theta = add_2pi(theta);
         }
     } else if (theta > kM2PiDownF) {
         while (theta > kM2PiDownF) {
             if (++it > kMaxWrap) { atomicOr(err, F_WRAP_BOUND); break; }
-            theta = __double2float_rn(__dsub_rn((double)theta, kM2Pi));
+            theta = sub_2pi(theta);
         }
     }
     const int rounded = __float2int_rz(roundf(__fmul_rn(theta, g.td_div_2pi)));
-    return (int)((unsigned)rounded % g.td);
+    return (unsigned)rounded < g.td ? rounded : (int)((unsigned)rounded % g.td);
 }
 
 // GiantLUTCast::calc_range, RangeLib.h:1869-1881; NaN arguments give max_range
@@ -651,6 +748,7 @@ __global__ void k_cddt_pair(CastParams p, float x, float y, float heading, float
 // ------------------------------------------------------------- dispatch
 template <int KIND, int LAYOUT, int PF = 0>
 __device__ __forceinline__ float cast_one(const CastParams& p, float x, float y, float h, long long ray) {
+    if (KIND == K_CDDT && PF == 3) return cddt_cast_index(p, x, y, h);
     if (KIND == K_CDDT) return cddt_cast<PF == 2>(p, x, y, h);   // PF 2: sector search
     if (KIND == K_GLT) return glt_cast(p, x, y, h);
     float c, s;
@@ -926,6 +1024,7 @@ __device__ __forceinline__ float cast_ray(const CastParams& p, const float* __re
     }
     if (p.kind == K_BL) return cast_one<K_BL, DT_LINEAR, 0>(p, ax, ay, h, ray);
     if (p.kind == K_GLT) return cast_one<K_GLT, DT_LINEAR, 0>(p, ax, ay, h, ray);
+    if (p.cddt.index) return cast_one<K_CDDT, DT_LINEAR, 3>(p, ax, ay, h, ray);
     return cast_one<K_CDDT, DT_LINEAR, 0>(p, ax, ay, h, ray);
 }
 
@@ -1092,7 +1191,7 @@ __device__ __forceinline__ void wide_tile(const CastParams& p, const SensorDev& 
             const float an = ang[(k & 1) * C + a];
             float d;
             if (KIND == K_CDDT) {
-                d = cddt_cast<PF == 2>(p, pose.x, pose.y, __fsub_rn(pose.z, an));
+                d = cast_one<K_CDDT, LAYOUT, PF>(p, pose.x, pose.y, __fsub_rn(pose.z, an), 0);
             } else if (KIND == K_GLT) {
                 d = glt_cast(p, pose.x, pose.y, __fsub_rn(pose.z, an));
             } else {
@@ -1605,6 +1704,7 @@ cudaError_t dispatch(int kind, int layout, int pf, Args... args) {
     if (kind == K_GLT) return F<K_GLT, DT_LINEAR, 0>::run(args...);
     if (pf == 1) return F<K_CDDT, DT_LINEAR, 1>::run(args...);   // warp-cooperative bin search
     if (pf == 2) return F<K_CDDT, DT_LINEAR, 2>::run(args...);   // sector search
+    if (pf == 3) return F<K_CDDT, DT_LINEAR, 3>::run(args...);   // the table's index
     return F<K_CDDT, DT_LINEAR, 0>::run(args...);
 }
 
@@ -1656,13 +1756,16 @@ cudaError_t set_smem(K kernel, size_t bytes) {
 // than the shorter blocks gain.  Ray marching on a 2048^2 corridor map, us per call before / wide:
 // 20,000 x 1,081 1365 / 379, 4,000 x 1,081 329 / 140, 4,000 x 271 88 / 60, 2,000 x 1,081 178 / 107,
 // 2,000 x 300 61 / 48, 6,000 x 150 70 / 51, 2,000 x 150 41 / 35; below the line 1,000 x 1,081
-// 100 / 97, 1,000 x 300 38 / 43, 600 x 150 28 / 30, 20,000 x 61 62 / 68.  CDDT: 8,000 x 1,081
-// 634 / 187, 4,000 x 271 97 / 46.  Bresenham's walks are too uneven for a barrier per chunk (8,000 x
+// 100 / 97, 1,000 x 300 38 / 43, 600 x 150 28 / 30, 20,000 x 61 62 / 68.  Table queries are short, so
+// that the products weigh more: CDDT 8,000 x 1,081 595 / 128, 4,000 x 271 96 / 30, 2,000 x 150
+// 40 / 18, 1,000 x 300 28 / 24, 5,000 x 61 21 / 18; below the line 4,000 x 61 12.6 / 13.6, 8,000 x 35
+// 12.3 / 14.1, 600 x 200 15.3 / 17.1; GLT 20,000 x 200 253 / 39, 8,000 x 61 15.6 / 13.1, 4,000 x 61
+// 11.6 / 13.3.  Bresenham's walks are too uneven for a barrier per chunk (8,000 x
 // 1,081 722 / 869).
 inline bool fused_wide(int kind, int n, int na) {
     const long long rays = (long long)n * na;
-    if (kind == K_BL || n < 2000) return false;
-    return kind == K_RM ? na >= 128 && rays >= (1ll << 18) : na >= 192 && rays >= (1ll << 20);
+    if (kind == K_BL || rays < (1ll << 18)) return false;
+    return kind == K_RM ? na >= 128 && n >= 2000 : na >= 48;
 }
 // Its shape: as few particles per block as keep all blocks resident at once.  Up to kWideFactors
 // particles the rays' threads read the table factors themselves (a lone product chain that reads
@@ -1678,7 +1781,7 @@ struct RunFused {
                            const float* obs, double* w, int n, int na, int block, int tile, bool pick, cudaStream_t s) {
         if (n <= 0) return cudaSuccess;
         // the kernels that a call without a schedule can come to (pick_layout)
-        constexpr bool kPicked = KIND == K_GLT || (KIND == K_CDDT && PF == 0) ||
+        constexpr bool kPicked = KIND == K_GLT || (KIND == K_CDDT && (PF == 0 || PF == 3)) ||
                                  (KIND == K_RM && PF == 0 && (LAYOUT == DT_STEP || LAYOUT == DT_RUNS));
         if constexpr (kPicked) {
             if (pick && fused_wide(KIND, n, na)) {

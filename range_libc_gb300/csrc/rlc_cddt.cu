@@ -17,6 +17,7 @@
 // owns zeros [bin_start[b], bin_start[b+1]).  All offsets are uint32.
 #include "rlc_internal.cuh"
 
+#include <cmath>
 #include <cstdio>
 #include <vector>
 
@@ -354,6 +355,65 @@ __global__ void k_remap_starts(const uint32_t* __restrict__ old_start, const uin
     if (b <= nb) new_start[b] = pos[old_start[b]];
 }
 
+// ------------------------------------------------------------------ index
+// one warp per bin: its zero points after -inf and before +inf, in whole quads, and for every bucket k of its slice where
+// the zero points with a bucket >= k begin; *bad is set by zero points that are not finite and sorted
+struct IndexSlice {   // CddtDev::slices
+    float c, s, trans, v0;
+    uint32_t width, base, row, unused;
+};
+
+// first quad of bin b: at least n + 2 values before the next bin's
+__device__ __forceinline__ size_t index_quad(const uint32_t* start, uint32_t b) { return (size_t)(start[b] >> 2) + 2 * (size_t)b; }
+
+__global__ void __launch_bounds__(256) k_index_fill(const IndexSlice* __restrict__ sl,
+                                                    const uint32_t* __restrict__ slice_base, int td, uint32_t nb,
+                                                    const uint32_t* __restrict__ start, const float* __restrict__ zeros,
+                                                    float* __restrict__ qz, uint32_t* __restrict__ index,
+                                                    unsigned* __restrict__ bad) {
+    const uint32_t b = (uint32_t)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+    const int lane = threadIdx.x & 31;
+    if (b >= nb) return;
+    const uint32_t lo = start[b], n = start[b + 1] - lo;
+    const float* z = zeros + lo;
+    const size_t q0 = index_quad(start, b) * 4, q1 = index_quad(start, b + 1) * 4;
+    float* q = qz + q0;
+    const float inf = __int_as_float(0x7f800000);
+    bool ok = true;
+    for (uint32_t i = lane; i < (uint32_t)(q1 - q0); i += 32) {
+        float v = i == 0 ? -inf : inf;
+        if (i >= 1 && i <= n) {
+            v = z[i - 1];
+            ok = ok && isfinite(v) && (i == 1 || z[i - 2] <= v);
+        }
+        q[i] = v;
+    }
+    if (!ok) *bad = 1u;
+    int s0 = 0, s1 = td - 1;   // the bin's slice: the last with slice_base <= b
+    while (s0 < s1) {
+        const int mid = (s0 + s1 + 1) >> 1;
+        if (slice_base[mid] <= b) s0 = mid; else s1 = mid - 1;
+    }
+    const IndexSlice S = sl[s0];
+    for (uint32_t k = lane; k < S.row; k += 32) {
+        uint32_t i = 0, e = n;
+        if (k + 1 == S.row) i = n;   // the end: the upper sentinel
+        else
+            while (i < e) {   // first zero point whose bucket is >= k (the last bucket holds what lies beyond)
+                const uint32_t mid = (i + e) >> 1;
+                const int bk = min(max(cddt_bucket(z[mid], S.v0), 0), (int)S.row - 2);
+                if (bk >= (int)k) e = mid; else i = mid + 1;
+            }
+        index[S.base + (size_t)(b - slice_base[s0]) * S.row + k] = (uint32_t)q0 + 1 + i;
+    }
+}
+
+__global__ void k_gather_u32(const uint32_t* __restrict__ v, const uint32_t* __restrict__ at, uint32_t n,
+                             uint32_t* __restrict__ out) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) out[i] = v[at[i]];
+}
+
 struct DevBuf {
     void* p = nullptr;
     ~DevBuf() { if (p) cudaFree(p); }
@@ -506,6 +566,70 @@ cudaError_t cddt_build(const uint64_t* d_bits, int W, int H, int TY, unsigned td
     out->zeros = d_zeros;
     out->total_bins = nb;
     out->nzeros = nz;
+    return cudaSuccess;
+}
+
+void cddt_index_free(CddtIndex* ix) {
+    cudaFree(ix->mem);
+    *ix = CddtIndex{};
+}
+
+cudaError_t cddt_index_build(const CddtBuild& tab, int W, int H, unsigned td, const int* h_widths, const float* h_trans,
+                             const float* h_cos, const float* h_sin, const uint32_t* h_slice_base, CddtIndex* ix,
+                             cudaStream_t s) {
+    cddt_index_free(ix);
+    const uint32_t nb = tab.total_bins;
+    const unsigned long long nq = 4 * ((unsigned long long)(tab.nzeros >> 2) + 2ull * nb);
+    if (nb == 0 || nq + 8 >= (1ull << 32)) return cudaSuccess;
+    // slices without zero points (all from td / 2 on, unless a loaded table fills them) have no entries
+    std::vector<uint32_t> slice_zero(td + 1);
+    DevBuf firsts;
+    RLC_TRY(firsts.alloc((td + 1) * sizeof(uint32_t)));
+    k_gather_u32<<<blocks_for(td + 1, 256), 256, 0, s>>>(tab.bin_start, tab.slice_base, td + 1, firsts.as<uint32_t>());
+    RLC_TRY(cudaGetLastError());
+    RLC_TRY(cudaMemcpyAsync(slice_zero.data(), firsts.p, (td + 1) * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+    RLC_TRY(cudaStreamSynchronize(s));
+    std::vector<IndexSlice> sl(td);
+    unsigned long long entries = 0;
+    for (unsigned a = 0; a < td; ++a) {
+        IndexSlice& S = sl[a];
+        const float cx = (float)W * h_cos[a], sy = -((float)H * h_sin[a]);
+        const float lo = fminf(0.0f, fminf(cx, fminf(sy, cx + sy))), hi = fmaxf(0.0f, fmaxf(cx, fmaxf(sy, cx + sy)));
+        const bool used = slice_zero[a + 1] > slice_zero[a] && hi - lo < 1e9f;
+        if (slice_zero[a + 1] > slice_zero[a] && !used) return cudaSuccess;
+        S = IndexSlice{h_cos[a], h_sin[a], h_trans[a], lo, (uint32_t)h_widths[a], (uint32_t)entries,
+                       used ? (uint32_t)((hi - lo) / kCddtBucket) + 2u : 0u, 0u};
+        entries += (unsigned long long)h_widths[a] * S.row;
+        if (entries >= (1ull << 32)) return cudaSuccess;
+    }
+    auto up = [](size_t b) { return (b + 255) & ~(size_t)255; };
+    const size_t o_q = up(td * sizeof(IndexSlice)), o_i = o_q + up(nq * sizeof(float));
+    const size_t o_bad = o_i + up(entries * sizeof(uint32_t)), total = o_bad + 256;
+    char* mem = nullptr;
+    if (cudaMalloc(&mem, total) != cudaSuccess) {
+        cudaGetLastError();
+        return cudaSuccess;
+    }
+    unsigned* bad = reinterpret_cast<unsigned*>(mem + o_bad);
+    unsigned h_bad = 0;
+    cudaError_t e = cudaMemcpyAsync(mem, sl.data(), td * sizeof(IndexSlice), cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess) e = cudaMemsetAsync(bad, 0, sizeof(unsigned), s);
+    if (e == cudaSuccess) {
+        k_index_fill<<<blocks_for((long long)nb * 32, 256), 256, 0, s>>>(
+            reinterpret_cast<const IndexSlice*>(mem), tab.slice_base, (int)td, nb, tab.bin_start, tab.zeros,
+            reinterpret_cast<float*>(mem + o_q), reinterpret_cast<uint32_t*>(mem + o_i), bad);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&h_bad, bad, sizeof(unsigned), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (e != cudaSuccess || h_bad) {
+        cudaFree(mem);
+        return e;
+    }
+    ix->mem = mem;
+    ix->slices = reinterpret_cast<const float4*>(mem);
+    ix->qz = reinterpret_cast<const float*>(mem + o_q);
+    ix->index = reinterpret_cast<const uint32_t*>(mem + o_i);
     return cudaSuccess;
 }
 

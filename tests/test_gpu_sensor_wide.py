@@ -1,8 +1,8 @@
 """The sensor model's kernels at the sizes where they change shape.
 
-eval_sensor_model takes 32 particles per block and 32 beams per chunk; the fused update of 2,000
-particles or more (128 beams and 256 K rays up, no schedule set) takes up to 32 particles per block
-through chunks of beams, with table factors or bins in shared memory.  Both must give the oracle's weights bit for bit, and a call without a
+eval_sensor_model takes 32 particles per block and 32 beams per chunk; the fused update of 256 K rays
+or more (no schedule set; ray marching from 2,000 particles x 128 beams, tables from 48 beams) takes
+up to 32 particles per block through chunks of beams, with table factors or bins in shared memory.  Both must give the oracle's weights bit for bit, and a call without a
 schedule those of the same call with one.
 """
 import os
@@ -49,7 +49,8 @@ def test_eval_sensor_model_edges(small, n, na):
 # particles per block 2, 3, 8 (factors), 9 and 17 (bins) on 152 SMs, a last block of one particle, a
 # chunk's last beam alone, several chunks, two waves of blocks
 @pytest.mark.parametrize("n,na", [(2000, 132), (2049, 512), (2049, 513), (2433, 433), (5461, 193), (9728, 129),
-                                   (9729, 128), (3000, 1081), (20673, 137), (39000, 192)])
+                                   (9729, 128), (3000, 1081), (20673, 137), (39000, 192),
+                                   (5500, 48), (250, 1081)])
 @pytest.mark.parametrize("kind", ["rm", "cddt", "glt"])
 def test_wide_fused_update(rl, oracle_mod, kind, n, na):
     side, mr = 300, 60.0
