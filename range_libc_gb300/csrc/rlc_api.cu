@@ -75,11 +75,29 @@ struct rlc_map {
     std::atomic<int> refs{1};
     std::mutex mu;
 
+    uint8_t* d_free = nullptr;
     void* d_layouts = nullptr;    // one allocation behind every distance-transform layout
 
     ~rlc_map() {
         cudaFree(d_bits);
         cudaFree(d_layouts);
+        cudaFree(d_free);
+    }
+    // the free distances of Bresenham's walk on first use (two bytes per cell, one of them scratch)
+    int ensure_free() {
+        std::lock_guard<std::mutex> lk(mu);
+        const size_t cells = step_map_cells(W, H), scratch = ((size_t)W * H + 255) & ~(size_t)255;
+        if (d_free || cells == 0) return RLC_OK;
+        uint8_t* base = nullptr;
+        cudaError_t e = cudaMalloc(&base, cells + scratch);
+        if (e == cudaSuccess) e = launch_free_map(d_bits, W, H, TY, base + cells, base, 0);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(0);
+        if (e != cudaSuccess) {
+            cudaFree(base);
+            return cuda_fail(e, "free distances");
+        }
+        d_free = base;
+        return RLC_OK;
     }
     // Distance transform and its layouts on first use (RayMarching constructor, RangeLib.h:924).
     // All of them share one allocation (a cudaMalloc + cudaFree pair of 4 MB or more costs ~110 us
@@ -212,6 +230,7 @@ struct rlc_method {
         p.map.step = map->d_step;
         p.map.runs = map->d_runs;
         p.map.bits = map->d_bits;
+        p.map.free = map->d_free;
         p.cddt.td = td;
         p.cddt.td_div_2pi = td_div_2pi;
         p.cddt.twopi_div_td = twopi_div_td;
@@ -565,6 +584,7 @@ static int method_create(rlc_map* map, int kind, float max_range, unsigned td, c
     if (e == cudaSuccess) e = cudaMemset(m->d_err, 0, sizeof(unsigned));
     if (e != cudaSuccess) rc = cuda_fail(e, "method state");
     if (!rc && (m->dkind == K_RM || glt)) rc = map->ensure_dt();
+    if (!rc && m->dkind == K_BL) rc = map->ensure_free();
     if (!rc && glt) rc = glt_build(m, cos_tab, sin_tab);
     if (!rc && cddt) {
         cddt_constants(m, cos_tab, sin_tab);

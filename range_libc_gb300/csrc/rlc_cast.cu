@@ -297,8 +297,9 @@ struct BitCache {   // x, y in the grid; maps hold at most 2^31 cells (rlc_map_c
     }
 };
 
-__device__ float bl_cast(const MapDev& m, float mr, float x, float y, float c, float s, unsigned* err,
-                         int* steps = nullptr) {
+// The walk for any coordinates, one cell at a time.
+__device__ __noinline__ float bl_walk(const MapDev& m, float mr, float x, float y, float c, float s, unsigned* err,
+                                      int* steps) {
     if (isnan(x) || isnan(y)) return mr;
     if (occ_at(m, __float2int_rz(x), __float2int_rz(y))) return 0.0f;
     if (isnan(c) || isnan(s)) return mr;   // the reference never terminates on a NaN heading
@@ -361,6 +362,124 @@ __device__ float bl_cast(const MapDev& m, float mr, float x, float y, float c, f
         }
     }
     return mr;
+}
+
+// floor of v for |v| < 2^22: rounding down to a multiple of 1 beside 1.5 * 2^23
+__device__ __forceinline__ int floor_small(float v) {
+    return __float_as_int(__fadd_rd(v, 12582912.0f)) - 0x4B400000;
+}
+
+// The same walk over the free-distance map (MapDev::free: a byte per cell, the Chebyshev distance to
+// the nearest occupied cell, 0 on it), for coordinates below 2^22.  kBlSteps cells are stepped at once
+// without looking at memory, and their bytes read together and tested by their least: a block waits
+// for one read where the walk above waits for its slowest lane's at almost every step.  The last byte
+// then says how far the walk is free: a step moves each coordinate by 1, and float rounding (once per
+// power of two that a coordinate crosses, less than 1 in all below 2^22) can move a cell's index one
+// further, so the next r - 2 steps need no test, and as far as they stay two short of the walk's end
+// no end test either: they are the error accumulation alone, 5 instructions.  Halving and doubling are
+// exact at these sizes, so 2 * error >= deltax is error >= deltax / 2; below 2^22 a longer side is never
+// reached, so the grid test is the integers' (off the grid a position reads the map's one more row or
+// column, 1).  10,000 queries on 512^2 62 -> 35 us a call (blocks of 4 / 8 / 16 steps 40 / 35 / 34), 1 M
+// 363 -> 149, 1 M on 2048^2 403 -> 197, 4,000 x 61 fused 77 -> 44, 8,000 x 1,081 (wide) 722 -> 415.
+constexpr int kBlSteps = 8;
+
+__device__ __forceinline__ float bl_cast(const MapDev& m, float mr, float x, float y, float c, float s, unsigned* err) {
+    const float x1w = __fadd_rn(y, __fmul_rn(mr, s)), y1w = __fadd_rn(x, __fmul_rn(mr, c));
+    const float dx0 = fabsf(__fsub_rn(x1w, y)), dy0 = fabsf(__fsub_rn(y1w, x));
+    // NaN, infinite and far coordinates, walks without length, maps without the free distances
+    const float far = fmaxf(fmaxf(fabsf(x), fabsf(y)), fmaxf(fabsf(x1w), fabsf(y1w)));
+    if (m.free == nullptr || isnan(x) || isnan(y) || isnan(c) || isnan(s) || !(far < 0x1p22f) ||
+        !(fmaxf(dx0, dy0) > 0x1p-60f))
+        return bl_walk(m, mr, x, y, c, s, err, nullptr);
+    if (occ_at(m, __float2int_rz(x), __float2int_rz(y))) return 0.0f;
+    const bool steep = dy0 > dx0;   // the walk goes along x
+    const float x0 = steep ? x : y, y0 = steep ? y : x;
+    const float x1 = steep ? y1w : x1w, y1 = steep ? x1w : y1w;
+    const float deltax = steep ? dy0 : dx0, deltaerr = steep ? dx0 : dy0, half = __fmul_rn(deltax, 0.5f);
+    const float xstep = (x0 < x1) ? 1.0f : -1.0f, ystep = (y0 < y1) ? 1.0f : -1.0f;
+    const int end = __float2int_rz(__fadd_rn(x1, xstep)), bound = (int)deltax + 4;
+    // the walk's axes: the first is the map's x where steep, else its y
+    const unsigned bu = (unsigned)(steep ? m.W : m.H), bv = (unsigned)(steep ? m.H : m.W);
+    const unsigned su = steep ? (unsigned)m.H + 1u : 1u, sv = steep ? 1u : (unsigned)m.H + 1u;
+    float _x = x0, _y = y0, error = 0.0f;
+    int n = 0;
+    const auto step = [&]() {
+        _x = __fadd_rn(_x, xstep);
+        error = __fadd_rn(error, deltaerr);
+        if (error >= half) {
+            _y = __fadd_rn(_y, ystep);
+            error = __fsub_rn(error, deltax);
+        }
+    };
+    const auto cell = [&](int fu, int fv) { return min((unsigned)fu, bu) * su + min((unsigned)fv, bv) * sv; };
+    const auto range = [&]() {
+        const float xd = __fsub_rn(_x, x0), yd = __fsub_rn(_y, y0);
+        return __fsqrt_rn(__fadd_rn(__fmul_rn(xd, xd), __fmul_rn(yd, yd)));
+    };
+    // past the grid's edge in the direction of motion: no occupied cell is left on the walk
+    const auto gone = [&](int fu, int fv) {
+        return (xstep > 0.0f ? fu >= (int)bu : fu < 0) || (ystep > 0.0f ? fv >= (int)bv : fv < 0);
+    };
+    for (;;) {
+        const int xi = __float2int_rz(_x), left = xstep > 0.0f ? end - xi : xi - end;
+        if (left < kBlSteps + 2) break;   // rounding can bring the end one cell nearer
+        n += kBlSteps;
+        const float _x_at = _x, _y_at = _y, error_at = error;
+        unsigned r[kBlSteps];
+        int fu = 0, fv = 0;
+#pragma unroll
+        for (int i = 0; i < kBlSteps; ++i) {
+            step();
+            fu = floor_small(_x);
+            fv = floor_small(_y);
+            r[i] = __ldg(m.free + cell(fu, fv));
+        }
+        unsigned least = r[0];
+#pragma unroll
+        for (int i = 1; i < kBlSteps; ++i) least = min(least, r[i]);
+        if (least == 0u) {   // an occupied cell: its coordinates by the steps up to the first
+            _x = _x_at;
+            _y = _y_at;
+            error = error_at;
+            do step(); while (__ldg(m.free + cell(floor_small(_x), floor_small(_y))) != 0u);
+            return range();
+        }
+        if (gone(fu, fv)) return mr;
+        if (min((int)r[kBlSteps - 1], left - kBlSteps) - 2 >= kBlSteps) {   // once: more would hold up the other lanes
+            n += kBlSteps;
+#pragma unroll
+            for (int i = 0; i < kBlSteps; ++i) step();
+        }
+    }
+    for (;;) {   // around the end cell: the same blocks, noting where the walk ends
+        const float _x_at = _x, _y_at = _y, error_at = error;
+        unsigned r[kBlSteps];
+        int fu = 0, fv = 0, ends = kBlSteps;
+#pragma unroll
+        for (int i = 0; i < kBlSteps; ++i) {
+            if (ends == kBlSteps && (__float2int_rz(_x) == end || n + i > bound)) ends = i;
+            step();
+            fu = floor_small(_x);
+            fv = floor_small(_y);
+            r[i] = i < ends ? __ldg(m.free + cell(fu, fv)) : 1u;
+        }
+        unsigned least = r[0];
+#pragma unroll
+        for (int i = 1; i < kBlSteps; ++i) least = min(least, r[i]);
+        if (least == 0u || ends < kBlSteps) {   // step again, up to the occupied cell or the walk's end
+            _x = _x_at;
+            _y = _y_at;
+            error = error_at;
+            for (int i = 0; i < ends; ++i) {
+                step();
+                if (least == 0u && __ldg(m.free + cell(floor_small(_x), floor_small(_y))) == 0u) return range();
+            }
+            if (__float2int_rz(_x) != end) atomicOr(err, F_BL_BOUND);
+            return mr;
+        }
+        if (gone(fu, fv)) return mr;
+        n += kBlSteps;
+    }
 }
 
 // ------------------------------------------------------------------ CDDT
@@ -1038,7 +1157,7 @@ __device__ __forceinline__ float cast_ray(const CastParams& p, const float* __re
 // threads), so that a particle-filter step's blocks of 128 threads stay resident at 16 per SM
 // in one wave; the CDDT searches keep their registers.
 template <int KIND, int LAYOUT, int PF>
-__global__ void __launch_bounds__(512, KIND == K_CDDT ? 1 : 4) k_fused(CastParams p, SensorDev sm, const float* __restrict__ ins,
+__global__ void __launch_bounds__(512, KIND == K_CDDT ? 1 : KIND == K_BL ? 2 : 4) k_fused(CastParams p, SensorDev sm, const float* __restrict__ ins,
                                                const float* __restrict__ angles, const float* __restrict__ obs,
                                                double* __restrict__ weights, int n, int na, int P) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1110,6 +1229,9 @@ __device__ __forceinline__ void tile_bins4(const uint16_t* tile, int P, int li, 
 // issue slots used).  Now 384 us.
 constexpr int kWideThreads = 256;
 constexpr int kWideParticles = 32;
+
+// blocks per SM: the registers of the table search and of Bresenham's blocks of steps
+__host__ __device__ constexpr int wide_blocks(int kind) { return kind == K_CDDT || kind == K_BL ? 4 : 8; }
 
 struct WideSmem {   // byte offsets of the dynamic shared memory
     int part, beam, ang, row, bins, total;
@@ -1215,7 +1337,7 @@ __device__ __forceinline__ void wide_tile(const CastParams& p, const SensorDev& 
 }
 
 template <int KIND, int LAYOUT, int PF, bool FACTORS>
-__global__ void __launch_bounds__(kWideThreads, KIND == K_CDDT ? 4 : 8)
+__global__ void __launch_bounds__(kWideThreads, wide_blocks(KIND))
 k_fused_wide(CastParams p, SensorDev sm, const float* __restrict__ ins, const float* __restrict__ angles,
              const float* __restrict__ obs, double* __restrict__ weights, int n, int na, int P, int C) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1676,7 +1798,7 @@ __global__ void __launch_bounds__(256) k_count_steps(CastParams p, const float* 
         float c, s;
         if (p.trig) { c = p.trig[2 * g]; s = p.trig[2 * g + 1]; } else rlc_trig::sincos_cr(h, &s, &c);
         if (KIND == K_RM) rm_cast<DT_LINEAR>(p.map, p.mr, ax, ay, c, s, &steps);
-        else bl_cast(p.map, p.mr, ax, ay, c, s, p.err, &steps);
+        else bl_walk(p.map, p.mr, ax, ay, c, s, p.err, &steps);
     }
     for (int o = 16; o; o >>= 1) steps += __shfl_xor_sync(0xffffffffu, steps, o);
     if ((threadIdx.x & 31) == 0 && steps) atomicAdd(total, (unsigned long long)steps);
@@ -1760,12 +1882,11 @@ cudaError_t set_smem(K kernel, size_t bytes) {
 // that the products weigh more: CDDT 8,000 x 1,081 595 / 128, 4,000 x 271 96 / 30, 2,000 x 150
 // 40 / 18, 1,000 x 300 28 / 24, 5,000 x 61 21 / 18; below the line 4,000 x 61 12.6 / 13.6, 8,000 x 35
 // 12.3 / 14.1, 600 x 200 15.3 / 17.1; GLT 20,000 x 200 253 / 39, 8,000 x 61 15.6 / 13.1, 4,000 x 61
-// 11.6 / 13.3.  Bresenham's walks are too uneven for a barrier per chunk (8,000 x
-// 1,081 722 / 869).
+// 11.6 / 13.3.  Bresenham 8,000 x 1,081 617 / 416, 4,000 x 271 133 / 100.
 inline bool fused_wide(int kind, int n, int na) {
     const long long rays = (long long)n * na;
-    if (kind == K_BL || rays < (1ll << 18)) return false;
-    return kind == K_RM ? na >= 128 && n >= 2000 : na >= 48;
+    if (rays < (1ll << 18)) return false;
+    return kind == K_RM || kind == K_BL ? na >= 128 && n >= 2000 : na >= 48;
 }
 // Its shape: as few particles per block as keep all blocks resident at once.  Up to kWideFactors
 // particles the rays' threads read the table factors themselves (a lone product chain that reads
@@ -1781,7 +1902,7 @@ struct RunFused {
                            const float* obs, double* w, int n, int na, int block, int tile, bool pick, cudaStream_t s) {
         if (n <= 0) return cudaSuccess;
         // the kernels that a call without a schedule can come to (pick_layout)
-        constexpr bool kPicked = KIND == K_GLT || (KIND == K_CDDT && (PF == 0 || PF == 3)) ||
+        constexpr bool kPicked = KIND == K_GLT || KIND == K_BL || (KIND == K_CDDT && (PF == 0 || PF == 3)) ||
                                  (KIND == K_RM && PF == 0 && (LAYOUT == DT_STEP || LAYOUT == DT_RUNS));
         if constexpr (kPicked) {
             if (pick && fused_wide(KIND, n, na)) {
@@ -1789,7 +1910,7 @@ struct RunFused {
                 cudaError_t e = cudaGetDevice(&dev);
                 if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
                 if (e != cudaSuccess) return e;
-                const long long resident = (long long)sms * (KIND == K_CDDT ? 4 : 8);
+                const long long resident = (long long)sms * wide_blocks(KIND);
                 const long long waves = (n + resident * kWideParticles - 1) / (resident * kWideParticles);
                 const int P = (int)((n + resident * waves - 1) / (resident * waves));
                 const bool factors = P <= kWideFactors;

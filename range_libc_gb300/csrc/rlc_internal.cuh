@@ -51,7 +51,15 @@ struct MapDev {
     // -y, +x and -x (bits 0-7, 8-15, 16-23, 24-31; at most 255)
     const uint32_t* runs;
     const uint64_t* bits;     // occupancy bit tiles
+    // free distance per cell (a Bresenham method's map): the Chebyshev distance to the nearest occupied
+    // cell, 0 on it and at most kFreeMost, in a (W + 1) x (H + 1) grid whose last row and column are 1;
+    // null where that grid's index needs more than 32 bits
+    const uint8_t* free;
 };
+constexpr int kFreeMost = 64;
+// d_scratch: W * H bytes
+cudaError_t launch_free_map(const uint64_t* d_bits, int W, int H, int tiles_y, uint8_t* d_scratch, uint8_t* d_free,
+                            cudaStream_t s);
 
 struct CddtDev {
     unsigned td;

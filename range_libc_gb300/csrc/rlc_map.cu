@@ -683,6 +683,47 @@ __global__ void k_unpack_bits(const uint64_t* __restrict__ bits, int W, int H, i
     occ[i] = occ_bit(bits, TY, x, y) ? 1 : 0;
 }
 
+// ---- free distances (Bresenham's walk)
+// Distance along y to the nearest occupied cell of the column, at most kFreeMost: the bytes of the
+// column's tiles, outward.
+__global__ void __launch_bounds__(256) k_free_y(const uint64_t* __restrict__ bits, int W, int H, int TY,
+                                                uint8_t* __restrict__ g) {
+    const unsigned yb = ((unsigned)H + 31u) >> 5, bx = blockIdx.x / yb;   // 32 y x 8 x cells per block
+    const int x = (int)(bx * 8 + threadIdx.y), y = (int)((blockIdx.x - bx * yb) * 32 + threadIdx.x);
+    if (x >= W || y >= H) return;
+    const uint64_t* col = bits + (size_t)(x >> 3) * TY;
+    const int sh = (x & 7) << 3, c = y >> 3, in = y & 7;
+    const unsigned b = (unsigned)(__ldg(col + c) >> sh) & 0xFFu;
+    const unsigned lo = b & ((2u << in) - 1u), hi = b >> in;
+    int d = kFreeMost;
+    if (lo) d = min(d, in - edt_msb(lo));
+    if (hi) d = min(d, edt_lsb(hi));
+    for (int k = 1; 8 * k - 7 < d && (c - k >= 0 || c + k < TY); ++k) {
+        const unsigned l = c - k >= 0 ? (unsigned)(__ldg(col + c - k) >> sh) & 0xFFu : 0u;
+        const unsigned r = c + k < TY ? (unsigned)(__ldg(col + c + k) >> sh) & 0xFFu : 0u;
+        if (l) d = min(d, 8 * k + in - edt_msb(l));
+        if (r) d = min(d, 8 * k - in + edt_lsb(r));
+    }
+    g[(size_t)x * H + y] = (uint8_t)d;
+}
+
+// Chebyshev distance: the least over dx of max(|dx|, distance along y at x + dx); a (W + 1) x (H + 1) grid
+// with 1 in its last row and column.
+__global__ void __launch_bounds__(256) k_free_x(const uint8_t* __restrict__ g, int W, int H, uint8_t* __restrict__ out) {
+    const unsigned yb = ((unsigned)H + 32u) >> 5, bx = blockIdx.x / yb;
+    const int x = (int)(bx * 8 + threadIdx.y), y = (int)((blockIdx.x - bx * yb) * 32 + threadIdx.x);
+    if (x > W || y > H) return;
+    int d = 1;
+    if (x < W && y < H) {
+        d = __ldg(g + (size_t)x * H + y);
+        for (int e = 1; e < d; ++e) {
+            if (x - e >= 0) d = min(d, max(e, (int)__ldg(g + (size_t)(x - e) * H + y)));
+            if (x + e < W) d = min(d, max(e, (int)__ldg(g + (size_t)(x + e) * H + y)));
+        }
+    }
+    out[(size_t)x * (H + 1) + y] = (uint8_t)d;
+}
+
 inline unsigned blocks_for(long long n, int b) { return (unsigned)((n + b - 1) / b); }
 
 }  // namespace
@@ -772,6 +813,17 @@ cudaError_t launch_step_runs(const float* d_step, int W, int H, uint32_t* d_eq, 
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     k_step_runs<<<blocks_for(H, 32) * blocks_for(W, 8), dim3(32, 8), 0, s>>>(eqx, eqy, W, H, HW, d_runs);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_free_map(const uint64_t* d_bits, int W, int H, int TY, uint8_t* d_scratch, uint8_t* d_free,
+                            cudaStream_t s) {
+    if ((long long)W * H == 0) return cudaSuccess;
+    k_free_y<<<blocks_for(H, 32) * blocks_for(W, 8), dim3(32, 8), 0, s>>>(d_bits, W, H, TY, d_scratch);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    k_free_x<<<blocks_for((long long)H + 1, 32) * blocks_for((long long)W + 1, 8), dim3(32, 8), 0, s>>>(d_scratch, W, H,
+                                                                                                       d_free);
     return cudaGetLastError();
 }
 
