@@ -28,6 +28,8 @@
 #include <cstring>
 #include <vector>
 
+#define TRY(x) do { cudaError_t _e = (x); if (_e != cudaSuccess) return _e; } while (0)
+
 namespace rlc {
 namespace {
 
@@ -50,25 +52,16 @@ __host__ __device__ inline int layer_in(int l) { return l == 0 ? kFeat : kHidden
 constexpr size_t kOutW = kW0 + kHidden + 3 * (kWh + kHidden);  // output weights [256], then bias [1]
 
 // -------------------------------------------------------------------- GEMM
-enum Epi : int { EPI_F32 = 0, EPI_FWD = 1, EPI_BWD = 2, EPI_F32_ADD = 3 };
-
 struct GemmArgs {
-    const bf16* A;   // A[m * lda + k] (a_t and b_t must be 0: both operands K-major)
-    const bf16* B;   // B[n * ldb + k]
+    const bf16* A;   // A[m * lda + k] (K-major), or with a_t A[k * lda + m] (M-major)
+    const bf16* B;   // B[n * ldb + k], or with b_t B[k * ldb + n]
     int lda, ldb, a_t, b_t;
     int M, N, K;
-    int ksplit;         // K range of blockIdx.z: [z * ksplit, (z + 1) * ksplit)
-    int epi;
+    int ksplit;          // K range of blockIdx.z: [z * ksplit, min((z + 1) * ksplit, K))
+    float* C;            // C[m * ldc + n], of split z at C + z * part_stride; 16-byte aligned
     int ldc;
-    float* C32;         // EPI_F32: C[m * ldc + n]; EPI_F32_ADD: C[m * ldc + n] += (split-K partials)
-    const float* bias;  // EPI_FWD
-    bf16* Zout;         // EPI_FWD: pre-activation
-    bf16* Hout;         // EPI_FWD: GELU(z)
-    const bf16* Zin;    // EPI_BWD: pre-activation of the layer below
-    bf16* dZ;           // EPI_BWD: acc * GELU'(Zin)
-    bf16* HoutT;        // EPI_FWD (optional): GELU(z) transposed, [n * ldt + m]
-    bf16* dZT;          // EPI_BWD (optional): dZ transposed, [n * ldt + m]
-    int ldt;
+    size_t part_stride;
+    float* k_sums;       // with a_t: also the sums over k of A[k][m], at k_sums[z * part_stride + m]
     unsigned* err;
 };
 
@@ -81,63 +74,138 @@ __device__ __forceinline__ float tanh_sfu(float x) {
     return y;
 }
 
-__device__ __forceinline__ float gelu(float z) {
-    const float k0 = 0.7978845608028654f, k1 = 0.044715f;
-    return 0.5f * z * (1.0f + tanh_sfu(k0 * (z + k1 * z * z * z)));
+// Two floats per register pair: one issue slot for both (each rounded as by itself).  The network's
+// elementwise work is issue-bound (k_top for 65,536 rays: 25.7 -> 23.8 us).
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float a, float b) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
 }
+__device__ __forceinline__ float2 unpack2(f32x2 v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ f32x2 both(float a) { return pack2(a, a); }
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f32x2 tanh2(f32x2 x) {
+    const float2 v = unpack2(x);
+    return pack2(tanh_sfu(v.x), tanh_sfu(v.y));
+}
+constexpr float kGelu0 = 0.7978845608028654f, kGelu1 = 0.044715f;
 
-__device__ __forceinline__ float gelu_grad(float z) {
-    const float k0 = 0.7978845608028654f, k1 = 0.044715f;
-    float u = k0 * (z + k1 * z * z * z);
-    float th = tanh_sfu(u);
-    return 0.5f * (1.0f + th) + 0.5f * z * (1.0f - th * th) * k0 * (1.0f + 3.0f * k1 * z * z);
+// The assembler contracts mul.rn.f32x2 + add.rn.f32x2 to one rounding, also without -fmad.  A product
+// that is added to something is therefore an fma with a -0 that it cannot see: a * b rounded as by itself.
+__constant__ float c_neg_zero = -0.0f;
+__device__ __forceinline__ f32x2 mul2_then(f32x2 a, f32x2 b) { return fma2(a, b, both(c_neg_zero)); }
+
+// tanh(k0 (z + k1 z^3))
+__device__ __forceinline__ f32x2 gelu_tanh(f32x2 z) {
+    return tanh2(mul2(both(kGelu0), add2(z, mul2_then(mul2(mul2(both(kGelu1), z), z), z))));
+}
+// 0.5 z (1 + tanh(..))
+__device__ __forceinline__ float2 gelu(f32x2 z) {
+    return unpack2(mul2(mul2(both(0.5f), z), add2(both(1.0f), gelu_tanh(z))));
+}
+// 0.5 (1 + th) + 0.5 z (1 - th^2) k0 (1 + 3 k1 z^2)
+__device__ __forceinline__ f32x2 gelu_grad(f32x2 z) {
+    const f32x2 one = both(1.0f), half = both(0.5f), th = gelu_tanh(z);
+    const f32x2 sech2 = fma2(mul2(th, th), both(-1.0f), one);   // 1 - th * th, rounded as those two steps
+    const f32x2 du = add2(one, mul2_then(mul2(both(3.0f * kGelu1), z), z));
+    return add2(mul2_then(half, add2(one, th)), mul2_then(mul2(mul2(mul2(half, z), sech2), both(kGelu0)), du));
 }
 
 // --------------------------------------------------------------- TMA GEMM
-// C tile [128 x 256] at (blockIdx.y * 128, blockIdx.x * 256) of C = A . B^T, both operands
-// K-major in global memory (A[m * lda + k], B[n * ldb + k]), K range [z * ksplit, (z+1) * ksplit).
+// C tile [128 x BN] at (blockIdx.y * 128, blockIdx.x * BN) of C = A . B^T in fp32, K range
+// [z * ksplit, min((z + 1) * ksplit, K)): the weight gradients, whose K is the batch.  Either operand
+// may lie K-major or, as the batch's rows do here, M/N-major: the tensor cores read both, so no
+// transposed copy of an activation or gradient is ever written (before, the epilogues stored a second
+// copy two bytes at a time, and three transposes ran per step).
 //
-// Warp-specialised (192 threads, pipeline stages of 48 KB):
-//   warp 0     TMA producer: per 64-wide K chunk, one tile load of A (128 rows x 128 bytes) and
-//              one of B (256 rows) into stage s, completing on full[s]; it reuses a stage once the
-//              MMAs that read it have committed to empty[s];
-//   warp 1     allocates 256 TMEM columns; one thread issues the chunk's four
+// Warp-specialised (10 warps, 192 KB of pipeline stages):
+//   warp 0     TMA producer: per 64-wide K chunk, the tiles of A (128 rows or columns) and B (BN)
+//              into stage s, completing on full[s]; it reuses a stage once the MMAs that read it have
+//              committed to empty[s] (and the warps that sum it have arrived there);
+//   warp 1     allocates BN TMEM columns; one thread issues the chunk's four
 //              tcgen05.mma (K = 16 each) per stage and commits them to empty[s], and after the
 //              last chunk to `accum`;
-//   warps 2-5  epilogue: wait for `accum`, read the accumulator with tcgen05.ld (warp w reads
-//              TMEM lanes 32 (w % 4) .. + 31) and apply the epilogue.
-// Shared-memory operand layout (K-major, 128-byte swizzle, as the TMA writes it): row r of a
-// stage's tile at r * 128 bytes with its 16-byte chunks permuted by r & 7 (tc::make_desc_sw128).
+//   warps 2-9  with k_sums: add up the rows of every stage of A on its way (the bias gradients, which
+//              took four more passes over the gradients); then the epilogue: wait for `accum`, read
+//              half of the columns of 32 rows of the accumulator with tcgen05.ld (warp w reads TMEM
+//              lanes 32 (w % 4) .. + 31) and store it.
+// Shared-memory operand layouts, 128-byte swizzle, as the TMA writes them: K-major, row r of a tile at
+// r * 128 bytes (tc::make_desc_sw128); M/N-major, blocks of 64 columns, of which K row k lies at
+// k * 128 bytes (tc::make_desc_sw128_mn); 16-byte chunks permuted by the row & 7.
 // Every wait is bounded (about a second); a time-out sets bit 16 of *err, the remaining roles stop
 // at their next wait, and the CTA still frees its TMEM.
 //
-// kStages = 4 (one CTA per SM) for the long-K weight gradients; 2 (two CTAs per SM, so that one
-// CTA's epilogue overlaps the other's loads and MMAs) for the short-K forward and input-gradient
-// GEMMs (K = 256 or 512).
+// Bound by reading dZ and the layer's input: 67 MB for a hidden layer and 65,536 rays, 17 us (22 from the
+// transposed copies, which cost 32 us and more to write, and 27 us for the bias sums).
 constexpr uint32_t kStageA = kBM * tc::kKChunk * 2;   // 16 KB
-constexpr uint32_t kStageB = kBN * tc::kKChunk * 2;   // 32 KB
-template <int kStages>
-constexpr size_t tma_smem() { return kStages * (size_t)(kStageA + kStageB) + 1024; }   // + alignment slack
-constexpr int kGemmThreads = 192;
+constexpr uint32_t kBlockMN = 64 * tc::kKChunk * 2;   // an M/N-major block of 64 columns x 64 K: 8 KB
+constexpr size_t kGemmSmem = 196608 + 1024;           // the stages, + alignment slack
+constexpr int kEpiWarps = 8;
+constexpr int kGemmThreads = 64 + 32 * kEpiWarps;
 
-template <int kStages>
-__global__ void __launch_bounds__(kGemmThreads, kStages <= 2 ? 2 : 1)
+// 32 bytes per lane and instruction: whole sectors although the lanes' rows lie apart
+__device__ __forceinline__ void store32(void* p, const uint32_t* v) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(v[0]), "r"(v[1]), "r"(v[2]),
+                 "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+                 : "memory");
+}
+__device__ __forceinline__ void load32(const void* p, uint32_t* v) {
+    asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+                 : "l"(p));
+}
+__device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
+    const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
+    return *reinterpret_cast<const uint32_t*>(&v);
+}
+__device__ __forceinline__ f32x2 widen_bf16(uint32_t u) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(u << 16), "r"(u & 0xffff0000u));
+    return r;
+}
+__device__ __forceinline__ float2 unpack_bf16(uint32_t u) { return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u)); }
+
+template <int BN>
+__global__ void __launch_bounds__(kGemmThreads, 1)
 k_gemm_tma(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, GemmArgs g) {
+    constexpr uint32_t kStageB = BN * tc::kKChunk * 2;
+    constexpr int kStages = 196608 / (kStageA + kStageB);
     extern __shared__ uint8_t smem_raw[];
     __shared__ __align__(8) uint64_t full[kStages], empty[kStages], accum;
     __shared__ uint32_t tmem_base;
     __shared__ int abort_flag, n_issued, n_consumed;
+    __shared__ __align__(16) float s_sums[kEpiWarps / 2][kBM];
     uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     const uint32_t sbase = tc::smem_addr(smem);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int m0 = blockIdx.y * kBM, n0 = blockIdx.x * kBN;
+    const int m0 = blockIdx.y * kBM, n0 = blockIdx.x * BN;
     const int kbase = blockIdx.z * g.ksplit;
-    const int nchunks = g.ksplit / tc::kKChunk;
-    if (warp == 1) tc::tmem_alloc(tc::smem_addr(&tmem_base), 256);
+    const int nchunks = min(g.ksplit, g.K - kbase) / tc::kKChunk;
+    const bool sums = g.k_sums != nullptr && g.a_t && blockIdx.x == 0;
+    if (warp == 1) tc::tmem_alloc(tc::smem_addr(&tmem_base), BN);
     if (threadIdx.x == 0) {
         for (int i = 0; i < kStages; ++i) {
             tc::mbar_init(tc::smem_addr(&full[i]), 1);
-            tc::mbar_init(tc::smem_addr(&empty[i]), 1);
+            tc::mbar_init(tc::smem_addr(&empty[i]), sums ? 1 + kEpiWarps : 1);   // the MMAs' commit, and the summing warps
         }
         tc::mbar_init(tc::smem_addr(&accum), 1);
         abort_flag = 0;
@@ -155,46 +223,91 @@ k_gemm_tma(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
         // ---- producer
         tc::tma_prefetch_map(&tmA);
         tc::tma_prefetch_map(&tmB);
-        for (int c = 0; c < nchunks; ++c) {
-            const int st = c % kStages;
-            if (c >= kStages && !tc::mbar_wait(tc::smem_addr(&empty[st]), ((c / kStages) - 1) & 1)) {
+        int c = 0;
+        for (int st = 0, phase = 1, k = kbase; c < nchunks; ++c, k += tc::kKChunk) {
+            if (c >= kStages && !tc::mbar_wait(tc::smem_addr(&empty[st]), phase)) {
                 atomicOr(g.err, 16u);
                 atomicExch(&abort_flag, 1);
                 break;
             }
-            if (*(volatile int*)&abort_flag) break;
             const uint32_t fb = tc::smem_addr(&full[st]);
             tc::mbar_arrive_expect_tx(fb, kStageA + kStageB);
-            const int k0 = kbase + c * tc::kKChunk;
-            tc::tma_load_2d(stage_a(st), &tmA, k0, m0, fb);
-            tc::tma_load_2d(stage_b(st), &tmB, k0, n0, fb);
-            n_issued = c + 1;
+            tc::tma_load_3d(stage_a(st), &tmA, g.a_t ? 0 : k, g.a_t ? k : m0, g.a_t ? m0 / 64 : 0, fb);
+            tc::tma_load_3d(stage_b(st), &tmB, g.b_t ? 0 : k, g.b_t ? k : n0, g.b_t ? n0 / 64 : 0, fb);
+            if (++st == kStages) {
+                st = 0;
+                phase ^= 1;
+            }
         }
+        n_issued = c;
     } else if (warp == 1 && lane == 0) {
         // ---- MMA issuer
-        const uint32_t idesc = tc::make_idesc(kBM, kBN);
-        for (int c = 0; c < nchunks; ++c) {
-            const int st = c % kStages;
-            if (!tc::mbar_wait(tc::smem_addr(&full[st]), (c / kStages) & 1)) {
+        const uint32_t idesc = tc::make_idesc(kBM, BN) | (g.a_t ? tc::kIdescTransposeA : 0u) | (g.b_t ? tc::kIdescTransposeB : 0u);
+        // descriptors of stage 0; a stage and a K step of 16 further are additions to their address field
+        const uint64_t a0 = g.a_t ? tc::make_desc_sw128_mn(stage_a(0), kBlockMN) : tc::make_desc_sw128(stage_a(0));
+        const uint64_t b0 = g.b_t ? tc::make_desc_sw128_mn(stage_b(0), kBlockMN) : tc::make_desc_sw128(stage_b(0));
+        const uint32_t a_step = (g.a_t ? 16 * 128 : 32) >> 4, b_step = (g.b_t ? 16 * 128 : 32) >> 4;
+        int c = 0;
+        for (int st = 0, phase = 0; c < nchunks; ++c) {
+            if (!tc::mbar_wait(tc::smem_addr(&full[st]), phase)) {
                 atomicOr(g.err, 16u);
                 atomicExch(&abort_flag, 1);
                 break;
             }
             tc::fence_after_sync();
+            const uint32_t at = (uint32_t)st * ((kStageA + kStageB) >> 4);
 #pragma unroll
-            for (int ks = 0; ks < tc::kKChunk / 16; ++ks) {
-                const uint64_t ad = tc::make_desc_sw128(stage_a(st) + ks * 32);
-                const uint64_t bd = tc::make_desc_sw128(stage_b(st) + ks * 32);
-                tc::mma_bf16(tmem, ad, bd, idesc, (c > 0 || ks > 0) ? 1u : 0u);
-            }
+            for (int ks = 0; ks < tc::kKChunk / 16; ++ks)
+                tc::mma_bf16(tmem, a0 + (at + ks * a_step), b0 + (at + ks * b_step), idesc, (c > 0 || ks > 0) ? 1u : 0u);
             tc::mma_commit(tc::smem_addr(&empty[st]));
-            n_consumed = c + 1;
+            if (++st == kStages) {
+                st = 0;
+                phase ^= 1;
+            }
         }
+        n_consumed = c;
         // `accum` completes once every MMA issued above has (also with none issued)
         tc::mma_commit(tc::smem_addr(&accum));
     } else if (warp >= 2) {
+        if (sums) {
+            // ---- sums over K of A's columns: two columns and a quarter of a stage's rows per thread
+            constexpr int kRows = tc::kKChunk / (kEpiWarps / 2);
+            const int pair = (threadIdx.x - 64) & 63, part = (threadIdx.x - 64) >> 6, r0 = part * kRows;
+            const uint32_t at = (uint32_t)(pair >> 5) * kBlockMN + (uint32_t)(pair & 3) * 4u, chunk = (pair & 31) >> 2;
+            float a0 = 0.0f, a1 = 0.0f;
+            bool ok = true;
+            for (int c = 0; c < nchunks && ok; ++c) {
+                const int st = c % kStages;
+                ok = __all_sync(0xffffffffu, tc::mbar_wait(tc::smem_addr(&full[st]), (c / kStages) & 1));
+                if (ok) {
+                    const uint8_t* tile = smem + (size_t)st * (kStageA + kStageB) + at;
+#pragma unroll
+                    for (int r = r0; r < r0 + kRows; ++r) {
+                        const float2 v = unpack_bf16(*reinterpret_cast<const uint32_t*>(tile + r * 128 + ((chunk ^ (r & 7)) << 4)));
+                        a0 += v.x;
+                        a1 += v.y;
+                    }
+                }
+                __syncwarp();
+                if (lane == 0) tc::mbar_arrive(tc::smem_addr(&empty[st]));
+            }
+            if (!ok) {
+                atomicOr(g.err, 16u);
+                atomicExch(&abort_flag, 1);
+            }
+            // the parts of the rows, in a fixed order
+            *reinterpret_cast<float2*>(&s_sums[part][2 * pair]) = make_float2(a0, a1);
+            asm volatile("bar.sync 1, %0;" ::"n"(32 * kEpiWarps) : "memory");
+            const int col = threadIdx.x - 64;
+            if (col < kBM) {
+                float sum = s_sums[0][col];
+#pragma unroll
+                for (int q = 1; q < kEpiWarps / 2; ++q) sum += s_sums[q][col];
+                g.k_sums[(size_t)blockIdx.z * g.part_stride + m0 + col] = sum;
+            }
+        }
         // ---- epilogue
-        const bool ok = tc::mbar_wait(tc::smem_addr(&accum), 0);
+        const bool ok = __all_sync(0xffffffffu, tc::mbar_wait(tc::smem_addr(&accum), 0));
         tc::fence_after_sync();
         if (!ok) {
             if (lane == 0) atomicOr(g.err, 16u);
@@ -202,58 +315,19 @@ k_gemm_tma(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
             const int lq = warp & 3;   // TMEM lane quarter this warp may read
             const int row = m0 + lq * 32 + lane;
             const uint32_t lane_addr = tmem + ((uint32_t)(lq * 32) << 16);
-            for (int cb = 0; cb < kBN; cb += 32) {
+            constexpr int kCols = BN / (kEpiWarps / 4);
+            const int c0 = (warp - 2) / 4 * kCols;   // this warp's columns
+            float* out = g.C + (size_t)blockIdx.z * g.part_stride + (size_t)row * g.ldc + n0;
+            for (int cb = c0; cb < c0 + kCols; cb += 32) {
                 float v[32];
                 tc::tmem_ld32(lane_addr + cb, v);
-                const int col0 = n0 + cb;
-                if (g.epi == EPI_F32) {
-                    float* out = g.C32 + (size_t)row * g.ldc + col0;
+                if (g.part_stride) {   // the workspace of partial sums
 #pragma unroll
-                    for (int i = 0; i < 32; i += 4) *reinterpret_cast<float4*>(out + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
-                } else if (g.epi == EPI_F32_ADD) {   // split-K partial sums: 16-byte vector reductions
-                    float* out = g.C32 + (size_t)row * g.ldc + col0;
+                    for (int i = 0; i < 32; i += 8) store32(out + cb + i, reinterpret_cast<const uint32_t*>(v + i));
+                } else {
 #pragma unroll
                     for (int i = 0; i < 32; i += 4)
-                        asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(out + i), "f"(v[i]),
-                                     "f"(v[i + 1]), "f"(v[i + 2]), "f"(v[i + 3])
-                                     : "memory");
-                } else if (g.epi == EPI_FWD) {
-                    __nv_bfloat162 zp[16], hp[16];
-#pragma unroll
-                    for (int i = 0; i < 32; i += 2) {
-                        const float z0 = v[i] + __ldg(g.bias + col0 + i), z1 = v[i + 1] + __ldg(g.bias + col0 + i + 1);
-                        zp[i / 2] = __floats2bfloat162_rn(z0, z1);
-                        const float2 zf = __bfloat1622float2(zp[i / 2]);   // GELU of the stored (rounded) pre-activation
-                        hp[i / 2] = __floats2bfloat162_rn(gelu(zf.x), gelu(zf.y));
-                        if (g.HoutT) {   // transposed copy [column][row] for the weight-gradient GEMMs
-                            g.HoutT[(size_t)(col0 + i) * g.ldt + row] = __low2bfloat16(hp[i / 2]);
-                            g.HoutT[(size_t)(col0 + i + 1) * g.ldt + row] = __high2bfloat16(hp[i / 2]);
-                        }
-                    }
-                    uint4* zo = reinterpret_cast<uint4*>(g.Zout + (size_t)row * g.ldc + col0);
-                    uint4* ho = reinterpret_cast<uint4*>(g.Hout + (size_t)row * g.ldc + col0);
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        zo[q] = *reinterpret_cast<const uint4*>(zp + 4 * q);
-                        ho[q] = *reinterpret_cast<const uint4*>(hp + 4 * q);
-                    }
-                } else {
-                    const uint4* zi = reinterpret_cast<const uint4*>(g.Zin + (size_t)row * g.ldc + col0);
-                    __nv_bfloat162 zin[16], dp[16];
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) *reinterpret_cast<uint4*>(zin + 4 * q) = zi[q];
-#pragma unroll
-                    for (int i = 0; i < 32; i += 2) {
-                        const float2 z = __bfloat1622float2(zin[i / 2]);
-                        dp[i / 2] = __floats2bfloat162_rn(v[i] * gelu_grad(z.x), v[i + 1] * gelu_grad(z.y));
-                        if (g.dZT) {
-                            g.dZT[(size_t)(col0 + i) * g.ldt + row] = __low2bfloat16(dp[i / 2]);
-                            g.dZT[(size_t)(col0 + i + 1) * g.ldt + row] = __high2bfloat16(dp[i / 2]);
-                        }
-                    }
-                    uint4* dz = reinterpret_cast<uint4*>(g.dZ + (size_t)row * g.ldc + col0);
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) dz[q] = *reinterpret_cast<const uint4*>(dp + 4 * q);
+                        *reinterpret_cast<float4*>(out + cb + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
                 }
             }
         }
@@ -266,29 +340,7 @@ k_gemm_tma(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
         for (int c = n_consumed; c < n_issued; ++c) (void)tc::mbar_wait(tc::smem_addr(&full[c % kStages]), (c / kStages) & 1);
     }
     __syncthreads();
-    if (warp == 1) tc::tmem_dealloc(tmem, 256);
-}
-
-// [rows x cols] -> [cols x rows] (bf16), 32 x 32 tiles through shared memory
-__global__ void k_transpose_bf16(const bf16* __restrict__ src, int rows, int cols, int lds, bf16* __restrict__ dst,
-                                 int ldd) {
-    __shared__ bf16 t[32][33];
-    const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
-    for (int i = threadIdx.y; i < 32; i += blockDim.y) {
-        const int r = r0 + i, c = c0 + threadIdx.x;
-        if (r < rows && c < cols) t[i][threadIdx.x] = src[(size_t)r * lds + c];
-    }
-    __syncthreads();
-    for (int i = threadIdx.y; i < 32; i += blockDim.y) {
-        const int c = c0 + i, r = r0 + threadIdx.x;
-        if (r < rows && c < cols) dst[(size_t)c * ldd + r] = t[threadIdx.x][i];
-    }
-}
-
-cudaError_t transpose_bf16(const bf16* src, int rows, int cols, int lds, bf16* dst, int ldd, cudaStream_t s) {
-    if (rows <= 0 || cols <= 0) return cudaSuccess;
-    k_transpose_bf16<<<dim3((cols + 31) / 32, (rows + 31) / 32), dim3(32, 8), 0, s>>>(src, rows, cols, lds, dst, ldd);
-    return cudaGetLastError();
+    if (warp == 1) tc::tmem_dealloc(tmem, BN);
 }
 
 // cuTensorMapEncodeTiled through the runtime's driver entry point (no link to the driver library)
@@ -311,40 +363,265 @@ EncodeTiledFn encode_tiled() {
     return fn;
 }
 
-// tensor map of a K-major bf16 operand [rows x K] (row stride ld elements): boxes of 64 K x
-// box_rows, 128-byte swizzled in shared memory
-cudaError_t operand_map(CUtensorMap* map, const bf16* base, int rows, int K, int ld, int box_rows) {
+// Tensor map of a bf16 operand of `rows` rows (or columns) x K with row stride ld, 128-byte swizzled in
+// shared memory, as three dimensions so that one load brings a tile's K chunk either way: K-major
+// {K, rows, 1} in boxes of 64 x box_rows; M/N-major (element (k, r) at k * ld + r) {64, K, rows / 64} in
+// boxes of 64 x 64 x box_rows / 64, blocks of 64 columns one after the other.
+cudaError_t operand_map(CUtensorMap* map, const bf16* base, bool mn_major, int rows, int K, int ld, int box_rows) {
     EncodeTiledFn enc = encode_tiled();
     if (!enc) return cudaErrorNotSupported;
     if (((uintptr_t)base & 15) || (ld * 2) % 16) return cudaErrorInvalidValue;
-    const cuuint64_t dim[2] = {(cuuint64_t)K, (cuuint64_t)rows};
-    const cuuint64_t stride[1] = {(cuuint64_t)ld * 2};
-    const cuuint32_t box[2] = {(cuuint32_t)tc::kKChunk, (cuuint32_t)box_rows};   // 128-byte rows
-    const cuuint32_t estr[2] = {1, 1};
-    const CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<bf16*>(base), dim, stride, box, estr,
+    const cuuint64_t dim[3] = {(cuuint64_t)(mn_major ? 64 : K), (cuuint64_t)(mn_major ? K : rows),
+                               (cuuint64_t)(mn_major ? rows / 64 : 1)};
+    const cuuint64_t stride[2] = {(cuuint64_t)ld * 2, 128};
+    const cuuint32_t box[3] = {64u, (cuuint32_t)(mn_major ? tc::kKChunk : box_rows), (cuuint32_t)(mn_major ? box_rows / 64 : 1)};
+    const cuuint32_t estr[3] = {1, 1, 1};
+    const CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<bf16*>(base), dim, stride, box, estr,
                            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                            CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
+template <int BN>
+cudaError_t launch_gemm(const GemmArgs& g, cudaStream_t s) {
+    CUtensorMap ta, tb;
+    TRY(operand_map(&ta, g.A, g.a_t, g.M, g.K, g.lda, kBM));
+    TRY(operand_map(&tb, g.B, g.b_t, g.N, g.K, g.ldb, BN));
+    static std::atomic<unsigned long long> attr{0};
+    TRY(ensure_smem_attr(k_gemm_tma<BN>, (int)kGemmSmem, attr));
+    k_gemm_tma<BN><<<dim3(g.N / BN, g.M / kBM, (g.K + g.ksplit - 1) / g.ksplit), kGemmThreads, kGemmSmem, s>>>(ta, tb, g);
+    return cudaGetLastError();
+}
+
+// The widest tiles that still give two thirds of the SMs a CTA: A is read once per tile column, but a
+// batch that splits badly (the single chain of an odd number of 128-ray tiles) leaves most SMs idle:
+// two steps of 32,640 rays take 2.0 ms so, 2.7 in 256-wide tiles, 2.5 before.
 cudaError_t gemm(GemmArgs g, cudaStream_t s) {
     if (g.M % kBM || g.N % kBN || g.K % tc::kKChunk || g.K <= 0) return cudaErrorInvalidValue;
-    if (g.a_t || g.b_t) return cudaErrorInvalidValue;   // operands are K-major (transposed copies are made)
     if (g.ksplit <= 0) g.ksplit = g.K;
-    if (g.K % g.ksplit || g.ksplit % tc::kKChunk) return cudaErrorInvalidValue;
-    if (g.ksplit != g.K && g.epi != EPI_F32_ADD) return cudaErrorInvalidValue;
-    CUtensorMap ta, tb;
-    if (cudaError_t e = operand_map(&ta, g.A, g.M, g.K, g.lda, kBM)) return e;
-    if (cudaError_t e = operand_map(&tb, g.B, g.N, g.K, g.ldb, kBN)) return e;
-    static std::atomic<unsigned long long> attr2{0}, attr4{0};
-    dim3 grid(g.N / kBN, g.M / kBM, g.K / g.ksplit);
-    if (g.ksplit / tc::kKChunk > 8) {
-        if (cudaError_t e = ensure_smem_attr(k_gemm_tma<4>, (int)tma_smem<4>(), attr4)) return e;
-        k_gemm_tma<4><<<grid, kGemmThreads, tma_smem<4>(), s>>>(ta, tb, g);
-    } else {
-        if (cudaError_t e = ensure_smem_attr(k_gemm_tma<2>, (int)tma_smem<2>(), attr2)) return e;
-        k_gemm_tma<2><<<grid, kGemmThreads, tma_smem<2>(), s>>>(ta, tb, g);
+    if (g.ksplit % tc::kKChunk || (g.ksplit < g.K && !g.part_stride)) return cudaErrorInvalidValue;
+    const long long tiles = (long long)(g.M / kBM) * (g.N / kBN) * ((g.K + g.ksplit - 1) / g.ksplit);
+    return tiles >= 96 ? launch_gemm<256>(g, s) : tiles >= 48 ? launch_gemm<128>(g, s) : launch_gemm<64>(g, s);
+}
+
+// ------------------------------------------------------------ layer GEMM
+// The forward and input-gradient GEMMs of one layer: `rows` rows of A [rows x K] against the layer's
+// weights, K = 512 or 256, as a persistent kernel, one CTA per SM.  Its weights (128 KB: all 256
+// columns for K = 256, half of them for K = 512) stay in shared memory; the rows come through a ring
+// of five 16 KB stages, and the accumulator has two buffers in TMEM, so that the tensor cores and the
+// loads of the next 128 rows run beside the epilogue of these.  Bound by its bytes (a forward layer of
+// 65,536 rays reads 33 and writes 67 MB); one CTA per tile, with its weights read again each time and
+// nothing beside its epilogue, took 32 us for it (45-49 with the transposed copies), this 25; input gradients 46 -> 26.
+//   FWD:  z = acc + bias, rounded to bf16, to Zout; GELU of it to Hout.  Weights [out x in], K-major.
+//   else: acc * GELU'(Zin) to dZ.  The weights as they lie, [K = out][N = in]: N-major.
+// Roles as in k_gemm_tma; the waits are bounded in the same way.
+struct LayerArgs {
+    int rows;
+    const float* bias;   // FWD
+    bf16 *Zout, *Hout;
+    const bf16* Zin;     // input gradients
+    bf16* dZ;
+    unsigned* err;
+};
+constexpr int kLayerStages = 5;
+constexpr uint32_t kWeightBytes = 131072;
+constexpr size_t kLayerSmem = kWeightBytes + kLayerStages * (size_t)kStageA + 1024;
+
+template <int BN, int K, bool FWD>
+__global__ void __launch_bounds__(kGemmThreads, 1)
+k_layer(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmW, LayerArgs g) {
+    static_assert(BN * K * 2 == kWeightBytes && kHidden % BN == 0, "weights of a CTA");
+    constexpr int kChunks = K / tc::kKChunk, kParts = kHidden / BN;
+    constexpr uint32_t kWChunk = BN * tc::kKChunk * 2;
+    extern __shared__ uint8_t smem_raw[];
+    __shared__ __align__(8) uint64_t full[kLayerStages], empty[kLayerStages], wfull[kChunks], acc_full[2], acc_empty[2], drained;
+    __shared__ uint32_t tmem_base;
+    __shared__ int abort_flag, n_issued, n_consumed;
+    __shared__ __align__(16) float s_bias[BN];
+    uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    const uint32_t sW = tc::smem_addr(smem), sA = sW + kWeightBytes;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int n0 = (int)(blockIdx.x % kParts) * BN;
+    const int tile0 = blockIdx.x / kParts, tiles = g.rows / kBM, step = gridDim.x / kParts;
+    if (warp == 1) tc::tmem_alloc(tc::smem_addr(&tmem_base), 2 * BN);
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < kLayerStages; ++i) {
+            tc::mbar_init(tc::smem_addr(&full[i]), 1);
+            tc::mbar_init(tc::smem_addr(&empty[i]), 1);
+        }
+        for (int c = 0; c < kChunks; ++c) tc::mbar_init(tc::smem_addr(&wfull[c]), 1);
+        for (int i = 0; i < 2; ++i) {
+            tc::mbar_init(tc::smem_addr(&acc_full[i]), 1);
+            tc::mbar_init(tc::smem_addr(&acc_empty[i]), kEpiWarps);
+        }
+        tc::mbar_init(tc::smem_addr(&drained), 1);
+        abort_flag = 0;
+        n_issued = 0;
+        n_consumed = 0;
+        tc::fence_mbar_init();
     }
+    if (FWD)
+        for (int i = threadIdx.x; i < BN; i += kGemmThreads) s_bias[i] = __ldg(g.bias + n0 + i);
+    tc::fence_before_sync();
+    __syncthreads();
+    tc::fence_after_sync();
+    const uint32_t tmem = tmem_base;
+    auto aborted = [&]() { return *(volatile int*)&abort_flag != 0; };
+    auto give_up = [&]() {
+        atomicOr(g.err, 16u);
+        atomicExch(&abort_flag, 1);
+    };
+    if (warp == 0 && lane == 0) {
+        // ---- producer: the chunks of the CTA's row tiles, one after the other, go round the stages
+        tc::tma_prefetch_map(&tmA);
+        tc::tma_prefetch_map(&tmW);
+        int n = 0, st = 0, phase = 1;
+        bool ok = true;
+        for (int t = tile0; t < tiles && ok; t += step) {
+            for (int c = 0; c < kChunks; ++c, ++n) {
+                if (n >= kLayerStages && !tc::mbar_wait(tc::smem_addr(&empty[st]), phase)) {
+                    give_up();
+                    ok = false;
+                    break;
+                }
+                if (t == tile0) {   // the weights of this K chunk come with the first tile's
+                    const uint32_t wb = tc::smem_addr(&wfull[c]);
+                    tc::mbar_arrive_expect_tx(wb, kWChunk);
+                    tc::tma_load_3d(sW + c * kWChunk, &tmW, FWD ? c * tc::kKChunk : 0, FWD ? n0 : c * tc::kKChunk, FWD ? 0 : n0 / 64, wb);
+                }
+                const uint32_t fb = tc::smem_addr(&full[st]);
+                tc::mbar_arrive_expect_tx(fb, kStageA);
+                tc::tma_load_3d(sA + st * kStageA, &tmA, c * tc::kKChunk, t * kBM, 0, fb);
+                if (++st == kLayerStages) {
+                    st = 0;
+                    phase ^= 1;
+                }
+            }
+        }
+        n_issued = n;
+    } else if (warp == 1 && lane == 0) {
+        // ---- MMA issuer: the CTA's i-th tile accumulates in TMEM buffer i & 1
+        const uint32_t idesc = tc::make_idesc(kBM, BN) | (FWD ? 0u : tc::kIdescTransposeB);
+        const uint64_t a0 = tc::make_desc_sw128(sA);
+        const uint64_t w0 = FWD ? tc::make_desc_sw128(sW) : tc::make_desc_sw128_mn(sW, kBlockMN);
+        constexpr uint32_t kWStep = (FWD ? 32 : 16 * 128) >> 4;
+        int n = 0, i = 0, st = 0, phase = 0;
+        bool ok = true;
+        for (int t = tile0; t < tiles && ok; t += step, ++i) {
+            const uint32_t acc = tmem + (uint32_t)(i & 1) * BN;
+            if (i >= 2) ok = tc::mbar_wait(tc::smem_addr(&acc_empty[i & 1]), ((i >> 1) - 1) & 1);
+            tc::fence_after_sync();
+            for (int c = 0; c < kChunks && ok; ++c) {
+                if (i == 0) ok = tc::mbar_wait(tc::smem_addr(&wfull[c]), 0);
+                if (ok) ok = tc::mbar_wait(tc::smem_addr(&full[st]), phase);
+                if (!ok) break;
+                tc::fence_after_sync();
+#pragma unroll
+                for (int ks = 0; ks < tc::kKChunk / 16; ++ks)
+                    tc::mma_bf16(acc, a0 + (uint32_t)(st * (kStageA >> 4) + ks * 2), w0 + (c * (kWChunk >> 4) + ks * kWStep), idesc,
+                                 (c > 0 || ks > 0) ? 1u : 0u);
+                tc::mma_commit(tc::smem_addr(&empty[st]));
+                ++n;
+                if (++st == kLayerStages) {
+                    st = 0;
+                    phase ^= 1;
+                }
+            }
+            if (ok) tc::mma_commit(tc::smem_addr(&acc_full[i & 1]));
+        }
+        n_consumed = n;
+        if (!ok) {   // let what was issued end before the TMEM is freed
+            give_up();
+            tc::mma_commit(tc::smem_addr(&drained));
+            (void)tc::mbar_wait(tc::smem_addr(&drained), 0);
+        }
+    } else if (warp >= 2) {
+        // ---- epilogue
+        constexpr int kCols = BN / (kEpiWarps / 4);
+        const int lq = warp & 3, c0 = (warp - 2) / 4 * kCols;   // TMEM lane quarter and columns of this warp
+        int i = 0;
+        for (int t = tile0; t < tiles; t += step, ++i) {
+            const size_t at = (size_t)(t * kBM + lq * 32 + lane) * kHidden + n0 + c0;
+            uint32_t zin[16];
+            if (!FWD) {
+                load32(g.Zin + at, zin);
+                load32(g.Zin + at + 16, zin + 8);
+            }
+            const bool ok = __all_sync(0xffffffffu, tc::mbar_wait(tc::smem_addr(&acc_full[i & 1]), (i >> 1) & 1) && !aborted());
+            tc::fence_after_sync();
+            if (!ok) {
+                if (lane == 0) give_up();
+                break;
+            }
+            const uint32_t acc = tmem + (uint32_t)(i & 1) * BN + ((uint32_t)(lq * 32) << 16) + c0;
+#pragma unroll
+            for (int cb = 0; cb < kCols; cb += 32) {
+                float v[32];
+                tc::tmem_ld32(acc + cb, v);
+                if (cb + 32 == kCols) {   // the accumulator is read: the next but one tile may have it
+                    tc::fence_before_sync();
+                    __syncwarp();
+                    if (lane == 0) tc::mbar_arrive(tc::smem_addr(&acc_empty[i & 1]));
+                }
+                if (FWD) {
+                    uint32_t zp[16], hp[16];
+#pragma unroll
+                    for (int q = 0; q < 32; q += 4) {
+                        const float4 b = *reinterpret_cast<const float4*>(s_bias + c0 + cb + q);
+                        const float2 a0 = unpack2(add2(pack2(v[q], v[q + 1]), pack2(b.x, b.y)));
+                        const float2 a1 = unpack2(add2(pack2(v[q + 2], v[q + 3]), pack2(b.z, b.w)));
+                        zp[q / 2] = pack_bf16(a0.x, a0.y);
+                        zp[q / 2 + 1] = pack_bf16(a1.x, a1.y);
+                        // GELU of the stored (rounded) pre-activation
+                        const float2 h0 = gelu(widen_bf16(zp[q / 2])), h1 = gelu(widen_bf16(zp[q / 2 + 1]));
+                        hp[q / 2] = pack_bf16(h0.x, h0.y);
+                        hp[q / 2 + 1] = pack_bf16(h1.x, h1.y);
+                    }
+                    store32(g.Zout + at + cb, zp);
+                    store32(g.Zout + at + cb + 16, zp + 8);
+                    store32(g.Hout + at + cb, hp);
+                    store32(g.Hout + at + cb + 16, hp + 8);
+                } else {
+                    uint32_t dp[16];
+#pragma unroll
+                    for (int q = 0; q < 32; q += 2) {
+                        const float2 d = unpack2(mul2(pack2(v[q], v[q + 1]), gelu_grad(widen_bf16(zin[q / 2]))));
+                        dp[q / 2] = pack_bf16(d.x, d.y);
+                    }
+                    if (cb + 32 < kCols) {   // the next columns' pre-activations beside this store and TMEM read
+                        load32(g.Zin + at + cb + 32, zin);
+                        load32(g.Zin + at + cb + 48, zin + 8);
+                    }
+                    store32(g.dZ + at + cb, dp);
+                    store32(g.dZ + at + cb + 16, dp + 8);
+                }
+            }
+        }
+    }
+    tc::fence_before_sync();
+    __syncthreads();
+    if (abort_flag && threadIdx.x == 0) {
+        // loads issued but never waited for are still landing in this CTA's shared memory: wait for
+        // them (bounded) before the CTA exits
+        for (int c = 0; c < min(kChunks, n_issued); ++c) (void)tc::mbar_wait(tc::smem_addr(&wfull[c]), 0);
+        for (int n = n_consumed; n < n_issued; ++n)
+            (void)tc::mbar_wait(tc::smem_addr(&full[n % kLayerStages]), (n / kLayerStages) & 1);
+    }
+    __syncthreads();
+    if (warp == 1) tc::tmem_dealloc(tmem, 2 * BN);
+}
+
+// rows: a multiple of 128; A [rows x K], W the layer's weights [256 x K] (FWD) or [K][256]
+template <int BN, int K, bool FWD>
+cudaError_t layer(const bf16* A, const bf16* W, const LayerArgs& g, cudaStream_t s) {
+    CUtensorMap ta, tw;
+    TRY(operand_map(&ta, A, false, g.rows, K, K, kBM));
+    TRY(operand_map(&tw, W, !FWD, kHidden, K, FWD ? K : kHidden, BN));
+    static std::atomic<unsigned long long> attr{0};
+    TRY(ensure_smem_attr(k_layer<BN, K, FWD>, (int)kLayerSmem, attr));
+    constexpr int kParts = kHidden / BN;
+    const int grid = std::min(152 / kParts, g.rows / kBM) * kParts;
+    k_layer<BN, K, FWD><<<grid, kGemmThreads, kLayerSmem, s>>>(ta, tw, g);
     return cudaGetLastError();
 }
 
@@ -354,33 +631,44 @@ struct FeatParams {
     float freq[64];
 };
 
-__device__ __forceinline__ void ray_features(const FeatParams& fp, float x, float y, float th, bf16* out) {
-    float s, c;
-    sincosf(th, &s, &c);
-    const float u[4] = {x * fp.inv_w, y * fp.inv_h, c, s};
+// Features of grid-frame rays (x, y, theta), one row per warp at a time: lane l computes frequencies l
+// and l + 32 of each input, so that a row's 1 KB leaves in whole lines (one row per thread before: 108
+// us for 65,536 rows, now 22).  Rows from n on are zero.
+constexpr int kFeatRows = 8;   // rows per warp
+
+__global__ void __launch_bounds__(256) k_features(FeatParams fp, const float* __restrict__ xyt, int n, int n_pad,
+                                                  bf16* __restrict__ X) {
+    __shared__ float s_freq[64];
+    if (threadIdx.x < 64) s_freq[threadIdx.x] = fp.freq[threadIdx.x];
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    const float f0 = s_freq[lane], f1 = s_freq[lane + 32];
+    const int r0 = (blockIdx.x * 8 + (threadIdx.x >> 5)) * kFeatRows;
+    for (int r = r0; r < min(r0 + kFeatRows, n_pad); ++r) {
+        uint32_t* out = reinterpret_cast<uint32_t*>(X + (size_t)r * kFeat) + lane;
+        if (r >= n) {
 #pragma unroll
-    for (int d = 0; d < 4; ++d) {
-        for (int k = 0; k < 64; k += 2) {
+            for (int j = 0; j < kFeat / 64; ++j) out[j * 32] = 0u;
+            continue;
+        }
+        float s, c;
+        sincosf(__ldg(xyt + 3 * (size_t)r + 2), &s, &c);
+        const float u[4] = {__ldg(xyt + 3 * (size_t)r) * fp.inv_w, __ldg(xyt + 3 * (size_t)r + 1) * fp.inv_h, c, s};
+#pragma unroll
+        for (int d = 0; d < 4; ++d) {
             float s0, c0, s1, c1;
-            sincospif(fp.freq[k] * u[d], &s0, &c0);
-            sincospif(fp.freq[k + 1] * u[d], &s1, &c1);
-            __nv_bfloat162* o = reinterpret_cast<__nv_bfloat162*>(out + d * 128 + k * 2);
-            o[0] = __floats2bfloat162_rn(s0, c0);
-            o[1] = __floats2bfloat162_rn(s1, c1);
+            sincospif(f0 * u[d], &s0, &c0);
+            sincospif(f1 * u[d], &s1, &c1);
+            out[d * 64] = pack_bf16(s0, c0);
+            out[d * 64 + 32] = pack_bf16(s1, c1);
         }
     }
 }
 
-// rays given as grid-frame (x, y, theta) triples
-__global__ void k_features(FeatParams fp, const float* __restrict__ xyt, int n, int n_pad, bf16* __restrict__ X) {
-    int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= n_pad) return;
-    bf16* out = X + (size_t)r * kFeat;
-    if (r >= n) {
-        for (int j = 0; j < kFeat; j += 8) *reinterpret_cast<uint4*>(out + j) = make_uint4(0, 0, 0, 0);
-        return;
-    }
-    ray_features(fp, xyt[3 * (size_t)r], xyt[3 * (size_t)r + 1], xyt[3 * (size_t)r + 2], out);
+cudaError_t launch_features(const FeatParams& fp, const float* xyt, int n, int rows, bf16* X, cudaStream_t s) {
+    if (rows <= 0) return cudaSuccess;
+    k_features<<<(rows + 8 * kFeatRows - 1) / (8 * kFeatRows), 256, 0, s>>>(fp, xyt, n, rows, X);
+    return cudaGetLastError();
 }
 
 // ------------------------------------------------------ fused forward pass
@@ -570,9 +858,8 @@ __global__ void __launch_bounds__(kFwdThreads, 2) k_mlp_forward(FeatParams fp, c
 #pragma unroll
             for (int i = 0; i < 32; i += 2) {
                 const float z0 = v[i] + __ldg(bias + cb + i), z1 = v[i + 1] + __ldg(bias + cb + i + 1);
-                const float2 zf = __bfloat1622float2(__floats2bfloat162_rn(z0, z1));
-                *reinterpret_cast<__nv_bfloat162*>(sH + act_offset(row, cb + i)) =
-                    __floats2bfloat162_rn(gelu(zf.x), gelu(zf.y));
+                const float2 h = gelu(widen_bf16(pack_bf16(z0, z1)));
+                *reinterpret_cast<uint32_t*>(sH + act_offset(row, cb + i)) = pack_bf16(h.x, h.y);
             }
         }
         tc::fence_before_sync();   // TMEM reads done before the next layer's MMAs overwrite it
@@ -637,80 +924,96 @@ __global__ void k_out_layer(const bf16* __restrict__ H, const float* __restrict_
 }
 
 // --------------------------------------------------------------- training
-// Huber loss (delta 1 px) against the target, mean over the batch; dy per ray.
-__global__ void k_loss(const float* __restrict__ y, const float* __restrict__ t, int n, float* __restrict__ dy,
-                       float* __restrict__ loss_sum) {
-    int r = blockIdx.x * blockDim.x + threadIdx.x;
-    float l = 0.0f;
-    if (r < n) {
-        const float e = y[r] - t[r];
-        const float ae = fabsf(e);
-        l = ae <= 1.0f ? 0.5f * e * e : ae - 0.5f;
-        dy[r] = (ae <= 1.0f ? e : copysignf(1.0f, e)) / (float)n;
-    }
-    for (int o = 16; o; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
-    if ((threadIdx.x & 31) == 0 && l != 0.0f) atomicAdd(loss_sum, l);
-}
+// The output layer of a training step in one pass over its activations H and pre-activations Z, a row
+// per warp: y = H . w + b (in k_out_layer's order), the Huber loss (delta 1 px) against the target and
+// its gradient dy (mean over the batch), dZ = dy * w * GELU'(Z), and the block's share of the layer's
+// gradients and of the loss in part[block] = {d w [256], d b, loss}.  Bound by its 3 x 512 bytes a row;
+// five kernels before (loss, backward, two column sums and the output layer: 113 us for 65,536 rows,
+// now 24).
+constexpr int kTopBlocks = 2 * 152, kTopThreads = 512;
+constexpr int kTopPart = kHidden + 2;
 
-// dZ of the last hidden layer = dy * w_out * GELU'(Z)
-__global__ void k_out_backward(const float* __restrict__ dy, const bf16* __restrict__ Z,
-                               const float* __restrict__ params, int n, bf16* __restrict__ dZ) {
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (warp >= n) return;
-    const float g = dy[warp];
-    const float* w = params + kOutW;
-    for (int j = lane; j < kHidden; j += 32) {
-        const size_t idx = (size_t)warp * kHidden + j;
-        dZ[idx] = __float2bfloat16_rn(g * w[j] * gelu_grad(__bfloat162float(Z[idx])));
-    }
-}
-
-// Column sums over rows of a [n x 256] bf16 matrix, each row weighted by w[r] (or 1): a block of
-// 128 threads covers the 256 columns two per thread (one 4-byte load per row), its rows strided by
-// the grid and four in flight per thread, then one atomic per column and block.
-constexpr int kColSumBlocks = 4 * 152;
-__device__ __forceinline__ void column_sums(const bf16* __restrict__ M, const float* __restrict__ w, int n,
-                                            float* __restrict__ out, float* __restrict__ wsum) {
-    const int c = 2 * threadIdx.x;
-    float a0 = 0.0f, a1 = 0.0f, s = 0.0f;
-    int r = blockIdx.x;
-    for (; r + 3 * (int)gridDim.x < n; r += 4 * gridDim.x) {
-        float2 v[4];
-        float g[4];
+__global__ void __launch_bounds__(kTopThreads) k_top(const bf16* __restrict__ H, const bf16* __restrict__ Z,
+                                                     const float* __restrict__ params, const float* __restrict__ target,
+                                                     int n, bf16* __restrict__ dZ, float* __restrict__ part) {
+    __shared__ float s_part[kTopThreads / 32][kTopPart];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const float* wo = params + kOutW;
+    float w[8], dw[8], db = 0.0f, loss = 0.0f;
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int ru = r + u * gridDim.x;
-            v[u] = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(M + (size_t)ru * kHidden + c));
-            g[u] = w ? __ldg(w + ru) : 1.0f;
+    for (int i = 0; i < 8; ++i) {
+        w[i] = __ldg(wo + lane + 32 * i);
+        dw[i] = 0.0f;
+    }
+    const float b = __ldg(wo + kHidden);
+    const int warps = gridDim.x * (kTopThreads / 32);
+#pragma unroll 2
+    for (int r = blockIdx.x * (kTopThreads / 32) + warp; r < n; r += warps) {
+        const size_t base = (size_t)r * kHidden + lane;
+        float h[8], z[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            h[i] = __bfloat162float(H[base + 32 * i]);
+            z[i] = __bfloat162float(Z[base + 32 * i]);
+        }
+        const float t = __ldg(target + r);
+        float acc = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) acc += h[i] * w[i];
+        for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        const float e = (acc + b) - t, ae = fabsf(e);
+        const float dy = (ae <= 1.0f ? e : copysignf(1.0f, e)) / (float)n;
+        loss += ae <= 1.0f ? 0.5f * e * e : ae - 0.5f;
+        db += dy;
+#pragma unroll
+        for (int i = 0; i < 8; i += 2) {
+            const float2 d = unpack2(mul2(mul2(both(dy), pack2(w[i], w[i + 1])), gelu_grad(pack2(z[i], z[i + 1]))));
+            dZ[base + 32 * i] = __float2bfloat16_rn(d.x);
+            dZ[base + 32 * i + 32] = __float2bfloat16_rn(d.y);
         }
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            a0 += g[u] * v[u].x;
-            a1 += g[u] * v[u].y;
-            s += g[u];
+        for (int i = 0; i < 8; ++i) {
+            dw[i] += dy * h[i];
         }
     }
-    for (; r < n; r += gridDim.x) {
-        const float2 v = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(M + (size_t)r * kHidden + c));
-        const float g = w ? __ldg(w + r) : 1.0f;
-        a0 += g * v.x;
-        a1 += g * v.y;
-        s += g;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) s_part[warp][lane + 32 * i] = dw[i];
+    if (lane == 0) {
+        s_part[warp][kHidden] = db;
+        s_part[warp][kHidden + 1] = loss;
     }
-    atomicAdd(out + c, a0);
-    atomicAdd(out + c + 1, a1);
-    if (wsum && threadIdx.x == 0) atomicAdd(wsum, s);
+    __syncthreads();
+    for (int j = threadIdx.x; j < kTopPart; j += kTopThreads) {
+        float sum = 0.0f;
+        for (int k = 0; k < kTopThreads / 32; ++k) sum += s_part[k][j];
+        part[(size_t)blockIdx.x * kTopPart + j] = sum;
+    }
 }
 
-// output-layer gradients: d w_out[j] = sum_r dy[r] H[r][j], d b_out = sum_r dy[r]
-__global__ void __launch_bounds__(128) k_out_wgrad(const float* __restrict__ dy, const bf16* __restrict__ H, int n,
-                                                   float* __restrict__ grads) {
-    column_sums(H, dy, n, grads + kOutW, grads + kOutW + kHidden);
-}
-
-// column sums of dZ [n x 256] -> bias gradient
-__global__ void __launch_bounds__(128) k_bias_grad(const bf16* __restrict__ dZ, int n, float* __restrict__ gb) {
-    column_sums(dZ, nullptr, n, gb, nullptr);
+// The gradients from their partial sums, always added in the same order: the hidden layers' from the
+// K splits of the weight-gradient GEMMs (part[z][kOutW], the flat parameter layout), the output
+// layer's and the loss from k_top's blocks.  A run repeats bit for bit; the sums were atomic before.
+__global__ void __launch_bounds__(256) k_reduce_grads(const float* __restrict__ part, int splits,
+                                                      const float* __restrict__ top, float* __restrict__ grads,
+                                                      float* __restrict__ loss) {
+    constexpr unsigned kHiddenBlocks = (unsigned)(kOutW / 256);
+    if (blockIdx.x < kHiddenBlocks) {
+        const size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;
+        float sum = 0.0f;
+#pragma unroll 16
+        for (int z = 0; z < splits; ++z) sum += __ldg(part + (size_t)z * kOutW + i);
+        grads[i] = sum;
+        return;
+    }
+    const int j = (int)(blockIdx.x - kHiddenBlocks) * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (j >= kTopPart) return;
+    float sum = 0.0f;
+    for (int k = lane; k < kTopBlocks; k += 32) sum += __ldg(top + (size_t)k * kTopPart + j);
+    for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if (lane == 0) {
+        if (j <= kHidden) grads[kOutW + j] = sum;
+        else *loss = sum;
+    }
 }
 
 // Adam (bias-corrected), fp32 master weights; refreshes the bf16 copies
@@ -761,17 +1064,26 @@ __global__ void k_init_params(float* __restrict__ p, uint32_t seed, float init_b
 // t = max_range when the ray leaves the map or runs out of range.
 __device__ float march_t(const MapDev& m, float mr, float x0, float y0, float c, float s, float* range) {
     float t = 0.0f;
+    const unsigned W = (unsigned)m.W, H = (unsigned)m.H;
     while (t < mr) {
-        int px = __float2int_rz(__fadd_rn(x0, __fmul_rn(c, t)));
-        int py = __float2int_rz(__fadd_rn(y0, __fmul_rn(s, t)));
-        if ((unsigned)px >= (unsigned)m.W || (unsigned)py >= (unsigned)m.H) break;
-        float d = __ldg(m.dt + (size_t)px * m.H + py);
-        if (d <= 0.0f) {
-            float xd = __fsub_rn(__int2float_rn(px), x0), yd = __fsub_rn(__int2float_rn(py), y0);
+        unsigned px = (unsigned)__float2int_rz(__fadd_rn(x0, __fmul_rn(c, t)));
+        unsigned py = (unsigned)__float2int_rz(__fadd_rn(y0, __fmul_rn(s, t)));
+        float st;
+        if (m.step) {   // NaN on occupied cells, +inf off the grid (MapDev::step)
+            px = min(px, W);
+            py = min(py, H);
+            st = __ldg(m.step + (px * (H + 1u) + py));
+        } else {
+            if (px >= W || py >= H) break;
+            const float d = __ldg(m.dt + (size_t)px * m.H + py);
+            st = d <= 0.0f ? __int_as_float(0x7fc00000) : fmaxf(__fmul_rn(d, 0.999f), 1.0f);
+        }
+        if (isnan(st)) {
+            float xd = __fsub_rn(__int2float_rn((int)px), x0), yd = __fsub_rn(__int2float_rn((int)py), y0);
             *range = __fsqrt_rn(__fadd_rn(__fmul_rn(xd, xd), __fmul_rn(yd, yd)));
             return t;
         }
-        t = __fadd_rn(t, fmaxf(__fmul_rn(d, 0.999f), 1.0f));
+        t = __fadd_rn(t, st);
     }
     *range = mr;
     return mr;
@@ -880,8 +1192,6 @@ __global__ void k_world_rays(WorldDev w, const float* __restrict__ ins, const fl
 
 inline unsigned blocks_for(long long n, int b) { return (unsigned)((n + b - 1) / b); }
 
-#define TRY(x) do { cudaError_t _e = (x); if (_e != cudaSuccess) return _e; } while (0)
-
 }  // namespace
 
 // ================================================================ host side
@@ -903,14 +1213,10 @@ struct LearnedModel {
     bf16* Z[kLayers] = {};             // pre-activations [cap x 256]
     bf16* Hh[kLayers] = {};            // activations
     bf16* dZ[2] = {};                  // ping-pong gradients
-    // transposed copies, [column x cap]: the K-major operands of the weight-gradient GEMMs
-    bf16* XT = nullptr;                // features [512 x cap]
-    bf16* HT[kLayers - 1] = {};        // activations of layers 0-2 [256 x cap]
-    bf16* dZT = nullptr;               // the current layer's gradient [256 x cap]
-    bf16* wbfT = nullptr;              // weights of layers 1-3 transposed [in x out] (input gradients)
+    float* wpart = nullptr;            // partial gradients of the hidden layers [kMaxSplits][kOutW]
+    float* tpart = nullptr;            // and of the output layer [kTopBlocks][kTopPart]
     float* y = nullptr;
-    float* dy = nullptr;
-    float* loss = nullptr;
+    float* loss = nullptr;             // of the last kLossSlots steps
     float* ray_xyt = nullptr;          // the rays of a training step [cap x 3] and their targets
     float* ray_t = nullptr;
     uint32_t* free_cells = nullptr;
@@ -938,11 +1244,9 @@ struct LearnedModel {
         cudaFree(X);
         for (int l = 0; l < kLayers; ++l) { cudaFree(Z[l]); cudaFree(Hh[l]); Z[l] = Hh[l] = nullptr; }
         cudaFree(dZ[0]); cudaFree(dZ[1]);
-        cudaFree(XT); cudaFree(dZT); cudaFree(wbfT);
-        for (int l = 0; l < kLayers - 1; ++l) { cudaFree(HT[l]); HT[l] = nullptr; }
-        cudaFree(y); cudaFree(dy); cudaFree(loss); cudaFree(ray_xyt); cudaFree(ray_t);
-        X = nullptr; dZ[0] = dZ[1] = nullptr; y = dy = loss = ray_xyt = ray_t = nullptr;
-        XT = dZT = wbfT = nullptr;
+        cudaFree(wpart); cudaFree(tpart);
+        cudaFree(y); cudaFree(loss); cudaFree(ray_xyt); cudaFree(ray_t);
+        X = nullptr; dZ[0] = dZ[1] = nullptr; y = loss = ray_xyt = ray_t = wpart = tpart = nullptr;
         cap = 0;
     }
     ~LearnedModel() {
@@ -962,23 +1266,24 @@ struct LearnedModel {
         }
         TRY(cudaMalloc(&dZ[0], (size_t)rows * kHidden * sizeof(bf16)));
         TRY(cudaMalloc(&dZ[1], (size_t)rows * kHidden * sizeof(bf16)));
-        TRY(cudaMalloc(&XT, (size_t)rows * kFeat * sizeof(bf16)));
-        for (int l = 0; l < kLayers - 1; ++l) TRY(cudaMalloc(&HT[l], (size_t)rows * kHidden * sizeof(bf16)));
-        TRY(cudaMalloc(&dZT, (size_t)rows * kHidden * sizeof(bf16)));
-        TRY(cudaMalloc(&wbfT, (size_t)(kLayers - 1) * kWh * sizeof(bf16)));
+        TRY(cudaMalloc(&wpart, (size_t)std::min(kMaxSplits, std::max(1, rows / 256)) * kOutW * sizeof(float)));
+        TRY(cudaMalloc(&tpart, (size_t)kTopBlocks * kTopPart * sizeof(float)));
         TRY(cudaMalloc(&y, (size_t)rows * sizeof(float)));
-        TRY(cudaMalloc(&dy, (size_t)rows * sizeof(float)));
-        TRY(cudaMalloc(&loss, sizeof(float)));
+        TRY(cudaMalloc(&loss, (kLossSlots + 1) * sizeof(float)));
         TRY(cudaMalloc(&ray_xyt, (size_t)rows * 3 * sizeof(float)));
         TRY(cudaMalloc(&ray_t, (size_t)rows * sizeof(float)));
         cap = rows;
         return cudaSuccess;
     }
 
-    // K split of the weight-gradient GEMMs: chunks of >= 256 rows, at most 64 splits
+    // K split of the weight-gradient GEMMs: equal chunks of >= 256 rows, at most kMaxSplits.  The split
+    // is part of the result: where a gradient nearly cancels, Adam turns another order of its sum into
+    // another step.
+    static constexpr int kMaxSplits = 64;
+    static constexpr int kLossSlots = 20;
     static int split_k(int rows) {
         int sp = rows;
-        for (int parts = 64; parts > 1; parts >>= 1)
+        for (int parts = kMaxSplits; parts > 1; parts >>= 1)
             if (rows % (parts * 256) == 0) { sp = rows / parts; break; }
         return sp;
     }
@@ -991,67 +1296,55 @@ struct LearnedModel {
 
     // forward over `rows` rays whose features are in X; predictions in y
     cudaError_t forward(int rows, cudaStream_t s) {
-        const bf16* in = X;
-        for (int l = 0; l < kLayers; ++l) {
-            GemmArgs g = base_args();
-            g.A = in; g.lda = layer_in(l); g.a_t = 0;
-            g.B = wbf + w_offset(l); g.ldb = layer_in(l); g.b_t = 0;   // W [out x in]: N x K, K-major
-            g.M = rows; g.N = kHidden; g.K = layer_in(l);
-            g.epi = EPI_FWD; g.ldc = kHidden;
-            g.bias = params + b_offset(l);
-            g.Zout = Z[l]; g.Hout = Hh[l];
-            if (l < kLayers - 1) { g.HoutT = HT[l]; g.ldt = cap; }
-            TRY(gemm(g, s));
-            in = Hh[l];
-        }
+        TRY(forward_hidden(rows, s));
         k_out_layer<<<blocks_for((long long)rows * 32, 256), 256, 0, s>>>(Hh[kLayers - 1], params, rows, y);
         return cudaGetLastError();
     }
 
-    // backward from dy (rows rays, features in X, forward state in Z/Hh); gradients into grads
-    cudaError_t backward(int rows, cudaStream_t s) {
-        TRY(cudaMemsetAsync(grads, 0, kParamCount * sizeof(float), s));
-        k_out_backward<<<blocks_for((long long)rows * 32, 256), 256, 0, s>>>(dy, Z[kLayers - 1], params, rows, dZ[0]);
-        TRY(cudaGetLastError());
-        k_out_wgrad<<<kColSumBlocks, 128, 0, s>>>(dy, Hh[kLayers - 1], rows, grads);
-        TRY(cudaGetLastError());
-        // K-major operands of the weight and input gradients: features and the top gradient
-        // transposed here, the hidden activations by the forward epilogue, the weights of layers 1-3
-        TRY(transpose_bf16(X, rows, kFeat, kFeat, XT, cap, s));
-        TRY(transpose_bf16(dZ[0], rows, kHidden, kHidden, dZT, cap, s));
-        for (int l = 1; l < kLayers; ++l)
-            TRY(transpose_bf16(wbf + w_offset(l), kHidden, kHidden, kHidden, wbfT + (size_t)(l - 1) * kWh, kHidden, s));
-        int cur = 0;
-        for (int l = kLayers - 1; l >= 0; --l) {
-            // weight gradient: dW [out x in] = dZ^T . input  (K = rows)
-            GemmArgs gw = base_args();
-            gw.A = dZT; gw.lda = cap;                               // A[m=out][k=row] = dZ[row][out]
-            gw.B = l == 0 ? XT : HT[l - 1]; gw.ldb = cap;           // B[n=in][k=row] = input[row][in]
-            gw.M = kHidden; gw.N = layer_in(l); gw.K = rows;
-            gw.ksplit = split_k(rows);                              // split the batch across CTAs
-            gw.epi = EPI_F32_ADD; gw.ldc = layer_in(l); gw.C32 = grads + w_offset(l);
-            TRY(gemm(gw, s));
-            k_bias_grad<<<kColSumBlocks, 128, 0, s>>>(dZ[cur], rows, grads + b_offset(l));
-            TRY(cudaGetLastError());
-            if (l == 0) break;
-            // input gradient: dH = dZ . W, then times GELU'(Z[l-1])
-            GemmArgs gx = base_args();
-            gx.A = dZ[cur]; gx.lda = kHidden;                       // A[m=row][k=out]
-            gx.B = wbfT + (size_t)(l - 1) * kWh; gx.ldb = kHidden;  // B[n=in][k=out] = W[out][in]
-            gx.M = rows; gx.N = layer_in(l); gx.K = kHidden;
-            gx.epi = EPI_BWD; gx.ldc = kHidden;
-            gx.Zin = Z[l - 1]; gx.dZ = dZ[cur ^ 1];
-            gx.dZT = dZT; gx.ldt = cap;                             // the next layer's weight-gradient operand
-            TRY(gemm(gx, s));
-            cur ^= 1;
+    cudaError_t forward_hidden(int rows, cudaStream_t s) {
+        LayerArgs g{};
+        g.rows = rows;
+        g.err = err;
+        for (int l = 0; l < kLayers; ++l) {
+            g.bias = params + b_offset(l); g.Zout = Z[l]; g.Hout = Hh[l];
+            if (l == 0) TRY((layer<128, kFeat, true>(X, wbf, g, s)));
+            else TRY((layer<256, kHidden, true>(Hh[l - 1], wbf + w_offset(l), g, s)));
         }
         return cudaSuccess;
     }
 
-    cudaError_t features(const float* xyt, int n, cudaStream_t s) {
-        const int rows = (n + kBM - 1) / kBM * kBM;
-        k_features<<<blocks_for(rows, 128), 128, 0, s>>>(fp, xyt, n, rows, X);
+    // the output layer's forward and the whole backward pass of `rows` rays (features in X, the hidden
+    // layers' forward state in Z/Hh, targets t); gradients into grads, the summed loss into loss[slot]
+    cudaError_t backward(const float* t, int rows, int slot, cudaStream_t s) {
+        k_top<<<kTopBlocks, kTopThreads, 0, s>>>(Hh[kLayers - 1], Z[kLayers - 1], params, t, rows, dZ[0], tpart);
+        TRY(cudaGetLastError());
+        int cur = 0;
+        const int ks = split_k(rows);
+        for (int l = kLayers - 1; l >= 0; --l) {
+            // weight gradient: dW [out x in] = dZ^T . input (K = rows, split across CTAs), both operands as
+            // they lie; the bias gradient on the way
+            GemmArgs gw = base_args();
+            gw.A = dZ[cur]; gw.lda = kHidden; gw.a_t = 1;                        // dZ[k=row][m=out]
+            gw.B = l == 0 ? X : Hh[l - 1]; gw.ldb = layer_in(l); gw.b_t = 1;      // input[k=row][n=in]
+            gw.M = kHidden; gw.N = layer_in(l); gw.K = rows;
+            gw.ksplit = ks;
+            gw.ldc = layer_in(l); gw.C = wpart + w_offset(l); gw.part_stride = kOutW;
+            gw.k_sums = wpart + b_offset(l);
+            TRY(gemm(gw, s));
+            if (l == 0) break;
+            // input gradient: dH = dZ . W, then times GELU'(Z[l-1])
+            LayerArgs gx{};
+            gx.rows = rows; gx.Zin = Z[l - 1]; gx.dZ = dZ[cur ^ 1]; gx.err = err;
+            TRY((layer<256, kHidden, false>(dZ[cur], wbf + w_offset(l), gx, s)));
+            cur ^= 1;
+        }
+        k_reduce_grads<<<(unsigned)(kOutW / 256) + blocks_for(kTopPart, 8), 256, 0, s>>>(wpart, rows / ks, tpart, grads,
+                                                                                        loss + slot);
         return cudaGetLastError();
+    }
+
+    cudaError_t features(const float* xyt, int n, cudaStream_t s) {
+        return launch_features(fp, xyt, n, (n + kBM - 1) / kBM * kBM, X, s);
     }
 
     cudaError_t adam_step(float lr, cudaStream_t s) {
@@ -1216,8 +1509,7 @@ int rlc_learned_predict_layered(rlc_learned* L, const float* d_xyt, int n, float
 // Test hook: the bf16 features of n grid-frame rays into d_out [n x 512] (device).
 int rlc_learned_features(rlc_learned* L, const float* d_xyt, int n, void* d_out) {
     if (!L || n <= 0 || !d_xyt || !d_out) return lfail(RLC_ERR_ARG, "bad argument");
-    k_features<<<blocks_for(n, 128), 128>>>(L->m.fp, d_xyt, n, n, (bf16*)d_out);
-    LTRY(cudaGetLastError(), "features");
+    LTRY(launch_features(L->m.fp, d_xyt, n, n, (bf16*)d_out, 0), "features");
     LTRY(cudaDeviceSynchronize(), "features");
     return RLC_OK;
 }
@@ -1231,11 +1523,8 @@ int rlc_learned_gradients(rlc_learned* L, const float* d_xyt, const float* d_t, 
     LearnedModel& M = L->m;
     LTRY(M.ensure(n), "gradient buffers");
     LTRY(M.features(d_xyt, n, 0), "features");
-    LTRY(M.forward(n, 0), "forward");
-    LTRY(cudaMemset(M.loss, 0, sizeof(float)), "loss");
-    k_loss<<<blocks_for(n, 256), 256>>>(M.y, d_t, n, M.dy, M.loss);
-    LTRY(cudaGetLastError(), "loss");
-    LTRY(M.backward(n, 0), "backward");
+    LTRY(M.forward_hidden(n, 0), "forward");
+    LTRY(M.backward(d_t, n, 0, 0), "backward");
     LTRY(cudaDeviceSynchronize(), "gradients");
     unsigned err = 0;
     LTRY(cudaMemcpy(&err, M.err, sizeof(unsigned), cudaMemcpyDeviceToHost), "gradients");
@@ -1267,25 +1556,21 @@ int rlc_learned_train(rlc_learned* L, int steps, int batch, float lr, unsigned s
                                                              (long long)st * batch, batch, xyt, tt, nullptr);
         e = cudaGetLastError();
         if (e == cudaSuccess) e = M.features(xyt, batch, s);
-        if (e == cudaSuccess) e = M.forward(batch, s);
-        if (e == cudaSuccess) e = cudaMemsetAsync(M.loss, 0, sizeof(float), s);
-        if (e == cudaSuccess) {
-            k_loss<<<blocks_for(batch, 256), 256, 0, s>>>(M.y, tt, batch, M.dy, M.loss);
-            e = cudaGetLastError();
-        }
-        if (e == cudaSuccess) e = M.backward(batch, s);
+        if (e == cudaSuccess) e = M.forward_hidden(batch, s);
+        const int slot = st - (steps - LearnedModel::kLossSlots);   // the last steps' losses are reported
+        if (e == cudaSuccess) e = M.backward(tt, batch, slot >= 0 ? slot : LearnedModel::kLossSlots, s);
         const float cosine = 0.5f * (1.0f + cosf(3.14159265f * (float)st / (float)(steps > 1 ? steps : 1)));
         if (e == cudaSuccess) e = M.adam_step(lr * (0.05f + 0.95f * cosine), s);
-        if (e == cudaSuccess && st >= steps - 20) {
-            float l = 0.0f;
-            e = cudaMemcpyAsync(&l, M.loss, sizeof(float), cudaMemcpyDeviceToHost, s);
-            if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-            loss_acc += l / (float)batch;
-            ++loss_n;
-        }
     }
+    float losses[LearnedModel::kLossSlots] = {};
+    if (e == cudaSuccess && steps > 0)
+        e = cudaMemcpyAsync(losses, M.loss, sizeof(losses), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return lfail(RLC_ERR_CUDA, "training", e);
+    for (int st = std::max(0, steps - LearnedModel::kLossSlots); st < steps; ++st) {
+        loss_acc += losses[st - (steps - LearnedModel::kLossSlots)] / (float)batch;
+        ++loss_n;
+    }
     unsigned err = 0;
     LTRY(cudaMemcpy(&err, M.err, sizeof(unsigned), cudaMemcpyDeviceToHost), "training");
     if (err) return lfail(RLC_ERR_CUDA, "tensor-core GEMM timed out waiting for its MMAs");
@@ -1343,32 +1628,28 @@ int rlc_tc_gemm(const void* d_a, const void* d_b, float* d_c, int M, int N, int 
     if (M <= 0 || N <= 0 || K <= 0 || M % kBM || N % kBN || K % tc::kKChunk)
         return lfail(RLC_ERR_ARG, "M must be a multiple of 128, N of 256, K of 64");
     unsigned* err = nullptr;
-    bf16 *at = nullptr, *bt = nullptr;   // K-major copies of transposed operands
     const cudaStream_t s = (cudaStream_t)stream;
     LTRY(cudaMalloc(&err, sizeof(unsigned)), "gemm");
     cudaError_t e = cudaMemset(err, 0, sizeof(unsigned));
+    bf16* copy[2] = {};   // of transposed operands that do not lie on the tile loads' 16 bytes
+    auto aligned = [&](const void* p, size_t elems, int which) -> const bf16* {
+        if (e != cudaSuccess || !((uintptr_t)p & 15)) return (const bf16*)p;
+        e = cudaMalloc(&copy[which], elems * sizeof(bf16));
+        if (e == cudaSuccess) e = cudaMemcpyAsync(copy[which], p, elems * sizeof(bf16), cudaMemcpyDeviceToDevice, s);
+        return copy[which];
+    };
     GemmArgs g{};
-    g.A = (const bf16*)d_a; g.lda = K;
-    g.B = (const bf16*)d_b; g.ldb = K;
-    if (e == cudaSuccess && a_t) {   // A given as [K x M]
-        e = cudaMalloc(&at, (size_t)M * K * sizeof(bf16));
-        if (e == cudaSuccess) e = transpose_bf16((const bf16*)d_a, K, M, M, at, K, s);
-        g.A = at;
-    }
-    if (e == cudaSuccess && b_t) {   // B given as [K x N]
-        e = cudaMalloc(&bt, (size_t)N * K * sizeof(bf16));
-        if (e == cudaSuccess) e = transpose_bf16((const bf16*)d_b, K, N, N, bt, K, s);
-        g.B = bt;
-    }
+    g.A = a_t ? aligned(d_a, (size_t)M * K, 0) : (const bf16*)d_a; g.lda = a_t ? M : K; g.a_t = a_t != 0;   // [M x K], or [K x M]
+    g.B = b_t ? aligned(d_b, (size_t)N * K, 1) : (const bf16*)d_b; g.ldb = b_t ? N : K; g.b_t = b_t != 0;
     g.M = M; g.N = N; g.K = K;
-    g.epi = EPI_F32; g.ldc = N; g.C32 = d_c; g.err = err;
+    g.ldc = N; g.C = d_c; g.err = err;
     if (e == cudaSuccess) e = gemm(g, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     unsigned h = 0;
     if (e == cudaSuccess) e = cudaMemcpy(&h, err, sizeof(unsigned), cudaMemcpyDeviceToHost);
     cudaFree(err);
-    cudaFree(at);
-    cudaFree(bt);
+    cudaFree(copy[0]);
+    cudaFree(copy[1]);
     if (e != cudaSuccess) return lfail(RLC_ERR_CUDA, "tensor-core gemm", e);
     if (h) return lfail(RLC_ERR_CUDA, "tensor-core GEMM timed out waiting for its MMAs");
     return RLC_OK;

@@ -55,6 +55,23 @@ __device__ __forceinline__ uint64_t make_desc_sw128(uint32_t saddr) {
     return d;
 }
 
+// Descriptor of an M/N-major operand in the layout that TMA loads of 64-column (128-byte) boxes with
+// 128-byte swizzle write: per block of 64 columns, K row k at k * 128 bytes, its 16-byte chunks permuted
+// by k & 7; groups of 8 K rows 1024 bytes apart (SBO), blocks of 64 columns block_bytes apart (LBO);
+// blocks 1024-byte aligned.  Successive 16-element K steps start 16 rows further.
+__device__ __forceinline__ uint64_t make_desc_sw128_mn(uint32_t saddr, uint32_t block_bytes) {
+    uint64_t d = 0;
+    d |= (uint64_t)((saddr >> 4) & 0x3FFF);
+    d |= (uint64_t)((block_bytes >> 4) & 0x3FFF) << 16;
+    d |= (uint64_t)(1024 >> 4) << 32;
+    d |= (uint64_t)1 << 46;                        // version
+    d |= (uint64_t)2 << 61;                        // 128-byte swizzle
+    return d;
+}
+
+// instruction descriptor bits of an M-major A and an N-major B
+constexpr uint32_t kIdescTransposeA = 1u << 15, kIdescTransposeB = 1u << 16;
+
 // kind::f16 instruction descriptor: D f32, A and B bf16, both K-major, M x N
 __host__ __device__ constexpr uint32_t make_idesc(int M, int N) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
@@ -79,24 +96,34 @@ __device__ __forceinline__ void mbar_init(uint32_t mbar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(mbar), "r"(count) : "memory");
 }
 
+__device__ __forceinline__ void mbar_arrive(uint32_t mbar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(mbar) : "memory");
+}
+
 __device__ __forceinline__ void fence_mbar_init() {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
 
+__device__ __forceinline__ bool mbar_try(uint32_t mbar, uint32_t parity) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}\n"
+        : "=r"(done)
+        : "r"(mbar), "r"(parity)
+        : "memory");
+    return done != 0;
+}
+
 // Wait for phase `parity` of the mbarrier, giving up after ~2^31 clock
-// cycles (about one second): returns false on time-out.
+// cycles (about one second): returns false on time-out.  The clock is read
+// only once a first try has failed: the issuing threads wait per K chunk.
 __device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity) {
+    if (mbar_try(mbar, parity)) return true;
     const long long t0 = clock64();
     for (;;) {
-        uint32_t done;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}\n"
-            : "=r"(done)
-            : "r"(mbar), "r"(parity)
-            : "memory");
-        if (done) return true;
+        if (mbar_try(mbar, parity)) return true;
         if (clock64() - t0 > (1ll << 31)) return false;
     }
 }
@@ -149,13 +176,13 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t mbar, uint32_t by
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mbar), "r"(bytes) : "memory");
 }
 
-// 2-D tiled TMA load of the box at (x = innermost coordinate, y) of the tensor map into shared
-// memory at dst, completing `bytes` of transaction count on the mbarrier.  x times the element
+// 3-D tiled TMA load of the box at (x = innermost coordinate, y, z) of the tensor map into shared
+// memory at dst, completing on the mbarrier's transaction count.  x times the element
 // size must be a multiple of 16 bytes; dst 128-byte aligned.
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const void* tmap, int x, int y, uint32_t mbar) {
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const void* tmap, int x, int y, int z, uint32_t mbar) {
     asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-        ::"r"(dst), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(x), "r"(y), "r"(mbar)
+        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+        ::"r"(dst), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(x), "r"(y), "r"(z), "r"(mbar)
         : "memory");
 }
 
