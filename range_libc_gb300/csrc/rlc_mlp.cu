@@ -366,14 +366,16 @@ EncodeTiledFn encode_tiled() {
 // Tensor map of a bf16 operand of `rows` rows (or columns) x K with row stride ld, 128-byte swizzled in
 // shared memory, as three dimensions so that one load brings a tile's K chunk either way: K-major
 // {K, rows, 1} in boxes of 64 x box_rows; M/N-major (element (k, r) at k * ld + r) {64, K, rows / 64} in
-// boxes of 64 x 64 x box_rows / 64, blocks of 64 columns one after the other.
-cudaError_t operand_map(CUtensorMap* map, const bf16* base, bool mn_major, int rows, int K, int ld, int box_rows) {
+// boxes of 64 x 64 x box_rows / 64, blocks of 64 columns one after the other.  K-major only: the third
+// dimension may count `batch` such operands, `pitch` elements apart.
+cudaError_t operand_map(CUtensorMap* map, const bf16* base, bool mn_major, int rows, int K, int ld, int box_rows,
+                        int batch = 1, size_t pitch = 64) {
     EncodeTiledFn enc = encode_tiled();
     if (!enc) return cudaErrorNotSupported;
-    if (((uintptr_t)base & 15) || (ld * 2) % 16) return cudaErrorInvalidValue;
+    if (((uintptr_t)base & 15) || (ld * 2) % 16 || (pitch * 2) % 16) return cudaErrorInvalidValue;
     const cuuint64_t dim[3] = {(cuuint64_t)(mn_major ? 64 : K), (cuuint64_t)(mn_major ? K : rows),
-                               (cuuint64_t)(mn_major ? rows / 64 : 1)};
-    const cuuint64_t stride[2] = {(cuuint64_t)ld * 2, 128};
+                               (cuuint64_t)(mn_major ? rows / 64 : batch)};
+    const cuuint64_t stride[2] = {(cuuint64_t)ld * 2, (cuuint64_t)pitch * 2};
     const cuuint32_t box[3] = {64u, (cuuint32_t)(mn_major ? tc::kKChunk : box_rows), (cuuint32_t)(mn_major ? box_rows / 64 : 1)};
     const cuuint32_t estr[3] = {1, 1, 1};
     const CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<bf16*>(base), dim, stride, box, estr,
@@ -672,242 +674,293 @@ cudaError_t launch_features(const FeatParams& fp, const float* xyt, int n, int r
 }
 
 // ------------------------------------------------------ fused forward pass
-// Inference of the whole network for 128 rays per CTA without leaving the SM:
-// the features of one 32-wide K stage are computed straight into the A
-// operand (shared memory, core-matrix layout), each layer accumulates its
-// 128 x 256 output in TMEM, and the epilogue (bias, BF16 rounding, GELU)
-// writes the next layer's A operand back into shared memory; the output
-// layer is a per-row dot product in the last epilogue.  Only the rays' poses
-// come in and one float per ray goes out (the layer-by-layer path moves
-// ~3.1 KB per ray through HBM).  Weights stream from L2 with cp.async into two
-// 16 KB stages of 256 x 32: stage c+1 is copied while the MMAs of stage c run.
-// Two threads share each TMEM lane (row) and split its features and epilogue
-// columns.  Every MMA operand, rounding point and summation order matches the
-// layer-by-layer path, so the predictions are bit-identical to it.
-// 96 KB of shared memory and 256 TMEM columns per CTA: two CTAs per SM, so
-// one CTA's epilogue or operand loads overlap the other's MMAs.
-constexpr int kFwdThreads = 256;   // two threads per TMEM lane (row): column halves
-constexpr int kFK = 32;            // K elements per pipeline stage
-constexpr uint32_t kFStage = 512;  // bytes between 8-row groups of a 32-wide K tile (4 core matrices)
-constexpr size_t kFwdSmem = 2 * 16384 + 65536;   // two 256 x 32 weight stages + activations
+// Inference of the whole network without leaving the SM: only the rays' poses come in and one float per
+// ray goes out (the layer-by-layer path moves ~3.1 KB per ray through HBM).  One persistent CTA per SM
+// works on two tiles of 128 rays, each with its 64 KB of activations in shared memory and its 256 TMEM
+// columns:
+//   warp 0       TMA producer: the weights of every layer in K chunks of 64 (32 KB), round a ring of
+//                three stages, in the MMA warp's order;
+//   warp 1       allocates TMEM; one thread issues the MMAs, layer by layer, tile 0 and tile 1 in turn;
+//   warps 2-9    tile 0, warps 10-17 tile 1, two threads per ray (column halves): the features of a K
+//                chunk straight into the A operand (the activation buffer's four 64-wide blocks are the
+//                first layer's stages), each layer's epilogue (bias, bf16 rounding, GELU) from TMEM into
+//                the next layer's A operand, the last one into the output layer's sums.
+// The two tiles are out of step, so one's arithmetic fills the other's waits for its MMAs.  Bound by
+// issuing that arithmetic: per ray 256 sincospi and 1,024 GELUs (a tanh each: 8 cycles of the SFU per
+// warp).  Two CTAs per SM in step with their weights' copies before: 1.08 M rays 2.32 ms, 0.93 now.
+// Every MMA operand, rounding point and summation order matches the layer-by-layer path, so the
+// predictions are bit-identical to it.  Operands K-major with the 128-byte swizzle (tc::make_desc_sw128).
+// Waits are bounded as in k_gemm_tma; no role waits on a hardware barrier that another may leave.
+constexpr int kFwdTile = 8 * 32;                     // threads of a tile
+constexpr int kFwdThreads = 64 + 2 * kFwdTile;
+constexpr int kFwdStages = 3;
+constexpr uint32_t kFwdStage = kBN * tc::kKChunk * 2;     // 32 KB of weights
+constexpr uint32_t kActBlock = kBM * tc::kKChunk * 2;     // 16 KB: 64 columns of a tile's activations
+constexpr size_t kFwdSmem = kFwdStages * (size_t)kFwdStage + 2 * 4 * (size_t)kActBlock + 1024;
 
-// byte offset of element (row, k) (k < 32) in a 32-wide K tile of core matrices
-__device__ __forceinline__ uint32_t core32(int row, int k) {
-    return (uint32_t)((row >> 3) * kFStage + (k >> 3) * tc::kCoreBytes + (row & 7) * 16 + (k & 7) * 2);
-}
+// K chunks of a layer
+__host__ __device__ constexpr int layer_chunks(int l) { return (l == 0 ? kFeat : kHidden) / tc::kKChunk; }
 
-// bf16 element k (< 256) of row `row` of the activation buffer (4 K chunks of 64 in core layout)
-__device__ __forceinline__ uint32_t act_offset(int row, int k) {
-    return (uint32_t)(k >> 6) * 16384u + tc::core_offset(row, k & 63);
-}
-
-// 16 features [32c + 16h, 32c + 16h + 16) of a ray with inputs u: input d = c / 4,
-// frequencies (c % 4) * 16 + 8h .. + 8, as 2 rows of 16 bytes of the core layout
-__device__ __forceinline__ void feature_quarter(const FeatParams& fp, const float* u, int c, int h, uint4* out) {
-    const int d = c >> 2, k0 = (c & 3) * 16 + 8 * h;
-#pragma unroll
-    for (int v = 0; v < 2; ++v) {
-        __nv_bfloat162 hb[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            float sn, cs;
-            sincospif(fp.freq[k0 + 4 * v + q] * u[d], &sn, &cs);
-            hb[q] = __floats2bfloat162_rn(sn, cs);
-        }
-        out[v] = *reinterpret_cast<const uint4*>(hb);
-    }
-}
-
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
-// weight rows [0, 256) x K [k0, k0 + 32) of a layer (row-major [256][ld]) into a stage, asynchronously
-__device__ __forceinline__ void load_weights32(uint32_t dst, const bf16* __restrict__ w, int ld, int k0) {
-    for (int v = threadIdx.x; v < kBN * (kFK / 8); v += blockDim.x) {
-        const int row = v >> 2, kv = v & 3;
-        cp_async16(dst + (uint32_t)((row >> 3) * kFStage + kv * tc::kCoreBytes + (row & 7) * 16),
-                   w + (size_t)row * ld + k0 + kv * 8);
-    }
-}
-
-// One layer's MMA chunks, pipelined: the weights of chunk c + 1 are copied into
-// the other stage while the MMAs of chunk c run; a stage is refilled only after
-// the MMAs that read it have completed (one mbarrier per stage).  Layer 0
-// computes its A operand (features) per chunk into sA[c % 2] inside the
-// activation buffer; hidden layers read A from the activations.
-struct FwdPipe {
-    uint32_t sB[2], mbar[2], par[2];
-    uint32_t tmem, idesc;
-};
-
-template <bool FEATURES>
-__device__ __forceinline__ bool fwd_layer(FwdPipe& P, const bf16* __restrict__ w, int K, uint32_t sH, uint8_t* sA_gen,
-                                          const FeatParams& fp, const float* u, bool live, int row, int half) {
-    const int C = K / kFK;
-    bool ok = true;
-    load_weights32(P.sB[0], w, K, 0);
-    cp_async_commit();
-    for (int c = 0; c < C; ++c) {
-        const int st = c & 1;
-        if (c + 1 < C) {
-            if (c >= 1) {   // stage st ^ 1 was read by the MMAs of chunk c - 1
-                const bool wt = tc::mbar_wait(P.mbar[st ^ 1], P.par[st ^ 1]);
-                P.par[st ^ 1] ^= 1u;
-                if (!__syncthreads_and(wt)) return false;
-            }
-            load_weights32(P.sB[st ^ 1], w, K, (c + 1) * kFK);
-            cp_async_commit();
-        }
-        uint32_t a0;
-        if (FEATURES) {   // A stage st (inside the activation buffer) was read by chunk c - 2, complete by now
-            uint4 f[2];
-            if (live) {
-                feature_quarter(fp, u, c, half, f);
-            } else {
-                f[0] = f[1] = make_uint4(0, 0, 0, 0);
-            }
-            uint8_t* sa = sA_gen + st * 8192;
-            *reinterpret_cast<uint4*>(sa + core32(row, 16 * half)) = f[0];
-            *reinterpret_cast<uint4*>(sa + core32(row, 16 * half + 8)) = f[1];
-            a0 = tc::smem_addr(sa);
-        } else {
-            a0 = sH + (uint32_t)(c >> 1) * 16384u + (uint32_t)(c & 1) * 4u * tc::kCoreBytes;
-        }
-        if (c + 1 < C) cp_async_wait<1>(); else cp_async_wait<0>();
-        tc::fence_async_smem();
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            tc::fence_after_sync();
-            const uint32_t sbo_a = FEATURES ? kFStage : tc::kRowBlockBytes;
-#pragma unroll
-            for (int ks = 0; ks < kFK / 16; ++ks) {
-                const uint64_t ad = tc::make_desc(a0 + ks * 2 * tc::kCoreBytes, tc::kCoreBytes, sbo_a);
-                const uint64_t bd = tc::make_desc(P.sB[st] + ks * 2 * tc::kCoreBytes, tc::kCoreBytes, kFStage);
-                tc::mma_bf16(P.tmem, ad, bd, P.idesc, (c > 0 || ks > 0) ? 1u : 0u);
-            }
-            tc::mma_commit(P.mbar[st]);
-        }
-    }
-    // the loop waited for the MMAs of chunks 0 .. C - 3; wait for the last two
-    for (int q = C >= 2 ? C - 2 : 0; q < C; ++q) {
-        const int st = q & 1;
-        const bool wt = tc::mbar_wait(P.mbar[st], P.par[st]);
-        P.par[st] ^= 1u;
-        ok = (__syncthreads_and(wt) != 0) && ok;
-    }
-    tc::fence_after_sync();
-    return ok;
-}
-
-__global__ void __launch_bounds__(kFwdThreads, 2) k_mlp_forward(FeatParams fp, const float* __restrict__ xyt, int n,
-                                                                 const bf16* __restrict__ wbf,
-                                                                 const float* __restrict__ params,
-                                                                 float* __restrict__ y, unsigned* err) {
-    extern __shared__ __align__(1024) uint8_t smem[];
-    __shared__ __align__(8) uint64_t mbar[2];
+__global__ void __launch_bounds__(kFwdThreads, 1)
+k_mlp_forward(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ CUtensorMap tmH, FeatParams fp,
+              const float* __restrict__ xyt, int n, const float* __restrict__ params, float* __restrict__ y, unsigned* err) {
+    extern __shared__ uint8_t smem_raw[];
+    __shared__ __align__(8) uint64_t w_full[kFwdStages], w_empty[kFwdStages];
+    __shared__ __align__(8) uint64_t a_full[2][4], a_free[2][4], acc_full[2], out_full[2], drained;
     __shared__ uint32_t tmem_base;
-    uint8_t* sB0 = smem;                 // weight stages: 2 x (256 rows x 32)
-    uint8_t* sH = smem + 2 * 16384;      // activations: 4 K chunks of 128 x 64 (layer 0: feature stages)
-    const int warp = threadIdx.x >> 5;
-    const int row = threadIdx.x & 127;   // TMEM lane = ray of the tile (warp % 4 owns lanes 32 (warp % 4) ..)
-    const int half = threadIdx.x >> 7;   // columns [128 half, 128 half + 128) of every layer
-    if (warp == 0) tc::tmem_alloc(tc::smem_addr(&tmem_base), 256);
+    __shared__ int abort_flag, n_issued, n_consumed;
+    __shared__ __align__(16) float s_freq[64];
+    uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    const uint32_t sW = tc::smem_addr(smem), sAct = sW + kFwdStages * kFwdStage;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    // tile i of group g is (2 i + g) * gridDim.x + blockIdx.x: few rays spread over the SMs first
+    const int tiles = (n + kBM - 1) / kBM, G = gridDim.x;
+    const int rounds = (tiles - (int)blockIdx.x + 2 * G - 1) / (2 * G);
+    auto has_tile = [&](int i, int g) { return (2 * i + g) * G + (int)blockIdx.x < tiles; };
+    if (warp == 1) tc::tmem_alloc(tc::smem_addr(&tmem_base), 512);
     if (threadIdx.x == 0) {
-        tc::mbar_init(tc::smem_addr(&mbar[0]), 1);
-        tc::mbar_init(tc::smem_addr(&mbar[1]), 1);
+        for (int i = 0; i < kFwdStages; ++i) {
+            tc::mbar_init(tc::smem_addr(&w_full[i]), 1);
+            tc::mbar_init(tc::smem_addr(&w_empty[i]), 1);
+        }
+        for (int g = 0; g < 2; ++g) {
+            for (int i = 0; i < 4; ++i) {
+                tc::mbar_init(tc::smem_addr(&a_full[g][i]), kFwdTile / 32);
+                tc::mbar_init(tc::smem_addr(&a_free[g][i]), 1);
+            }
+            tc::mbar_init(tc::smem_addr(&acc_full[g]), 1);
+            tc::mbar_init(tc::smem_addr(&out_full[g]), kFwdTile / 64);
+        }
+        tc::mbar_init(tc::smem_addr(&drained), 1);
+        abort_flag = 0;
+        n_issued = 0;
+        n_consumed = 0;
         tc::fence_mbar_init();
     }
+    if (threadIdx.x < 64) s_freq[threadIdx.x] = fp.freq[threadIdx.x];
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
-    FwdPipe P;
-    P.sB[0] = tc::smem_addr(sB0);
-    P.sB[1] = tc::smem_addr(sB0 + 16384);
-    P.mbar[0] = tc::smem_addr(&mbar[0]);
-    P.mbar[1] = tc::smem_addr(&mbar[1]);
-    P.par[0] = P.par[1] = 0u;
-    P.tmem = tmem_base;
-    P.idesc = tc::make_idesc(kBM, kBN);
-    const uint32_t lane_addr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
-    const uint32_t sHa = tc::smem_addr(sH);
-
-    const int r = blockIdx.x * kBM + row;
-    float u[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-    const bool live = r < n;
-    if (live) {
-        float sn, cs;
-        sincosf(__ldg(xyt + 3 * (size_t)r + 2), &sn, &cs);
-        u[0] = __ldg(xyt + 3 * (size_t)r) * fp.inv_w;
-        u[1] = __ldg(xyt + 3 * (size_t)r + 1) * fp.inv_h;
-        u[2] = cs;
-        u[3] = sn;
-    }
-    bool ok = fwd_layer<true>(P, wbf + w_offset(0), kFeat, sHa, sH, fp, u, live, row, half);
-    for (int l = 0; l < kLayers && ok; ++l) {
-        if (l > 0) ok = fwd_layer<false>(P, wbf + w_offset(l), kHidden, sHa, sH, fp, u, live, row, half);
-        if (!ok) break;
-        // epilogue of layer l: z = acc + b, rounded to bf16; h = bf16(GELU(z)) into sH
-        const float* bias = params + b_offset(l);
-        for (int cb = 128 * half; cb < 128 * half + 128; cb += 32) {
-            float v[32];
-            tc::tmem_ld32(lane_addr + cb, v);
-#pragma unroll
-            for (int i = 0; i < 32; i += 2) {
-                const float z0 = v[i] + __ldg(bias + cb + i), z1 = v[i + 1] + __ldg(bias + cb + i + 1);
-                const float2 h = gelu(widen_bf16(pack_bf16(z0, z1)));
-                *reinterpret_cast<uint32_t*>(sH + act_offset(row, cb + i)) = pack_bf16(h.x, h.y);
-            }
-        }
-        tc::fence_before_sync();   // TMEM reads done before the next layer's MMAs overwrite it
-    }
-    if (ok) {
-        // output layer on the last activations, in k_out_layer's summation order: partial
-        // sums over j = i (mod 32) in increasing j, then the xor butterfly
-        __syncthreads();
-        if (half == 0 && live) {
-            const float* wout = params + kOutW;
-            float part[32];
-#pragma unroll
-            for (int i = 0; i < 32; ++i) part[i] = 0.0f;
-            for (int cb = 0; cb < kHidden; cb += 32) {
-#pragma unroll
-                for (int i = 0; i < 32; i += 8) {
-                    const uint4 q = *reinterpret_cast<const uint4*>(sH + act_offset(row, cb + i));
-                    const __nv_bfloat162* hb = reinterpret_cast<const __nv_bfloat162*>(&q);
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        const float2 hf = __bfloat1622float2(hb[e]);
-                        part[i + 2 * e] = __fadd_rn(part[i + 2 * e], __fmul_rn(hf.x, __ldg(wout + cb + i + 2 * e)));
-                        part[i + 2 * e + 1] =
-                            __fadd_rn(part[i + 2 * e + 1], __fmul_rn(hf.y, __ldg(wout + cb + i + 2 * e + 1)));
+    const uint32_t tmem = tmem_base;
+    auto aborted = [&]() { return *(volatile int*)&abort_flag != 0; };
+    auto give_up = [&]() {
+        atomicOr(err, 16u);
+        atomicExch(&abort_flag, 1);
+    };
+    if (warp == 0 && lane == 0) {
+        // ---- producer
+        tc::tma_prefetch_map(&tm0);
+        tc::tma_prefetch_map(&tmH);
+        int c_all = 0, st = 0, phase = 1;
+        bool ok = true;
+        for (int i = 0; i < rounds && ok; ++i)
+            for (int lg = 0; lg < 2 * kLayers && ok; ++lg) {
+                const int l = lg >> 1;
+                if (!has_tile(i, lg & 1)) continue;
+                for (int c = 0; c < layer_chunks(l); ++c, ++c_all) {
+                    if (c_all >= kFwdStages && !tc::mbar_wait(tc::smem_addr(&w_empty[st]), phase)) {
+                        give_up();
+                        ok = false;
+                        break;
+                    }
+                    const uint32_t fb = tc::smem_addr(&w_full[st]);
+                    tc::mbar_arrive_expect_tx(fb, kFwdStage);
+                    tc::tma_load_3d(sW + st * kFwdStage, l == 0 ? &tm0 : &tmH, c * tc::kKChunk, 0, l == 0 ? 0 : l - 1, fb);
+                    if (++st == kFwdStages) {
+                        st = 0;
+                        phase ^= 1;
                     }
                 }
             }
+        n_issued = c_all;
+    } else if (warp == 1 && lane == 0) {
+        // ---- MMA issuer.  uses[g]: how often tile g's A blocks have been filled (all four alike)
+        const uint32_t idesc = tc::make_idesc(kBM, kBN);
+        const uint64_t w0 = tc::make_desc_sw128(sW), a0 = tc::make_desc_sw128(sAct);
+        int c_all = 0, st = 0, phase = 0;
+        unsigned uses[2] = {0, 0};
+        bool ok = true;
+        for (int i = 0; i < rounds && ok; ++i)
+            for (int l = 0; l < kLayers && ok; ++l)
 #pragma unroll
-            for (int o = 16; o; o >>= 1)
+                for (int g = 0; g < 2; ++g) {
+                    if (!has_tile(i, g) || !ok) continue;
+                    for (int c = 0; c < layer_chunks(l); ++c) {
+                        const int b = c & 3;
+                        ok = tc::mbar_wait(tc::smem_addr(&a_full[g][b]), (uses[g] + (c >> 2)) & 1) &&
+                             tc::mbar_wait(tc::smem_addr(&w_full[st]), phase);
+                        if (!ok) break;
+                        tc::fence_after_sync();
 #pragma unroll
-                for (int i = 0; i < o; ++i) part[i] = __fadd_rn(part[i], part[i + o]);
-            y[r] = __fadd_rn(part[0], __ldg(wout + kHidden));
+                        for (int ks = 0; ks < tc::kKChunk / 16; ++ks)
+                            tc::mma_bf16(tmem + g * kBN, a0 + (uint32_t)((g * 4 + b) * (kActBlock >> 4) + ks * 2),
+                                         w0 + (uint32_t)(st * (kFwdStage >> 4) + ks * 2), idesc, (c > 0 || ks > 0) ? 1u : 0u);
+                        tc::mma_commit(tc::smem_addr(&w_empty[st]));
+                        if (l == 0 && c < 4) tc::mma_commit(tc::smem_addr(&a_free[g][b]));
+                        ++c_all;
+                        if (++st == kFwdStages) {
+                            st = 0;
+                            phase ^= 1;
+                        }
+                    }
+                    if (ok) tc::mma_commit(tc::smem_addr(&acc_full[g]));
+                    uses[g] += layer_chunks(l) / 4;
+                }
+        n_consumed = c_all;
+        if (!ok) {   // let what was issued end before the TMEM is freed
+            give_up();
+            tc::mma_commit(tc::smem_addr(&drained));
+            (void)tc::mbar_wait(tc::smem_addr(&drained), 0);
         }
-    } else if (threadIdx.x == 0) {
-        atomicOr(err, 16u);
+    } else if (warp >= 2) {
+        // ---- features and epilogues
+        const int g = (warp - 2) >> 3, half = ((warp - 2) >> 2) & 1;
+        const int row = (warp & 3) * 32 + lane;   // TMEM lanes 32 (warp % 4) .. + 31
+        uint8_t* act = smem + kFwdStages * kFwdStage + g * 4 * kActBlock + row * 128;
+        const uint32_t acc = tmem + g * kBN + ((uint32_t)((warp & 3) * 32) << 16);
+        const int swz = row & 7;
+        const float* wout = params + kOutW;
+        auto wait = [&](uint64_t* bar, uint32_t parity) {
+            const bool ok = __all_sync(0xffffffffu, tc::mbar_wait(tc::smem_addr(bar), parity) && !aborted());
+            if (!ok && lane == 0) give_up();
+            tc::fence_after_sync();
+            return ok;
+        };
+        bool ok = true;
+        unsigned layers_done = 0;
+        for (int i = 0; i < rounds && ok && has_tile(i, g); ++i) {
+            const int r = ((2 * i + g) * G + (int)blockIdx.x) * kBM + row;
+            const bool live = r < n;
+            float u0 = 0.0f, u1 = 0.0f, u2 = 0.0f, u3 = 0.0f;
+            if (live) {
+                sincosf(__ldg(xyt + 3 * (size_t)r + 2), &u3, &u2);
+                u0 = __ldg(xyt + 3 * (size_t)r) * fp.inv_w;
+                u1 = __ldg(xyt + 3 * (size_t)r + 1) * fp.inv_h;
+            }
+            // features [64 c, 64 c + 64): input c / 2, frequencies 32 (c % 2) .. + 31, a thread 16 of them
+#pragma unroll 1
+            for (int c = 0; c < kFeat / tc::kKChunk; ++c) {
+                if (c >= 4 && !(ok = wait(&a_free[g][c & 3], i & 1))) break;
+                const float u = c < 2 ? u0 : c < 4 ? u1 : c < 6 ? u2 : u3;
+                const float* f = s_freq + (c & 1) * 32 + half * 16;
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const float4 fq = *reinterpret_cast<const float4*>(f + 4 * q);
+                    uint4 o;
+                    float sn, cs;
+                    sincospif(fq.x * u, &sn, &cs);
+                    o.x = pack_bf16(sn, cs);
+                    sincospif(fq.y * u, &sn, &cs);
+                    o.y = pack_bf16(sn, cs);
+                    sincospif(fq.z * u, &sn, &cs);
+                    o.z = pack_bf16(sn, cs);
+                    sincospif(fq.w * u, &sn, &cs);
+                    o.w = pack_bf16(sn, cs);
+                    if (!live) o = make_uint4(0u, 0u, 0u, 0u);
+                    *reinterpret_cast<uint4*>(act + (c & 3) * kActBlock + (((half * 4 + q) ^ swz) << 4)) = o;
+                }
+                tc::fence_async_smem();
+                tc::fence_before_sync();
+                __syncwarp();
+                if (lane == 0) tc::mbar_arrive(tc::smem_addr(&a_full[g][c & 3]));
+            }
+            // hidden layers: z = acc + b, rounded to bf16; h = bf16(GELU(z)) into the A blocks
+#pragma unroll 1
+            for (int l = 0; l < kLayers - 1 && ok; ++l) {
+                if (!(ok = wait(&acc_full[g], layers_done++ & 1))) break;
+                const float4* bias = reinterpret_cast<const float4*>(params + b_offset(l));
+#pragma unroll 1
+                for (int cb = 128 * half; cb < 128 * half + 128; cb += 32) {
+                    float v[32];
+                    tc::tmem_ld32(acc + cb, v);
+                    uint32_t h[16];
+#pragma unroll
+                    for (int q = 0; q < 32; q += 4) {
+                        const float4 b = __ldg(bias + (cb + q) / 4);
+                        const float2 z0 = unpack2(add2(pack2(v[q], v[q + 1]), pack2(b.x, b.y)));
+                        const float2 z1 = unpack2(add2(pack2(v[q + 2], v[q + 3]), pack2(b.z, b.w)));
+                        const float2 h0 = gelu(widen_bf16(pack_bf16(z0.x, z0.y))), h1 = gelu(widen_bf16(pack_bf16(z1.x, z1.y)));
+                        h[q / 2] = pack_bf16(h0.x, h0.y);
+                        h[q / 2 + 1] = pack_bf16(h1.x, h1.y);
+                    }
+#pragma unroll
+                    for (int q = 0; q < 4; ++q)
+                        *reinterpret_cast<uint4*>(act + (cb >> 6) * kActBlock + ((((cb & 32) / 8 + q) ^ swz) << 4)) =
+                            make_uint4(h[4 * q], h[4 * q + 1], h[4 * q + 2], h[4 * q + 3]);
+                }
+                tc::fence_async_smem();
+                tc::fence_before_sync();
+                __syncwarp();
+                if (lane < 4) tc::mbar_arrive(tc::smem_addr(&a_full[g][lane]));
+            }
+            // the last layer and the output layer in k_out_layer's summation order: sums over the columns
+            // j = e (mod 32) in increasing j, of which this thread has e = 16 half .. + 15, then the xor butterfly
+            if (!ok || !(ok = wait(&acc_full[g], layers_done++ & 1))) break;
+            const float4* bias = reinterpret_cast<const float4*>(params + b_offset(kLayers - 1));
+            f32x2 part[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) part[e] = 0ull;
+#pragma unroll 1
+            for (int cb = 16 * half; cb < kHidden; cb += 32) {
+                float v[16];
+                tc::tmem_ld16(acc + cb, v);
+#pragma unroll
+                for (int q = 0; q < 16; q += 4) {
+                    const float4 b = __ldg(bias + (cb + q) / 4), w = __ldg(reinterpret_cast<const float4*>(wout + cb + q));
+                    const float2 z0 = unpack2(add2(pack2(v[q], v[q + 1]), pack2(b.x, b.y)));
+                    const float2 z1 = unpack2(add2(pack2(v[q + 2], v[q + 3]), pack2(b.z, b.w)));
+                    const float2 h0 = gelu(widen_bf16(pack_bf16(z0.x, z0.y))), h1 = gelu(widen_bf16(pack_bf16(z1.x, z1.y)));
+                    part[q / 2] = add2(part[q / 2], mul2_then(widen_bf16(pack_bf16(h0.x, h0.y)), pack2(w.x, w.y)));
+                    part[q / 2 + 1] = add2(part[q / 2 + 1], mul2_then(widen_bf16(pack_bf16(h1.x, h1.y)), pack2(w.z, w.w)));
+                }
+            }
+            float p[16];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                const float2 t = unpack2(part[e]);
+                p[2 * e] = t.x;
+                p[2 * e + 1] = t.y;
+            }
+            if (half) {   // through TMEM columns 16 .. 31, which only this thread reads
+                tc::tmem_st16(acc + 16, p);
+                tc::fence_before_sync();
+                __syncwarp();
+                if (lane == 0) tc::mbar_arrive(tc::smem_addr(&out_full[g]));
+            } else {
+                if (!(ok = wait(&out_full[g], i & 1))) break;
+                float o[16];
+                tc::tmem_ld16(acc + 16, o);
+#pragma unroll
+                for (int e = 0; e < 16; ++e) p[e] = __fadd_rn(p[e], o[e]);
+#pragma unroll
+                for (int s = 8; s; s >>= 1)
+#pragma unroll
+                    for (int e = 0; e < s; ++e) p[e] = __fadd_rn(p[e], p[e + s]);
+                if (live) y[r] = __fadd_rn(p[0], __ldg(wout + kHidden));
+            }
+        }
     }
-    cp_async_wait<0>();
     tc::fence_before_sync();
     __syncthreads();
-    if (warp == 0) tc::tmem_dealloc(P.tmem, 256);
+    if (abort_flag && threadIdx.x == 0) {
+        // loads issued but never waited for are still landing in this CTA's shared memory: wait for
+        // them (bounded) before the CTA exits
+        for (int c = n_consumed; c < n_issued; ++c)
+            (void)tc::mbar_wait(tc::smem_addr(&w_full[c % kFwdStages]), (c / kFwdStages) & 1);
+    }
+    __syncthreads();
+    if (warp == 1) tc::tmem_dealloc(tmem, 512);
 }
 
 cudaError_t mlp_forward(const FeatParams& fp, const float* xyt, int n, const bf16* wbf, const float* params, float* y,
                         unsigned* err, cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
+    CUtensorMap t0, th;
+    TRY(operand_map(&t0, wbf, false, kHidden, kFeat, kFeat, kHidden));
+    TRY(operand_map(&th, wbf + w_offset(1), false, kHidden, kHidden, kHidden, kHidden, kLayers - 1, w_offset(2) - w_offset(1)));
     static std::atomic<unsigned long long> attr{0};
-    if (cudaError_t e = ensure_smem_attr(k_mlp_forward, (int)kFwdSmem, attr)) return e;
-    k_mlp_forward<<<(n + kBM - 1) / kBM, kFwdThreads, kFwdSmem, s>>>(fp, xyt, n, wbf, params, y, err);
+    TRY(ensure_smem_attr(k_mlp_forward, (int)kFwdSmem, attr));
+    k_mlp_forward<<<std::min(152, (n - 1) / kBM + 1), kFwdThreads, kFwdSmem, s>>>(t0, th, fp, xyt, n, params, y, err);
     return cudaGetLastError();
 }
 

@@ -2,12 +2,6 @@
 // as inline PTX: shared-memory matrix descriptors, the kind::f16 instruction
 // descriptor, TMEM allocation, MMA issue/commit, mbarrier waits with a time
 // bound, TMEM loads, and TMA tile loads.
-//
-// Shared-memory operand layout used throughout (no swizzle, K-major): a tile
-// of R rows x 64 K (bf16) is stored as 8x8 "core matrices" of 128 contiguous
-// bytes (8 rows x 16 B); core matrix (i, j) -- rows 8i..8i+7, k 8j..8j+7 --
-// sits at byte (i * 8 + j) * 128.  Adjacent core matrices along K are 128 B
-// apart (leading byte offset), along M/N 1024 B apart (stride byte offset).
 #pragma once
 
 #include <cuda_bf16.h>
@@ -17,27 +11,9 @@ namespace rlc {
 namespace tc {
 
 constexpr int kKChunk = 64;                   // K elements per smem stage
-constexpr uint32_t kCoreBytes = 128;          // one 8x8 bf16 core matrix
-constexpr uint32_t kRowBlockBytes = 8 * kCoreBytes;   // 8 core matrices along K
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) {
     return (uint32_t)__cvta_generic_to_shared(p);
-}
-
-// byte offset of element (row, k) of a K-major core-matrix tile (k < 64)
-__device__ __forceinline__ uint32_t core_offset(int row, int k) {
-    return (uint32_t)(((row >> 3) * 8 + (k >> 3)) * kCoreBytes + (row & 7) * 16 + (k & 7) * 2);
-}
-
-// Shared-memory matrix descriptor: start address, leading / stride byte
-// offsets (all >> 4), descriptor version 1, no swizzle.
-__device__ __forceinline__ uint64_t make_desc(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
-    uint64_t d = 0;
-    d |= (uint64_t)((saddr >> 4) & 0x3FFF);
-    d |= (uint64_t)((lbo >> 4) & 0x3FFF) << 16;
-    d |= (uint64_t)((sbo >> 4) & 0x3FFF) << 32;
-    d |= (uint64_t)1 << 46;   // version
-    return d;                 // base offset 0, layout type 0 (no swizzle)
 }
 
 // Descriptor of a K-major operand in the 128-byte swizzled layout that a TMA load with
@@ -168,6 +144,32 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* v) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
     for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
+}
+
+// the same with 16 columns, and the store of 16 columns back
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
+    uint32_t r[16];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+}
+
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const float* v) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+        "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr),
+        "r"(__float_as_uint(v[0])), "r"(__float_as_uint(v[1])), "r"(__float_as_uint(v[2])), "r"(__float_as_uint(v[3])),
+        "r"(__float_as_uint(v[4])), "r"(__float_as_uint(v[5])), "r"(__float_as_uint(v[6])), "r"(__float_as_uint(v[7])),
+        "r"(__float_as_uint(v[8])), "r"(__float_as_uint(v[9])), "r"(__float_as_uint(v[10])), "r"(__float_as_uint(v[11])),
+        "r"(__float_as_uint(v[12])), "r"(__float_as_uint(v[13])), "r"(__float_as_uint(v[14])), "r"(__float_as_uint(v[15]))
+        : "memory");
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 
 // ---- TMA (cp.async.bulk.tensor) ---------------------------------------------
