@@ -173,6 +173,7 @@ __device__ __forceinline__ void load32(const void* p, uint32_t* v) {
                  : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
                  : "l"(p));
 }
+__device__ __forceinline__ bool same_bits(float a, float b) { return __float_as_uint(a) == __float_as_uint(b); }
 __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
     const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
     return *reinterpret_cast<const uint32_t*>(&v);
@@ -687,7 +688,10 @@ cudaError_t launch_features(const FeatParams& fp, const float* xyt, int n, int r
 //                the next layer's A operand, the last one into the output layer's sums.
 // The two tiles are out of step, so one's arithmetic fills the other's waits for its MMAs.  Bound by
 // issuing that arithmetic: per ray 256 sincospi and 1,024 GELUs (a tanh each: 8 cycles of the SFU per
-// warp).  Two CTAs per SM in step with their weights' copies before: 1.08 M rays 2.32 ms, 0.93 now.
+// warp).  Two CTAs per SM in step with their weights' copies before: 1.08 M rays 2.32 ms; this 0.93,
+// with x and y features computed once for the beams of a pose and TMEM read ahead 0.79.  Not better:
+// a stream of half-size weight stages for each tile (0.96), the tiles half a tile apart (0.99), their
+// feature chunks in turn (0.82).
 // Every MMA operand, rounding point and summation order matches the layer-by-layer path, so the
 // predictions are bit-identical to it.  Operands K-major with the 128-byte swizzle (tc::make_desc_sw128).
 // Waits are bounded as in k_gemm_tma; no role waits on a hardware barrier that another may leave.
@@ -837,56 +841,84 @@ k_mlp_forward(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ C
                 u0 = __ldg(xyt + 3 * (size_t)r) * fp.inv_w;
                 u1 = __ldg(xyt + 3 * (size_t)r + 1) * fp.inv_h;
             }
-            // features [64 c, 64 c + 64): input c / 2, frequencies 32 (c % 2) .. + 31, a thread 16 of them
+            // features [64 c, 64 c + 64): input c / 2, frequencies 32 (c % 2) .. + 31, a thread 16 of them.
+            // Where the warp's rays come from at most two positions, as 32 beams or more of a pose do, lane
+            // l computes frequency l % 16 of x and y for the first (l < 16) or the second, once for them all.
+            const float ax = __shfl_sync(0xffffffffu, u0, 0), ay = __shfl_sync(0xffffffffu, u1, 0);
+            const float bx = __shfl_sync(0xffffffffu, u0, 31), by = __shfl_sync(0xffffffffu, u1, 31);
+            const bool first = same_bits(u0, ax) && same_bits(u1, ay);
+            const bool shared = __all_sync(0xffffffffu, first || (same_bits(u0, bx) && same_bits(u1, by)));
 #pragma unroll 1
             for (int c = 0; c < kFeat / tc::kKChunk; ++c) {
                 if (c >= 4 && !(ok = wait(&a_free[g][c & 3], i & 1))) break;
-                const float u = c < 2 ? u0 : c < 4 ? u1 : c < 6 ? u2 : u3;
                 const float* f = s_freq + (c & 1) * 32 + half * 16;
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const float4 fq = *reinterpret_cast<const float4*>(f + 4 * q);
-                    uint4 o;
+                uint8_t* out = act + (c & 3) * kActBlock;
+                if (c < 4 && shared) {
                     float sn, cs;
-                    sincospif(fq.x * u, &sn, &cs);
-                    o.x = pack_bf16(sn, cs);
-                    sincospif(fq.y * u, &sn, &cs);
-                    o.y = pack_bf16(sn, cs);
-                    sincospif(fq.z * u, &sn, &cs);
-                    o.z = pack_bf16(sn, cs);
-                    sincospif(fq.w * u, &sn, &cs);
-                    o.w = pack_bf16(sn, cs);
-                    if (!live) o = make_uint4(0u, 0u, 0u, 0u);
-                    *reinterpret_cast<uint4*>(act + (c & 3) * kActBlock + (((half * 4 + q) ^ swz) << 4)) = o;
+                    sincospif(f[lane & 15] * (lane < 16 ? (c < 2 ? ax : ay) : (c < 2 ? bx : by)), &sn, &cs);
+                    const uint32_t v = pack_bf16(sn, cs);   // (rows past the end take either)
+                    const int from = first ? 0 : 16;
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        uint32_t o[4];
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) o[e] = __shfl_sync(0xffffffffu, v, from + 4 * q + e);
+                        *reinterpret_cast<uint4*>(out + (((half * 4 + q) ^ swz) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
+                    }
+                } else {
+                    const float u = c < 2 ? u0 : c < 4 ? u1 : c < 6 ? u2 : u3;
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const float4 fq = *reinterpret_cast<const float4*>(f + 4 * q);
+                        uint4 o;
+                        float sn, cs;
+                        sincospif(fq.x * u, &sn, &cs);
+                        o.x = pack_bf16(sn, cs);
+                        sincospif(fq.y * u, &sn, &cs);
+                        o.y = pack_bf16(sn, cs);
+                        sincospif(fq.z * u, &sn, &cs);
+                        o.z = pack_bf16(sn, cs);
+                        sincospif(fq.w * u, &sn, &cs);
+                        o.w = pack_bf16(sn, cs);
+                        if (!live) o = make_uint4(0u, 0u, 0u, 0u);
+                        *reinterpret_cast<uint4*>(out + (((half * 4 + q) ^ swz) << 4)) = o;
+                    }
                 }
                 tc::fence_async_smem();
                 tc::fence_before_sync();
                 __syncwarp();
                 if (lane == 0) tc::mbar_arrive(tc::smem_addr(&a_full[g][c & 3]));
             }
+            if (!ok) break;
             // hidden layers: z = acc + b, rounded to bf16; h = bf16(GELU(z)) into the A blocks
 #pragma unroll 1
             for (int l = 0; l < kLayers - 1 && ok; ++l) {
                 if (!(ok = wait(&acc_full[g], layers_done++ & 1))) break;
                 const float4* bias = reinterpret_cast<const float4*>(params + b_offset(l));
-#pragma unroll 1
-                for (int cb = 128 * half; cb < 128 * half + 128; cb += 32) {
-                    float v[32];
-                    tc::tmem_ld32(acc + cb, v);
-                    uint32_t h[16];
+                const int c0 = 128 * half;
+                uint32_t v[2][32];   // the next 32 columns are on their way while these are computed
+                tc::tmem_ld32_issue(acc + c0, v[0]);
 #pragma unroll
-                    for (int q = 0; q < 32; q += 4) {
-                        const float4 b = __ldg(bias + (cb + q) / 4);
-                        const float2 z0 = unpack2(add2(pack2(v[q], v[q + 1]), pack2(b.x, b.y)));
-                        const float2 z1 = unpack2(add2(pack2(v[q + 2], v[q + 3]), pack2(b.z, b.w)));
-                        const float2 h0 = gelu(widen_bf16(pack_bf16(z0.x, z0.y))), h1 = gelu(widen_bf16(pack_bf16(z1.x, z1.y)));
-                        h[q / 2] = pack_bf16(h0.x, h0.y);
-                        h[q / 2 + 1] = pack_bf16(h1.x, h1.y);
+                for (int k = 0; k < 4; ++k) {
+                    uint32_t* a = v[k & 1];
+                    tc::tmem_ld32_wait(a);
+                    if (k < 3) tc::tmem_ld32_issue(acc + c0 + 32 * k + 32, v[(k + 1) & 1]);
+                    uint8_t* out = act + ((c0 >> 6) + (k >> 1)) * kActBlock;
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        uint32_t h[4];
+#pragma unroll
+                        for (int e = 0; e < 2; ++e) {
+                            const int j = 8 * q + 4 * e;
+                            const float4 b = __ldg(bias + (c0 + 32 * k + j) / 4);
+                            const float2 z0 = unpack2(add2(pack2(__uint_as_float(a[j]), __uint_as_float(a[j + 1])), pack2(b.x, b.y)));
+                            const float2 z1 = unpack2(add2(pack2(__uint_as_float(a[j + 2]), __uint_as_float(a[j + 3])), pack2(b.z, b.w)));
+                            const float2 h0 = gelu(widen_bf16(pack_bf16(z0.x, z0.y))), h1 = gelu(widen_bf16(pack_bf16(z1.x, z1.y)));
+                            h[2 * e] = pack_bf16(h0.x, h0.y);
+                            h[2 * e + 1] = pack_bf16(h1.x, h1.y);
+                        }
+                        *reinterpret_cast<uint4*>(out + ((((k & 1) * 4 + q) ^ swz) << 4)) = make_uint4(h[0], h[1], h[2], h[3]);
                     }
-#pragma unroll
-                    for (int q = 0; q < 4; ++q)
-                        *reinterpret_cast<uint4*>(act + (cb >> 6) * kActBlock + ((((cb & 32) / 8 + q) ^ swz) << 4)) =
-                            make_uint4(h[4 * q], h[4 * q + 1], h[4 * q + 2], h[4 * q + 3]);
                 }
                 tc::fence_async_smem();
                 tc::fence_before_sync();
@@ -1112,34 +1144,48 @@ __global__ void k_init_params(float* __restrict__ p, uint32_t seed, float init_b
     p[i] = val;
 }
 
+// the reference's range: from (x0, y0) to the corner of cell (px, py)
+__device__ __forceinline__ float corner_range(unsigned px, unsigned py, float x0, float y0) {
+    const float xd = __fsub_rn(__int2float_rn((int)px), x0), yd = __fsub_rn(__int2float_rn((int)py), y0);
+    return __fsqrt_rn(__fadd_rn(__fmul_rn(xd, xd), __fmul_rn(yd, yd)));
+}
+
 // ---------------------------------------------------- rays from the marcher
 // The exact march (RangeLib.h:927-962) also reporting t at the hit step;
 // t = max_range when the ray leaves the map or runs out of range.
 __device__ float march_t(const MapDev& m, float mr, float x0, float y0, float c, float s, float* range) {
-    float t = 0.0f;
     const unsigned W = (unsigned)m.W, H = (unsigned)m.H;
-    while (t < mr) {
-        unsigned px = (unsigned)__float2int_rz(__fadd_rn(x0, __fmul_rn(c, t)));
-        unsigned py = (unsigned)__float2int_rz(__fadd_rn(y0, __fmul_rn(s, t)));
-        float st;
-        if (m.step) {   // NaN on occupied cells, +inf off the grid (MapDev::step)
-            px = min(px, W);
-            py = min(py, H);
-            st = __ldg(m.step + (px * (H + 1u) + py));
-        } else {
+    float t = 0.0f, at = mr;
+    unsigned px = 0, py = 0;
+    bool hit = false;
+    if (m.step) {   // NaN on occupied cells, +inf off the grid (MapDev::step): one comparison ends the march
+        while (t < mr) {
+            at = t;
+            px = (unsigned)__float2int_rz(__fadd_rn(x0, __fmul_rn(c, t)));
+            py = (unsigned)__float2int_rz(__fadd_rn(y0, __fmul_rn(s, t)));
+            t = __fadd_rn(t, __ldg(m.step + (min(px, W) * (H + 1u) + min(py, H))));
+        }
+        hit = isnan(t);
+    } else {
+        while (t < mr) {
+            at = t;
+            px = (unsigned)__float2int_rz(__fadd_rn(x0, __fmul_rn(c, t)));
+            py = (unsigned)__float2int_rz(__fadd_rn(y0, __fmul_rn(s, t)));
             if (px >= W || py >= H) break;
             const float d = __ldg(m.dt + (size_t)px * m.H + py);
-            st = d <= 0.0f ? __int_as_float(0x7fc00000) : fmaxf(__fmul_rn(d, 0.999f), 1.0f);
+            if (d <= 0.0f) {
+                hit = true;
+                break;
+            }
+            t = __fadd_rn(t, fmaxf(__fmul_rn(d, 0.999f), 1.0f));
         }
-        if (isnan(st)) {
-            float xd = __fsub_rn(__int2float_rn((int)px), x0), yd = __fsub_rn(__int2float_rn((int)py), y0);
-            *range = __fsqrt_rn(__fadd_rn(__fmul_rn(xd, xd), __fmul_rn(yd, yd)));
-            return t;
-        }
-        t = __fadd_rn(t, st);
     }
-    *range = mr;
-    return mr;
+    if (!hit) {
+        *range = mr;
+        return mr;
+    }
+    *range = corner_range(px, py, x0, y0);
+    return at;
 }
 
 // random free-cell poses, uniform heading; xyt (grid frame), t target, exact range
@@ -1183,48 +1229,76 @@ __device__ __forceinline__ bool occ_cell(const MapDev& m, int x, int y) {
     return (w >> (((x & 7) << 3) | (y & 7))) & 1ull;
 }
 
-// prediction -> accept check -> range (the reference's distance to the hit
-// cell's corner); rejected rays are appended to the recast list
-__global__ void k_accept(MapDev m, float mr, const float* __restrict__ xyt, const float* __restrict__ pred, int n,
-                         float scale, float* __restrict__ outs, uint8_t* __restrict__ accepted,
-                         int* __restrict__ recast, int* __restrict__ n_recast) {
-    int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= n) return;
-    const float x0 = xyt[3 * (size_t)r], y0 = xyt[3 * (size_t)r + 1], th = xyt[3 * (size_t)r + 2];
-    const float t = pred[r];
-    bool ok = false;
-    float rg = 0.0f;
-    if (t > 1.0f && t < 0.999f * mr && isfinite(t)) {
-        float s, c;
-        rlc_trig::sincos_cr(th, &s, &c);
-        const int hx = __float2int_rz(x0 + c * t), hy = __float2int_rz(y0 + s * t);
-        const int bx = __float2int_rz(x0 + c * (t - 1.0f)), by = __float2int_rz(y0 + s * (t - 1.0f));
-        if (occ_cell(m, hx, hy) && !occ_cell(m, bx, by)) {
-            const float xd = __fsub_rn(__int2float_rn(hx), x0), yd = __fsub_rn(__int2float_rn(hy), y0);
-            rg = __fsqrt_rn(__fadd_rn(__fmul_rn(xd, xd), __fmul_rn(yd, yd)));
-            ok = true;
+// A ray whose predicted hit cell is occupied and the cell a step before it free is accepted: the range to
+// that cell's corner.  The block's other rays are collected with their direction and marched exactly, 32
+// at a time per warp as warps come free (lanes taking rays one by one: 98 us).  (Two passes with a list in memory, and the march's two tests a
+// step: 103 us for 1.08 M rays of which all are recast, now 86.)
+constexpr int kResolveRays = 1024, kResolveThreads = 256;
+
+__global__ void __launch_bounds__(kResolveThreads) k_resolve(MapDev m, float mr, const float* __restrict__ xyt,
+                                                             const float* __restrict__ pred, int n, float scale,
+                                                             float* __restrict__ outs, uint8_t* __restrict__ accepted,
+                                                             int* __restrict__ n_recast) {
+    __shared__ float4 s_ray[kResolveRays];
+    __shared__ unsigned short s_id[kResolveRays];
+    __shared__ int s_count, s_next;
+    if (threadIdx.x == 0) s_count = s_next = 0;
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    const long long base = (long long)blockIdx.x * kResolveRays;
+#pragma unroll
+    for (int j = 0; j < kResolveRays / kResolveThreads; ++j) {
+        const int id = j * kResolveThreads + (int)threadIdx.x;
+        const long long r = base + id;
+        bool recast = false;
+        float x0 = 0.0f, y0 = 0.0f, s = 0.0f, c = 0.0f;
+        if (r < n) {
+            x0 = __ldg(xyt + 3 * r);
+            y0 = __ldg(xyt + 3 * r + 1);
+            rlc_trig::sincos_cr(__ldg(xyt + 3 * r + 2), &s, &c);
+            const float t = __ldg(pred + r);
+            bool ok = false;
+            if (t > 1.0f && t < 0.999f * mr && isfinite(t)) {
+                const int hx = __float2int_rz(x0 + c * t), hy = __float2int_rz(y0 + s * t);
+                const int bx = __float2int_rz(x0 + c * (t - 1.0f)), by = __float2int_rz(y0 + s * (t - 1.0f));
+                if (occ_cell(m, hx, hy) && !occ_cell(m, bx, by)) {
+                    outs[r] = __fmul_rn(corner_range((unsigned)hx, (unsigned)hy, x0, y0), scale);
+                    ok = true;
+                }
+            }
+            if (accepted) accepted[r] = ok ? 1 : 0;
+            recast = !ok;
+        }
+        const unsigned who = __ballot_sync(0xffffffffu, recast);
+        if (who) {
+            int slot = 0;
+            if (lane == 0) slot = atomicAdd(&s_count, __popc(who));
+            slot = __shfl_sync(0xffffffffu, slot, 0) + __popc(who & ((1u << lane) - 1u));
+            if (recast) {
+                s_ray[slot] = make_float4(x0, y0, c, s);
+                s_id[slot] = (unsigned short)id;
+            }
         }
     }
-    if (accepted) accepted[r] = ok ? 1 : 0;
-    if (ok) {
-        outs[r] = __fmul_rn(rg, scale);
-    } else {
-        int slot = atomicAdd(n_recast, 1);
-        recast[slot] = r;
+    __syncthreads();
+    const int count = s_count;
+    if (threadIdx.x == 0 && count) atomicAdd(n_recast, count);
+    for (;;) {
+        int i = 0;
+        if (lane == 0) i = atomicAdd(&s_next, 32);
+        i = __shfl_sync(0xffffffffu, i, 0);
+        if (i >= count) break;
+        i += lane;
+        if (i < count) {
+            const float4 q = s_ray[i];
+            float rg;
+            march_t(m, mr, q.x, q.y, q.z, q.w, &rg);
+            outs[base + s_id[i]] = __fmul_rn(rg, scale);
+        }
     }
 }
 
-__global__ void k_recast(MapDev m, float mr, const float* __restrict__ xyt, const int* __restrict__ list,
-                         const int* __restrict__ count, float scale, float* __restrict__ outs) {
-    int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= *count) return;
-    const int r = list[j];
-    const float x0 = xyt[3 * (size_t)r], y0 = xyt[3 * (size_t)r + 1], th = xyt[3 * (size_t)r + 2];
-    float s, c, rg;
-    rlc_trig::sincos_cr(th, &s, &c);
-    march_t(m, mr, x0, y0, c, s, &rg);
-    outs[r] = __fmul_rn(rg, scale);
-}
+
 
 // world-frame particles x beams -> grid-frame rays (RangeLib.h:482-520)
 __global__ void k_world_rays(WorldDev w, const float* __restrict__ ins, const float* __restrict__ angles, int n,
@@ -1278,16 +1352,14 @@ struct LearnedModel {
     long long qcap = 0;
     float* q_xyt = nullptr;
     float* q_pred = nullptr;
-    int* q_list = nullptr;
     int* q_cnt = nullptr;
 
     cudaError_t ensure_query(long long rays) {
         if (rays <= qcap) return cudaSuccess;
-        cudaFree(q_xyt); cudaFree(q_pred); cudaFree(q_list); cudaFree(q_cnt);
-        q_xyt = q_pred = nullptr; q_list = q_cnt = nullptr; qcap = 0;
+        cudaFree(q_xyt); cudaFree(q_pred); cudaFree(q_cnt);
+        q_xyt = q_pred = nullptr; q_cnt = nullptr; qcap = 0;
         TRY(cudaMalloc(&q_xyt, (size_t)rays * 3 * sizeof(float)));
         TRY(cudaMalloc(&q_pred, (size_t)rays * sizeof(float)));
-        TRY(cudaMalloc(&q_list, (size_t)rays * sizeof(int)));
         TRY(cudaMalloc(&q_cnt, sizeof(int)));
         qcap = rays;
         return cudaSuccess;
@@ -1306,7 +1378,7 @@ struct LearnedModel {
         free_work();
         cudaFree(params); cudaFree(adam_m); cudaFree(adam_v); cudaFree(grads); cudaFree(wbf); cudaFree(err);
         cudaFree(free_cells);
-        cudaFree(q_xyt); cudaFree(q_pred); cudaFree(q_list); cudaFree(q_cnt);
+        cudaFree(q_xyt); cudaFree(q_pred); cudaFree(q_cnt);
     }
     cudaError_t ensure(int rows) {
         rows = (rows + kBM - 1) / kBM * kBM;
@@ -1647,7 +1719,6 @@ int rlc_learned_calc_range_repeat_angles(rlc_learned* L, const float* d_ins, con
     LTRY(M.ensure_query(rays), "learned query buffers");
     float* xyt = M.q_xyt;
     float* pred = M.q_pred;
-    int* list = M.q_list;
     int* cnt = M.q_cnt;
     cudaError_t e = cudaMemsetAsync(cnt, 0, sizeof(int), s);
     if (e == cudaSuccess) {
@@ -1657,12 +1728,8 @@ int rlc_learned_calc_range_repeat_angles(rlc_learned* L, const float* d_ins, con
     int rc = RLC_OK;
     if (e == cudaSuccess) rc = rlc_learned_predict(L, xyt, (int)rays, pred, stream);
     if (e == cudaSuccess && !rc) {
-        k_accept<<<blocks_for(rays, 256), 256, 0, s>>>(M.map, M.mr, xyt, pred, (int)rays, M.world.s, d_outs,
-                                                       d_accepted, list, cnt);
-        e = cudaGetLastError();
-    }
-    if (e == cudaSuccess && !rc) {
-        k_recast<<<blocks_for(rays, 256), 256, 0, s>>>(M.map, M.mr, xyt, list, cnt, M.world.s, d_outs);
+        k_resolve<<<blocks_for(rays, kResolveRays), kResolveThreads, 0, s>>>(M.map, M.mr, xyt, pred, (int)rays, M.world.s,
+                                                                             d_outs, d_accepted, cnt);
         e = cudaGetLastError();
     }
     int h_cnt = 0;

@@ -16,3 +16,16 @@ def test_fused_forward_at_grid_edges(rl, learned_setup, n):  # noqa: F811
     L.train(steps=3, batch=1024)
     xyt, _, _ = L.sample_rays(n, seed=n)
     assert torch.equal(L.predict(xyt), L.predict(xyt, layered=True))
+
+
+@pytest.mark.parametrize("na", [1, 7, 30, 31, 32, 33, 108])
+def test_fused_forward_of_shared_positions(rl, learned_setup, na):  # noqa: F811
+    """Runs of rays from one position (features of x and y computed once where a warp's rays have at most two)."""
+    _, _, rm = learned_setup
+    L = rl.PyLearnedRM(rm, seed=9)
+    L.train(steps=3, batch=1024)
+    poses, _, _ = L.sample_rays(5000 // na + 1, seed=na)
+    xyt = poses.repeat_interleave(na, dim=0)
+    xyt[:, 2] += torch.linspace(-2.0, 2.0, na, device=xyt.device).repeat(len(poses))
+    xyt = xyt[3:].contiguous()
+    assert torch.equal(L.predict(xyt), L.predict(xyt, layered=True))
