@@ -149,8 +149,8 @@ _fast = None   # None: not looked for yet; False: not built
 
 def fast():
     """The CPython entry points of the per-call methods (csrc/rlc_py.c), or None where they were
-    not built.  They call the same C ABI; -1 from them means "argument not a plain buffer of the
-    expected type and shape", and the caller takes its checked ctypes path."""
+    not built.  They call the same C ABI; -1 from them means "arguments not all plain buffers, or
+    all plain CUDA tensors, of the expected type and shape", and the caller takes its checked ctypes path."""
     global _fast
     if _fast is None:
         lib()   # the library first, so that the module binds to this loaded copy

@@ -382,7 +382,7 @@ class _RangeMethod:
 
     def calc_range_many(self, ins, outs) -> None:
         F = _lib.fast()
-        if F is not None:   # numpy buffers straight to the C ABI; -1: not a plain buffer, check below
+        if F is not None:   # plain buffers or tensors straight to the C ABI; -1: neither, check below
             rc = F.calc_range_many(self._h.value, ins, outs)
             if rc != -1:
                 return _lib.check(rc)
