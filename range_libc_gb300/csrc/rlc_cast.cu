@@ -673,16 +673,6 @@ __device__ float cddt_cast(const CastParams& p, float x, float y, float heading)
                                     : bound_g(q.bin, q.n, q.lx, upper));
 }
 
-// A query by the table's index (CddtDev::index; schedules that name a search keep theirs).  The
-// index holds, for every bin and every kCddtBucket pixels along it, where in the query's copy of the
-// zero points (CddtDev::qz: per bin -inf, the zero points, +inf up to a whole quad) those at or past
-// the bucket's start begin.  Bucket numbers are a monotone function of the position, so the bound
-// lies between the bucket's start and the next one's whatever that function rounds.  A query reads
-// the slice's two records (L1), one index entry and a quad or two of zero points, in which it keeps
-// the last value not past lx and the first past it without branches: 3 dependent reads and ~5
-// scattered requests, against ~10 and ~20 for slice entries, bin bounds, bin ends and a binary
-// search.  1 M queries on 2048^2, td 108: 42 -> 24.5 us (binary search / index; the sector search 39),
-// td 216 48 -> 31, pruned 36 -> 21, 512^2 32 -> 21; 4,000 x 500 beams and their weights 52 -> 46.
 __device__ __forceinline__ float cddt_cast_index(const CastParams& p, float x, float y, float heading) {
     const CddtDev& c = p.cddt;
     const float mr = p.mr, inf = __int_as_float(0x7f800000);
@@ -790,6 +780,16 @@ __device__ __forceinline__ int glt_discretize(const GltDev& g, float theta, unsi
     return (unsigned)rounded < g.td ? rounded : (int)((unsigned)rounded % g.td);
 }
 
+// A lookup table entry, from device memory in 64 bytes: a plain load of a line that is not in L2 brings
+// most of its 128.  1 M random rays on a 226 MB table read 74 instead of 131 MB, 25.7 instead of 26.6 us;
+// what is left is the rate of random DRAM accesses (2, 4 or 8 rays per thread change nothing).  Not for
+// the CDDT index, whose next entries are often needed (30.2 instead of 28.7 us).
+__device__ __forceinline__ uint16_t load_entry(const uint16_t* p) {
+    uint16_t v;
+    asm("ld.global.nc.L2::64B.u16 %0, [%1];" : "=h"(v) : "l"(p));
+    return v;
+}
+
 // GiantLUTCast::calc_range, RangeLib.h:1869-1881; NaN arguments give max_range
 __device__ __forceinline__ float glt_cast(const CastParams& p, float x, float y, float heading) {
     if (isnan(x) || isnan(y) || isnan(heading)) return p.mr;
@@ -797,7 +797,7 @@ __device__ __forceinline__ float glt_cast(const CastParams& p, float x, float y,
     const GltDev& g = p.glt;
     const int b = glt_discretize(g, heading, p.err);
     const size_t cell = (size_t)__float2int_rz(x) * p.map.H + __float2int_rz(y);
-    return __fmul_rn(__int2float_rn(__ldg(g.lut + cell * g.td + b)), g.max_div_limits);
+    return __fmul_rn(__int2float_rn(load_entry(g.lut + cell * g.td + b)), g.max_div_limits);
 }
 
 // one ray per (cell corner, angle bin), angle bins fastest: lut[(x * H + y) * td + i]
