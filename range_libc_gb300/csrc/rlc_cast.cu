@@ -943,6 +943,7 @@ __global__ void __launch_bounds__(256) k_cddt_radial(CastParams p, const float* 
 template <int KIND, int LAYOUT, int PF, bool WORLD>
 __global__ void __launch_bounds__(256) k_calc_range_many(CastParams p, const float* __restrict__ ins,
                                                          float* __restrict__ outs, int n) {
+    after_previous();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (KIND == K_CDDT && PF == 1) {   // warp-cooperative bin search: every lane of the warp takes part
         const bool act = i < n;
@@ -975,6 +976,7 @@ template <int KIND, int LAYOUT, int PF>
 __global__ void __launch_bounds__(256) k_repeat_angles(CastParams p, const float* __restrict__ ins,
                                                        const float* __restrict__ angles,
                                                        float* __restrict__ outs, int n, int na) {
+    after_previous();
     long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (KIND == K_CDDT && PF == 1) {   // warp-cooperative bin search
         const bool act = g < (long long)n * na;
@@ -1068,6 +1070,7 @@ __global__ void __launch_bounds__(32 * kEvalWarps) k_eval_sensor(CastParams p, S
                                                                  const float* __restrict__ ranges,
                                                                  double* __restrict__ outs, int na, int n) {
     __shared__ double s_f[2][kEvalBeams][33];   // [beam][particle]; a row is 33 doubles: no bank conflicts either way
+    after_previous();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int first = blockIdx.x * 32, np = min(32, n - first);
     const float* rows = ranges + (size_t)first * na;
@@ -1161,6 +1164,7 @@ __global__ void __launch_bounds__(512, KIND == K_CDDT ? 1 : KIND == K_BL ? 2 : 4
                                                const float* __restrict__ angles, const float* __restrict__ obs,
                                                double* __restrict__ weights, int n, int na, int P) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    after_previous();
     double* sf = reinterpret_cast<double*>(smem_raw);
     const int first = blockIdx.x * P, nr = P * na;
     const float inv_na = __frcp_rn(__int2float_rn(na));
@@ -1342,6 +1346,7 @@ k_fused_wide(CastParams p, SensorDev sm, const float* __restrict__ ins, const fl
              const float* __restrict__ obs, double* __restrict__ weights, int n, int na, int P, int C) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ unsigned s_next[2];
+    after_previous();
     const int first = blockIdx.x * P;
     wide_tile<KIND, LAYOUT, PF, FACTORS>(p, sm, ins, angles, obs, nullptr, weights, first, min(P, n - first), na, P, C,
                                          smem_raw, s_next);
@@ -1834,9 +1839,8 @@ template <int KIND, int LAYOUT, int PF>
 struct RunMany {
     static cudaError_t run(const CastParams& p, bool world, const float* ins, float* outs, int n, cudaStream_t s) {
         if (n <= 0) return cudaSuccess;
-        if (world) k_calc_range_many<KIND, LAYOUT, PF, true><<<blocks_for(n, 256), 256, 0, s>>>(p, ins, outs, n);
-        else k_calc_range_many<KIND, LAYOUT, PF, false><<<blocks_for(n, 256), 256, 0, s>>>(p, ins, outs, n);
-        return cudaGetLastError();
+        return launch_next(world ? k_calc_range_many<KIND, LAYOUT, PF, true> : k_calc_range_many<KIND, LAYOUT, PF, false>,
+                           dim3(blocks_for(n, 256)), 256, 0, s, p, ins, outs, n);
     }
 };
 
@@ -1846,8 +1850,7 @@ struct RunAngles {
                            cudaStream_t s) {
         long long total = (long long)n * na;
         if (total <= 0) return cudaSuccess;
-        k_repeat_angles<KIND, LAYOUT, PF><<<blocks_for(total, 256), 256, 0, s>>>(p, ins, angles, outs, n, na);
-        return cudaGetLastError();
+        return launch_next(k_repeat_angles<KIND, LAYOUT, PF>, dim3(blocks_for(total, 256)), 256, 0, s, p, ins, angles, outs, n, na);
     }
 };
 
@@ -1917,8 +1920,7 @@ struct RunFused {
                 const int C = min(factors ? (P <= 2 ? 256 : 128) : max(32, (kWideChunk / P + 31) / 32 * 32), (na + 3) / 4 * 4);
                 const int smem = wide_smem(P, C, factors).total;
                 const auto kernel = factors ? k_fused_wide<KIND, LAYOUT, PF, true> : k_fused_wide<KIND, LAYOUT, PF, false>;
-                kernel<<<blocks_for(n, P), kWideThreads, smem, s>>>(p, sm, ins, angles, obs, w, n, na, P, C);
-                return cudaGetLastError();
+                return launch_next(kernel, dim3(blocks_for(n, P)), kWideThreads, smem, s, p, sm, ins, angles, obs, w, n, na, P, C);
             }
         }
         int P, threads;
@@ -1926,8 +1928,7 @@ struct RunFused {
         const size_t smem = (size_t)P * na * sizeof(double);
         cudaError_t e = set_smem(k_fused<KIND, LAYOUT, PF>, smem);
         if (e != cudaSuccess) return e;
-        k_fused<KIND, LAYOUT, PF><<<blocks_for(n, P), threads, smem, s>>>(p, sm, ins, angles, obs, w, n, na, P);
-        return cudaGetLastError();
+        return launch_next(k_fused<KIND, LAYOUT, PF>, dim3(blocks_for(n, P)), threads, smem, s, p, sm, ins, angles, obs, w, n, na, P);
     }
 };
 
@@ -1946,8 +1947,7 @@ cudaError_t launch_repeat_angles(const CastParams& p, int layout, int pf, const 
 cudaError_t launch_eval_sensor(const CastParams& p, const SensorDev& sm, const float* obs, const float* ranges,
                                double* outs, int na, int n, cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
-    k_eval_sensor<<<blocks_for(n, 32), 32 * kEvalWarps, 0, s>>>(p, sm, obs, ranges, outs, na, n);
-    return cudaGetLastError();
+    return launch_next(k_eval_sensor, dim3(blocks_for(n, 32)), 32 * kEvalWarps, 0, s, p, sm, obs, ranges, outs, na, n);
 }
 
 cudaError_t launch_fused(const CastParams& p, int layout, int pf, const SensorDev& sm, const float* ins,

@@ -51,27 +51,6 @@ __host__ __device__ inline size_t b_offset(int l) { return w_offset(l) + (l == 0
 __host__ __device__ inline int layer_in(int l) { return l == 0 ? kFeat : kHidden; }
 constexpr size_t kOutW = kW0 + kHidden + 3 * (kWh + kHidden);  // output weights [256], then bias [1]
 
-// ------------------------------------------------------------------ launches
-// A training step is a chain of 15 kernels of 17-30 us.  Each is launched while the one before it drains,
-// sets itself up (barriers, TMEM, empty sums) and waits for the other's end and writes with after_previous()
-// before it touches memory: 0.73 instead of 0.80 ms for two steps of 65,536 rays.  Launched any other way the wait is nothing.
-__device__ __forceinline__ void after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
-template <class... P, class... A>
-cudaError_t launch_next(void (*kernel)(P...), dim3 grid, int block, size_t smem, cudaStream_t s, const A&... a) {
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t c{};
-    c.gridDim = grid;
-    c.blockDim = dim3(block);
-    c.dynamicSmemBytes = smem;
-    c.stream = s;
-    c.attrs = &at;
-    c.numAttrs = 1;
-    return cudaLaunchKernelEx(&c, kernel, static_cast<P>(a)...);
-}
-
 // -------------------------------------------------------------------- GEMM
 struct GemmArgs {
     const bf16* A;   // A[m * lda + k] (K-major), or with a_t A[k * lda + m] (M-major)
