@@ -72,6 +72,7 @@ struct rlc_map {
     uint8_t* d_dt8 = nullptr;
     float* d_step = nullptr;
     uint32_t* d_runs = nullptr;   // equal-step runs of the step map (DT_RUNS)
+    bool long_runs = true;        // enough of them to be worth reading (ensure_dt)
     std::atomic<int> refs{1};
     std::mutex mu;
 
@@ -116,7 +117,7 @@ struct rlc_map {
         const size_t steps = step_map_cells(W, H);
         const size_t o_dt = room(n * sizeof(float)), o_step = room(steps * sizeof(float));
         const size_t o_tiled = room(tiled * sizeof(float)), o_u16 = room(tiled * sizeof(uint16_t)), o_u8 = room(tiled);
-        const size_t o_runs = room(n * sizeof(uint32_t)), o_eq = room(step_eq_words(W, H) * sizeof(uint32_t));
+        const size_t o_runs = room(n * sizeof(uint32_t)), o_eq = room(step_eq_words(W, H) * sizeof(uint32_t)), o_share = room(8);
         const size_t sb = edt_scratch_bytes(W, H);
         void* extra = nullptr;   // maps with a side above 16384 need more scratch than the run map holds
         char* base = nullptr;
@@ -130,7 +131,9 @@ struct rlc_map {
         o.u8 = (uint8_t*)(base + o_u8);
         uint32_t* runs = (uint32_t*)(base + o_runs);
         if (e == cudaSuccess) e = launch_edt(d_bits, W, H, TY, o, extra ? extra : runs, sb, 0);
-        if (e == cudaSuccess && steps) e = launch_step_runs(o.step, W, H, (uint32_t*)(base + o_eq), runs, 0);
+        unsigned long long share = 0, *d_share = (unsigned long long*)(base + o_share);
+        if (e == cudaSuccess && steps && n) e = launch_step_runs(o.step, W, H, (uint32_t*)(base + o_eq), runs, d_share, 0);
+        if (e == cudaSuccess && steps && n) e = cudaMemcpyAsync(&share, d_share, sizeof(share), cudaMemcpyDeviceToHost, 0);
         if (e == cudaSuccess) e = cudaStreamSynchronize(0);
         cudaFree(extra);
         if (e != cudaSuccess) {
@@ -144,6 +147,11 @@ struct rlc_map {
         d_dt8 = o.u8;
         d_step = o.step;
         d_runs = runs;
+        // Runs are long where walls lie along the axes: in a quarter to a half of the free cells of the
+        // rectangles-and-disks maps, three quarters of the corridor maps', but 8 % on the reference's
+        // basement map, where reading them costs more than it saves (200,000 queries of 300 px from free
+        // cells linear / step / runs 42 / 40 / 48 us, 2 M of 500 px 101 / 99 / 105 us).  The line is at a sixth.
+        long_runs = 6 * (share & 0xffffffffull) >= share >> 32;
         return RLC_OK;
     }
     void retain() { refs.fetch_add(1); }
@@ -399,6 +407,7 @@ int cast_layout(const rlc_method* m) { return m->layout == DT_STAGED ? DT_LINEAR
 // 43 / 41 / 46 us, 20,000 x 1,081 267 / 257 / 336 us).
 int cast_layout(const rlc_method* m, long long rays, bool independent) {
     if (!m->pick || m->dkind != K_RM) return cast_layout(m);
+    if (!m->map->long_runs) return map_layout(m->map, DT_STEP);
     return map_layout(m->map, independent || (rays >= (1ll << 14) && rays < (1ll << 18)) ? DT_RUNS : DT_STEP);
 }
 
@@ -412,6 +421,7 @@ int cast_search(const rlc_method* m) { return m->pick && m->dkind == K_CDDT && m
 // 4,000 x 1,081 - / 140 / 157, 20,000 x 1,081 438 / 423 / 496 us.
 int fused_layout(const rlc_method* m, int n, int na) {
     if (!m->pick || m->dkind != K_RM) return cast_layout(m);
+    if (!m->map->long_runs) return map_layout(m->map, DT_STEP);
     return map_layout(m->map, (long long)n * na < (2ll << 20) && (na < 512 || n >= 2000) ? DT_RUNS : DT_STEP);
 }
 
@@ -1295,15 +1305,16 @@ struct rlc_batch {
         CUDA_OR_FAIL(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "batch setup");
         run = Schedule{layout, prefetch, block, tile, separate, false};
         bool steps = true;   // every ray-marching filter's map has a step map
-        long long particles = 0;
+        long long particles = 0, run_rays = 0;   // rays on maps with long equal-step runs
         for (const rlc_filter_desc& d : descs) {
             if (d.method->dkind == K_RM && map_layout(d.method->map, DT_STEP) != DT_STEP) steps = false;
             particles += d.n_particles;
+            if (d.method->map->long_runs) run_rays += (long long)d.n_particles * d.n_angles;
         }
         if (!steps && (layout == DT_STEP || layout == DT_RUNS)) run.layout = DT_LINEAR;
         if (pick && rm_only && steps) {
             if (rays < (48ll << 20))
-                run = Schedule{rays < (2ll << 20) ? DT_RUNS : DT_STEP, 0, 256, batch_wide_tile(particles, sms), false, true};
+                run = Schedule{rays < (2ll << 20) && 2 * run_rays >= rays ? DT_RUNS : DT_STEP, 0, 256, batch_wide_tile(particles, sms), false, true};
             else
                 run = Schedule{DT_STEP, 0, 256, 8, true, false};
         }

@@ -138,7 +138,9 @@ constexpr size_t edt_scratch_bound(size_t cells, size_t side) {
 size_t step_map_cells(int W, int H);
 // equal-step run lengths of the step map along both axes (MapDev::runs); d_eq: step_eq_words scratch
 size_t step_eq_words(int W, int H);
-cudaError_t launch_step_runs(const float* d_step, int W, int H, uint32_t* d_eq, uint32_t* d_runs, cudaStream_t s);
+// d_share: free cells sampled << 32 | those with a run that a ray may skip
+cudaError_t launch_step_runs(const float* d_step, int W, int H, uint32_t* d_eq, uint32_t* d_runs, unsigned long long* d_share,
+                             cudaStream_t s);
 cudaError_t launch_edge_map(const uint64_t* d_bits, int W, int H, int tiles_y, uint8_t* d_edge, cudaStream_t s);
 cudaError_t launch_unpack_bits(const uint64_t* d_bits, int W, int H, int tiles_y, uint8_t* d_occ, cudaStream_t s);
 

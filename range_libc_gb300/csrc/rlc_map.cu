@@ -590,8 +590,10 @@ __global__ void __launch_bounds__(256) k_dt_layouts(const float* __restrict__ li
 // (y >> 5)] is step(x, y - 1) == step(x, y), bit x & 31 of eqx[(x >> 5) * H + y] is step(x - 1, y)
 // == step(x, y).  A warp reads a 32 x 32 patch once, 32 independent coalesced rows.
 __global__ void __launch_bounds__(256) k_step_eq(const float* __restrict__ step, int W, int H, int HW,
-                                                 uint32_t* __restrict__ eqx, uint32_t* __restrict__ eqy) {
+                                                 uint32_t* __restrict__ eqx, uint32_t* __restrict__ eqy,
+                                                 unsigned long long* __restrict__ share) {
     const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (w == 0 && threadIdx.x == 0) *share = 0ull;
     const int lane = threadIdx.x & 31, XW = (W + 31) >> 5;
     if (w >= (long long)XW * HW) return;
     const int xw = (int)(w / HW), yw = (int)(w - (long long)xw * HW), x0 = xw << 5, y = (yw << 5) + lane;
@@ -648,15 +650,28 @@ __device__ __forceinline__ unsigned bits_up(const Word& word, int j, int nw) {
 // runs[x * H + y]: how many cells after (x, y) along +y, -y, +x and -x have its step (bits 0-7,
 // 8-15, 16-23, 24-31; at most 255 each), counted in the bit lines: one or two words per direction
 // where a thread per line walked the map before.  2048^2: 2106 us -> 51 us with k_step_eq.
+// *share, zeroed before: over a sixteenth of the blocks, the free cells (upper half) and those of them with
+// a run that a ray may skip (kLongRun; lower half).
+constexpr uint32_t kLongRun = 12;
+
 __global__ void __launch_bounds__(256) k_step_runs(const uint32_t* __restrict__ eqx, const uint32_t* __restrict__ eqy,
-                                                   int W, int H, int HW, uint32_t* __restrict__ runs) {
+                                                   const float* __restrict__ step, int W, int H, int HW,
+                                                   uint32_t* __restrict__ runs, unsigned long long* __restrict__ share) {
     const unsigned yb = ((unsigned)H + 31u) >> 5, bx = blockIdx.x / yb;   // 32 y x 8 x cells per block
     const int x = (int)(bx * 8 + threadIdx.y), y = (int)((blockIdx.x - bx * yb) * 32 + threadIdx.x);
-    if (x >= W || y >= H) return;
-    const auto wx = [&](int w) { return __ldg(eqx + (size_t)w * H + y); };
-    const auto wy = [&](int w) { return __ldg(eqy + (size_t)x * HW + w); };
-    runs[(size_t)x * H + y] = bits_up(wy, y + 1, HW) | bits_down(wy, y) << 8 | bits_up(wx, x + 1, (W + 31) >> 5) << 16 |
-              bits_down(wx, x) << 24;
+    const bool in = x < W && y < H;
+    uint32_t word = 0;
+    if (in) {
+        const auto wx = [&](int w) { return __ldg(eqx + (size_t)w * H + y); };
+        const auto wy = [&](int w) { return __ldg(eqy + (size_t)x * HW + w); };
+        word = bits_up(wy, y + 1, HW) | bits_down(wy, y) << 8 | bits_up(wx, x + 1, (W + 31) >> 5) << 16 |
+               bits_down(wx, x) << 24;
+        runs[(size_t)x * H + y] = word;
+    }
+    if ((blockIdx.x * 0x9E3779B1u) >> 28) return;
+    const int free = __syncthreads_count(in && !isnan(__ldg(step + (size_t)x * (H + 1) + y)));
+    const int lng = __syncthreads_count(in && __vcmpgeu4(word, kLongRun * 0x01010101u) != 0u);
+    if (threadIdx.x == 0 && threadIdx.y == 0 && free) atomicAdd(share, ((unsigned long long)free << 32) + (unsigned)lng);
 }
 
 // RangeLib.h:293-312: an occupied cell with any in-grid free 8-neighbour.
@@ -804,15 +819,16 @@ size_t step_eq_words(int W, int H) {
     return (size_t)W * ((H + 31) >> 5) + (size_t)((W + 31) >> 5) * H;
 }
 
-cudaError_t launch_step_runs(const float* d_step, int W, int H, uint32_t* d_eq, uint32_t* d_runs, cudaStream_t s) {
+cudaError_t launch_step_runs(const float* d_step, int W, int H, uint32_t* d_eq, uint32_t* d_runs, unsigned long long* d_share,
+                             cudaStream_t s) {
     if ((long long)W * H == 0) return cudaSuccess;
     const int HW = (H + 31) >> 5, XW = (W + 31) >> 5;
     uint32_t* eqy = d_eq;
     uint32_t* eqx = d_eq + (size_t)W * HW;
-    k_step_eq<<<blocks_for((long long)XW * HW, 8), 256, 0, s>>>(d_step, W, H, HW, eqx, eqy);
+    k_step_eq<<<blocks_for((long long)XW * HW, 8), 256, 0, s>>>(d_step, W, H, HW, eqx, eqy, d_share);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    k_step_runs<<<blocks_for(H, 32) * blocks_for(W, 8), dim3(32, 8), 0, s>>>(eqx, eqy, W, H, HW, d_runs);
+    k_step_runs<<<blocks_for(H, 32) * blocks_for(W, 8), dim3(32, 8), 0, s>>>(eqx, eqy, d_step, W, H, HW, d_runs, d_share);
     return cudaGetLastError();
 }
 
