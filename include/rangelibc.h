@@ -219,7 +219,7 @@ RLC_API int rlc_count_steps(rlc_method* m, const float* ins, const float* angles
 /* ---- tuning ------------------------------------------------------------ */
 /* Schedule of the kernels: dt_layout 0 = linear x-major distance transform, 1 = 8x8 tiles,
  * 2 = compact 16-bit squared distances, 4 = linear map of each cell's march step
- * max(d * 0.999, 1) (0 on occupied cells), 5 = that step map plus, per cell, how many cells after
+ * max(d * 0.999, 1) (a marker on occupied cells), 5 = that step map plus, per cell, how many cells after
  * it along each axis have the same step, so that a ray repeating one step beside a wall (6 times
  * in a row) skips the rest of the run in one go (exactly: the skipped steps' parameters are formed by the reference's own float
  * additions and the landing cell is checked), 3 = beam-major fused update that stages each bundle's
@@ -230,7 +230,9 @@ RLC_API int rlc_count_steps(rlc_method* m, const float* ins, const float* angles
  * step, ballot; calc_range_many and calc_range_repeat_angles), 2 by 32-byte sectors for bins of
  * more than 32 zero points (fewer dependent reads; pays when queries spread over the map); tile =
  * particles per tile of the fused and batched kernels (0 = automatic).  Results are identical
- * under every schedule. */
+ * under every schedule.  Until a schedule is set or tuned, every call picks its kernel by its size
+ * and map (layouts 4 and 5, a wide kernel for large fused updates, the CDDT table's index);
+ * get_schedule then reports the values that set_schedule would start from. */
 RLC_API int rlc_method_set_schedule(rlc_method* m, int dt_layout, int fused_block, int prefetch, int tile);
 RLC_API int rlc_method_get_schedule(const rlc_method* m, int* dt_layout, int* fused_block, int* prefetch,
                                     int* tile);
@@ -290,7 +292,9 @@ RLC_API int rlc_batch_run(rlc_batch* b, void* stream);
 /* Schedule of the persistent launch: distance-transform layout (0 linear, 1 tiled, 2 compact
  * 16-bit, 4 step map, 5 step map with equal-step runs) and prefetch of every ray-marching filter,
  * threads per block, particles per tile
- * (0 = 32).  Results are identical under every schedule. */
+ * (0 = 32).  Results are identical under every schedule.  Until a schedule, a product mode or a block
+ * size is given, a batch of ray marchers picks its launch by its size (one wide launch with the
+ * products inside below 48 M rays). */
 RLC_API int rlc_batch_set_schedule(rlc_batch* b, int dt_layout, int prefetch, int block, int tile);
 RLC_API int rlc_batch_get_schedule(const rlc_batch* b, int* dt_layout, int* prefetch, int* block, int* tile);
 /* Where the per-particle products run: RLC_PRODUCTS_OVERLAPPED -- inside the persistent kernel,
