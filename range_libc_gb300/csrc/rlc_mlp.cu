@@ -138,10 +138,10 @@ __device__ __forceinline__ f32x2 gelu_grad(f32x2 z) {
 // copy two bytes at a time, and three transposes ran per step).
 //
 // Warp-specialised (10 warps, 192 KB of pipeline stages):
-//   warp 0     TMA producer: per 64-wide K chunk, the tiles of A (128 rows or columns) and B (BN)
+//   warp 0     TMA producer: per K chunk of KS, the tiles of A (128 rows or columns) and B (BN)
 //              into stage s, completing on full[s]; it reuses a stage once the MMAs that read it have
 //              committed to empty[s] (and the warps that sum it have arrived there);
-//   warp 1     allocates BN TMEM columns; one thread issues the chunk's four
+//   warp 1     allocates BN TMEM columns; one thread issues the chunk's
 //              tcgen05.mma (K = 16 each) per stage and commits them to empty[s], and after the
 //              last chunk to `accum`;
 //   warps 2-9  with k_sums: add up the rows of every stage of A on its way (the bias gradients, which
@@ -153,6 +153,10 @@ __device__ __forceinline__ f32x2 gelu_grad(f32x2 z) {
 // k * 128 bytes (tc::make_desc_sw128_mn); 16-byte chunks permuted by the row & 7.
 // Every wait is bounded (about a second); a time-out sets bit 16 of *err, the remaining roles stop
 // at their next wait, and the CTA still frees its TMEM.
+//
+// KS: K of a stage.  64, or 128 where both operands are M/N-major and few CTAs each have a long chain:
+// there the issuing threads set the pace (a step of 32,640 rays: 0.93 ms in stages of 64, 0.84 in stages of
+// 128, 0.78 with the issuing warps kept together, so that their loops run in uniform registers).
 //
 // Bound by reading dZ and the layer's input: 67 MB for a hidden layer and 65,536 rays, 17 us (22 from the
 // transposed copies, which cost 32 us and more to write, and 27 us for the bias sums).
@@ -185,10 +189,10 @@ __device__ __forceinline__ f32x2 widen_bf16(uint32_t u) {
 }
 __device__ __forceinline__ float2 unpack_bf16(uint32_t u) { return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u)); }
 
-template <int BN>
+template <int BN, int KS>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 k_gemm_tma(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, GemmArgs g) {
-    constexpr uint32_t kStageB = BN * tc::kKChunk * 2;
+    constexpr uint32_t kStageA = kBM * KS * 2, kStageB = BN * KS * 2, kBlock = 64 * KS * 2;   // kBlock: 64 columns, M/N-major
     constexpr int kStages = 196608 / (kStageA + kStageB);
     extern __shared__ uint8_t smem_raw[];
     __shared__ __align__(8) uint64_t full[kStages], empty[kStages], accum;
@@ -200,7 +204,7 @@ k_gemm_tma(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int m0 = blockIdx.y * kBM, n0 = blockIdx.x * BN;
     const int kbase = blockIdx.z * g.ksplit;
-    const int nchunks = min(g.ksplit, g.K - kbase) / tc::kKChunk;
+    const int nchunks = min(g.ksplit, g.K - kbase) / KS;
     const bool sums = g.k_sums != nullptr && g.a_t && blockIdx.x == 0;
     if (warp == 1) tc::tmem_alloc(tc::smem_addr(&tmem_base), BN);
     if (threadIdx.x == 0) {
@@ -221,61 +225,71 @@ k_gemm_tma(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
     const uint32_t tmem = tmem_base;
     auto stage_a = [&](int st) { return sbase + (uint32_t)st * (kStageA + kStageB); };
     auto stage_b = [&](int st) { return stage_a(st) + kStageA; };
-    if (warp == 0 && lane == 0) {
-        // ---- producer
+    if (warp == 0) {
+        // ---- producer; the warp keeps together, so that the loop runs in uniform registers
         tc::tma_prefetch_map(&tmA);
         tc::tma_prefetch_map(&tmB);
         int c = 0;
-        for (int st = 0, phase = 1, k = kbase; c < nchunks; ++c, k += tc::kKChunk) {
-            if (c >= kStages && !tc::mbar_wait(tc::smem_addr(&empty[st]), phase)) {
-                atomicOr(g.err, 16u);
-                atomicExch(&abort_flag, 1);
+        for (int st = 0, phase = 1, k = kbase; c < nchunks; ++c, k += KS) {
+            if (c >= kStages && !__all_sync(0xffffffffu, tc::mbar_wait(tc::smem_addr(&empty[st]), phase))) {
+                if (lane == 0) {
+                    atomicOr(g.err, 16u);
+                    atomicExch(&abort_flag, 1);
+                }
                 break;
             }
             const uint32_t fb = tc::smem_addr(&full[st]);
-            tc::mbar_arrive_expect_tx(fb, kStageA + kStageB);
-            tc::tma_load_3d(stage_a(st), &tmA, g.a_t ? 0 : k, g.a_t ? k : m0, g.a_t ? m0 / 64 : 0, fb);
-            tc::tma_load_3d(stage_b(st), &tmB, g.b_t ? 0 : k, g.b_t ? k : n0, g.b_t ? n0 / 64 : 0, fb);
+            if (tc::elect_one()) {
+                tc::mbar_arrive_expect_tx(fb, kStageA + kStageB);
+                tc::tma_load_3d(stage_a(st), &tmA, g.a_t ? 0 : k, g.a_t ? k : m0, g.a_t ? m0 / 64 : 0, fb);
+                tc::tma_load_3d(stage_b(st), &tmB, g.b_t ? 0 : k, g.b_t ? k : n0, g.b_t ? n0 / 64 : 0, fb);
+            }
+            __syncwarp();
             if (++st == kStages) {
                 st = 0;
                 phase ^= 1;
             }
         }
-        n_issued = c;
-    } else if (warp == 1 && lane == 0) {
+        if (lane == 0) n_issued = c;
+    } else if (warp == 1) {
         // ---- MMA issuer
         const uint32_t idesc = tc::make_idesc(kBM, BN) | (g.a_t ? tc::kIdescTransposeA : 0u) | (g.b_t ? tc::kIdescTransposeB : 0u);
         // descriptors of stage 0; a stage and a K step of 16 further are additions to their address field
-        const uint64_t a0 = g.a_t ? tc::make_desc_sw128_mn(stage_a(0), kBlockMN) : tc::make_desc_sw128(stage_a(0));
-        const uint64_t b0 = g.b_t ? tc::make_desc_sw128_mn(stage_b(0), kBlockMN) : tc::make_desc_sw128(stage_b(0));
+        const uint64_t a0 = g.a_t ? tc::make_desc_sw128_mn(stage_a(0), kBlock) : tc::make_desc_sw128(stage_a(0));
+        const uint64_t b0 = g.b_t ? tc::make_desc_sw128_mn(stage_b(0), kBlock) : tc::make_desc_sw128(stage_b(0));
         const uint32_t a_step = (g.a_t ? 16 * 128 : 32) >> 4, b_step = (g.b_t ? 16 * 128 : 32) >> 4;
         int c = 0;
         for (int st = 0, phase = 0; c < nchunks; ++c) {
-            if (!tc::mbar_wait(tc::smem_addr(&full[st]), phase)) {
-                atomicOr(g.err, 16u);
-                atomicExch(&abort_flag, 1);
+            if (!__all_sync(0xffffffffu, tc::mbar_wait(tc::smem_addr(&full[st]), phase))) {
+                if (lane == 0) {
+                    atomicOr(g.err, 16u);
+                    atomicExch(&abort_flag, 1);
+                }
                 break;
             }
             tc::fence_after_sync();
             const uint32_t at = (uint32_t)st * ((kStageA + kStageB) >> 4);
+            if (tc::elect_one()) {
 #pragma unroll
-            for (int ks = 0; ks < tc::kKChunk / 16; ++ks)
-                tc::mma_bf16(tmem, a0 + (at + ks * a_step), b0 + (at + ks * b_step), idesc, (c > 0 || ks > 0) ? 1u : 0u);
-            tc::mma_commit(tc::smem_addr(&empty[st]));
+                for (int ks = 0; ks < KS / 16; ++ks)
+                    tc::mma_bf16(tmem, a0 + (at + ks * a_step), b0 + (at + ks * b_step), idesc, (c > 0 || ks > 0) ? 1u : 0u);
+                tc::mma_commit(tc::smem_addr(&empty[st]));
+            }
+            __syncwarp();
             if (++st == kStages) {
                 st = 0;
                 phase ^= 1;
             }
         }
-        n_consumed = c;
+        if (lane == 0) n_consumed = c;
         // `accum` completes once every MMA issued above has (also with none issued)
-        tc::mma_commit(tc::smem_addr(&accum));
+        if (tc::elect_one()) tc::mma_commit(tc::smem_addr(&accum));   // (the thread that issued them)
     } else if (warp >= 2) {
         if (sums) {
             // ---- sums over K of A's columns: two columns and a quarter of a stage's rows per thread
-            constexpr int kRows = tc::kKChunk / (kEpiWarps / 2);
+            constexpr int kRows = KS / (kEpiWarps / 2);
             const int pair = (threadIdx.x - 64) & 63, part = (threadIdx.x - 64) >> 6, r0 = part * kRows;
-            const uint32_t at = (uint32_t)(pair >> 5) * kBlockMN + (uint32_t)(pair & 3) * 4u, chunk = (pair & 31) >> 2;
+            const uint32_t at = (uint32_t)(pair >> 5) * kBlock + (uint32_t)(pair & 3) * 4u, chunk = (pair & 31) >> 2;
             float a0 = 0.0f, a1 = 0.0f;
             bool ok = true;
             for (int c = 0; c < nchunks && ok; ++c) {
@@ -368,17 +382,17 @@ EncodeTiledFn encode_tiled() {
 // Tensor map of a bf16 operand of `rows` rows (or columns) x K with row stride ld, 128-byte swizzled in
 // shared memory, as three dimensions so that one load brings a tile's K chunk either way: K-major
 // {K, rows, 1} in boxes of 64 x box_rows; M/N-major (element (k, r) at k * ld + r) {64, K, rows / 64} in
-// boxes of 64 x 64 x box_rows / 64, blocks of 64 columns one after the other.  K-major only: the third
+// boxes of 64 x mn_k x box_rows / 64, blocks of 64 columns one after the other.  K-major only: the third
 // dimension may count `batch` such operands, `pitch` elements apart.
 cudaError_t operand_map(CUtensorMap* map, const bf16* base, bool mn_major, int rows, int K, int ld, int box_rows,
-                        int batch = 1, size_t pitch = 64) {
+                        int batch = 1, size_t pitch = 64, int mn_k = tc::kKChunk) {
     EncodeTiledFn enc = encode_tiled();
     if (!enc) return cudaErrorNotSupported;
     if (((uintptr_t)base & 15) || (ld * 2) % 16 || (pitch * 2) % 16) return cudaErrorInvalidValue;
     const cuuint64_t dim[3] = {(cuuint64_t)(mn_major ? 64 : K), (cuuint64_t)(mn_major ? K : rows),
                                (cuuint64_t)(mn_major ? rows / 64 : batch)};
     const cuuint64_t stride[2] = {(cuuint64_t)ld * 2, (cuuint64_t)pitch * 2};
-    const cuuint32_t box[3] = {64u, (cuuint32_t)(mn_major ? tc::kKChunk : box_rows), (cuuint32_t)(mn_major ? box_rows / 64 : 1)};
+    const cuuint32_t box[3] = {64u, (cuuint32_t)(mn_major ? mn_k : box_rows), (cuuint32_t)(mn_major ? box_rows / 64 : 1)};
     const cuuint32_t estr[3] = {1, 1, 1};
     const CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<bf16*>(base), dim, stride, box, estr,
                            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
@@ -386,26 +400,28 @@ cudaError_t operand_map(CUtensorMap* map, const bf16* base, bool mn_major, int r
     return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
-template <int BN>
+template <int BN, int KS>
 cudaError_t launch_gemm(const GemmArgs& g, cudaStream_t s) {
     CUtensorMap ta, tb;
-    TRY(operand_map(&ta, g.A, g.a_t, g.M, g.K, g.lda, kBM));
-    TRY(operand_map(&tb, g.B, g.b_t, g.N, g.K, g.ldb, BN));
+    TRY(operand_map(&ta, g.A, g.a_t, g.M, g.K, g.lda, kBM, 1, 64, KS));
+    TRY(operand_map(&tb, g.B, g.b_t, g.N, g.K, g.ldb, BN, 1, 64, KS));
     static std::atomic<unsigned long long> attr{0};
-    TRY(ensure_smem_attr(k_gemm_tma<BN>, (int)kGemmSmem, attr));
-    return launch_next(k_gemm_tma<BN>, dim3(g.N / BN, g.M / kBM, (g.K + g.ksplit - 1) / g.ksplit), kGemmThreads, kGemmSmem, s,
+    TRY(ensure_smem_attr(k_gemm_tma<BN, KS>, (int)kGemmSmem, attr));
+    return launch_next(k_gemm_tma<BN, KS>, dim3(g.N / BN, g.M / kBM, (g.K + g.ksplit - 1) / g.ksplit), kGemmThreads, kGemmSmem, s,
                        ta, tb, g);
 }
 
 // The widest tiles that still give two thirds of the SMs a CTA: A is read once per tile column, but a
 // batch that splits badly (the single chain of an odd number of 128-ray tiles) leaves most SMs idle:
-// two steps of 32,640 rays take 2.0 ms so, 2.7 in 256-wide tiles, 2.5 before.
+// two steps of 32,640 rays take 1.56 ms so (2.7 in 256-wide tiles, 2.5 before).
 cudaError_t gemm(GemmArgs g, cudaStream_t s) {
     if (g.M % kBM || g.N % kBN || g.K % tc::kKChunk || g.K <= 0) return cudaErrorInvalidValue;
     if (g.ksplit <= 0) g.ksplit = g.K;
     if (g.ksplit % tc::kKChunk || (g.ksplit < g.K && !g.part_stride)) return cudaErrorInvalidValue;
     const long long tiles = (long long)(g.M / kBM) * (g.N / kBN) * ((g.K + g.ksplit - 1) / g.ksplit);
-    return tiles >= 96 ? launch_gemm<256>(g, s) : tiles >= 48 ? launch_gemm<128>(g, s) : launch_gemm<64>(g, s);
+    if (tiles >= 96) return launch_gemm<256, 64>(g, s);
+    if (tiles >= 48) return launch_gemm<128, 64>(g, s);
+    return g.a_t && g.b_t && g.ksplit % 128 == 0 && g.K % 128 == 0 ? launch_gemm<64, 128>(g, s) : launch_gemm<64, 64>(g, s);
 }
 
 // ------------------------------------------------------------ layer GEMM

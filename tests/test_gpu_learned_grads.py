@@ -60,3 +60,16 @@ def test_transposed_operands(rl, M, N, K, a_t, b_t, shift):
     c = rl.tc_gemm(put(a, a_t), put(b, b_t), M, N, K, bool(a_t), bool(b_t))
     torch.cuda.synchronize()
     assert np.array_equal(c.cpu().numpy(), a @ b.T)
+
+
+@pytest.mark.parametrize("K", [128, 384, 640, 4224])   # stages of 128 K: fewer than, as many as and more than the ring
+def test_transposed_operands_long_stages(rl, K):
+    """Small whole numbers: products and sums are exact in float32."""
+    M, N = 256, 256
+    rng = np.random.default_rng(K)
+    a = rng.integers(-3, 4, (M, K)).astype(np.float32)
+    b = rng.integers(-3, 4, (N, K)).astype(np.float32)
+    put = lambda x: torch.from_numpy(np.ascontiguousarray(x.T)).cuda().to(torch.bfloat16)  # noqa: E731
+    c = rl.tc_gemm(put(a), put(b), M, N, K, True, True)
+    torch.cuda.synchronize()
+    assert np.array_equal(c.cpu().numpy(), a @ b.T)
