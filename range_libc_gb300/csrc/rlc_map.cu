@@ -316,8 +316,9 @@ __host__ __device__ void fh_line_exact(const In& f, const Out& out, unsigned n, 
 
 // ---- the searches
 constexpr unsigned kEdtNone = 0xFFFFu;   // "no occupied cell in the column"
-constexpr int kEdtNear = 32;             // distances searched one by one before whole blocks
-constexpr int kEdtBlock = 32;            // cells of a row whose least pass-1 distance is kept together
+constexpr int kEdtNear = 8;              // distances searched one by one before whole blocks
+constexpr int kEdtBlock = 8;             // cells of a row whose least pass-1 distance is kept together,
+constexpr int kEdtFar = 64;              // and whose least blocks' distance is, for the search beyond kEdtFar
 
 // f of a pass-1 distance d: the float square (pass 1 stores 0 + (q - v)^2), FLT_MAX for none
 __host__ __device__ __forceinline__ float edt_f(unsigned d) {
@@ -349,16 +350,52 @@ __host__ __device__ __forceinline__ unsigned edt_col_search(int prev, unsigned n
     return (unsigned)(at < q ? q - at : at - q);
 }
 
+// The blocks beyond kEdtNear of q in growing distance, until near(gap) says that columns `gap` or more away
+// cannot win; columns(first, end) looks into a block for which worth(gap, its least distance) holds.
+template <class Near, class Worth, class Columns, class GMin, class GFar>
+__host__ __device__ __forceinline__ void edt_blocks(const Near& near, const Worth& worth, const Columns& columns,
+                                                    const GMin& gmin, const GFar& gfar, int W, int q) {
+    const int nb = (W + kEdtBlock - 1) / kEdtBlock, nf = (W + kEdtFar - 1) / kEdtFar, ratio = kEdtFar / kEdtBlock;
+    auto block = [&](int b) {
+        const int gap = b * kEdtBlock > q ? b * kEdtBlock - q : q - (b * kEdtBlock + kEdtBlock - 1);
+        if (!near(gap)) return false;
+        const unsigned m = gmin(b);
+        if (m != kEdtNone && worth(gap, m)) columns(b * kEdtBlock, b * kEdtBlock + kEdtBlock < W ? b * kEdtBlock + kEdtBlock : W);
+        return true;
+    };
+    bool open = true;
+    for (int k = 1, own = q / kEdtBlock; k <= ratio && open; ++k) {
+        open = own - k >= 0 && block(own - k);
+        if (own + k < nb && block(own + k)) open = true;
+    }
+    for (int k = 1, own = q / kEdtFar; open; ++k) {
+        open = false;
+        for (int side = 0; side < 2; ++side) {
+            const int f = side ? own + k : own - k;
+            if (f < 0 || f >= nf) continue;
+            const int gap = side ? f * kEdtFar - q : q - (f * kEdtFar + kEdtFar - 1);
+            if (!near(gap)) continue;
+            open = true;
+            const unsigned m = gfar(f);
+            if (m == kEdtNone || !worth(gap, m)) continue;
+            for (int b = f * ratio; b < (f + 1) * ratio && b < nb; ++b) (void)block(b);
+        }
+    }
+}
+
 // Pass 2 at column q of a row of W pass-1 distances g(p): the value whose square root is the
-// distance transform.  gmin(b): the least distance of columns [32 b, 32 b + 32).  Distances up to
-// kEdtNear are searched one by one (most cells of a map with walls end there), farther ones a
-// block at a time, so that an empty map costs W / 32 block reads per cell and not W.
+// distance transform.  gmin(b): the least distance of columns [8 b, 8 b + 8), gfar(b) of [64 b, 64 b + 64).
+// Distances up to kEdtNear are searched one by one, then blocks of 8 columns up to 64, then of 64, each
+// looked into only where its least distance could win: a cell 50 px from the walls asks 14 blocks and not
+// 100 columns, and an empty map costs W / 64 reads per cell.  Map and marcher set up, us, one by one to 32
+// and blocks of 32 / this: corridor 2048^2 382 / 343, rectangles and disks 368 / 340, 8192^2 5819 / 4570, a
+// single obstacle 578 / 468 (with blocks of 8 alone 338, 342, 4550, 941).
 //
 // Keys below 2^24: the value is the least f(p) + (p - q)^2, and which p gives it does not matter.
 // So the near search runs in groups of four distances with one exit test, and a position past the
 // row's end reads its last cell instead (which at that distance is never less than it is itself).
-template <class G, class GMin>
-__host__ __device__ __forceinline__ float edt_row_search_exact(const G& g, const GMin& gmin, int W, int q) {
+template <class G, class GMin, class GFar>
+__host__ __device__ __forceinline__ float edt_row_search_exact(const G& g, const GMin& gmin, const GFar& gfar, int W, int q) {
     // 65535^2 + e^2 < 2^32 for e <= 256 stands for "none"; every true value is below 2^24
     unsigned best = g(q) * g(q);
     int e = 1;
@@ -381,36 +418,24 @@ __host__ __device__ __forceinline__ float edt_row_search_exact(const G& g, const
             best = m < best ? m : best;
         }
     }
-    if (e > kEdtNear && (unsigned)(e * e) < best) {
-        const int own = q / kEdtBlock, nb = (W + kEdtBlock - 1) / kEdtBlock;
-        for (int k = 1;; ++k) {
-            bool open = false;
-            for (int side = 0; side < 2; ++side) {
-                const int b = side ? own + k : own - k;
-                if (b < 0 || b >= nb) continue;
-                const unsigned gap = (unsigned)(side ? b * kEdtBlock - q : q - (b * kEdtBlock + kEdtBlock - 1));
-                if (gap * gap >= best) continue;
-                open = true;
-                const unsigned m = gmin(b);
-                if (m == kEdtNone || gap * gap + m * m >= best) continue;
-                const int end = b * kEdtBlock + kEdtBlock < W ? b * kEdtBlock + kEdtBlock : W;
-                for (int p = b * kEdtBlock; p < end; ++p) {
-                    const unsigned d = g(p);
-                    if (d == kEdtNone) continue;
-                    const unsigned c = d * d + (unsigned)((p - q) * (p - q));
-                    best = c < best ? c : best;
-                }
-            }
-            if (!open) break;
-        }
-    }
+    if (e > kEdtNear && (unsigned)(e * e) < best)
+        edt_blocks([&](int gap) { return (unsigned)(gap * gap) < best; },
+                   [&](int gap, unsigned m) { return (unsigned)(gap * gap) + m * m < best; },
+                   [&](int p, int end) {
+                       for (; p < end; ++p) {
+                           const unsigned d = g(p), c = d * d + (unsigned)((p - q) * (p - q));
+                           best = d != kEdtNone && c < best ? c : best;
+                       }
+                   },
+                   gmin, gfar, W, q);
     return best < (1u << 24) ? (float)best : FLT_MAX;
 }
 
 // Keys that round: they are formed as the reference rounds them, `slack` bounds e, and the smallest
 // p of the least keys is the one taken.
-template <class G, class GMin>
-__host__ __device__ __forceinline__ float edt_row_search_rounded(const G& g, const GMin& gmin, int W, int q, int slack) {
+template <class G, class GMin, class GFar>
+__host__ __device__ __forceinline__ float edt_row_search_rounded(const G& g, const GMin& gmin, const GFar& gfar, int W, int q,
+                                                                  int slack) {
     int best = 0x7FFFFFFF, at = q;   // best: K(p) - 2 p q + q q
     unsigned d_at = kEdtNone;
     auto take = [&](int p) {
@@ -429,32 +454,21 @@ __host__ __device__ __forceinline__ float edt_row_search_rounded(const G& g, con
         if (q - e >= 0) take(q - e);
         if (q + e < W) take(q + e);
     }
-    if (e > kEdtNear && e * e - slack <= best) {
-        const int own = q / kEdtBlock, nb = (W + kEdtBlock - 1) / kEdtBlock;
-        for (int k = 1;; ++k) {
-            bool open = false;
-            for (int side = 0; side < 2; ++side) {
-                const int b = side ? own + k : own - k;
-                if (b < 0 || b >= nb) continue;
-                const int gap = side ? b * kEdtBlock - q : q - (b * kEdtBlock + kEdtBlock - 1);
-                if (gap * gap - slack > best) continue;
-                open = true;
-                const unsigned m = gmin(b);
-                if (m == kEdtNone || gap * gap - slack > best - (int)edt_f(m)) continue;
-                const int end = b * kEdtBlock + kEdtBlock < W ? b * kEdtBlock + kEdtBlock : W;
-                for (int p = b * kEdtBlock; p < end; ++p) take(p);
-            }
-            if (!open) break;
-        }
-    }
+    if (e > kEdtNear && e * e - slack <= best)
+        edt_blocks([&](int gap) { return gap * gap - slack <= best; },
+                   [&](int gap, unsigned m) { return gap * gap - slack <= best - (int)edt_f(m); },
+                   [&](int p, int end) {
+                       for (; p < end; ++p) take(p);
+                   },
+                   gmin, gfar, W, q);
     if (d_at == kEdtNone) return FLT_MAX;
     const float dq = edt_fsub((float)q, (float)at);
     return edt_fadd(edt_f(d_at), edt_fmul(dq, dq));
 }
 
-template <bool EXACT, class G, class GMin>
-__host__ __device__ __forceinline__ float edt_row_search(const G& g, const GMin& gmin, int W, int q, int slack) {
-    return EXACT ? edt_row_search_exact(g, gmin, W, q) : edt_row_search_rounded(g, gmin, W, q, slack);
+template <bool EXACT, class G, class GMin, class GFar>
+__host__ __device__ __forceinline__ float edt_row_search(const G& g, const GMin& gmin, const GFar& gfar, int W, int q, int slack) {
+    return EXACT ? edt_row_search_exact(g, gmin, gfar, W, q) : edt_row_search_rounded(g, gmin, gfar, W, q, slack);
 }
 
 // Pass 1, a few blocks per 8 columns (a row of bit tiles), each answering a share of the rows.  Bound by its 2 bytes per cell written.  A
@@ -512,16 +526,21 @@ __global__ void __launch_bounds__(256) k_edt_cols(const uint64_t* __restrict__ b
     }
 }
 
-// the least pass-1 distance of every block of kEdtBlock columns, per row: gmin[b * H + y]
+// the least pass-1 distance of every block of kEdtBlock columns and of every kEdtFar, per row:
+// gmin[b * H + y], gfar[b * H + y]
 __global__ void __launch_bounds__(256) k_edt_block_min(const uint16_t* __restrict__ g, int W, int H,
-                                                       uint16_t* __restrict__ gmin) {
-    const int y = blockIdx.x * blockDim.x + threadIdx.x, b = blockIdx.y;
+                                                       uint16_t* __restrict__ gmin, uint16_t* __restrict__ gfar) {
+    const int y = blockIdx.x * blockDim.x + threadIdx.x, f = blockIdx.y;
     if (y >= H) return;
-    const int x0 = b * kEdtBlock, x1 = min(x0 + kEdtBlock, W);
-    unsigned m = kEdtNone;
-#pragma unroll 8
-    for (int x = x0; x < x1; ++x) m = min(m, (unsigned)__ldg(g + (size_t)x * H + y));
-    gmin[(size_t)b * H + y] = (uint16_t)m;
+    unsigned least = kEdtNone;
+    for (int b = f * (kEdtFar / kEdtBlock); b < (f + 1) * (kEdtFar / kEdtBlock) && b * kEdtBlock < W; ++b) {
+        unsigned m = kEdtNone;
+#pragma unroll
+        for (int j = 0; j < kEdtBlock; ++j) m = min(m, (unsigned)__ldg(g + (size_t)min(b * kEdtBlock + j, W - 1) * H + y));
+        gmin[(size_t)b * H + y] = (uint16_t)m;
+        least = min(least, m);
+    }
+    gfar[(size_t)f * H + y] = (uint16_t)least;
 }
 
 // Every form of the distance transform at cell (x, y), value dt; padding cells of the tiles too.
@@ -555,17 +574,19 @@ __device__ __forceinline__ void store_layouts(const DtOut& o, int W, int H, int 
 
 // Pass 2, one thread per cell, 32 consecutive y per warp (the searched distances of a warp are
 // whole 64-byte pieces) x 8 x per block (which share them in the L1).  Bound by the search's
-// instructions: about 2 x (mean distance) reads per cell.  ALL: writes every layout, straight from
+// instructions: about 16 + (mean distance) / 4 reads per cell.  ALL: writes every layout, straight from
 // the search (60 MB at 2048^2; four more kernels read the linear one back before).
-// 2048^2 with the layouts: 1553 + 117 us with one thread per row -> 118 us.
+// 2048^2 with the layouts: 1553 + 117 us with one thread per row, 121 with blocks of 32 columns, now 88.
 template <bool EXACT, bool ALL>
 __global__ void __launch_bounds__(256) k_edt_rows(const uint16_t* __restrict__ g, const uint16_t* __restrict__ gmin,
+                                                  const uint16_t* __restrict__ gfar,
                                                   int W, int H, int TY, int slack, DtOut o) {
     const int y = blockIdx.x * 32 + threadIdx.x, x = blockIdx.y * 8 + threadIdx.y;
     float dt = 0.0f;
     if (x < W && y < H)
         dt = __fsqrt_rn(edt_row_search<EXACT>([&](int p) { return (unsigned)__ldg(g + (size_t)p * H + y); },
-                                              [&](int b) { return (unsigned)__ldg(gmin + (size_t)b * H + y); }, W, x,
+                                              [&](int b) { return (unsigned)__ldg(gmin + (size_t)b * H + y); },
+                                              [&](int b) { return (unsigned)__ldg(gfar + (size_t)b * H + y); }, W, x,
                                               slack));
     if (ALL) {
         if ((y >> 3) < TY) store_layouts(o, W, H, TY, x, y, dt);
@@ -754,7 +775,8 @@ cudaError_t launch_pack_bits(const uint8_t* d_occ, int W, int H, bool rows, uint
 
 size_t edt_scratch_bytes(int W, int H) {
     if (W <= kEdtIntSide && H <= kEdtIntSide)   // pass-1 distances and their block minima, uint16
-        return ((size_t)W + (size_t)((W + kEdtBlock - 1) / kEdtBlock)) * H * sizeof(uint16_t);
+        return ((size_t)W + (size_t)((W + kEdtBlock - 1) / kEdtBlock) + (size_t)((W + kEdtFar - 1) / kEdtFar)) * H *
+               sizeof(uint16_t);
     // pass-1 output g (W*H floats) + per-line v (n uint32) and z (n+1 doubles);
     // both passes reuse the same v/z region sized for the larger pass
     size_t g = (size_t)W * H * sizeof(float);
@@ -773,6 +795,7 @@ cudaError_t launch_edt(const uint64_t* d_bits, int W, int H, int TY, const DtOut
     if (W <= kEdtIntSide && H <= kEdtIntSide) {
         uint16_t* g = reinterpret_cast<uint16_t*>(base);
         uint16_t* gmin = g + (size_t)W * H;
+        uint16_t* gfar = gmin + (size_t)((W + kEdtBlock - 1) / kEdtBlock) * H;
         const size_t smem = (size_t)8 * 2 * TY * sizeof(uint16_t);   // at most 64 KB
         static std::atomic<unsigned long long> attr_done{0};
         cudaError_t e = ensure_smem_attr(k_edt_cols, 8 * 2 * (kEdtIntSide / 8) * (int)sizeof(uint16_t), attr_done);
@@ -780,17 +803,17 @@ cudaError_t launch_edt(const uint64_t* d_bits, int W, int H, int TY, const DtOut
         k_edt_cols<<<dim3((W + 7) >> 3, min(4, (H + 255) / 256)), 256, smem, s>>>(d_bits, W, H, TY, g);
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;
-        k_edt_block_min<<<dim3(blocks_for(H, 256), (W + kEdtBlock - 1) / kEdtBlock), 256, 0, s>>>(g, W, H, gmin);
+        k_edt_block_min<<<dim3(blocks_for(H, 256), (W + kEdtFar - 1) / kEdtFar), 256, 0, s>>>(g, W, H, gmin, gfar);
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;
         const dim3 grid(blocks_for((long long)TY * 8, 32), (W + 7) >> 3), block(32, 8);
         // keys below 2^24 are exact; see above for the bounds of what rounding adds
         const bool exact = (long long)(W - 1) * (W - 1) + (long long)(H - 1) * (H - 1) < (1ll << 24);
         const int slack = exact ? 0 : (W <= kEdtExactSide && H <= kEdtExactSide ? 1 : 24);
-        if (exact && all) k_edt_rows<true, true><<<grid, block, 0, s>>>(g, gmin, W, H, TY, slack, o);
-        else if (exact) k_edt_rows<true, false><<<grid, block, 0, s>>>(g, gmin, W, H, TY, slack, o);
-        else if (all) k_edt_rows<false, true><<<grid, block, 0, s>>>(g, gmin, W, H, TY, slack, o);
-        else k_edt_rows<false, false><<<grid, block, 0, s>>>(g, gmin, W, H, TY, slack, o);
+        if (exact && all) k_edt_rows<true, true><<<grid, block, 0, s>>>(g, gmin, gfar, W, H, TY, slack, o);
+        else if (exact) k_edt_rows<true, false><<<grid, block, 0, s>>>(g, gmin, gfar, W, H, TY, slack, o);
+        else if (all) k_edt_rows<false, true><<<grid, block, 0, s>>>(g, gmin, gfar, W, H, TY, slack, o);
+        else k_edt_rows<false, false><<<grid, block, 0, s>>>(g, gmin, gfar, W, H, TY, slack, o);
         return cudaGetLastError();
     }
     float* g = reinterpret_cast<float*>(base);

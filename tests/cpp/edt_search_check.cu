@@ -24,8 +24,8 @@ int cases = 0, fails = 0;
 void check(const std::vector<uint8_t>& occ, int W, int H, const char* what) {
     std::vector<float> ref((size_t)W * H);
     orc_edt(occ.data(), W, H, ref.data());
-    const int nb = (W + rlc::kEdtBlock - 1) / rlc::kEdtBlock;
-    std::vector<uint16_t> g((size_t)W * H), gmin((size_t)nb * H, 0xFFFF);
+    const int nb = (W + rlc::kEdtBlock - 1) / rlc::kEdtBlock, nf = (W + rlc::kEdtFar - 1) / rlc::kEdtFar;
+    std::vector<uint16_t> g((size_t)W * H), gmin((size_t)nb * H, 0xFFFF), gfar((size_t)nf * H, 0xFFFF);
     for (int x = 0; x < W; ++x) {
         const uint8_t* col = occ.data() + (size_t)x * H;
         std::vector<int> prev(H);
@@ -38,6 +38,8 @@ void check(const std::vector<uint8_t>& occ, int W, int H, const char* what) {
             g[(size_t)x * H + q] = (uint16_t)rlc::edt_col_search(prev[q], next[q], q, H, [&](int r) { return col[r] != 0; });
             uint16_t& m = gmin[(size_t)(x / rlc::kEdtBlock) * H + q];
             m = std::min(m, g[(size_t)x * H + q]);
+            uint16_t& f = gfar[(size_t)(x / rlc::kEdtFar) * H + q];
+            f = std::min(f, g[(size_t)x * H + q]);
         }
     }
     const bool exact = (long long)(W - 1) * (W - 1) + (long long)(H - 1) * (H - 1) < (1ll << 24);
@@ -47,9 +49,10 @@ void check(const std::vector<uint8_t>& occ, int W, int H, const char* what) {
         for (int y = 0; y < H; ++y) {
             const auto gy = [&](int q) { return (unsigned)g[(size_t)q * H + y]; };
             const auto my = [&](int b) { return (unsigned)gmin[(size_t)b * H + y]; };
+            const auto fy = [&](int b) { return (unsigned)gfar[(size_t)b * H + y]; };
             for (int x = 0; x < W; ++x) {
-                const float v = sqrtf(form == 0 ? rlc::edt_row_search<true>(gy, my, W, x, 0)
-                                                : rlc::edt_row_search<false>(gy, my, W, x, slack));
+                const float v = sqrtf(form == 0 ? rlc::edt_row_search<true>(gy, my, fy, W, x, 0)
+                                                : rlc::edt_row_search<false>(gy, my, fy, W, x, slack));
                 const float* r = &ref[(size_t)x * H + y];
                 if (memcmp(&v, r, sizeof(float)) != 0 && bad++ == 0)
                     printf("mismatch %s %dx%d form %d at (%d, %d): %.9g vs %.9g\n", what, W, H, form, x, y, v, *r);
