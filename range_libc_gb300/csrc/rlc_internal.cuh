@@ -255,7 +255,9 @@ cudaError_t launch_next(void (*kernel)(P...), dim3 grid, int block, size_t smem,
     c.stream = s;
     c.attrs = &at;
     c.numAttrs = 1;
-    return cudaLaunchKernelEx(&c, kernel, static_cast<P>(a)...);
+    const cudaError_t e = cudaLaunchKernelEx(&c, kernel, static_cast<P>(a)...);
+    if (e != cudaSuccess) (void)cudaGetLastError();   // returned here, not to the next call that asks
+    return e;
 }
 
 // Bytes of a CDDT zero-point array of nz entries: whole 32-byte sectors, so that the bin search
