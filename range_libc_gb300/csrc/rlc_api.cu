@@ -178,7 +178,9 @@ struct rlc_method {
     float* d_sin = nullptr;
     CddtBuild tab;
     CddtIndex index;
-    unsigned table_gen = 0;   // counts the tables of this method (a batch holds their device pointers)
+    // counts the changes to what a batch's filter table holds of this method: its CDDT table, trig override
+    // and sensor model
+    unsigned generation = 0;
     // GiantLUTCast
     uint16_t* d_lut = nullptr;
     float max_div_limits = 0.0f, limits_div_max = 0.0f;
@@ -264,7 +266,7 @@ struct rlc_method {
 
     // the index of the current CDDT table
     cudaError_t build_index() {
-        ++table_gen;
+        ++generation;
         return cddt_index_build(tab, map->W, map->H, td, h_widths.data(), h_trans.data(), h_cos.data(), h_sin.data(),
                                 h_slice_base.data(), &index, 0);
     }
@@ -732,6 +734,7 @@ int rlc_cddt_table_load(rlc_method* m, const float* trans, const int64_t* bin_le
 
 int rlc_method_set_trig_override(rlc_method* m, const float* trig, int64_t count) {
     if (int rc = check_method(m)) return rc;
+    ++m->generation;
     cudaFree(m->d_trig);
     m->d_trig = nullptr;
     m->trig_count = 0;
@@ -902,10 +905,15 @@ int rlc_set_sensor_model(rlc_method* m, const double* table, int K) {
     if (int rc = check_method(m)) return rc;
     if (!table || K <= 0) return fail(RLC_ERR_ARG, "sensor model needs a K x K table with K > 0");
     if ((long long)K * K > (1ll << 28)) return fail(RLC_ERR_ARG, "sensor table too large");
+    ++m->generation;
     cudaFree(m->d_table);
     m->d_table = nullptr;
     m->K = 0;
-    if (int rc = upload((void**)&m->d_table, table, (size_t)K * K * sizeof(double), "sensor model")) return rc;
+    if (int rc = upload((void**)&m->d_table, table, (size_t)K * K * sizeof(double), "sensor model")) {
+        cudaFree(m->d_table);
+        m->d_table = nullptr;
+        return rc;
+    }
     m->K = K;
     return RLC_OK;
 }
@@ -1278,8 +1286,7 @@ struct rlc_batch {
     cudaStream_t cap = nullptr;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
-    // each method's trig override and CDDT table when the device table was built
-    std::vector<std::pair<const float*, unsigned>> seen;
+    std::vector<unsigned> seen;   // each method's generation in the device table; empty: no table
 
     void drop_graph() {
         if (exec) cudaGraphExecDestroy(exec);
@@ -1300,6 +1307,13 @@ struct rlc_batch {
     // (re)build the device filter table for the current schedule
     int build() {
         drop_graph();
+        seen.clear();
+        for (size_t i = 0; i < descs.size(); ++i) {
+            const rlc_method* m = descs[i].method;
+            if (!m->d_table) return fail(RLC_ERR_STATE, "filter %d: sensor model not set", (int)i);
+            if (m->d_trig && m->trig_count < (long long)descs[i].n_particles * descs[i].n_angles)
+                return fail(RLC_ERR_ARG, "filter %d: trig override too short", (int)i);
+        }
         int dev = 0, sms = 0;
         CUDA_OR_FAIL(cudaGetDevice(&dev), "batch setup");
         CUDA_OR_FAIL(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "batch setup");
@@ -1372,8 +1386,6 @@ struct rlc_batch {
             it.cost = (double)it.f.ppb * (d.n_angles > 0 ? d.n_angles : 1) * (double)(m->mr > 1.0f ? m->mr : 1.0f);
             items.push_back(it);
         }
-        seen.clear();
-        for (const rlc_filter_desc& d : descs) seen.emplace_back(d.method->d_trig, d.method->table_gen);
         std::stable_sort(items.begin(), items.end(), [](const Item& a, const Item& b) { return a.cost > b.cost; });
         unsigned long long tiles = 0, parts = 0;
         std::vector<FilterDev> hf;
@@ -1405,22 +1417,19 @@ struct rlc_batch {
         long long g = (long long)sms * per_sm;
         if (g > (long long)tiles) g = (long long)tiles;
         grid = (int)(g > 0 ? g : 1);
+        for (const rlc_filter_desc& d : descs) seen.push_back(d.method->generation);
         return RLC_OK;
     }
 
     // queue reset + persistent kernel, captured once as a CUDA graph
     int launch(cudaStream_t stream) {
         if (total_tiles == 0) return RLC_OK;
-        // a method whose trig override was set or cleared, or whose CDDT table was pruned or loaded, since
-        // the build: the device table holds the old (freed) one, so rebuild it (and the graph) first
-        for (size_t i = 0; i < descs.size(); ++i) {
-            const rlc_method* m = descs[i].method;
-            if (i < seen.size() && seen[i] == std::make_pair((const float*)m->d_trig, m->table_gen)) continue;
-            if (m->d_trig && m->trig_count < (long long)descs[i].n_particles * descs[i].n_angles)
-                return fail(RLC_ERR_ARG, "filter %d: trig override too short", (int)i);
+        // a method whose trig override, sensor model or CDDT table was replaced since the build: the device
+        // table holds the old (freed) one, so rebuild it (and the graph) first
+        bool current = !seen.empty();
+        for (size_t i = 0; i < seen.size(); ++i) current = current && descs[i].method->generation == seen[i];
+        if (!current)
             if (int rc = build()) return rc;
-            break;
-        }
         if (!exec) {
             CUDA_OR_FAIL(cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal), "batch capture");
             cudaError_t e = cudaMemsetAsync(d_queue, 0, sizeof(unsigned), cap);
@@ -1460,14 +1469,11 @@ int rlc_batch_create(const rlc_filter_desc* fd, int nf, int block, rlc_batch** o
         const rlc_filter_desc& d = fd[i];
         rlc_method* m = d.method;
         if (!m) return fail(RLC_ERR_ARG, "filter %d: null method", i);
-        if (!m->d_table) return fail(RLC_ERR_STATE, "filter %d: sensor model not set", i);
         if (d.n_particles < 0 || d.n_angles < 0) return fail(RLC_ERR_ARG, "filter %d: negative size", i);
         if (d.n_angles > 16384) return fail(RLC_ERR_ARG, "filter %d: at most 16384 beams", i);
         if (d.n_particles > 0 && (!d.ins || !d.weights || (d.n_angles > 0 && (!d.angles || !d.obs))))
             return fail(RLC_ERR_ARG, "filter %d: null array", i);
         if ((long long)d.n_particles * d.n_angles > (1ll << 31) - 1) return fail(RLC_ERR_ARG, "filter %d: too many rays", i);
-        if (m->d_trig && m->trig_count < (long long)d.n_particles * d.n_angles)
-            return fail(RLC_ERR_ARG, "filter %d: trig override too short", i);
         rays += (long long)d.n_particles * d.n_angles;
         if (m->dkind != K_RM) rm_only = false;
     }

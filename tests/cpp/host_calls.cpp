@@ -1,0 +1,217 @@
+// The library's host code on a stand-in for the CUDA runtime: every runtime function that
+// librangelibc_gb300.so imports is defined here, so that no GPU is needed and none is touched.
+// "Device" memory is host memory that is filled with ones and never given back (a pointer into a freed
+// block stays recognisable), kernels do not run but are recorded, allocations can be made to fail, and
+// a kernel's time is what the scenario says.
+//
+//   host_calls <scenario>     prints "ok", or what was wrong, and exits non-zero then
+#include "rangelibc.h"
+
+#include <cuda_runtime_api.h>
+#include <cxxabi.h>
+
+#include <cstdio>
+#include <cstdlib>
+#include <cstring>
+#include <functional>
+#include <map>
+#include <string>
+#include <vector>
+
+namespace {
+
+struct Block { size_t bytes; bool live; };
+std::map<char*, Block> blocks;                    // by address, freed ones too
+std::map<const void*, std::string>& kernels() {   // host function -> demangled name; filled before this file's own globals are made
+    static std::map<const void*, std::string> m;
+    return m;
+}
+size_t refuse_from = ~(size_t)0;                  // allocations of this many bytes or more fail
+long long calls = 0;                              // runtime calls of any kind
+std::function<void(const std::string&, void**)> on_launch = [](const std::string&, void**) {};
+std::function<float(const std::string&)> kernel_ms = [](const std::string&) { return 1.0f; };
+float clock_ms = 0.0f;
+std::map<cudaEvent_t, float> events;
+std::map<const void*, int> smem_limit;
+int lowered = 0;                                  // times a kernel's shared-memory limit went down
+
+struct Launch { std::string name; std::vector<void*> words; };   // the first parameter, where it is a pointer
+bool capturing = false;
+std::vector<Launch> recorded;
+
+void launched(const void* f, void** args) {
+    const std::string& name = kernels()[f];
+    clock_ms += kernel_ms(name);
+    on_launch(name, args);
+    if (capturing) recorded.push_back(Launch{name, {args ? *(void**)args[0] : nullptr}});
+}
+
+// the words of the block at p that point into freed memory
+int stale_words(void* p) {
+    auto it = blocks.find((char*)p);
+    if (it == blocks.end()) return 0;
+    int n = 0;
+    for (size_t i = 0; i + sizeof(char*) <= it->second.bytes; i += sizeof(char*)) {
+        char* w;
+        memcpy(&w, it->first + i, sizeof(w));
+        auto at = blocks.upper_bound(w);
+        if (at == blocks.begin()) continue;
+        --at;
+        if (!at->second.live && w < at->first + at->second.bytes) ++n;
+    }
+    return n;
+}
+
+}  // namespace
+
+extern "C" {
+cudaError_t cudaMalloc(void** p, size_t n) {
+    ++calls;
+    *p = nullptr;
+    if (n >= refuse_from) return cudaErrorMemoryAllocation;
+    char* b = (char*)aligned_alloc(256, (n + 255) / 256 * 256);
+    memset(b, 1, n);
+    blocks[b] = Block{n, true};
+    *p = b;
+    return cudaSuccess;
+}
+cudaError_t cudaFree(void* p) {
+    ++calls;
+    if (p) blocks[(char*)p].live = false;
+    return cudaSuccess;
+}
+cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind) { ++calls; memcpy(d, s, n); return cudaSuccess; }
+cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cudaStream_t) { ++calls; memcpy(d, s, n); return cudaSuccess; }
+cudaError_t cudaMemset(void* d, int v, size_t n) { ++calls; memset(d, v, n); return cudaSuccess; }
+cudaError_t cudaMemsetAsync(void* d, int v, size_t n, cudaStream_t) { ++calls; memset(d, v, n); return cudaSuccess; }
+cudaError_t cudaGetLastError(void) { return cudaSuccess; }
+const char* cudaGetErrorString(cudaError_t) { return "stand-in error"; }
+cudaError_t cudaGetDevice(int* d) { ++calls; *d = 0; return cudaSuccess; }
+cudaError_t cudaSetDevice(int) { ++calls; return cudaSuccess; }
+cudaError_t cudaGetDeviceCount(int* n) { *n = 1; return cudaSuccess; }
+cudaError_t cudaDeviceSynchronize(void) { ++calls; return cudaSuccess; }
+cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr a, int) {
+    *v = a == cudaDevAttrMultiProcessorCount ? 152 : a == cudaDevAttrL2CacheSize ? 1 << 20 : a == cudaDevAttrPageableMemoryAccess;
+    return cudaSuccess;
+}
+cudaError_t cudaEventCreate(cudaEvent_t* e) { *e = (cudaEvent_t)malloc(1); return cudaSuccess; }
+cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }
+cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t) { events[e] = clock_ms; return cudaSuccess; }
+cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
+cudaError_t cudaEventElapsedTime(float* ms, cudaEvent_t a, cudaEvent_t b) { *ms = events[b] - events[a]; return cudaSuccess; }
+cudaError_t cudaFuncSetAttribute(const void* f, cudaFuncAttribute a, int v) {
+    ++calls;
+    if (a == cudaFuncAttributeMaxDynamicSharedMemorySize) {
+        if (smem_limit.count(f) && v < smem_limit[f]) ++lowered;
+        smem_limit[f] = v;
+    }
+    return cudaSuccess;
+}
+cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int* n, const void*, int, size_t, unsigned) { *n = 4; return cudaSuccess; }
+static int encode(...) { return 0; }
+cudaError_t cudaGetDriverEntryPointByVersion(const char*, void** p, unsigned, unsigned long long, cudaDriverEntryPointQueryResult* q) {
+    *p = (void*)encode;
+    *q = cudaDriverEntryPointSuccess;
+    return cudaSuccess;
+}
+cudaError_t cudaGetSymbolAddress(void** p, const void*) { return cudaMalloc(p, 1024); }
+cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void*) { memset(a, 0, sizeof(*a)); return cudaSuccess; }
+cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) { *s = (cudaStream_t)malloc(1); return cudaSuccess; }
+cudaError_t cudaStreamDestroy(cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaStreamSynchronize(cudaStream_t) { ++calls; return cudaSuccess; }
+cudaError_t cudaStreamBeginCapture(cudaStream_t, cudaStreamCaptureMode) { capturing = true; recorded.clear(); return cudaSuccess; }
+cudaError_t cudaStreamEndCapture(cudaStream_t, cudaGraph_t* g) {
+    capturing = false;
+    *g = (cudaGraph_t) new std::vector<Launch>(recorded);
+    return cudaSuccess;
+}
+cudaError_t cudaGraphInstantiate(cudaGraphExec_t* e, cudaGraph_t g, unsigned long long) {
+    *e = (cudaGraphExec_t) new std::vector<Launch>(*(std::vector<Launch>*)g);
+    return cudaSuccess;
+}
+cudaError_t cudaGraphDestroy(cudaGraph_t) { return cudaSuccess; }
+cudaError_t cudaGraphExecDestroy(cudaGraphExec_t) { return cudaSuccess; }
+static std::vector<Launch> last_graph;
+cudaError_t cudaGraphLaunch(cudaGraphExec_t e, cudaStream_t) {
+    last_graph = *(std::vector<Launch>*)e;
+    for (const Launch& l : last_graph) clock_ms += kernel_ms(l.name);
+    return cudaSuccess;
+}
+cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t*, const void* f, void** args) { ++calls; launched(f, args); return cudaSuccess; }
+// what nvcc's host code calls to register and launch kernels
+cudaError_t __cudaGetKernel(void** k, const void* f) { *k = (void*)f; return cudaSuccess; }
+cudaError_t __cudaLaunchKernel(void* k, dim3, dim3, void** args, size_t, cudaStream_t) { ++calls; launched(k, args); return cudaSuccess; }
+unsigned __cudaPushCallConfiguration(dim3, dim3, size_t, cudaStream_t) { return 0; }
+cudaError_t __cudaPopCallConfiguration(dim3*, dim3*, size_t*, void*) { return cudaSuccess; }
+void** __cudaRegisterFatBinary(void*) { static void* h; return &h; }
+void __cudaRegisterFatBinaryEnd(void**) {}
+void __cudaUnregisterFatBinary(void**) {}
+void __cudaRegisterVar(void**, char*, char*, const char*, int, size_t, int, int) {}
+void __cudaRegisterFunction(void**, const char* f, char*, const char* name, int, void*, void*, void*, void*, int*) {
+    int st = 0;
+    char* d = abi::__cxa_demangle(name, nullptr, nullptr, &st);
+    kernels()[f] = d ? d : name;
+    free(d);
+}
+}
+
+namespace {
+
+int wrong(const char* what) {
+    printf("%s (%s)\n", what, rlc_last_error());
+    return 1;
+}
+#define CHECK(c) do { if (!(c)) return wrong(#c); } while (0)
+
+rlc_method* method(int kind, int W = 64, int H = 48, unsigned td = 0) {
+    std::vector<uint8_t> occ((size_t)W * H, 0);
+    rlc_map* map = nullptr;
+    rlc_method* m = nullptr;
+    if (rlc_map_create(occ.data(), W, H, &map) == RLC_OK) rlc_method_create(map, kind, 40.0f, td, &m);
+    return m;
+}
+
+int sensor(rlc_method* m, int K) { return rlc_set_sensor_model(m, std::vector<double>((size_t)K * K, 0.5).data(), K); }
+
+// A batch whose method gets another sensor table, trig override or none runs on what the method has now.
+int batch_tables() {
+    for (int kind : {RLC_RM, RLC_BL}) {
+        rlc_method *a = method(kind), *b = method(kind);
+        CHECK(a && b && sensor(a, 41) == RLC_OK && sensor(b, 41) == RLC_OK);
+        std::vector<float> x(4000, 1.0f);
+        std::vector<double> w(100);
+        const rlc_filter_desc d[2] = {{a, x.data(), x.data(), x.data(), nullptr, w.data(), 50, 7},
+                                      {b, x.data(), x.data(), x.data(), nullptr, w.data(), 50, 7}};
+        rlc_batch* q = nullptr;
+        CHECK(rlc_batch_create(d, 2, 0, &q) == RLC_OK && rlc_batch_run(q, nullptr) == RLC_OK);
+        auto fresh = [&]() { return !last_graph.empty() && stale_words(last_graph.back().words[0]) == 0; };
+        CHECK(fresh());
+        CHECK(sensor(b, 33) == RLC_OK && rlc_batch_run(q, nullptr) == RLC_OK && fresh());
+        CHECK(rlc_method_set_trig_override(a, x.data(), 350) == RLC_OK);
+        CHECK(rlc_batch_run(q, nullptr) == RLC_OK && fresh());
+        // every changed method is looked at, not only the first
+        CHECK(sensor(a, 30) == RLC_OK && rlc_method_set_trig_override(b, x.data(), 349) == RLC_OK);
+        CHECK(rlc_batch_run(q, nullptr) == RLC_ERR_ARG);
+        CHECK(rlc_method_set_trig_override(b, nullptr, 0) == RLC_OK && rlc_batch_run(q, nullptr) == RLC_OK && fresh());
+        // a table that could not be uploaded: refused until there is one
+        refuse_from = 8 * 60 * 60;
+        CHECK(sensor(a, 60) != RLC_OK);
+        refuse_from = ~(size_t)0;
+        CHECK(rlc_batch_run(q, nullptr) == RLC_ERR_STATE && rlc_batch_set_schedule(q, 0, 0, 256, 0) == RLC_ERR_STATE);
+        CHECK(rlc_batch_run(q, nullptr) == RLC_ERR_STATE);
+        CHECK(sensor(a, 60) == RLC_OK && rlc_batch_run(q, nullptr) == RLC_OK && fresh());
+        rlc_batch_destroy(q);
+    }
+    return 0;
+}
+
+}  // namespace
+
+int main(int argc, char** argv) {
+    const std::map<std::string, int (*)()> scenarios = {{"batch_tables", batch_tables}};
+    const auto it = scenarios.find(argc > 1 ? argv[1] : "");
+    if (it == scenarios.end()) return wrong("no such scenario");
+    if (const int rc = it->second()) return rc;
+    printf("ok\n");
+    return 0;
+}
