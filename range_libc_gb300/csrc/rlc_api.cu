@@ -1314,6 +1314,7 @@ struct rlc_batch {
             if (m->d_trig && m->trig_count < (long long)descs[i].n_particles * descs[i].n_angles)
                 return fail(RLC_ERR_ARG, "filter %d: trig override too short", (int)i);
         }
+        if (d_filters) CUDA_OR_FAIL(cudaDeviceSynchronize(), "batch setup");   // a run may still be reading the table
         int dev = 0, sms = 0;
         CUDA_OR_FAIL(cudaGetDevice(&dev), "batch setup");
         CUDA_OR_FAIL(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "batch setup");

@@ -35,6 +35,9 @@ std::map<cudaEvent_t, float> events;
 std::map<const void*, int> smem_limit;
 int lowered = 0;                                  // times a kernel's shared-memory limit went down
 
+std::map<void*, bool> in_flight;                  // blocks that a launched graph may still be reading
+int torn = 0;                                     // copies into one of them
+
 struct Launch { std::string name; std::vector<void*> words; };   // the first parameter, where it is a pointer
 bool capturing = false;
 std::vector<Launch> recorded;
@@ -77,10 +80,18 @@ cudaError_t cudaMalloc(void** p, size_t n) {
 }
 cudaError_t cudaFree(void* p) {
     ++calls;
-    if (p) blocks[(char*)p].live = false;
+    if (p) {
+        blocks[(char*)p].live = false;
+        in_flight.clear();   // waits for the device
+    }
     return cudaSuccess;
 }
-cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind) { ++calls; memcpy(d, s, n); return cudaSuccess; }
+cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind) {
+    ++calls;
+    torn += (int)in_flight.count(d);   // (not ordered with streams that do not wait for the legacy one)
+    memcpy(d, s, n);
+    return cudaSuccess;
+}
 cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cudaStream_t) { ++calls; memcpy(d, s, n); return cudaSuccess; }
 cudaError_t cudaMemset(void* d, int v, size_t n) { ++calls; memset(d, v, n); return cudaSuccess; }
 cudaError_t cudaMemsetAsync(void* d, int v, size_t n, cudaStream_t) { ++calls; memset(d, v, n); return cudaSuccess; }
@@ -89,7 +100,7 @@ const char* cudaGetErrorString(cudaError_t) { return "stand-in error"; }
 cudaError_t cudaGetDevice(int* d) { ++calls; *d = 0; return cudaSuccess; }
 cudaError_t cudaSetDevice(int) { ++calls; return cudaSuccess; }
 cudaError_t cudaGetDeviceCount(int* n) { *n = 1; return cudaSuccess; }
-cudaError_t cudaDeviceSynchronize(void) { ++calls; return cudaSuccess; }
+cudaError_t cudaDeviceSynchronize(void) { ++calls; in_flight.clear(); return cudaSuccess; }
 cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr a, int) {
     *v = a == cudaDevAttrMultiProcessorCount ? 152 : a == cudaDevAttrL2CacheSize ? 1 << 20 : a == cudaDevAttrPageableMemoryAccess;
     return cudaSuccess;
@@ -134,7 +145,10 @@ cudaError_t cudaGraphExecDestroy(cudaGraphExec_t) { return cudaSuccess; }
 static std::vector<Launch> last_graph;
 cudaError_t cudaGraphLaunch(cudaGraphExec_t e, cudaStream_t) {
     last_graph = *(std::vector<Launch>*)e;
-    for (const Launch& l : last_graph) clock_ms += kernel_ms(l.name);
+    for (const Launch& l : last_graph) {
+        clock_ms += kernel_ms(l.name);
+        in_flight[l.words[0]] = true;
+    }
     return cudaSuccess;
 }
 cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t*, const void* f, void** args) { ++calls; launched(f, args); return cudaSuccess; }
@@ -205,10 +219,28 @@ int batch_tables() {
     return 0;
 }
 
+// The filter table is replaced only when no run reads it.
+int batch_in_flight() {
+    rlc_method* m = method(RLC_RM);
+    CHECK(m && sensor(m, 41) == RLC_OK);
+    std::vector<float> x(400, 1.0f);
+    std::vector<double> w(50);
+    const rlc_filter_desc d = {m, x.data(), x.data(), x.data(), nullptr, w.data(), 50, 7};
+    rlc_batch* q = nullptr;
+    CHECK(rlc_batch_create(&d, 1, 0, &q) == RLC_OK);
+    for (int layout : {0, 4, 5}) CHECK(rlc_batch_run(q, nullptr) == RLC_OK && rlc_batch_set_schedule(q, layout, 0, 256, 8) == RLC_OK);
+    CHECK(torn == 0);
+    // the first override of a method frees nothing, which would wait for the run
+    std::vector<float> trig(700, 0.5f);
+    CHECK(rlc_batch_run(q, nullptr) == RLC_OK && rlc_method_set_trig_override(m, trig.data(), 350) == RLC_OK);
+    CHECK(rlc_batch_run(q, nullptr) == RLC_OK && torn == 0);
+    return 0;
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
-    const std::map<std::string, int (*)()> scenarios = {{"batch_tables", batch_tables}};
+    const std::map<std::string, int (*)()> scenarios = {{"batch_tables", batch_tables}, {"batch_in_flight", batch_in_flight}};
     const auto it = scenarios.find(argc > 1 ? argv[1] : "");
     if (it == scenarios.end()) return wrong("no such scenario");
     if (const int rc = it->second()) return rc;
