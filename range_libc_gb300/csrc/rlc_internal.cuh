@@ -57,9 +57,7 @@ struct MapDev {
     const uint8_t* free;
 };
 constexpr int kFreeMost = 64;
-// d_scratch: W * H bytes
-cudaError_t launch_free_map(const uint64_t* d_bits, int W, int H, int tiles_y, uint8_t* d_scratch, uint8_t* d_free,
-                            cudaStream_t s);
+cudaError_t launch_free_map(const uint64_t* d_bits, int W, int H, int tiles_y, uint8_t* d_free, cudaStream_t s);
 
 struct CddtDev {
     unsigned td;

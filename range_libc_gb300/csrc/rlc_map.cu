@@ -720,13 +720,9 @@ __global__ void k_unpack_bits(const uint64_t* __restrict__ bits, int W, int H, i
 }
 
 // ---- free distances (Bresenham's walk)
-// Distance along y to the nearest occupied cell of the column, at most kFreeMost: the bytes of the
-// column's tiles, outward.
-__global__ void __launch_bounds__(256) k_free_y(const uint64_t* __restrict__ bits, int W, int H, int TY,
-                                                uint8_t* __restrict__ g) {
-    const unsigned yb = ((unsigned)H + 31u) >> 5, bx = blockIdx.x / yb;   // 32 y x 8 x cells per block
-    const int x = (int)(bx * 8 + threadIdx.y), y = (int)((blockIdx.x - bx * yb) * 32 + threadIdx.x);
-    if (x >= W || y >= H) return;
+// Distance along y from cell (x, y) to the nearest occupied cell of its column, at most kFreeMost: the
+// bytes of the column's tiles, outward.
+__device__ __forceinline__ int free_y(const uint64_t* __restrict__ bits, int TY, int x, int y) {
     const uint64_t* col = bits + (size_t)(x >> 3) * TY;
     const int sh = (x & 7) << 3, c = y >> 3, in = y & 7;
     const unsigned b = (unsigned)(__ldg(col + c) >> sh) & 0xFFu;
@@ -740,24 +736,36 @@ __global__ void __launch_bounds__(256) k_free_y(const uint64_t* __restrict__ bit
         if (l) d = min(d, 8 * k + in - edt_msb(l));
         if (r) d = min(d, 8 * k - in + edt_lsb(r));
     }
-    g[(size_t)x * H + y] = (uint8_t)d;
+    return d;
 }
 
 // Chebyshev distance: the least over dx of max(|dx|, distance along y at x + dx); a (W + 1) x (H + 1) grid
-// with 1 in its last row and column.
-__global__ void __launch_bounds__(256) k_free_x(const uint8_t* __restrict__ g, int W, int H, uint8_t* __restrict__ out) {
+// with 1 in its last row and column.  A block answers kFreeTile x 32 cells from the distances along y of
+// their columns and of kFreeMost - 1 on either side, in shared memory, so that the map needs no scratch
+// beside its result (two passes with one in memory before: a method on 2048^2 with walls made in 219 us, now
+// 190; with blocks of 8 warps, each on its rows in turn, 220, and 86 instead of 49 on 512^2).
+constexpr int kFreeTile = 128, kFreeReach = kFreeMost - 1, kFreeWarps = 32;
+
+__global__ void __launch_bounds__(32 * kFreeWarps) k_free(const uint64_t* __restrict__ bits, int W, int H, int TY,
+                                              uint8_t* __restrict__ out) {
+    __shared__ uint8_t s_y[kFreeTile + 2 * kFreeReach][32];
     const unsigned yb = ((unsigned)H + 32u) >> 5, bx = blockIdx.x / yb;
-    const int x = (int)(bx * 8 + threadIdx.y), y = (int)((blockIdx.x - bx * yb) * 32 + threadIdx.x);
-    if (x > W || y > H) return;
-    int d = 1;
-    if (x < W && y < H) {
-        d = __ldg(g + (size_t)x * H + y);
-        for (int e = 1; e < d; ++e) {
-            if (x - e >= 0) d = min(d, max(e, (int)__ldg(g + (size_t)(x - e) * H + y)));
-            if (x + e < W) d = min(d, max(e, (int)__ldg(g + (size_t)(x + e) * H + y)));
-        }
+    const int x0 = (int)(bx * kFreeTile), lane = threadIdx.x, y = (int)((blockIdx.x - bx * yb) * 32 + lane);
+    for (int i = threadIdx.y; i < kFreeTile + 2 * kFreeReach; i += kFreeWarps) {
+        const int x = x0 - kFreeReach + i;
+        s_y[i][lane] = (uint8_t)(x >= 0 && x < W && y < H ? free_y(bits, TY, x, y) : kFreeMost);
     }
-    out[(size_t)x * (H + 1) + y] = (uint8_t)d;
+    __syncthreads();
+    if (y > H) return;
+    for (int j = threadIdx.y; j < kFreeTile && x0 + j <= W; j += kFreeWarps) {
+        int d = 1;
+        if (x0 + j < W && y < H) {
+            d = s_y[j + kFreeReach][lane];
+            for (int e = 1; e < d; ++e)
+                d = min(d, max(e, (int)min(s_y[j + kFreeReach - e][lane], s_y[j + kFreeReach + e][lane])));
+        }
+        out[(size_t)(x0 + j) * (H + 1) + y] = (uint8_t)d;
+    }
 }
 
 inline unsigned blocks_for(long long n, int b) { return (unsigned)((n + b - 1) / b); }
@@ -855,14 +863,10 @@ cudaError_t launch_step_runs(const float* d_step, int W, int H, uint32_t* d_eq, 
     return cudaGetLastError();
 }
 
-cudaError_t launch_free_map(const uint64_t* d_bits, int W, int H, int TY, uint8_t* d_scratch, uint8_t* d_free,
-                            cudaStream_t s) {
+cudaError_t launch_free_map(const uint64_t* d_bits, int W, int H, int TY, uint8_t* d_free, cudaStream_t s) {
     if ((long long)W * H == 0) return cudaSuccess;
-    k_free_y<<<blocks_for(H, 32) * blocks_for(W, 8), dim3(32, 8), 0, s>>>(d_bits, W, H, TY, d_scratch);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    k_free_x<<<blocks_for((long long)H + 1, 32) * blocks_for((long long)W + 1, 8), dim3(32, 8), 0, s>>>(d_scratch, W, H,
-                                                                                                       d_free);
+    k_free<<<blocks_for((long long)H + 1, 32) * blocks_for((long long)W + 1, kFreeTile), dim3(32, kFreeWarps), 0, s>>>(
+        d_bits, W, H, TY, d_free);
     return cudaGetLastError();
 }
 

@@ -237,10 +237,33 @@ int batch_in_flight() {
     return 0;
 }
 
+size_t live_bytes() {
+    size_t n = 0;
+    for (const auto& b : blocks) n += b.second.live ? b.second.bytes : 0;
+    return n;
+}
+
+// A Bresenham method keeps one byte a cell of free distances, and does without where there is no room.
+int bresenham_memory() {
+    std::vector<uint8_t> occ(300 * 200, 0);
+    rlc_map* map = nullptr;
+    rlc_method *m = nullptr, *late = nullptr;
+    CHECK(rlc_map_create(occ.data(), 300, 200, &map) == RLC_OK);
+    const size_t before = live_bytes();
+    refuse_from = 300 * 200;
+    CHECK(rlc_method_create(map, RLC_BL, 40.0f, 0, &m) == RLC_OK && rlc_method_destroy(m) == RLC_OK);
+    CHECK(live_bytes() == before);
+    refuse_from = ~(size_t)0;
+    CHECK(rlc_method_create(map, RLC_BL, 40.0f, 0, &late) == RLC_OK);
+    CHECK(live_bytes() >= before + 301 * 201 && live_bytes() < before + 301 * 201 + 1024);
+    return 0;
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
-    const std::map<std::string, int (*)()> scenarios = {{"batch_tables", batch_tables}, {"batch_in_flight", batch_in_flight}};
+    const std::map<std::string, int (*)()> scenarios = {{"batch_tables", batch_tables}, {"batch_in_flight", batch_in_flight},
+                                                          {"bresenham_memory", bresenham_memory}};
     const auto it = scenarios.find(argc > 1 ? argv[1] : "");
     if (it == scenarios.end()) return wrong("no such scenario");
     if (const int rc = it->second()) return rc;
