@@ -10,7 +10,9 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <memory>
 #include <mutex>
+#include <new>
 #include <string>
 #include <vector>
 
@@ -66,6 +68,7 @@ struct rlc_map {
     int W = 0, H = 0, TY = 0;
     float world[6] = {1.0f, 0.0f, 0.0f, 0.0f, 0.0f, 1.0f};   // scale, angle, ox, oy, sin, cos
     uint64_t* d_bits = nullptr;
+    std::unique_ptr<uint64_t[]> h_bits;   // their copy, so that the occupancy can be asked for at any time
     float* d_dt = nullptr;
     float* d_dt_tiled = nullptr;
     uint16_t* d_dt16 = nullptr;
@@ -383,17 +386,6 @@ bool host_direct() {
     return c == 2;
 }
 
-// makes `device` current until the end of the scope
-struct DeviceGuard {
-    int before = -1;
-    explicit DeviceGuard(int device) {
-        if (cudaGetDevice(&before) != cudaSuccess || before == device || cudaSetDevice(device) != cudaSuccess) before = -1;
-    }
-    ~DeviceGuard() {
-        if (before >= 0) cudaSetDevice(before);
-    }
-};
-
 int finish_launch(cudaError_t e, const char* what) {
     if (e != cudaSuccess) return cuda_fail(e, what);
     return RLC_OK;
@@ -479,7 +471,9 @@ static int map_create(const uint8_t* occ, int width, int height, bool rows, rlc_
         if (e == cudaSuccess) e = cudaMemcpy(d_occ, occ, n, cudaMemcpyHostToDevice);
     }
     if (e == cudaSuccess) e = launch_pack_bits(direct ? occ : d_occ, width, height, rows, m->d_bits, 0);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(0);
+    m->h_bits.reset(new (std::nothrow) uint64_t[words]);
+    if (e == cudaSuccess && !m->h_bits) e = cudaErrorMemoryAllocation;
+    if (e == cudaSuccess) e = cudaMemcpy(m->h_bits.get(), m->d_bits, words * sizeof(uint64_t), cudaMemcpyDeviceToHost);
     cudaFree(d_occ);
     if (e != cudaSuccess) {
         delete m;
@@ -523,14 +517,19 @@ int rlc_map_size(const rlc_map* map, int* width, int* height) {
 
 int rlc_map_occupancy(rlc_map* map, uint8_t* occ_out) {
     if (!map || !occ_out) return fail(RLC_ERR_ARG, "null argument");
-    const DeviceGuard on(map->device);   // PyOMap.occupancy may be asked with another device current
-    size_t n = (size_t)map->W * map->H;
-    uint8_t* d = nullptr;
-    CUDA_OR_FAIL(cudaMalloc(&d, n), "occupancy export");
-    cudaError_t e = launch_unpack_bits(map->d_bits, map->W, map->H, map->TY, d, 0);
-    if (e == cudaSuccess) e = cudaMemcpy(occ_out, d, n, cudaMemcpyDeviceToHost);
-    cudaFree(d);
-    return finish_launch(e, "occupancy export");
+    for (int x = 0; x < map->W; ++x) {
+        uint8_t* col = occ_out + (size_t)x * map->H;
+        const uint64_t* tiles = map->h_bits.get() + (size_t)(x >> 3) * map->TY;
+        for (int y = 0; y < map->H; y += 8) {
+            // the tile's eight cells of this column, a byte each: the product puts bit k at bit 8 k (k < 7)
+            const uint64_t b = (tiles[y >> 3] >> ((x & 7) << 3)) & 0xFFu;
+            const uint64_t cells = (((b & 0x7Fu) * 0x40810204081ull) & 0x0101010101010101ull) | (b >> 7) << 56;
+            if (y + 8 <= map->H) std::memcpy(col + y, &cells, 8);
+            else
+                for (int k = 0; y + k < map->H; ++k) col[y + k] = (uint8_t)(cells >> (8 * k));
+        }
+    }
+    return RLC_OK;
 }
 
 int rlc_map_distance_transform(rlc_map* map, float* dt_out) {

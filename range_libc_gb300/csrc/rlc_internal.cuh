@@ -140,7 +140,6 @@ size_t step_eq_words(int W, int H);
 cudaError_t launch_step_runs(const float* d_step, int W, int H, uint32_t* d_eq, uint32_t* d_runs, unsigned long long* d_share,
                              cudaStream_t s);
 cudaError_t launch_edge_map(const uint64_t* d_bits, int W, int H, int tiles_y, uint8_t* d_edge, cudaStream_t s);
-cudaError_t launch_unpack_bits(const uint64_t* d_bits, int W, int H, int tiles_y, uint8_t* d_occ, cudaStream_t s);
 
 // ---- casting (rlc_cast.cu) ----
 // layout: DtLayout of the distance transform; pf: 1 = RM prefetching schedule

@@ -712,13 +712,6 @@ __global__ void k_edge_map(const uint64_t* __restrict__ bits, int W, int H, int 
     edge[i] = e;
 }
 
-__global__ void k_unpack_bits(const uint64_t* __restrict__ bits, int W, int H, int TY, uint8_t* __restrict__ occ) {
-    long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (long long)W * H) return;
-    int x = (int)(i / H), y = (int)(i - (long long)x * H);
-    occ[i] = occ_bit(bits, TY, x, y) ? 1 : 0;
-}
-
 // ---- free distances (Bresenham's walk)
 // Distance along y from cell (x, y) to the nearest occupied cell of its column, at most kFreeMost: the
 // bytes of the column's tiles, outward.
@@ -874,13 +867,6 @@ cudaError_t launch_edge_map(const uint64_t* d_bits, int W, int H, int TY, uint8_
     long long n = (long long)W * H;
     if (n == 0) return cudaSuccess;
     k_edge_map<<<blocks_for(n, 256), 256, 0, s>>>(d_bits, W, H, TY, d_edge);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_unpack_bits(const uint64_t* d_bits, int W, int H, int TY, uint8_t* d_occ, cudaStream_t s) {
-    long long n = (long long)W * H;
-    if (n == 0) return cudaSuccess;
-    k_unpack_bits<<<blocks_for(n, 256), 256, 0, s>>>(d_bits, W, H, TY, d_occ);
     return cudaGetLastError();
 }
 

@@ -251,7 +251,7 @@ class PyOMap:
             occ = self._from_png(str(arg1), float(arg2))
         elif isinstance(arg1, np.ndarray) and arg1.ndim == 2 and arg1.size:
             # handed over as it lies in memory, rows or columns; grid[x][y] is made on the device, and
-            # read back if it is asked for
+            # unpacked from the host's copy of its bits if it is asked for
             cells = arg1 if arg1.dtype.kind in "bui" and arg1.itemsize == 1 else arg1 != 0
             by_rows = cells.flags.c_contiguous or abs(cells.strides[0]) >= abs(cells.strides[1])
             grid = np.ascontiguousarray(cells if by_rows else cells.T)

@@ -259,11 +259,27 @@ int bresenham_memory() {
     return 0;
 }
 
+// A map's occupancy is given without the GPU (a capture may be under way, or this be a forked child).
+int occupancy() {
+    for (int mode : {RLC_HOST_AUTO, RLC_HOST_STAGED}) {
+        std::vector<uint8_t> occ(29 * 19, 0), got(29 * 19, 7);
+        rlc_map* map = nullptr;
+        CHECK(rlc_set_host_path(mode) == RLC_OK && rlc_map_create_rows(occ.data(), 29, 19, &map) == RLC_OK);
+        const long long before = calls;
+        CHECK(rlc_map_occupancy(map, got.data()) == RLC_OK && calls == before);
+        // the stand-in's tiles are bytes of 1: of eight rows, the first is occupied
+        for (int x = 0; x < 29; ++x)
+            for (int y = 0; y < 19; ++y) CHECK(got[x * 19 + y] == (y % 8 == 0));
+        CHECK(rlc_map_destroy(map) == RLC_OK && live_bytes() == 0);
+    }
+    return 0;
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
     const std::map<std::string, int (*)()> scenarios = {{"batch_tables", batch_tables}, {"batch_in_flight", batch_in_flight},
-                                                          {"bresenham_memory", bresenham_memory}};
+                                                          {"bresenham_memory", bresenham_memory}, {"occupancy", occupancy}};
     const auto it = scenarios.find(argc > 1 ? argv[1] : "");
     if (it == scenarios.end()) return wrong("no such scenario");
     if (const int rc = it->second()) return rc;
