@@ -1870,10 +1870,12 @@ inline void product_shape(int na, int block, int tile, int& P, int& threads) {
     if (threads < 32) threads = 32;
 }
 
+// room for `bytes` of dynamic shared memory; `done` is the kernel's own.  The limit is set to the most there
+// is and never lowered: it is the device's, not the launch's, and other threads launch the same kernel.
+constexpr int kSmemMost = 227 * 1024;
 template <class K>
-cudaError_t set_smem(K kernel, size_t bytes) {
-    if (bytes <= 48 * 1024) return cudaSuccess;
-    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+cudaError_t set_smem(K kernel, size_t bytes, std::atomic<unsigned long long>& done) {
+    return bytes <= 48 * 1024 ? cudaSuccess : ensure_smem_attr(kernel, kSmemMost, done);
 }
 
 // Which fused calls go wide, where the caller has not asked for a schedule: those where a block of
@@ -1926,7 +1928,8 @@ struct RunFused {
         int P, threads;
         product_shape(na, block, tile, P, threads);
         const size_t smem = (size_t)P * na * sizeof(double);
-        cudaError_t e = set_smem(k_fused<KIND, LAYOUT, PF>, smem);
+        static std::atomic<unsigned long long> attr{0};
+        cudaError_t e = set_smem(k_fused<KIND, LAYOUT, PF>, smem, attr);
         if (e != cudaSuccess) return e;
         return launch_next(k_fused<KIND, LAYOUT, PF>, dim3(blocks_for(n, P)), threads, smem, s, p, sm, ins, angles, obs, w, n, na, P);
     }
@@ -2032,7 +2035,8 @@ cudaError_t launch_fused_staged(const CastParams& p, const SensorDev& sm, const 
     if (e != cudaSuccess) return e;
     const int PB = max(1, min(32, (int)((kTileSmem - (size_t)na * sizeof(uint16_t)) / ((size_t)na * sizeof(double)))));
     const size_t wsmem = (((size_t)PB * na * sizeof(double) + (size_t)na * sizeof(uint16_t)) + 15) & ~(size_t)15;
-    e = set_smem(k_bm_weights, wsmem);
+    static std::atomic<unsigned long long> wattr{0};
+    e = set_smem(k_bm_weights, wsmem, wattr);
     if (e != cudaSuccess) return e;
     k_bm_weights<<<blocks_for(n, PB), 128, wsmem, s>>>(p, sm, obs, bins, n, na, PB, weights);
     return cudaGetLastError();
@@ -2091,27 +2095,23 @@ cudaError_t launch_batch_wide(const FilterDev* d_filters, int nf, unsigned total
     return cudaGetLastError();
 }
 
-size_t batch_smem(int block, bool rm_only) {
+size_t batch_smem(int block, bool rm_only) {   // 32 KB for the largest block
     return rm_only ? (size_t)((block + 31) / 32) * kBatchSlots * sizeof(RmRay) : 0;
 }
 
 cudaError_t batch_occupancy(int block, size_t smem, bool rm_only, int layout, int pf, bool separate,
                             int* blocks_per_sm) {
-    BatchKernel k = batch_kernel(rm_only, layout, pf, separate);
-    cudaError_t e = set_smem(k, smem);
-    if (e != cudaSuccess) return e;
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k, block, smem);
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, batch_kernel(rm_only, layout, pf, separate), block,
+                                                         smem);
 }
 
 cudaError_t launch_batch(const FilterDev* d_filters, int nf, unsigned total_tiles, unsigned* queue, int grid,
                          int block, size_t smem, bool rm_only, int layout, int pf, bool separate,
                          unsigned total_particles, cudaStream_t s) {
     if (total_tiles == 0 || nf == 0) return cudaSuccess;
-    BatchKernel k = batch_kernel(rm_only, layout, pf, separate);
-    cudaError_t e = set_smem(k, smem);
-    if (e != cudaSuccess) return e;
+    const BatchKernel k = batch_kernel(rm_only, layout, pf, separate);
     k_batch_obs_bins<<<nf, 256, 0, s>>>(d_filters, rm_only);
-    e = cudaGetLastError();
+    cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     if (rm_only && total_particles) {
         k_batch_particles<<<blocks_for(total_particles, 256), 256, 0, s>>>(d_filters, nf, total_particles);

@@ -267,6 +267,7 @@ __global__ void k_project(SliceGeom g, const uint32_t* __restrict__ edges, uint3
 // entries mostly share bins.  Counting and filling entry by entry in memory took 159 and 249 us for the
 // 7.2 M projections of a 2048 x 2048 map with 108 slices, now 88 and 177.
 constexpr int kProjectChunk = 8192, kProjectThreads = 512;
+constexpr size_t kProjectSmem = 100 * 1024;   // leaves an SM room for a second block
 
 template <int PASS>
 __global__ void __launch_bounds__(kProjectThreads) k_project_block(SliceGeom g, const uint32_t* __restrict__ edges,
@@ -395,6 +396,8 @@ __global__ void __launch_bounds__(256) k_sort_bins(const uint32_t* __restrict__ 
         longer[1 + atomicAdd(longer, 1u)] = b;
     }
 }
+
+constexpr size_t kSortSmem = 200 * 1024;
 
 // the listed bins, a block each: bitonic sort in shared memory, then de-duplicate in
 // place; ucount[b] receives the number of distinct values
@@ -683,12 +686,13 @@ cudaError_t cddt_build(const uint64_t* d_bits, int W, int H, int TY, unsigned td
     uint32_t most = 0;
     for (int a = 0; a < nslices; ++a) most = std::max(most, h_slice_base[a + 1] - h_slice_base[a]);
     const size_t bins_smem = (size_t)most * sizeof(uint32_t);
-    const bool by_block = work > 0 && bins_smem <= 100 * 1024 && nslices <= 65535;
+    const bool by_block = work > 0 && bins_smem <= kProjectSmem && nslices <= 65535;
     const dim3 pgrid((nedges + kProjectChunk - 1) / kProjectChunk, (unsigned)nslices);
     if (by_block) {
-        if (bins_smem > 48 * 1024) {
-            RLC_TRY(cudaFuncSetAttribute(k_project_block<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bins_smem));
-            RLC_TRY(cudaFuncSetAttribute(k_project_block<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bins_smem));
+        if (bins_smem > 48 * 1024) {   // the limits to the most a table may need: tables are built by several threads
+            static std::atomic<unsigned long long> attr0{0}, attr1{0};
+            RLC_TRY(ensure_smem_attr(k_project_block<0>, (int)kProjectSmem, attr0));
+            RLC_TRY(ensure_smem_attr(k_project_block<1>, (int)kProjectSmem, attr1));
         }
         k_project_block<0><<<pgrid, kProjectThreads, bins_smem, s>>>(g, edges.as<uint32_t>(), nedges, H,
                                                                      counts.as<uint32_t>(), nullptr, nullptr);
@@ -713,7 +717,7 @@ cudaError_t cddt_build(const uint64_t* d_bits, int W, int H, int TY, unsigned td
     size_t p2 = 1;
     while (p2 < mlen) p2 <<= 1;
     const size_t smem = p2 * sizeof(float);
-    if (smem > 200 * 1024) {
+    if (smem > kSortSmem) {
         snprintf(why, why_len, "CDDT bin of %u zero points exceeds the in-shared-memory sort (max 51200)", mlen);
         return cudaErrorInvalidValue;
     }
@@ -742,8 +746,8 @@ cudaError_t cddt_build(const uint64_t* d_bits, int W, int H, int TY, unsigned td
                                                       counts.as<uint32_t>());
         RLC_TRY(cudaGetLastError());
         if (mlen > 256) {
-            if (smem > 48 * 1024)
-                RLC_TRY(cudaFuncSetAttribute(k_sort_unique, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            static std::atomic<unsigned long long> attr{0};
+            if (smem > 48 * 1024) RLC_TRY(ensure_smem_attr(k_sort_unique, (int)kSortSmem, attr));
             k_sort_unique<<<2 * 152, 256, smem, s>>>(counts.as<uint32_t>(), start.as<uint32_t>(), raw.as<float>(),
                                                      ucount.as<uint32_t>());
             RLC_TRY(cudaGetLastError());

@@ -275,11 +275,45 @@ int occupancy() {
     return 0;
 }
 
+// A kernel's limit of shared memory is the device's, not the launch's: a call that lowered it could have it
+// lowered between another thread's call and that one's launch.
+int shared_memory_limits() {
+    long long longest = 0;
+    on_launch = [&](const std::string& name, void** args) {
+        if (name.find("k_edges") != std::string::npos) **(uint32_t**)args[6] = 5;
+        if (name.find("k_count_stats") != std::string::npos) {
+            unsigned long long* out = *(unsigned long long**)args[2];
+            out[0] = (unsigned long long)longest;
+            out[1] = 1000;
+        }
+    };
+    const int sides[] = {20000, 13000, 24000};
+    const long long bins[] = {30000, 9000, 20000};
+    for (int i = 0; i < 3; ++i) {
+        longest = bins[i];
+        CHECK(method(RLC_CDDT, sides[i], 8, 16));
+    }
+    for (int layout : {0, 3})
+        for (int na : {7000, 6500, 16384, 6400}) {
+            rlc_method* m = method(RLC_RM);
+            std::vector<float> x(50000, 1.0f);
+            double w[2];
+            CHECK(m && sensor(m, 41) == RLC_OK && rlc_method_set_schedule(m, layout, 0, 0, 0) == RLC_OK);
+            CHECK(rlc_calc_range_repeat_angles_eval_sensor_model(m, x.data(), x.data(), x.data(), w, 2, na, 0, nullptr) == RLC_OK);
+        }
+    int large = 0;
+    for (const auto& k : smem_limit) large += k.second > 48 * 1024;
+    CHECK(large >= 5);   // k_project_block twice, k_sort_unique, k_fused, k_bm_weights
+    CHECK(lowered == 0);
+    return 0;
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
     const std::map<std::string, int (*)()> scenarios = {{"batch_tables", batch_tables}, {"batch_in_flight", batch_in_flight},
-                                                          {"bresenham_memory", bresenham_memory}, {"occupancy", occupancy}};
+                                                          {"bresenham_memory", bresenham_memory}, {"occupancy", occupancy},
+                                                          {"shared_memory_limits", shared_memory_limits}};
     const auto it = scenarios.find(argc > 1 ? argv[1] : "");
     if (it == scenarios.end()) return wrong("no such scenario");
     if (const int rc = it->second()) return rc;
