@@ -327,7 +327,9 @@ RLC_API int rlc_learned_sample_rays(rlc_learned* l, long long first_id, unsigned
                                     float* d_t, float* d_range, void* stream);
 RLC_API int rlc_learned_train(rlc_learned* l, int steps, int batch, float lr, unsigned seed, float* final_loss,
                               void* stream);
-/* t of n grid-frame rays by the fused forward kernel (the whole network per 128-ray tile on one SM) */
+/* t of n grid-frame rays by the fused forward kernel (the whole network per 128-ray tile on one SM);
+ * queued on the stream.  A bounded wait that runs out in a learned kernel is RLC_ERR_CUDA from the call
+ * that waits for it: train, gradients, calc_range_repeat_angles, or the next of these after a predict. */
 RLC_API int rlc_learned_predict(rlc_learned* l, const float* d_xyt, int n, float* d_pred, void* stream);
 /* the same through the layer-by-layer GEMMs of the training path (bit-identical; test reference) */
 RLC_API int rlc_learned_predict_layered(rlc_learned* l, const float* d_xyt, int n, float* d_pred, void* stream);

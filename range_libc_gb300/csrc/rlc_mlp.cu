@@ -1358,7 +1358,7 @@ struct LearnedModel {
     float* adam_v = nullptr;
     float* grads = nullptr;
     bf16* wbf = nullptr;       // bf16 copy of params (weights used by the GEMMs)
-    unsigned* err = nullptr;
+    unsigned* err = nullptr;   // {bits raised by waits that ran out since they were last taken, recast rays of a query}
     long long adam_t = 0;
     // work buffers for a chunk of `cap` rays
     int cap = 0;
@@ -1378,15 +1378,13 @@ struct LearnedModel {
     long long qcap = 0;
     float* q_xyt = nullptr;
     float* q_pred = nullptr;
-    int* q_cnt = nullptr;
 
     cudaError_t ensure_query(long long rays) {
         if (rays <= qcap) return cudaSuccess;
-        cudaFree(q_xyt); cudaFree(q_pred); cudaFree(q_cnt);
-        q_xyt = q_pred = nullptr; q_cnt = nullptr; qcap = 0;
+        cudaFree(q_xyt); cudaFree(q_pred);
+        q_xyt = q_pred = nullptr; qcap = 0;
         TRY(cudaMalloc(&q_xyt, (size_t)rays * 3 * sizeof(float)));
         TRY(cudaMalloc(&q_pred, (size_t)rays * sizeof(float)));
-        TRY(cudaMalloc(&q_cnt, sizeof(int)));
         qcap = rays;
         return cudaSuccess;
     }
@@ -1404,7 +1402,7 @@ struct LearnedModel {
         free_work();
         cudaFree(params); cudaFree(adam_m); cudaFree(adam_v); cudaFree(grads); cudaFree(wbf); cudaFree(err);
         cudaFree(free_cells);
-        cudaFree(q_xyt); cudaFree(q_pred); cudaFree(q_cnt);
+        cudaFree(q_xyt); cudaFree(q_pred);
     }
     cudaError_t ensure(int rows) {
         rows = (rows + kBM - 1) / kBM * kBM;
@@ -1437,6 +1435,14 @@ struct LearnedModel {
         for (int parts = kMaxSplits; parts > 1; parts >>= 1)
             if (rows % (parts * 256) == 0) { sp = rows / parts; break; }
         return sp;
+    }
+
+    // Waits for the stream's work and takes the error word: words[0] the bits, which are cleared (a wait that
+    // ran out spoils what was under way, not the calls after), words[1] the count.
+    cudaError_t take(unsigned* words, cudaStream_t s) {
+        TRY(cudaMemcpyAsync(words, err, 2 * sizeof(unsigned), cudaMemcpyDeviceToHost, s));
+        TRY(cudaStreamSynchronize(s));
+        return words[0] ? cudaMemsetAsync(err, 0, sizeof(unsigned), s) : cudaSuccess;
     }
 
     GemmArgs base_args() const {
@@ -1516,6 +1522,7 @@ struct rlc_learned {
 
 namespace {
 char g_msg[512];
+constexpr const char* kTimedOut = "tensor-core GEMM timed out waiting for its MMAs";
 int lfail(int code, const char* what, cudaError_t e = cudaSuccess) {
     if (e != cudaSuccess) snprintf(g_msg, sizeof(g_msg), "%s: %s", what, cudaGetErrorString(e));
     else snprintf(g_msg, sizeof(g_msg), "%s", what);
@@ -1548,8 +1555,8 @@ int rlc_learned_create(const rlc_method* rm, unsigned seed, rlc_learned** out) {
     if (e == cudaSuccess) e = cudaMalloc(&M.adam_v, kParamCount * sizeof(float));
     if (e == cudaSuccess) e = cudaMalloc(&M.grads, kParamCount * sizeof(float));
     if (e == cudaSuccess) e = cudaMalloc(&M.wbf, kParamCount * sizeof(bf16));
-    if (e == cudaSuccess) e = cudaMalloc(&M.err, sizeof(unsigned));
-    if (e == cudaSuccess) e = cudaMemset(M.err, 0, sizeof(unsigned));
+    if (e == cudaSuccess) e = cudaMalloc(&M.err, 2 * sizeof(unsigned));
+    if (e == cudaSuccess) e = cudaMemset(M.err, 0, 2 * sizeof(unsigned));
     if (e == cudaSuccess) e = cudaMemset(M.adam_m, 0, kParamCount * sizeof(float));
     if (e == cudaSuccess) e = cudaMemset(M.adam_v, 0, kParamCount * sizeof(float));
     if (e == cudaSuccess) {
@@ -1673,10 +1680,9 @@ int rlc_learned_gradients(rlc_learned* L, const float* d_xyt, const float* d_t, 
     LTRY(M.features(d_xyt, n, 0), "features");
     LTRY(M.forward_hidden(n, 0), "forward");
     LTRY(M.backward(d_t, n, 0, AdamArgs{}, 0), "backward");
-    LTRY(cudaDeviceSynchronize(), "gradients");
-    unsigned err = 0;
-    LTRY(cudaMemcpy(&err, M.err, sizeof(unsigned), cudaMemcpyDeviceToHost), "gradients");
-    if (err) return lfail(RLC_ERR_CUDA, "tensor-core GEMM timed out waiting for its MMAs");
+    unsigned words[2];
+    LTRY(M.take(words, 0), "gradients");
+    if (words[0]) return lfail(RLC_ERR_CUDA, kTimedOut);
     if (host_grads) LTRY(cudaMemcpy(host_grads, M.grads, kParamCount * sizeof(float), cudaMemcpyDeviceToHost), "grads");
     if (host_loss) {
         float l = 0.0f;
@@ -1712,15 +1718,14 @@ int rlc_learned_train(rlc_learned* L, int steps, int batch, float lr, unsigned s
     float losses[LearnedModel::kLossSlots] = {};
     if (e == cudaSuccess && steps > 0)
         e = cudaMemcpyAsync(losses, M.loss, sizeof(losses), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    unsigned words[2] = {};
+    if (e == cudaSuccess) e = M.take(words, s);
     if (e != cudaSuccess) return lfail(RLC_ERR_CUDA, "training", e);
+    if (words[0]) return lfail(RLC_ERR_CUDA, kTimedOut);
     for (int st = std::max(0, steps - LearnedModel::kLossSlots); st < steps; ++st) {
         loss_acc += losses[st - (steps - LearnedModel::kLossSlots)] / (float)batch;
         ++loss_n;
     }
-    unsigned err = 0;
-    LTRY(cudaMemcpy(&err, M.err, sizeof(unsigned), cudaMemcpyDeviceToHost), "training");
-    if (err) return lfail(RLC_ERR_CUDA, "tensor-core GEMM timed out waiting for its MMAs");
     if (final_loss) *final_loss = loss_n ? loss_acc / loss_n : 0.0f;
     return RLC_OK;
 }
@@ -1741,7 +1746,7 @@ int rlc_learned_calc_range_repeat_angles(rlc_learned* L, const float* d_ins, con
     LTRY(M.ensure_query(rays), "learned query buffers");
     float* xyt = M.q_xyt;
     float* pred = M.q_pred;
-    int* cnt = M.q_cnt;
+    int* cnt = (int*)(M.err + 1);
     cudaError_t e = cudaMemsetAsync(cnt, 0, sizeof(int), s);
     if (e == cudaSuccess) {
         k_world_rays<<<blocks_for(rays, 256), 256, 0, s>>>(M.world, d_ins, d_angles, n, na, xyt);
@@ -1754,12 +1759,12 @@ int rlc_learned_calc_range_repeat_angles(rlc_learned* L, const float* d_ins, con
                                                                              d_outs, d_accepted, cnt);
         e = cudaGetLastError();
     }
-    int h_cnt = 0;
-    if (e == cudaSuccess && !rc) e = cudaMemcpyAsync(&h_cnt, cnt, sizeof(int), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess && !rc) e = cudaStreamSynchronize(s);
+    unsigned words[2] = {};
+    if (e == cudaSuccess && !rc) e = M.take(words, s);
     if (rc) return rc;
     if (e != cudaSuccess) return lfail(RLC_ERR_CUDA, "learned ranges", e);
-    if (n_recast) *n_recast = h_cnt;
+    if (words[0]) return lfail(RLC_ERR_CUDA, kTimedOut);   // predictions are missing: those of an older call were checked
+    if (n_recast) *n_recast = (int)words[1];
     return RLC_OK;
 }
 
@@ -1793,7 +1798,7 @@ int rlc_tc_gemm(const void* d_a, const void* d_b, float* d_c, int M, int N, int 
     cudaFree(copy[0]);
     cudaFree(copy[1]);
     if (e != cudaSuccess) return lfail(RLC_ERR_CUDA, "tensor-core gemm", e);
-    if (h) return lfail(RLC_ERR_CUDA, "tensor-core GEMM timed out waiting for its MMAs");
+    if (h) return lfail(RLC_ERR_CUDA, kTimedOut);
     return RLC_OK;
 }
 

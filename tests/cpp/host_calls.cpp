@@ -119,7 +119,10 @@ cudaError_t cudaFuncSetAttribute(const void* f, cudaFuncAttribute a, int v) {
     return cudaSuccess;
 }
 cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int* n, const void*, int, size_t, unsigned) { *n = 4; return cudaSuccess; }
-static int encode(...) { return 0; }
+// cuTensorMapEncodeTiled
+static int encode(void*, int, unsigned, void*, const void*, const void*, const unsigned*, const unsigned*, int, int, int, int) {
+    return 0;
+}
 cudaError_t cudaGetDriverEntryPointByVersion(const char*, void** p, unsigned, unsigned long long, cudaDriverEntryPointQueryResult* q) {
     *p = (void*)encode;
     *q = cudaDriverEntryPointSuccess;
@@ -308,12 +311,52 @@ int shared_memory_limits() {
     return 0;
 }
 
+// A kernel of the learned surrogate whose bounded wait runs out raises a bit and leaves its outputs
+// unwritten: the call that follows it up says so, once, and the next one is good again.
+int learned_timeouts() {
+    const char* raises = "";    // the kernel whose wait runs out (of a training step, k_top stands for its layers)
+    unsigned* word = nullptr;   // the model's error bits
+    on_launch = [&](const std::string& name, void** args) {
+        if (name.find("k_resolve") != std::string::npos) **(int**)args[8] = 5;
+        if (name.find("k_mlp_forward") != std::string::npos) word = *(unsigned**)args[7];
+        if (*raises && name.find(raises) != std::string::npos) *word |= 16u;
+    };
+    rlc_method* rm = method(RLC_RM);
+    rlc_learned* l = nullptr;
+    CHECK(rm && rlc_learned_create(rm, 1, &l) == RLC_OK);
+    std::vector<float> ins(30, 1.0f), out(60), grads((size_t)rlc_learned_param_count());
+    int64_t recast = 0;
+    float loss = 0;
+    auto query = [&]() { return rlc_learned_calc_range_repeat_angles(l, ins.data(), ins.data(), out.data(), 10, 6, nullptr, &recast, nullptr); };
+    std::vector<float> xyt(128 * 3, 1.0f), t(128, 1.0f);
+    auto train = [&]() { return rlc_learned_train(l, 1, 128, 1e-3f, 1, &loss, nullptr); };
+    auto gradients = [&]() { return rlc_learned_gradients(l, xyt.data(), t.data(), 128, grads.data(), &loss); };
+    CHECK(query() == RLC_OK && recast == 5 && train() == RLC_OK && gradients() == RLC_OK);
+    raises = "k_mlp_forward";
+    CHECK(query() == RLC_ERR_CUDA && std::string(rlc_last_error()).find("timed out") != std::string::npos);
+    raises = "";
+    CHECK(query() == RLC_OK && train() == RLC_OK && gradients() == RLC_OK);
+    for (auto& call : {std::function<int()>(train), std::function<int()>(gradients)}) {
+        raises = "k_top";
+        CHECK(call() == RLC_ERR_CUDA);
+        raises = "";
+        CHECK(call() == RLC_OK && query() == RLC_OK);
+    }
+    // a prediction does not wait: the next call that does reports it
+    raises = "k_mlp_forward";
+    CHECK(rlc_learned_predict(l, xyt.data(), 128, out.data(), nullptr) == RLC_OK);
+    raises = "";
+    CHECK(query() == RLC_ERR_CUDA && query() == RLC_OK);
+    return 0;
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
     const std::map<std::string, int (*)()> scenarios = {{"batch_tables", batch_tables}, {"batch_in_flight", batch_in_flight},
                                                           {"bresenham_memory", bresenham_memory}, {"occupancy", occupancy},
-                                                          {"shared_memory_limits", shared_memory_limits}};
+                                                          {"shared_memory_limits", shared_memory_limits},
+                                                          {"learned_timeouts", learned_timeouts}};
     const auto it = scenarios.find(argc > 1 ? argv[1] : "");
     if (it == scenarios.end()) return wrong("no such scenario");
     if (const int rc = it->second()) return rc;
