@@ -471,9 +471,14 @@ static int map_create(const uint8_t* occ, int width, int height, bool rows, rlc_
         if (e == cudaSuccess) e = cudaMemcpy(d_occ, occ, n, cudaMemcpyHostToDevice);
     }
     if (e == cudaSuccess) e = launch_pack_bits(direct ? occ : d_occ, width, height, rows, m->d_bits, 0);
-    m->h_bits.reset(new (std::nothrow) uint64_t[words]);
+    m->h_bits.reset(new (std::nothrow) uint64_t[words]());   // zeroed: its pages are made beside the kernel, not by the GPU's writes
     if (e == cudaSuccess && !m->h_bits) e = cudaErrorMemoryAllocation;
-    if (e == cudaSuccess) e = cudaMemcpy(m->h_bits.get(), m->d_bits, words * sizeof(uint64_t), cudaMemcpyDeviceToHost);
+    if (e == cudaSuccess && direct) {
+        e = launch_copy_bits(m->d_bits, words, m->h_bits.get(), 0);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(0);
+    } else if (e == cudaSuccess) {
+        e = cudaMemcpy(m->h_bits.get(), m->d_bits, words * sizeof(uint64_t), cudaMemcpyDeviceToHost);
+    }
     cudaFree(d_occ);
     if (e != cudaSuccess) {
         delete m;

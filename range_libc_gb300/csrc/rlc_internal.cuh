@@ -116,6 +116,7 @@ struct SensorDev {
 // ---- map preprocessing (rlc_map.cu) ----
 // rows: occ[y * W + x], else occ[x * H + y]
 cudaError_t launch_pack_bits(const uint8_t* d_occ, int W, int H, bool rows, uint64_t* d_bits, cudaStream_t s);
+cudaError_t launch_copy_bits(const uint64_t* d_bits, size_t words, uint64_t* out, cudaStream_t s);
 // the distance transform's device arrays: the linear floats, and (all but step, or none) the derived
 // layouts
 struct DtOut {

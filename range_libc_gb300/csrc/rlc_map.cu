@@ -66,6 +66,12 @@ __global__ void __launch_bounds__(256) k_pack_bits(const uint8_t* __restrict__ o
     bits[(size_t)tx * TY + ty] = w;
 }
 
+// the tiles into host memory that the GPU writes in place: 512 KB for 2048^2, where a copy by the runtime into
+// pageable memory took map creation 10 us longer
+__global__ void __launch_bounds__(256) k_copy_bits(const uint64_t* __restrict__ bits, size_t words, uint64_t* __restrict__ out) {
+    for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < words; i += (size_t)gridDim.x * 256) out[i] = bits[i];
+}
+
 __device__ __forceinline__ bool occ_bit(const uint64_t* __restrict__ bits, int TY, int x, int y) {
     uint64_t w = bits[(size_t)(x >> 3) * TY + (y >> 3)];
     return (w >> (((x & 7) << 3) | (y & 7))) & 1ull;
@@ -771,6 +777,12 @@ cudaError_t launch_pack_bits(const uint8_t* d_occ, int W, int H, bool rows, uint
     if (n == 0) return cudaSuccess;
     if (rows) k_pack_bits<true><<<blocks_for(n, 256), 256, 0, s>>>(d_occ, W, H, TY, d_bits);
     else k_pack_bits<false><<<blocks_for(n, 256), 256, 0, s>>>(d_occ, W, H, TY, d_bits);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_copy_bits(const uint64_t* d_bits, size_t words, uint64_t* out, cudaStream_t s) {
+    if (words == 0) return cudaSuccess;
+    k_copy_bits<<<min(blocks_for((long long)words, 256), 8u * 152u), 256, 0, s>>>(d_bits, words, out);
     return cudaGetLastError();
 }
 

@@ -267,6 +267,9 @@ int occupancy() {
     for (int mode : {RLC_HOST_AUTO, RLC_HOST_STAGED}) {
         std::vector<uint8_t> occ(29 * 19, 0), got(29 * 19, 7);
         rlc_map* map = nullptr;
+        on_launch = [](const std::string& name, void** args) {   // the tiles' copy into host memory
+            if (name.find("k_copy_bits") != std::string::npos) memcpy(*(void**)args[2], *(void**)args[0], 8 * *(size_t*)args[1]);
+        };
         CHECK(rlc_set_host_path(mode) == RLC_OK && rlc_map_create_rows(occ.data(), 29, 19, &map) == RLC_OK);
         const long long before = calls;
         CHECK(rlc_map_occupancy(map, got.data()) == RLC_OK && calls == before);
