@@ -780,8 +780,10 @@ def run_batch(args, emit=True, oracle_check=False):
         batch.autotune()
 
     def batched():
-        batch.run()   # one graph: observation bins, the persistent cast (+ the products launch when separate)
-        return 3 if batch.product_mode() == "separate" else 2
+        # one graph: observation bins, the persistent cast and the products launch when separate, else at least
+        # the one launch with the products inside
+        batch.run()
+        return 3 if batch.product_mode() == "separate" else 1
 
     def per_filter_fused():
         for m, ins, ang, obs, w in filters:

@@ -230,18 +230,21 @@ RLC_API int rlc_count_steps(rlc_method* m, const float* ins, const float* angles
  * step, ballot; calc_range_many and calc_range_repeat_angles), 2 by 32-byte sectors for bins of
  * more than 32 zero points (fewer dependent reads; pays when queries spread over the map); tile =
  * particles per tile of the fused and batched kernels (0 = automatic).  Results are identical
- * under every schedule.  Until a schedule is set or tuned, every call picks its kernel by its size
+ * under every schedule.  Until a schedule is set, every call picks its kernel by its size
  * and map (layouts 4 and 5, a wide kernel for large fused updates, the CDDT table's index);
- * get_schedule then reports the values that set_schedule would start from. */
+ * get_schedule then reports the values that set_schedule would start from.  Autotuning decides for
+ * the fused update alone. */
 RLC_API int rlc_method_set_schedule(rlc_method* m, int dt_layout, int fused_block, int prefetch, int tile);
 RLC_API int rlc_method_get_schedule(const rlc_method* m, int* dt_layout, int* fused_block, int* prefetch,
                                     int* tile);
-/* Time the schedule candidates on a workload (device pointers) and keep the fastest: the median
- * of 5 single launches for every candidate, then the median of 31 for the three fastest, taken
- * round-robin.  rlc_method_autotune_ex with RLC_TUNE_FLUSH_L2 writes twice the L2 size before
+/* Time the schedule candidates of the fused update on a workload (device pointers), and what it picks
+ * without a schedule, and keep the fastest: the median of 5 single launches for every candidate, then
+ * the median of 31 for the three fastest, taken round-robin.  rlc_method_autotune_ex with RLC_TUNE_FLUSH_L2 writes twice the L2 size before
  * every timed launch (for callers whose maps leave L2 between updates; it holds that buffer for
  * the call), and rlc_method_autotune_results returns the candidates of the last autotune:
- * schedules[4 i .. 4 i + 3] = (dt_layout, fused_block, prefetch, tile) and times_ms[2 i],
+ * schedules[4 i .. 4 i + 3] = (dt_layout, fused_block, prefetch, tile) -- (its layout, 0, 0, 0) for what
+ * the call picks, which get_schedule reports too (with the block left as it was) while that is kept,
+ * and which no set_schedule restores -- and times_ms[2 i],
  * times_ms[2 i + 1] = first-stage and final medians (0 when not a finalist); at most `max`
  * entries are written, *count gets the number of candidates. */
 enum rlc_tune_flags { RLC_TUNE_FLUSH_L2 = 1u };
@@ -286,7 +289,8 @@ typedef struct rlc_filter_desc {
 } rlc_filter_desc;
 
 /* The methods must outlive the batch.  block = threads per block (0 = 256).  A method's trig
- * override set or cleared after the batch was created is taken up by the next rlc_batch_run. */
+ * override, sensor model or CDDT table changed after the batch was created is taken up by the next
+ * rlc_batch_run. */
 RLC_API int rlc_batch_create(const rlc_filter_desc* filters, int n_filters, int block, rlc_batch** out);
 RLC_API int rlc_batch_run(rlc_batch* b, void* stream);
 /* Schedule of the persistent launch: distance-transform layout (0 linear, 1 tiled, 2 compact
@@ -294,7 +298,7 @@ RLC_API int rlc_batch_run(rlc_batch* b, void* stream);
  * threads per block, particles per tile
  * (0 = 32).  Results are identical under every schedule.  Until a schedule, a product mode or a block
  * size is given, a batch of ray marchers picks its launch by its size (one wide launch with the
- * products inside below 48 M rays). */
+ * products inside below 48 M rays), which rlc_batch_autotune times beside the schedules. */
 RLC_API int rlc_batch_set_schedule(rlc_batch* b, int dt_layout, int prefetch, int block, int tile);
 RLC_API int rlc_batch_get_schedule(const rlc_batch* b, int* dt_layout, int* prefetch, int* block, int* tile);
 /* Where the per-particle products run: RLC_PRODUCTS_OVERLAPPED -- inside the persistent kernel,
@@ -304,7 +308,8 @@ RLC_API int rlc_batch_get_schedule(const rlc_batch* b, int* dt_layout, int* pref
 enum rlc_product_mode { RLC_PRODUCTS_OVERLAPPED = 0, RLC_PRODUCTS_SEPARATE = 1 };
 RLC_API int rlc_batch_set_product_mode(rlc_batch* b, int mode);
 RLC_API int rlc_batch_get_product_mode(const rlc_batch* b, int* mode);
-/* Run the batch under each schedule candidate on `stream` and keep the fastest. */
+/* Run the batch under each schedule candidate and the launch that it picks without one on `stream`,
+ * and keep the fastest. */
 RLC_API int rlc_batch_autotune(rlc_batch* b, void* stream);
 RLC_API int rlc_batch_destroy(rlc_batch* b);
 /* rays = sum of n_particles * n_angles; tiles = work items of the device queue */

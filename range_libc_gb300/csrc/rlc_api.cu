@@ -210,12 +210,15 @@ struct rlc_method {
     int prefetch = 0;
     int fused_block = 256;
     int tile = 0;             // particles per tile of the fused kernels (0 = auto)
-    // no schedule asked for or autotuned yet: every call picks its kernels by size (results do not
-    // depend on the schedule; rlc_method_get_schedule reports the values above meanwhile)
-    bool pick = true;
+    // No schedule asked for: every call picks its kernels by size (results do not depend on the schedule;
+    // rlc_method_get_schedule reports the values above meanwhile).  The fused update has its own word,
+    // which autotune changes: it times that call and decides for no other.
+    bool pick = true, pick_fused = true;
     bool autotune_pending = false;
+    // a schedule of the fused update; pick: what the call chooses by itself
+    struct Fused { int layout, block, prefetch, tile; bool pick; };
     // the last autotune: every candidate's schedule and median times (ms) of both stages
-    struct TuneResult { int layout, block, prefetch, tile; float first_ms, final_ms; };
+    struct TuneResult { Fused f; float first_ms, final_ms; };
     std::vector<TuneResult> tune_results;
 
     ~rlc_method() {
@@ -236,14 +239,15 @@ struct rlc_method {
         if (map) map->release();
     }
 
-    CastParams params() const {
+    // dt_layout: the distance transform's layout that the call reads
+    CastParams params(int dt_layout = DT_LINEAR) const {
         CastParams p{};
         p.kind = dkind;
         p.mr = mr;
         p.map.W = map->W;
         p.map.H = map->H;
         p.map.tiles_y = map->TY;
-        p.map.dt = layout == DT_TILED ? map->d_dt_tiled : map->d_dt;   // linear for DT_U16 / DT_STAGED
+        p.map.dt = dt_layout == DT_TILED ? map->d_dt_tiled : map->d_dt;   // linear for DT_U16 / DT_STAGED
         p.map.dt16 = map->d_dt16;
         p.map.dt8 = map->d_dt8;
         p.map.step = map->d_step;
@@ -413,14 +417,15 @@ int cast_layout(const rlc_method* m, long long rays, bool independent) {
 
 // search of a CDDT method's queries (the prefetch schedule) or prefetch of a ray-marching one:
 // without a schedule, CDDT queries go by the table's index where it has one
-int cast_search(const rlc_method* m) { return m->pick && m->dkind == K_CDDT && m->index.index ? 3 : m->prefetch; }
+int picked_search(const rlc_method* m) { return m->dkind == K_CDDT && m->index.index ? 3 : 0; }
+int cast_search(const rlc_method* m) { return m->pick ? picked_search(m) : m->prefetch; }
 
-// layout of a fused call.  Without a schedule, ray marching takes the step map, with its equal-step
+// layout of a fused call without a schedule: ray marching takes the step map, with its equal-step
 // runs while the call waits for its longest rays and not for its products: 4,000 x 61 linear / step /
 // runs 43 / 43 / 34 us, 500 x 300 50 / 50 / 38, 4,000 x 271 - / 69 / 60; 637 x 849 72 / 72 / 78,
 // 4,000 x 1,081 - / 140 / 157, 20,000 x 1,081 438 / 423 / 496 us.
-int fused_layout(const rlc_method* m, int n, int na) {
-    if (!m->pick || m->dkind != K_RM) return cast_layout(m);
+int picked_fused_layout(const rlc_method* m, int n, int na) {
+    if (m->dkind != K_RM) return DT_LINEAR;
     if (!m->map->long_runs) return map_layout(m->map, DT_STEP);
     return map_layout(m->map, (long long)n * na < (2ll << 20) && (na < 512 || n >= 2000) ? DT_RUNS : DT_STEP);
 }
@@ -858,12 +863,13 @@ int rlc_calc_range_many(rlc_method* m, const float* ins, float* outs, int n, uns
     if (!ins || !outs) return fail(RLC_ERR_ARG, "null array");
     if (int rc = check_trig(m, n)) return rc;
     cudaStream_t s = (cudaStream_t)stream;
-    CastParams p = m->params();
+    const int layout = cast_layout(m, n, true);
+    CastParams p = m->params(layout);
     bool world = !(flags & RLC_NO_WORLD);
     if (flags & RLC_DEVICE_PTRS)
-        return finish_launch(launch_calc_range_many(p, cast_layout(m, n, true), cast_search(m), world, ins, outs, n, s), "calc_range_many");
+        return finish_launch(launch_calc_range_many(p, layout, cast_search(m), world, ins, outs, n, s), "calc_range_many");
     if (host_direct()) {
-        CUDA_OR_FAIL(launch_calc_range_many(p, cast_layout(m, n, true), cast_search(m), world, ins, outs, n, s), "calc_range_many");
+        CUDA_OR_FAIL(launch_calc_range_many(p, layout, cast_search(m), world, ins, outs, n, s), "calc_range_many");
         CUDA_OR_FAIL(cudaStreamSynchronize(s), "calc_range_many");
         return RLC_OK;
     }
@@ -873,7 +879,7 @@ int rlc_calc_range_many(rlc_method* m, const float* ins, float* outs, int n, uns
     float* d_in = (float*)st;
     float* d_out = (float*)((char*)st + bin);
     CUDA_OR_FAIL(cudaMemcpyAsync(d_in, ins, (size_t)n * 3 * sizeof(float), cudaMemcpyHostToDevice, s), "H2D");
-    CUDA_OR_FAIL(launch_calc_range_many(p, cast_layout(m, n, true), cast_search(m), world, d_in, d_out, n, s), "calc_range_many");
+    CUDA_OR_FAIL(launch_calc_range_many(p, layout, cast_search(m), world, d_in, d_out, n, s), "calc_range_many");
     CUDA_OR_FAIL(cudaMemcpyAsync(outs, d_out, (size_t)n * sizeof(float), cudaMemcpyDeviceToHost, s), "D2H");
     CUDA_OR_FAIL(cudaStreamSynchronize(s), "calc_range_many");
     return RLC_OK;
@@ -888,11 +894,12 @@ int rlc_calc_range_repeat_angles(rlc_method* m, const float* ins, const float* a
     if (!ins || !angles || !outs) return fail(RLC_ERR_ARG, "null array");
     if (int rc = check_trig(m, (long long)n * na)) return rc;
     cudaStream_t s = (cudaStream_t)stream;
-    CastParams p = m->params();
+    const int layout = cast_layout(m, (long long)n * na, false);
+    CastParams p = m->params(layout);
     if (flags & RLC_DEVICE_PTRS)
-        return finish_launch(launch_repeat_angles(p, cast_layout(m, (long long)n * na, false), cast_search(m), ins, angles, outs, n, na, s), "repeat_angles");
+        return finish_launch(launch_repeat_angles(p, layout, cast_search(m), ins, angles, outs, n, na, s), "repeat_angles");
     if (host_direct()) {
-        CUDA_OR_FAIL(launch_repeat_angles(p, cast_layout(m, (long long)n * na, false), cast_search(m), ins, angles, outs, n, na, s), "repeat_angles");
+        CUDA_OR_FAIL(launch_repeat_angles(p, layout, cast_search(m), ins, angles, outs, n, na, s), "repeat_angles");
         CUDA_OR_FAIL(cudaStreamSynchronize(s), "repeat_angles");
         return RLC_OK;
     }
@@ -905,7 +912,7 @@ int rlc_calc_range_repeat_angles(rlc_method* m, const float* ins, const float* a
     float* d_out = (float*)((char*)st + b0 + b1);
     CUDA_OR_FAIL(cudaMemcpyAsync(d_in, ins, (size_t)n * 3 * sizeof(float), cudaMemcpyHostToDevice, s), "H2D");
     CUDA_OR_FAIL(cudaMemcpyAsync(d_ang, angles, (size_t)na * sizeof(float), cudaMemcpyHostToDevice, s), "H2D");
-    CUDA_OR_FAIL(launch_repeat_angles(p, cast_layout(m, (long long)n * na, false), cast_search(m), d_in, d_ang, d_out, n, na, s), "repeat_angles");
+    CUDA_OR_FAIL(launch_repeat_angles(p, layout, cast_search(m), d_in, d_ang, d_out, n, na, s), "repeat_angles");
     CUDA_OR_FAIL(cudaMemcpyAsync(outs, d_out, (size_t)n * na * sizeof(float), cudaMemcpyDeviceToHost, s), "D2H");
     CUDA_OR_FAIL(cudaStreamSynchronize(s), "repeat_angles");
     return RLC_OK;
@@ -1014,6 +1021,20 @@ static int ensure_bins(rlc_method* m, size_t count) {
     return RLC_OK;
 }
 
+// the fused update under one schedule (ensure_bins first for DT_STAGED)
+static cudaError_t launch_fused_as(const rlc_method* m, const rlc_method::Fused& f, const float* ins, const float* angles,
+                                   const float* obs, double* w, int n, int na, cudaStream_t s) {
+    const SensorDev sm{m->d_table, m->K};
+    if (f.pick) {
+        const int layout = picked_fused_layout(m, n, na);
+        return launch_fused(m->params(layout), layout, picked_search(m), sm, ins, angles, obs, w, n, na, 0, 0, true, s);
+    }
+    if (f.layout == DT_STAGED && m->dkind == K_RM)
+        return launch_fused_staged(m->params(), sm, ins, angles, obs, w, n, na, f.tile, m->d_bins, s);
+    const int layout = f.layout == DT_STAGED ? DT_LINEAR : map_layout(m->map, f.layout);
+    return launch_fused(m->params(layout), layout, f.prefetch, sm, ins, angles, obs, w, n, na, f.block, f.tile, false, s);
+}
+
 static int fused_device(rlc_method* m, const float* ins, const float* angles, const float* obs, double* w, int n,
                         int na, cudaStream_t s) {
     if (m->autotune_pending) {
@@ -1021,16 +1042,10 @@ static int fused_device(rlc_method* m, const float* ins, const float* angles, co
         int rc = rlc_method_autotune(m, ins, angles, obs, w, n, na, s);
         if (rc) return rc;
     }
-    CastParams p = m->params();
-    SensorDev sm{m->d_table, m->K};
-    if (m->layout == DT_STAGED && m->dkind == K_RM) {
+    const rlc_method::Fused f{m->layout, m->fused_block, m->prefetch, m->tile, m->pick_fused};
+    if (!f.pick && f.layout == DT_STAGED && m->dkind == K_RM)
         if (int rc = ensure_bins(m, (size_t)n * na)) return rc;
-        return finish_launch(launch_fused_staged(p, sm, ins, angles, obs, w, n, na, m->tile, m->d_bins, s),
-                             "fused sensor model (staged)");
-    }
-    return finish_launch(launch_fused(p, fused_layout(m, n, na), cast_search(m), sm, ins, angles, obs, w, n, na,
-                                      m->fused_block, m->tile, m->pick, s),
-                         "fused sensor model");
+    return finish_launch(launch_fused_as(m, f, ins, angles, obs, w, n, na, s), "fused sensor model");
 }
 
 int rlc_trig_eval(const float* x, float* sincos, int64_t n, unsigned flags, void* stream) {
@@ -1099,7 +1114,7 @@ int rlc_method_set_schedule(rlc_method* m, int dt_layout, int fused_block, int p
         m->layout = dt_layout;
         m->prefetch = prefetch;
         m->tile = tile;
-        m->pick = false;
+        m->pick = m->pick_fused = false;
     }
     if (fused_block) m->fused_block = fused_block;
     return RLC_OK;
@@ -1125,7 +1140,7 @@ static float median_of(std::vector<float> v) {
 }
 
 // Times every schedule candidate (distance-transform layout x RM march variant or CDDT bin search
-// x block size x particles per tile, and the staged update) on the caller's workload with CUDA
+// x block size x particles per tile, the staged update, and what the call picks without a schedule) on the caller's workload with CUDA
 // events around single launches: the median of kTuneFirst launches for every candidate, then the
 // median of kTuneFinal launches for the kTuneFinalists fastest, taken round-robin so that clock
 // and neighbour drift falls on all of them alike.  With RLC_TUNE_FLUSH_L2 a write of twice the
@@ -1150,12 +1165,13 @@ int rlc_method_autotune_ex(rlc_method* m, const float* ins, const float* angles,
                     if (ti > 0 && tile_particles(na, blocks[bi], tiles[ti]) == tile_particles(na, blocks[bi], 0))
                         continue;   // same tile as the automatic choice
                     const int pf = (m->dkind == K_CDDT && pk) ? 2 : pk;
-                    cands.push_back(Cand{kLayouts[lk], blocks[bi], pf, tiles[ti], 0.0f, 0.0f});
+                    cands.push_back(Cand{{kLayouts[lk], blocks[bi], pf, tiles[ti], false}, 0.0f, 0.0f});
                 }
     if (rm) {   // beam-major update with staged windows
         if (int rc = ensure_bins(m, (size_t)n * na)) return rc;
-        cands.push_back(Cand{DT_STAGED, 0, 0, 0, 0.0f, 0.0f});
+        cands.push_back(Cand{{DT_STAGED, 0, 0, 0, false}, 0.0f, 0.0f});
     }
+    cands.push_back(Cand{{picked_fused_layout(m, n, na), 0, 0, 0, true}, 0.0f, 0.0f});   // the call's own choice
     void* flush = nullptr;
     size_t flush_bytes = 0;
     if (flags & RLC_TUNE_FLUSH_L2) {
@@ -1171,14 +1187,7 @@ int rlc_method_autotune_ex(rlc_method* m, const float* ins, const float* angles,
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     cudaError_t err = cudaEventCreate(&e0);
     if (err == cudaSuccess) err = cudaEventCreate(&e1);
-    SensorDev sm{m->d_table, m->K};
-    const int saved_layout = m->layout;
-    auto launch = [&](const Cand& c) -> cudaError_t {
-        m->layout = c.layout;
-        CastParams p = m->params();
-        if (c.layout == DT_STAGED) return launch_fused_staged(p, sm, ins, angles, obs, w, n, na, 0, m->d_bins, s);
-        return launch_fused(p, map_layout(m->map, c.layout), c.prefetch, sm, ins, angles, obs, w, n, na, c.block, c.tile, false, s);
-    };
+    auto launch = [&](const Cand& c) { return launch_fused_as(m, c.f, ins, angles, obs, w, n, na, s); };
     unsigned flush_round = 0;
     auto time_once = [&](const Cand& c, float* ms) -> cudaError_t {
         cudaError_t e = cudaSuccess;
@@ -1223,11 +1232,10 @@ int rlc_method_autotune_ex(rlc_method* m, const float* ins, const float* angles,
     if (e0) cudaEventDestroy(e0);
     if (e1) cudaEventDestroy(e1);
     if (flush) cudaFree(flush);
-    m->layout = saved_layout;
     if (err != cudaSuccess) return cuda_fail(err, "autotune");
     if (best >= 0) {
-        const Cand& b = cands[best];
-        m->pick = false;
+        const rlc_method::Fused& b = cands[best].f;
+        m->pick_fused = b.pick;
         m->layout = b.layout;
         if (b.block) m->fused_block = b.block;
         m->prefetch = b.prefetch;
@@ -1249,10 +1257,10 @@ int rlc_method_autotune_results(const rlc_method* m, int max, int* count, int* s
     for (int i = 0; i < max && i < *count; ++i) {
         const auto& r = m->tune_results[i];
         if (schedules) {
-            schedules[4 * i] = r.layout;
-            schedules[4 * i + 1] = r.block;
-            schedules[4 * i + 2] = r.prefetch;
-            schedules[4 * i + 3] = r.tile;
+            schedules[4 * i] = r.f.layout;
+            schedules[4 * i + 1] = r.f.block;
+            schedules[4 * i + 2] = r.f.prefetch;
+            schedules[4 * i + 3] = r.f.tile;
         }
         if (times_ms) {
             times_ms[2 * i] = r.first_ms;
@@ -1548,7 +1556,7 @@ int rlc_batch_get_schedule(const rlc_batch* b, int* dt_layout, int* prefetch, in
 int rlc_batch_autotune(rlc_batch* b, void* stream) {
     if (!b) return fail(RLC_ERR_ARG, "null batch handle");
     cudaStream_t s = (cudaStream_t)stream;
-    struct Cand { bool sep; int layout, pf, block, tile; float ms; };
+    struct Cand { bool sep; int layout, pf, block, tile; float ms; bool pick; };
     std::vector<Cand> cands;
     const int blocks[2] = {256, 512};
     const int tiles[3] = {8, 16, 32};
@@ -1559,12 +1567,21 @@ int rlc_batch_autotune(rlc_batch* b, void* stream) {
                 for (int bi = 0; bi < 2; ++bi)
                     for (int ti = 0; ti < 3; ++ti) {
                         if (!b->rm_only && (kLayouts[lk] != 0 || pf != 0)) continue;
-                        cands.push_back(Cand{sp != 0, kLayouts[lk], pf, blocks[bi], tiles[ti], 0.0f});
+                        cands.push_back(Cand{sp != 0, kLayouts[lk], pf, blocks[bi], tiles[ti], 0.0f, false});
                     }
+    if (b->rm_only) {   // the batch's own choice: the wide launch, where it comes to that
+        const bool pick = b->pick;
+        b->pick = true;
+        const int rc = b->build();
+        b->pick = pick;
+        if (rc) return rc;
+        const rlc_batch::Schedule& r = b->run;
+        if (r.wide) cands.push_back(Cand{r.separate, r.layout, r.prefetch, r.block, r.tile, 0.0f, true});
+    }
     const bool s0 = b->separate, pick0 = b->pick;
-    b->pick = false;
     const int l0 = b->layout, p0 = b->prefetch, b0 = b->block, t0 = b->tile;
     auto apply = [&](const Cand& c) {
+        b->pick = c.pick;
         b->separate = c.sep;
         b->layout = c.layout;
         b->prefetch = c.pf;

@@ -493,7 +493,8 @@ class _RangeMethod:
         return a.value, b.value, c.value, d.value
 
     def autotune(self, ins, angles, obs, weights, flush_l2: bool = False) -> None:
-        """Time the schedule candidates on this workload (CUDA tensors) and keep the fastest;
+        """Time the fused update's schedule candidates, and what it picks without one, on this workload
+        (CUDA tensors) and keep the fastest (the other calls go on choosing by size);
         flush_l2 writes twice the L2 size before every timed launch (maps that leave L2 between
         updates)."""
         ptrs = [_arg(a, dt, nd, nm) for a, dt, nd, nm in ((ins, np.float32, 2, "ins"), (angles, np.float32, 1, "angles"),
@@ -505,7 +506,8 @@ class _RangeMethod:
 
     def autotune_results(self):
         """Candidates of the last autotune: list of ((dt_layout, fused_block, prefetch, tile),
-        first-stage median ms, final median ms or None)."""
+        first-stage median ms, final median ms or None); (layout, 0, 0, 0) with another layout than 3
+        is the call's own choice."""
         n = C.c_int()
         call("rlc_method_autotune_results", self._h, 0, C.byref(n), None, None)
         sched = np.zeros((max(n.value, 1), 4), np.int32)
@@ -716,7 +718,8 @@ class PyFilterBatch:
         return tuple(x.value for x in v)
 
     def autotune(self) -> None:
-        """Run the batch under each schedule candidate and keep the fastest (outputs are rewritten)."""
+        """Run the batch under each schedule candidate and the launch it picks without one, and keep
+        the fastest (outputs are rewritten)."""
         call("rlc_batch_autotune", self._h, _stream_of(self._keep[0][1]))
 
     def info(self):

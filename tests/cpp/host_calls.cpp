@@ -42,8 +42,10 @@ struct Launch { std::string name; std::vector<void*> words; };   // the first pa
 bool capturing = false;
 std::vector<Launch> recorded;
 
+std::string last_kernel;
+
 void launched(const void* f, void** args) {
-    const std::string& name = kernels()[f];
+    const std::string& name = last_kernel = kernels()[f];
     clock_ms += kernel_ms(name);
     on_launch(name, args);
     if (capturing) recorded.push_back(Launch{name, {args ? *(void**)args[0] : nullptr}});
@@ -353,13 +355,72 @@ int learned_timeouts() {
     return 0;
 }
 
+// Tuning keeps what is fastest, the call's own choice without a schedule among it; it decides for the fused
+// update that it times, and the other calls go on choosing for themselves.
+int autotune() {
+    std::vector<float> x(9, 1.0f);   // (nothing reads the arrays)
+    std::vector<double> w(9);
+    const int n = 2100, na = 150;
+    auto ran = [](const char* part) { return last_kernel.find(part) != std::string::npos; };
+    for (int kind : {RLC_RM, RLC_CDDT, RLC_GLT, RLC_BL}) {
+        rlc_method* m = method(kind, 64, 48, kind == RLC_CDDT || kind == RLC_GLT ? 16 : 0);
+        CHECK(m && sensor(m, 41) == RLC_OK);
+        auto fused = [&]() { return rlc_calc_range_repeat_angles_eval_sensor_model(m, x.data(), x.data(), x.data(), w.data(), n, na, RLC_DEVICE_PTRS, nullptr); };
+        auto many = [&]() { return rlc_calc_range_many(m, x.data(), x.data(), n, RLC_DEVICE_PTRS, nullptr); };
+        auto tune = [&](const char* fast) {
+            kernel_ms = [=](const std::string& name) { return name.find(fast) != std::string::npos ? 1.0f : 2.0f; };
+            return rlc_method_autotune(m, x.data(), x.data(), x.data(), w.data(), n, na, nullptr);
+        };
+        CHECK(many() == RLC_OK);
+        const std::string own = last_kernel;
+        const char* listed = kind == RLC_RM ? "k_fused<1, 1, 8>" : kind == RLC_CDDT ? "k_fused<2, 0, 2>" : "k_fused<";
+        for (const char* fast : {"k_fused_wide<", listed, "k_fused_wide<"}) {
+            CHECK(tune(fast) == RLC_OK && fused() == RLC_OK && ran(fast));
+            CHECK(many() == RLC_OK && last_kernel == own);
+            int count = 0, finals = 0, match = 0, sch[4];
+            CHECK(rlc_method_autotune_results(m, 0, &count, nullptr, nullptr) == RLC_OK && count > 1);
+            std::vector<int> s(4 * (size_t)count);
+            std::vector<float> ms(2 * (size_t)count);
+            CHECK(rlc_method_autotune_results(m, count, &count, s.data(), ms.data()) == RLC_OK);
+            CHECK(rlc_method_get_schedule(m, sch, sch + 1, sch + 2, sch + 3) == RLC_OK);
+            for (int i = 0; i < count; ++i)
+                if (ms[2 * i + 1] > 0) {
+                    ++finals;
+                    match += s[4 * i] == sch[0] && s[4 * i + 2] == sch[2] && s[4 * i + 3] == sch[3];
+                }
+            CHECK(finals == 3 && match > 0);
+        }
+        // a schedule that was set holds for all calls
+        CHECK(rlc_method_set_schedule(m, 0, 128, 0, 0) == RLC_OK && fused() == RLC_OK && ran("k_fused<"));
+        CHECK(many() == RLC_OK && ran(kind == RLC_RM ? "k_calc_range_many<1, 0, 0" : kind == RLC_CDDT ? "k_calc_range_many<2, 0, 0" : "k_calc_range_many<"));
+    }
+    rlc_method* m = method(RLC_RM);
+    CHECK(m && sensor(m, 41) == RLC_OK);
+    const rlc_filter_desc d = {m, x.data(), x.data(), x.data(), nullptr, w.data(), 500, 70};
+    rlc_batch* q = nullptr;
+    CHECK(rlc_batch_create(&d, 1, 0, &q) == RLC_OK);
+    auto in_graph = [&](const char* part) {
+        for (const Launch& l : last_graph)
+            if (l.name.find(part) != std::string::npos) return true;
+        return false;
+    };
+    for (const char* fast : {"k_batch_wide<", "k_batch<", "k_batch_wide<"}) {
+        kernel_ms = [=](const std::string& name) {
+            if (name.find(fast) != std::string::npos) return 1.0f;
+            return name.find("k_batch_wide<") != std::string::npos || name.find("k_batch<") != std::string::npos ? 9.0f : 0.1f;
+        };
+        CHECK(rlc_batch_autotune(q, nullptr) == RLC_OK && rlc_batch_run(q, nullptr) == RLC_OK && in_graph(fast));
+    }
+    return 0;
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
     const std::map<std::string, int (*)()> scenarios = {{"batch_tables", batch_tables}, {"batch_in_flight", batch_in_flight},
                                                           {"bresenham_memory", bresenham_memory}, {"occupancy", occupancy},
                                                           {"shared_memory_limits", shared_memory_limits},
-                                                          {"learned_timeouts", learned_timeouts}};
+                                                          {"learned_timeouts", learned_timeouts}, {"autotune", autotune}};
     const auto it = scenarios.find(argc > 1 ? argv[1] : "");
     if (it == scenarios.end()) return wrong("no such scenario");
     if (const int rc = it->second()) return rc;

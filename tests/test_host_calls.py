@@ -29,7 +29,7 @@ def host_calls(tmp_path_factory):
 
 
 @pytest.mark.parametrize("scenario", ["batch_tables", "batch_in_flight", "bresenham_memory", "occupancy",
-                                      "shared_memory_limits", "learned_timeouts"])
+                                      "shared_memory_limits", "learned_timeouts", "autotune"])
 def test_host_calls(host_calls, scenario):
     r = subprocess.run([str(host_calls), scenario], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0 and r.stdout.strip() == "ok", r.stdout + r.stderr
