@@ -941,14 +941,14 @@ __global__ void __launch_bounds__(256) k_cddt_radial(CastParams p, const float* 
 
 // ---------------------------------------------------------------- kernels
 template <int KIND, int LAYOUT, int PF, bool WORLD>
-__global__ void __launch_bounds__(256) k_calc_range_many(CastParams p, const float* __restrict__ ins,
+__global__ void __launch_bounds__(256) k_calc_range_many(CastParams p, const float* ins,
                                                          float* __restrict__ outs, int n) {
     after_previous();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (KIND == K_CDDT && PF == 1) {   // warp-cooperative bin search: every lane of the warp takes part
         const bool act = i < n;
         float q0 = 0.0f, q1 = 0.0f, q2 = 0.0f;
-        if (act) { q0 = __ldg(ins + 3 * (size_t)i); q1 = __ldg(ins + 3 * (size_t)i + 1); q2 = __ldg(ins + 3 * (size_t)i + 2); }
+        if (act) { q0 = ins[3 * (size_t)i]; q1 = ins[3 * (size_t)i + 1]; q2 = ins[3 * (size_t)i + 2]; }
         float r;
         if (WORLD) {
             float ax, ay, th;
@@ -961,7 +961,7 @@ __global__ void __launch_bounds__(256) k_calc_range_many(CastParams p, const flo
         return;
     }
     if (i >= n) return;
-    float q0 = __ldg(ins + 3 * (size_t)i), q1 = __ldg(ins + 3 * (size_t)i + 1), q2 = __ldg(ins + 3 * (size_t)i + 2);
+    float q0 = ins[3 * (size_t)i], q1 = ins[3 * (size_t)i + 1], q2 = ins[3 * (size_t)i + 2];
     if (WORLD) {
         float ax, ay, th;
         world_to_grid(p.world, q0, q1, q2, ax, ay, th);
@@ -973,8 +973,8 @@ __global__ void __launch_bounds__(256) k_calc_range_many(CastParams p, const flo
 
 // RangeLib.h:482-520: rays are particle-major, ray = i * na + a
 template <int KIND, int LAYOUT, int PF>
-__global__ void __launch_bounds__(256) k_repeat_angles(CastParams p, const float* __restrict__ ins,
-                                                       const float* __restrict__ angles,
+__global__ void __launch_bounds__(256) k_repeat_angles(CastParams p, const float* ins,
+                                                       const float* angles,
                                                        float* __restrict__ outs, int n, int na) {
     after_previous();
     long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -984,9 +984,9 @@ __global__ void __launch_bounds__(256) k_repeat_angles(CastParams p, const float
         if (act) {   // n * na < 2^31 (the ABI refuses larger calls): 32-bit division
             const unsigned gu = (unsigned)g, i = gu / (unsigned)na, a = gu - i * (unsigned)na;
             float th;
-            world_to_grid(p.world, __ldg(ins + 3 * (size_t)i), __ldg(ins + 3 * (size_t)i + 1),
-                          __ldg(ins + 3 * (size_t)i + 2), ax, ay, th);
-            h = __fsub_rn(th, __ldg(angles + a));
+            world_to_grid(p.world, ins[3 * (size_t)i], ins[3 * (size_t)i + 1],
+                          ins[3 * (size_t)i + 2], ax, ay, th);
+            h = __fsub_rn(th, angles[a]);
         }
         const float r = cddt_cast_warp(p, act, ax, ay, h);
         if (act) outs[g] = __fmul_rn(r, p.world.s);
@@ -995,9 +995,9 @@ __global__ void __launch_bounds__(256) k_repeat_angles(CastParams p, const float
     if (g >= (long long)n * na) return;
     const unsigned gu = (unsigned)g, i = gu / (unsigned)na, a = gu - i * (unsigned)na;   // n * na < 2^31
     float ax, ay, th;
-    world_to_grid(p.world, __ldg(ins + 3 * (size_t)i), __ldg(ins + 3 * (size_t)i + 1),
-                  __ldg(ins + 3 * (size_t)i + 2), ax, ay, th);
-    float r = cast_one<KIND, LAYOUT, PF>(p, ax, ay, __fsub_rn(th, __ldg(angles + a)), g);
+    world_to_grid(p.world, ins[3 * (size_t)i], ins[3 * (size_t)i + 1],
+                  ins[3 * (size_t)i + 2], ax, ay, th);
+    float r = cast_one<KIND, LAYOUT, PF>(p, ax, ay, __fsub_rn(th, angles[a]), g);
     outs[g] = __fmul_rn(r, p.world.s);
 }
 
@@ -1066,8 +1066,8 @@ constexpr int kEvalWarps = 8;
 constexpr int kEvalRows = (32 + kEvalWarps - 2) / (kEvalWarps - 1);   // particles per preparing warp
 
 __global__ void __launch_bounds__(32 * kEvalWarps) k_eval_sensor(CastParams p, SensorDev sm,
-                                                                 const float* __restrict__ obs,
-                                                                 const float* __restrict__ ranges,
+                                                                 const float* obs,
+                                                                 const float* ranges,
                                                                  double* __restrict__ outs, int na, int n) {
     __shared__ double s_f[2][kEvalBeams][33];   // [beam][particle]; a row is 33 doubles: no bank conflicts either way
     after_previous();
@@ -1081,9 +1081,9 @@ __global__ void __launch_bounds__(32 * kEvalWarps) k_eval_sensor(CastParams p, S
         const auto request = [&](int k) {   // chunk k's ranges and observation, lane = beam
             const int a = k * kEvalBeams + lane;
             if (a < na) {
-                o = __ldg(obs + a);
+                o = obs[a];
 #pragma unroll
-                for (int u = 0; u < kEvalRows; ++u) r[u] = i0 + u < np ? __ldg(rows + (size_t)(i0 + u) * na + a) : 0.0f;
+                for (int u = 0; u < kEvalRows; ++u) r[u] = i0 + u < np ? rows[(size_t)(i0 + u) * na + a] : 0.0f;
             }
         };
         const auto factors = [&](int k) {
@@ -1122,13 +1122,13 @@ __global__ void __launch_bounds__(32 * kEvalWarps) k_eval_sensor(CastParams p, S
 
 // range of ray (particle i, beam a) in pixels (RangeLib.h:558-612)
 template <int KIND, int LAYOUT, int PF>
-__device__ __forceinline__ float cast_ray(const CastParams& p, const float* __restrict__ ins,
-                                          const float* __restrict__ angles, int i, int a, int na, int layout, int pf) {
+__device__ __forceinline__ float cast_ray(const CastParams& p, const float* ins,
+                                          const float* angles, int i, int a, int na, int layout, int pf) {
     float ax, ay, th;
-    world_to_grid(p.world, __ldg(ins + 3 * (size_t)i), __ldg(ins + 3 * (size_t)i + 1), __ldg(ins + 3 * (size_t)i + 2),
+    world_to_grid(p.world, ins[3 * (size_t)i], ins[3 * (size_t)i + 1], ins[3 * (size_t)i + 2],
                   ax, ay, th);
     const long long ray = (long long)i * na + a;
-    const float h = __fsub_rn(th, __ldg(angles + a));
+    const float h = __fsub_rn(th, angles[a]);
     if (KIND >= 0) return cast_one<KIND, LAYOUT, PF>(p, ax, ay, h, ray);
     if (KIND == kRmOnly) return cast_one<K_RM, LAYOUT, PF>(p, ax, ay, h, ray);   // every filter ray-marches
     // mixed kinds: dispatch at run time
@@ -1160,8 +1160,8 @@ __device__ __forceinline__ float cast_ray(const CastParams& p, const float* __re
 // threads), so that a particle-filter step's blocks of 128 threads stay resident at 16 per SM
 // in one wave; the CDDT searches keep their registers.
 template <int KIND, int LAYOUT, int PF>
-__global__ void __launch_bounds__(512, KIND == K_CDDT ? 1 : KIND == K_BL ? 2 : 4) k_fused(CastParams p, SensorDev sm, const float* __restrict__ ins,
-                                               const float* __restrict__ angles, const float* __restrict__ obs,
+__global__ void __launch_bounds__(512, KIND == K_CDDT ? 1 : KIND == K_BL ? 2 : 4) k_fused(CastParams p, SensorDev sm, const float* ins,
+                                               const float* angles, const float* obs,
                                                double* __restrict__ weights, int n, int na, int P) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     after_previous();
@@ -1171,7 +1171,7 @@ __global__ void __launch_bounds__(512, KIND == K_CDDT ? 1 : KIND == K_BL ? 2 : 4
     for (int r = threadIdx.x; r < nr; r += blockDim.x) {
         const int li = div_small(r, na, inv_na), a = r - li * na, i = first + li;
         if (i < n) {
-            const int ob = sensor_bin(__fmul_rn(__ldg(obs + a), p.world.inv_s), sm.K, p.err);
+            const int ob = sensor_bin(__fmul_rn(obs[a], p.world.inv_s), sm.K, p.err);
             const float d = cast_ray<KIND, LAYOUT, PF>(p, ins, angles, i, a, na, LAYOUT, PF);
             sf[r] = __ldg(sm.table + (size_t)ob * sm.K + sensor_bin(d, sm.K, p.err));
         }
@@ -1254,8 +1254,8 @@ __host__ __device__ inline WideSmem wide_smem(int P, int C, bool factors) {
 // Particles [first, first + np) of one filter through all its beams, by a whole block; ranges (pixels,
 // optional) as ranges[i * na + a].  s_next: two counters of the block.
 template <int KIND, int LAYOUT, int PF, bool FACTORS>
-__device__ __forceinline__ void wide_tile(const CastParams& p, const SensorDev& sm, const float* __restrict__ ins,
-                                          const float* __restrict__ angles, const float* __restrict__ obs,
+__device__ __forceinline__ void wide_tile(const CastParams& p, const SensorDev& sm, const float* ins,
+                                          const float* angles, const float* obs,
                                           float* __restrict__ ranges, double* __restrict__ weights, int first, int np,
                                           int na, int P, int C, unsigned char* smem, unsigned* s_next) {
     constexpr bool kTrig = KIND == K_RM || KIND == K_BL;
@@ -1270,16 +1270,16 @@ __device__ __forceinline__ void wide_tile(const CastParams& p, const SensorDev& 
     if ((int)threadIdx.x < np) {
         const float* q = ins + 3 * (size_t)(first + threadIdx.x);
         float ax, ay, th;
-        world_to_grid(p.world, __ldg(q), __ldg(q + 1), __ldg(q + 2), ax, ay, th);
+        world_to_grid(p.world, q[0], q[1], q[2], ax, ay, th);
         part[2 * threadIdx.x] = make_float4(ax, ay, th, 0.0f);
         if (kTrig && !p.trig) part[2 * threadIdx.x + 1] = trig_record(th);
     }
     const auto beams = [&](int k, int t) {   // records of chunk k's beams, thread t of 64
         for (int j = t; j < min(C, na - k * C); j += 64) {
-            const float an = __ldg(angles + k * C + j);
+            const float an = angles[k * C + j];
             ang[(k & 1) * C + j] = an;
             if (kTrig && !p.trig) beam[(k & 1) * C + j] = trig_record(an);
-            row[(k % 3) * C + j] = (uint16_t)sensor_bin(__fmul_rn(__ldg(obs + k * C + j), p.world.inv_s), sm.K, p.err);
+            row[(k % 3) * C + j] = (uint16_t)sensor_bin(__fmul_rn(obs[k * C + j], p.world.inv_s), sm.K, p.err);
         }
     };
     if (threadIdx.x >= kWideThreads - 64) beams(0, threadIdx.x - (kWideThreads - 64));
@@ -1342,8 +1342,8 @@ __device__ __forceinline__ void wide_tile(const CastParams& p, const SensorDev& 
 
 template <int KIND, int LAYOUT, int PF, bool FACTORS>
 __global__ void __launch_bounds__(kWideThreads, wide_blocks(KIND))
-k_fused_wide(CastParams p, SensorDev sm, const float* __restrict__ ins, const float* __restrict__ angles,
-             const float* __restrict__ obs, double* __restrict__ weights, int n, int na, int P, int C) {
+k_fused_wide(CastParams p, SensorDev sm, const float* ins, const float* angles,
+             const float* obs, double* __restrict__ weights, int n, int na, int P, int C) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ unsigned s_next[2];
     after_previous();

@@ -233,7 +233,11 @@ inline cudaError_t ensure_smem_attr(K kernel, int bytes, std::atomic<unsigned lo
 // A kernel that launch_next launches may come onto the SMs while the blocks of the one before it in the
 // stream are ending; it calls after_previous() before it touches memory, which waits for all of those and
 // their writes, and only then lets the next one do the same.  So at most two kernels of a stream are on
-// the SMs, and what the one before the previous wrote is there.  Launched any other way, or after
+// the SMs, and what the one before the previous wrote is there.  What the one before may have written, a call's
+// arrays and a training step's, is read by plain loads through pointers without __restrict__: __ldg and const
+// __restrict__ stand for the non-coherent path, which PTX allows only for memory that nobody writes while the
+// kernel lives, and this one lives beside its writer.  Maps, tables and parameters, written earlier than that,
+// may take it.  Launched any other way, or after
 // anything but such a kernel, the wait is nothing.  Calls in a row: 1 M lookups 25.7 -> 22.8 us each, a
 // cast and a product of 4,000 x 108 rays 18.1 -> 16.2; two training steps of 65,536 rays 0.80 -> 0.73 ms.
 __device__ __forceinline__ void after_previous() {

@@ -656,7 +656,7 @@ struct FeatParams {
 // us for 65,536 rows, now 22).  Rows from n on are zero.
 constexpr int kFeatRows = 8;   // rows per warp
 
-__global__ void __launch_bounds__(256) k_features(FeatParams fp, const float* __restrict__ xyt, int n, int n_pad,
+__global__ void __launch_bounds__(256) k_features(FeatParams fp, const float* xyt, int n, int n_pad,
                                                   bf16* __restrict__ X) {
     __shared__ float s_freq[64];
     if (threadIdx.x < 64) s_freq[threadIdx.x] = fp.freq[threadIdx.x];
@@ -673,8 +673,8 @@ __global__ void __launch_bounds__(256) k_features(FeatParams fp, const float* __
             continue;
         }
         float s, c;
-        sincosf(__ldg(xyt + 3 * (size_t)r + 2), &s, &c);
-        const float u[4] = {__ldg(xyt + 3 * (size_t)r) * fp.inv_w, __ldg(xyt + 3 * (size_t)r + 1) * fp.inv_h, c, s};
+        sincosf(xyt[3 * (size_t)r + 2], &s, &c);
+        const float u[4] = {xyt[3 * (size_t)r] * fp.inv_w, xyt[3 * (size_t)r + 1] * fp.inv_h, c, s};
 #pragma unroll
         for (int d = 0; d < 4; ++d) {
             float s0, c0, s1, c1;
@@ -1035,8 +1035,8 @@ __global__ void k_out_layer(const bf16* __restrict__ H, const float* __restrict_
 constexpr int kTopBlocks = 2 * 152, kTopThreads = 512;
 constexpr int kTopPart = kHidden + 2;
 
-__global__ void __launch_bounds__(kTopThreads) k_top(const bf16* __restrict__ H, const bf16* __restrict__ Z,
-                                                     const float* __restrict__ params, const float* __restrict__ target,
+__global__ void __launch_bounds__(kTopThreads) k_top(const bf16* H, const bf16* Z,
+                                                     const float* __restrict__ params, const float* target,
                                                      int n, bf16* __restrict__ dZ, float* __restrict__ part) {
     __shared__ float s_part[kTopThreads / 32][kTopPart];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1059,7 +1059,7 @@ __global__ void __launch_bounds__(kTopThreads) k_top(const bf16* __restrict__ H,
             h[i] = __bfloat162float(H[base + 32 * i]);
             z[i] = __bfloat162float(Z[base + 32 * i]);
         }
-        const float t = __ldg(target + r);
+        const float t = target[r];
         float acc = 0.0f;
 #pragma unroll
         for (int i = 0; i < 8; ++i) acc += h[i] * w[i];
@@ -1114,8 +1114,8 @@ __device__ __forceinline__ void adam(const AdamArgs& A, size_t i, float gi) {
     A.wbf[i] = __float2bfloat16_rn(pi);
 }
 
-__global__ void __launch_bounds__(256) k_reduce_grads(const float* __restrict__ part, int splits,
-                                                      const float* __restrict__ top, float* __restrict__ grads,
+__global__ void __launch_bounds__(256) k_reduce_grads(const float* part, int splits,
+                                                      const float* top, float* __restrict__ grads,
                                                       float* __restrict__ loss, AdamArgs A) {
     constexpr unsigned kHiddenBlocks = (unsigned)(kOutW / 256);
     after_previous();
@@ -1123,7 +1123,7 @@ __global__ void __launch_bounds__(256) k_reduce_grads(const float* __restrict__ 
         const size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;
         float sum = 0.0f;
 #pragma unroll 16
-        for (int z = 0; z < splits; ++z) sum += __ldg(part + (size_t)z * kOutW + i);
+        for (int z = 0; z < splits; ++z) sum += part[(size_t)z * kOutW + i];
         grads[i] = sum;
         if (A.p) adam(A, i, sum);
         return;
@@ -1131,7 +1131,7 @@ __global__ void __launch_bounds__(256) k_reduce_grads(const float* __restrict__ 
     const int j = (int)(blockIdx.x - kHiddenBlocks) * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (j >= kTopPart) return;
     float sum = 0.0f;
-    for (int k = lane; k < kTopBlocks; k += 32) sum += __ldg(top + (size_t)k * kTopPart + j);
+    for (int k = lane; k < kTopBlocks; k += 32) sum += top[(size_t)k * kTopPart + j];
     for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
     if (lane != 0) return;
     if (j <= kHidden) {
