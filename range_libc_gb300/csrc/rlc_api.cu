@@ -63,12 +63,58 @@ int rlc::set_last_error(int code, const char* msg) {
     return code;
 }
 
+// A block of host memory for a map's bits.  Fresh pages that the GPU writes, and their unmapping, cost 12 us
+// of a 2048^2 map's 0.6 ms, so the last block of up to kKeep words (1 MB) that a map gave back waits for the
+// next one that fits, until the process ends.
+struct HostBits {
+    static constexpr size_t kKeep = 1u << 17;
+    std::unique_ptr<uint64_t[]> p;
+    size_t words = 0;
+
+    // at least `n` words, or null; new ones zeroed, so that the GPU writes to pages that are there
+    void take(size_t n) {
+        Spare& s = spare();
+        {
+            std::lock_guard<std::mutex> lk(s.mu);
+            if (s.words >= n) {
+                p = std::move(s.p);
+                words = s.words;
+                s.words = 0;
+            }
+        }
+        if (!p) {
+            p.reset(new (std::nothrow) uint64_t[n]());
+            words = n;
+        }
+    }
+    ~HostBits() {
+        if (!p || words > kKeep) return;
+        Spare& s = spare();
+        std::lock_guard<std::mutex> lk(s.mu);
+        if (words > s.words) {
+            std::swap(p, s.p);
+            s.words = words;
+        }
+    }
+
+private:
+    struct Spare {
+        std::mutex mu;
+        std::unique_ptr<uint64_t[]> p;
+        size_t words = 0;
+    };
+    static Spare& spare() {
+        static Spare* s = new Spare;   // (a map may outlive this library's statics)
+        return *s;
+    }
+};
+
 struct rlc_map {
     int device = 0;
     int W = 0, H = 0, TY = 0;
     float world[6] = {1.0f, 0.0f, 0.0f, 0.0f, 0.0f, 1.0f};   // scale, angle, ox, oy, sin, cos
     uint64_t* d_bits = nullptr;
-    std::unique_ptr<uint64_t[]> h_bits;   // their copy, so that the occupancy can be asked for at any time
+    HostBits h_bits;              // their copy, so that the occupancy can be asked for at any time
     float* d_dt = nullptr;
     float* d_dt_tiled = nullptr;
     uint16_t* d_dt16 = nullptr;
@@ -476,13 +522,13 @@ static int map_create(const uint8_t* occ, int width, int height, bool rows, rlc_
         if (e == cudaSuccess) e = cudaMemcpy(d_occ, occ, n, cudaMemcpyHostToDevice);
     }
     if (e == cudaSuccess) e = launch_pack_bits(direct ? occ : d_occ, width, height, rows, m->d_bits, 0);
-    m->h_bits.reset(new (std::nothrow) uint64_t[words]());   // zeroed: its pages are made beside the kernel, not by the GPU's writes
-    if (e == cudaSuccess && !m->h_bits) e = cudaErrorMemoryAllocation;
+    m->h_bits.take(words);
+    if (e == cudaSuccess && !m->h_bits.p) e = cudaErrorMemoryAllocation;
     if (e == cudaSuccess && direct) {
-        e = launch_copy_bits(m->d_bits, words, m->h_bits.get(), 0);
+        e = launch_copy_bits(m->d_bits, words, m->h_bits.p.get(), 0);
         if (e == cudaSuccess) e = cudaStreamSynchronize(0);
     } else if (e == cudaSuccess) {
-        e = cudaMemcpy(m->h_bits.get(), m->d_bits, words * sizeof(uint64_t), cudaMemcpyDeviceToHost);
+        e = cudaMemcpy(m->h_bits.p.get(), m->d_bits, words * sizeof(uint64_t), cudaMemcpyDeviceToHost);
     }
     cudaFree(d_occ);
     if (e != cudaSuccess) {
@@ -529,7 +575,7 @@ int rlc_map_occupancy(rlc_map* map, uint8_t* occ_out) {
     if (!map || !occ_out) return fail(RLC_ERR_ARG, "null argument");
     for (int x = 0; x < map->W; ++x) {
         uint8_t* col = occ_out + (size_t)x * map->H;
-        const uint64_t* tiles = map->h_bits.get() + (size_t)(x >> 3) * map->TY;
+        const uint64_t* tiles = map->h_bits.p.get() + (size_t)(x >> 3) * map->TY;
         for (int y = 0; y < map->H; y += 8) {
             // the tile's eight cells of this column, a byte each: the product puts bit k at bit 8 k (k < 7)
             const uint64_t b = (tiles[y >> 3] >> ((x & 7) << 3)) & 0xFFu;
