@@ -156,7 +156,9 @@ __global__ void k_edt_pass_x(const float* g, int W, int H, float* dt, uint32_t* 
 // z[k + 1] < q) therefore has the outcome of the exact comparison of the quotients.
 //  * edt_col_exact and fh_line_exact are the reference's steps with those comparisons decided in
 //    integers, one line after the other; comparisons with a FLT_MAX key run in double as in the
-//    reference.  No kernel runs them: they state the rule that the searches below are tested with.
+//    reference.  No kernel runs them: they are this rule as code, checked against the reference's
+//    transform on the host (tests/cpp/edt_exact_check.cu).  The searches that the kernels run are
+//    checked against that transform by themselves (edt_search_check.cu, edt_search_maps.cu).
 //  * So the envelope is the exact lower envelope of the lines K(p) - 2 p q, and at an integer q it
 //    takes the smallest p among those with the least K(p) - 2 p q: `s <= z[k]` drops a vertex that
 //    is nowhere strictly least, `z[k + 1] < q` stays with the left vertex where two tie.  A
@@ -580,7 +582,8 @@ __device__ __forceinline__ void store_layouts(const DtOut& o, int W, int H, int 
 
 // Pass 2, one thread per cell, 32 consecutive y per warp (the searched distances of a warp are
 // whole 64-byte pieces) x 8 x per block (which share them in the L1).  Bound by the search's
-// instructions: about 16 + (mean distance) / 4 reads per cell.  ALL: writes every layout, straight from
+// instructions: up to 17 reads of columns per cell, then one for each block of 8 up to 64 columns away and
+// of 64 beyond, and the columns of those that could win.  ALL: writes every layout, straight from
 // the search (60 MB at 2048^2; four more kernels read the linear one back before).
 // 2048^2 with the layouts: 1553 + 117 us with one thread per row, 121 with blocks of 32 columns, now 88.
 template <bool EXACT, bool ALL>
