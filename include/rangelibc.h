@@ -220,8 +220,9 @@ RLC_API int rlc_count_steps(rlc_method* m, const float* ins, const float* angles
 /* Schedule of the kernels: dt_layout 0 = linear x-major distance transform, 1 = 8x8 tiles,
  * 2 = compact 16-bit squared distances, 4 = linear map of each cell's march step
  * max(d * 0.999, 1) (a marker on occupied cells), 5 = that step map plus, per cell, how many cells after
- * it along each axis have the same step, so that a ray repeating one step beside a wall (6 times
- * in a row) skips the rest of the run in one go (exactly: the skipped steps' parameters are formed by the reference's own float
+ * it along each axis have the same step, so that a ray repeating one step beside a wall (it looks at
+ * every fourth step, and at the run where that equals the one four steps before) skips the rest of the
+ * run in one go (exactly: the skipped steps' parameters are formed by the reference's own float
  * additions and the landing cell is checked), 3 = beam-major fused update that stages each bundle's
  * window of 8-bit squared distances in shared memory (RM only; tile = particle chunks per beam,
  * 0 = one block per SM) (-1 = autotune on the next fused call); fused_block = threads per block of the fused kernel

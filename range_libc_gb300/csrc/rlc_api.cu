@@ -451,10 +451,11 @@ int cast_layout(const rlc_method* m) { return m->layout == DT_STAGED ? DT_LINEAR
 
 // layout of a cast of `rays` rays.  Without a schedule, ray marching takes the step map, with its
 // equal-step runs where the call waits for its longest rays: independent queries (their warps mix
-// long and short rays: 2 M queries on 2048^2 linear / step / runs 121 / 119 / 94 us, 10,000 21 / 19 /
-// 17 us, 1,000 on 512^2 33 / 33 / 15 us), and repeat-angle calls between 16 K and 256 K rays (4,000 x
-// 61 27 / 27 / 21 us; 1 x 1,081 9.7 / 9.3 / 10.0 us, 1,588 x 199 29 / 29 / 31 us, 20,000 x 61
-// 43 / 41 / 46 us, 20,000 x 1,081 267 / 257 / 336 us).
+// long and short rays: 2 M queries on 2048^2 linear / step / runs 114 / 110 / 89 us, 200,000 35 / 34 /
+// 21, 10,000 19 / 19 / 14, 1,000 on 512^2 9.9 / 9.6 / 10.5), and repeat-angle calls between 16 K and
+// 256 K rays (4,000 x 61 23 / 22 / 14 us, 200 x 100 22 / 21 / 12; 1 x 1,081 4.9 / 4.8 / 4.8, 20,000 x
+// 1,081 249 / 236 / 256).  The upper line is older than the march that looks for runs at every fourth
+// step only: 1,588 x 199 26 / 24 / 18 us and 20,000 x 61 36 / 34 / 31 now lie on its wrong side.
 int cast_layout(const rlc_method* m, long long rays, bool independent) {
     if (!m->pick || m->dkind != K_RM) return cast_layout(m);
     if (!m->map->long_runs) return map_layout(m->map, DT_STEP);
@@ -467,9 +468,9 @@ int picked_search(const rlc_method* m) { return m->dkind == K_CDDT && m->index.i
 int cast_search(const rlc_method* m) { return m->pick ? picked_search(m) : m->prefetch; }
 
 // layout of a fused call without a schedule: ray marching takes the step map, with its equal-step
-// runs while the call waits for its longest rays and not for its products: 4,000 x 61 linear / step /
-// runs 43 / 43 / 34 us, 500 x 300 50 / 50 / 38, 4,000 x 271 - / 69 / 60; 637 x 849 72 / 72 / 78,
-// 4,000 x 1,081 - / 140 / 157, 20,000 x 1,081 438 / 423 / 496 us.
+// runs while the call waits for its longest rays and not for its products: 4,000 x 61 step / runs 24 /
+// 17 us, 500 x 300 31 / 27, 4,000 x 271 47 / 46, 8,000 x 200 49 / 48; 637 x 849 78 / 80, 4,000 x 1,081
+// 117 / 117, 20,000 x 1,081 333 / 342 us.
 int picked_fused_layout(const rlc_method* m, int n, int na) {
     if (m->dkind != K_RM) return DT_LINEAR;
     if (!m->map->long_runs) return map_layout(m->map, DT_STEP);

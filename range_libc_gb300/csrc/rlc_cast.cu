@@ -175,7 +175,8 @@ struct __align__(16) RmRay {
 // grid (a position off the grid reads that row or column) and at max_range alike, and what the cell
 // holds says which it was.  15 instructions a step instead of 24 with the grid tests and the hit
 // test beside it; the budget and the run map are looked at every kUnroll steps.  2 M queries on
-// 2048^2 with runs 94 -> 87 us, 20,000 x 1,081 fused 401 -> 365, 23 M rays batched 707 -> 649.
+// 2048^2 with runs 94 -> 87 us, 20,000 x 1,081 fused 401 -> 365 (with the rest of the kernel as it was
+// then), 23 M rays batched 707 -> 649.
 template <int LAYOUT, int PF, bool BUDGETED>
 __device__ __forceinline__ bool rm_advance_steps(const MapDev& m, float mr, RmRay& q, int budget, float* out, int* steps) {
     const float x0 = q.x0, y0 = q.y0, c = q.c, s = q.s;
@@ -1230,7 +1231,7 @@ __device__ __forceinline__ void tile_bins4(const uint16_t* tile, int P, int li, 
 // once per block, those of the beams once per chunk.  Before, blocks held 256 / na particles: from
 // 256 beams on a single lane multiplied, and since a double multiply costs the FP64 pipe ~19 cycles
 // whatever its active lanes, 20,000 x 1,081 rays took the pipe's 1.36 ms (82 % busy, 25 % of the
-// issue slots used).  Now 384 us.
+// issue slots used).  Now 333 to 352, by map and poses.
 constexpr int kWideThreads = 256;
 constexpr int kWideParticles = 32;
 
@@ -1880,14 +1881,14 @@ cudaError_t set_smem(K kernel, size_t bytes, std::atomic<unsigned long long>& do
 
 // Which fused calls go wide, where the caller has not asked for a schedule: those where a block of
 // k_fused would multiply with one or two lanes, from the particle count on at which that costs more
-// than the shorter blocks gain.  Ray marching on a 2048^2 corridor map, us per call before / wide:
-// 20,000 x 1,081 1365 / 379, 4,000 x 1,081 329 / 140, 4,000 x 271 88 / 60, 2,000 x 1,081 178 / 107,
-// 2,000 x 300 61 / 48, 6,000 x 150 70 / 51, 2,000 x 150 41 / 35; below the line 1,000 x 1,081
-// 100 / 97, 1,000 x 300 38 / 43, 600 x 150 28 / 30, 20,000 x 61 62 / 68.  Table queries are short, so
-// that the products weigh more: CDDT 8,000 x 1,081 595 / 128, 4,000 x 271 96 / 30, 2,000 x 150
-// 40 / 18, 1,000 x 300 28 / 24, 5,000 x 61 21 / 18; below the line 4,000 x 61 12.6 / 13.6, 8,000 x 35
-// 12.3 / 14.1, 600 x 200 15.3 / 17.1; GLT 20,000 x 200 253 / 39, 8,000 x 61 15.6 / 13.1, 4,000 x 61
-// 11.6 / 13.3.  Bresenham 8,000 x 1,081 617 / 416, 4,000 x 271 133 / 100.
+// than the shorter blocks gain.  Ray marching on a 2048^2 corridor map, us per call k_fused / wide:
+// 20,000 x 1,081 1364 / 333, 4,000 x 1,081 324 / 118, 4,000 x 271 87 / 46, 2,000 x 1,081 175 / 101,
+// 2,000 x 300 58 / 40, 6,000 x 150 70 / 38, 2,000 x 150 38 / 24; below the line 1,000 x 1,081
+// 101 / 96, 1,000 x 300 33 / 36, 600 x 150 20 / 23, 20,000 x 61 41 / 45.  Table queries are short, so
+// that the products weigh more: CDDT 8,000 x 1,081 605 / 123, 4,000 x 271 93 / 28, 2,000 x 150
+// 37 / 16, 1,000 x 300 28 / 23, 5,000 x 61 18 / 14; below the line 4,000 x 61 10.9 / 11.7, 8,000 x 35
+// 9.5 / 11.6, 600 x 200 12.5 / 15.9; GLT 20,000 x 200 249 / 37, 8,000 x 61 13.3 / 10.0, 4,000 x 61
+// 7.8 / 8.8.  Bresenham 8,000 x 1,081 701 / 477, 4,000 x 271 130 / 90.
 inline bool fused_wide(int kind, int n, int na) {
     const long long rays = (long long)n * na;
     if (rays < (1ll << 18)) return false;
@@ -1906,7 +1907,7 @@ struct RunFused {
     static cudaError_t run(const CastParams& p, const SensorDev& sm, const float* ins, const float* angles,
                            const float* obs, double* w, int n, int na, int block, int tile, bool pick, cudaStream_t s) {
         if (n <= 0) return cudaSuccess;
-        // the kernels that a call without a schedule can come to (pick_layout)
+        // the kernels that a call without a schedule can come to (picked_fused_layout, picked_search)
         constexpr bool kPicked = KIND == K_GLT || KIND == K_BL || (KIND == K_CDDT && (PF == 0 || PF == 3)) ||
                                  (KIND == K_RM && PF == 0 && (LAYOUT == DT_STEP || LAYOUT == DT_RUNS));
         if constexpr (kPicked) {

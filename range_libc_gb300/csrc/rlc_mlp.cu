@@ -13,7 +13,7 @@
 // A prediction t^ is accepted when the cell at x0 + t^ dir is occupied and
 // the cell at x0 + (t^ - 1) dir is free; the range returned is then the
 // reference's distance to that cell's corner, otherwise the ray is recast
-// exactly (compacted into a dense second pass).
+// exactly (k_resolve, which collects a block's rejected rays and marches them).
 #include "rangelibc.h"
 #include "rlc_internal.cuh"
 #include "rlc_tc.cuh"
